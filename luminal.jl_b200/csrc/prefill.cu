@@ -7,12 +7,12 @@
 // grouped kv heads; K and V are also appended to the decode cache.
 //
 // gemm_tc_kernel: acc[row, token] = sum_k W[row, k] * X[token, k]
-//   one CTA = 128 weight rows x 128 tokens, k in steps of 64 through a 6-stage ring:
-//   warp 5      : one thread issues, per step, a bulk copy of half a weight unit (16 KB, already in
+//   one CTA = 128 weight rows x 64, 128 or 256 tokens, k in steps of 64 through a ring of stages:
+//   warp 9      : one thread issues, per step, a bulk copy of half a weight unit (16 KB, already in
 //                 the tensor core's layout) and a 3-D TMA box of the row-major activations that lands
 //                 in the same layout,
-//   warp 4      : one thread issues tcgen05.mma 128 x 128 x 16,
-//   warps 0..3  : epilogue, one weight row per thread, tcgen05.ld 32 tokens at a time:
+//   warp 8      : one thread issues tcgen05.mma 128 x (tokens) x 16,
+//   warps 0..7  : epilogue, one weight row per thread, tcgen05.ld 32 tokens at a time:
 //                 store float32 / SiLU(gate) * up / RoPE + q, k, v (and the cache).
 #include <cuda.h>
 #include <math_constants.h>
@@ -33,7 +33,9 @@ bool flash_tc_supported(int64_t D);
 
 namespace {
 
-constexpr int kGemmThreads = 6 * 32;
+constexpr int kEpiWarps = 8;                   // two per quarter of the accumulator's lanes: each drains half of the tokens
+constexpr int kMmaWarp = kEpiWarps, kLoadWarp = kEpiWarps + 1;
+constexpr int kGemmThreads = (kEpiWarps + 2) * 32;
 constexpr int kUnitBytes = 32768;
 constexpr int kEpiStageBytes = 32 * 80;        // per epilogue warp: 32 tokens x 32 bf16 outputs, rows of 80 bytes
 constexpr float kInvLn2 = 1.4426950408889634f;
@@ -78,13 +80,35 @@ struct GemmParams {
 __device__ __forceinline__ float gelu_ref(float a) {
   const float inner = (0.7978845608f * a) * (1.0f + (0.044715f * a) * a);
   const float z = inner * 2.0f;
-  const float sg = 1.0f / (1.0f + exp2f((z * -1.0f) * kInvLn2));
+  const float sg = __fdividef(1.0f, 1.0f + exp2f((z * -1.0f) * kInvLn2));
   const float th = sg * 2.0f + -1.0f;
   return (a * 0.5f) * (1.0f + th);
 }
 
+// The warp's 32-token x (8 * PIECES)-feature block, staged as rows of kEpiPitch elements, to dst[token * pitch + feature].
+// PIECES lanes write one token's features as 16-byte vectors, so an instruction writes 32 / PIECES whole runs.
+constexpr int kEpiPitch = 40;                            // bf16 elements per staged token row (80 bytes: conflict-free both ways)
+template <int PIECES>
+__device__ __forceinline__ void store_block(__nv_bfloat16* dst, int64_t pitch, const __nv_bfloat16* st, int n_tok) {
+  const int lane = threadIdx.x & 31, pc = lane % PIECES;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int t = lane / PIECES + i * (32 / PIECES);
+    if (t < n_tok) *reinterpret_cast<uint4*>(dst + t * pitch + pc * 8) = *reinterpret_cast<const uint4*>(st + t * kEpiPitch + pc * 8);
+  }
+}
+// the same with a check per element: unaligned rows, or fewer than 8 * PIECES features left
+__device__ __forceinline__ void store_block_ragged(__nv_bfloat16* dst, int64_t pitch, const __nv_bfloat16* st, int n_tok, int n_feat) {
+  const int lane = threadIdx.x & 31;
+  if (lane >= n_tok) return;
+  for (int c = 0; c < n_feat; ++c) dst[lane * pitch + c] = st[lane * kEpiPitch + c];
+}
+__device__ __forceinline__ bool vector_rows(const __nv_bfloat16* dst, int64_t pitch) {
+  return (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (pitch & 7) == 0;
+}
+
 // GEMM_SEGMENTS: segments start on multiples of 32 rows, so a warp's 32 rows lie in one segment (or in none)
-__device__ __forceinline__ void segment_epilogue(const GemmParams& p, float (&v)[32], int row, int t0, int t_end, unsigned char* stage) {
+__device__ __forceinline__ void segment_epilogue(const GemmParams& p, float (&v)[32], int row, int t0, int t_end, __nv_bfloat16* st) {
   const int row0 = row & ~31, lane = threadIdx.x & 31;
   RowSeg sg;
   sg.rows = 0;
@@ -93,22 +117,22 @@ __device__ __forceinline__ void segment_epilogue(const GemmParams& p, float (&v)
     if (i < p.segs.n && row0 >= p.segs.s[i].row0 && row0 < p.segs.s[i].row0 + p.segs.s[i].rows) sg = p.segs.s[i];
   if (sg.rows == 0) return;                              // padding between segments
   const int r = row - sg.row0;
-  if (sg.kind == SEG_F32 || sg.kind == SEG_SOFTCAP) {
+  const int n_tok = min(32, t_end - t0);
+  if (sg.kind == SEG_F32 || sg.kind == SEG_SOFTCAP || sg.kind == SEG_DECAY) {
     if (r >= sg.rows) return;
-    float* out = reinterpret_cast<float*>(sg.dst);
-    const float cap = sg.kind == SEG_SOFTCAP ? p.segs.softcap : 0.f;
+    if (sg.kind == SEG_SOFTCAP && p.segs.softcap > 0.f) {
+      const float cap = p.segs.softcap;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = cap * tanhf(v[i] / cap);
+    } else if (sg.kind == SEG_DECAY) {
+      const float rate = -expf(sg.rate[r / sg.head]), bias = sg.bias[r];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = rate * softplus_f32(v[i] + bias);
+    }
+    float* out = reinterpret_cast<float*>(sg.dst) + (int64_t)t0 * sg.pitch + r;
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-      if (t0 + i < t_end) out[(int64_t)(t0 + i) * sg.pitch + r] = cap > 0.f ? cap * tanhf(v[i] / cap) : v[i];
-    return;
-  }
-  if (sg.kind == SEG_DECAY) {
-    if (r >= sg.rows) return;
-    float* out = reinterpret_cast<float*>(sg.dst);
-    const float rate = -expf(sg.rate[r / sg.head]), bias = sg.bias[r];
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (t0 + i < t_end) out[(int64_t)(t0 + i) * sg.pitch + r] = rate * softplus_f32(v[i] + bias);
+      if (i < n_tok) out[(int64_t)i * sg.pitch] = v[i];
     return;
   }
   if (sg.kind == SEG_GELU_TOKEN) {
@@ -122,122 +146,155 @@ __device__ __forceinline__ void segment_epilogue(const GemmParams& p, float (&v)
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = gelu_ref(v[i]) * __bfloat162float(e[i]);
-  }
-  if (sg.kind == SEG_ROT) {
+  } else if (sg.kind == SEG_ROT) {
     const int f = r % sg.rot_head - sg.rot_off;         // partner rows are neighbouring lanes
     const bool turn = f >= 0 && f < sg.rot_dims;
     const float sign = (f & 1) ? 1.f : -1.f;
     const float2* rot = sg.rot + (turn ? f >> 1 : 0);
     float2 cs[32];                                      // all table reads first: between stores the compiler could not move them
 #pragma unroll
-    for (int i = 0; i < 32; ++i) cs[i] = turn && t0 + i < t_end ? __ldg(rot + (int64_t)(t0 + i) * (sg.rot_dims >> 1)) : make_float2(1.f, 0.f);
+    for (int i = 0; i < 32; ++i) cs[i] = turn && i < n_tok ? __ldg(rot + (int64_t)(t0 + i) * (sg.rot_dims >> 1)) : make_float2(1.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       const float w = __shfl_xor_sync(0xffffffffu, v[i], 1);
       v[i] = v[i] * cs[i].x + sign * (w * cs[i].y);
     }
-  }
-  // bf16: the warp's 32 x 32 block is turned through shared memory, lane L then stores 32 consecutive features of token t0 + L
-  __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
-  constexpr int kPitch = 40;
+  } else if (sg.kind == SEG_RELU2) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float y = v[i];
-    if (sg.kind == SEG_RELU2) { y = fmaxf(y, 0.f); y = y * y; }
-    else if (sg.kind == SEG_SILU) y = y / (1.0f + expf(-y));
-    else if (sg.kind == SEG_SIGMOID) y = sigmoid_f32(y);
-    st[i * kPitch + lane] = __float2bfloat16_rn(y);
+    for (int i = 0; i < 32; ++i) { const float y = fmaxf(v[i], 0.f); v[i] = y * y; }
+  } else if (sg.kind == SEG_SILU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __fdividef(v[i], 1.0f + expf(-v[i]));
+  } else if (sg.kind == SEG_SIGMOID) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __fdividef(1.0f, 1.0f + expf(-v[i]));
   }
+  // bf16: the warp's 32 x 32 block is turned through shared memory and stored as runs of 64 bytes
+#pragma unroll
+  for (int i = 0; i < 32; ++i) st[i * kEpiPitch + lane] = __float2bfloat16_rn(v[i]);
   __syncwarp();
-  const int tL = t0 + lane, r0 = row0 - sg.row0;
-  if (tL < t_end) {
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(sg.dst) + (int64_t)tL * sg.pitch + r0;
-    if (r0 + 32 <= sg.rows && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-      const uint4* src = reinterpret_cast<const uint4*>(st + lane * kPitch);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) reinterpret_cast<uint4*>(dst)[c] = src[c];
-    } else {
-      for (int c = 0; c < 32 && r0 + c < sg.rows; ++c) dst[c] = st[lane * kPitch + c];
-    }
-  }
+  const int r0 = row0 - sg.row0;
+  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(sg.dst) + (int64_t)t0 * sg.pitch + r0;
+  if (r0 + 32 <= sg.rows && vector_rows(dst, sg.pitch)) store_block<4>(dst, sg.pitch, st, n_tok);
+  else store_block_ragged(dst, sg.pitch, st, n_tok, min(32, sg.rows - r0));
   __syncwarp();
 }
 
-// v[i] = accumulator of (row, token t0 + i).  Rows g and g+8 of a 16-row block, which the fused
-// epilogues combine, are 8 lanes apart.
-__device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32], int row, int t0, int t_end, unsigned char* stage) {
-  const int rb = row >> 4, rr = row & 15, g = rr & 7, hi = rr >> 3;
-  if (p.epi == GEMM_STORE_F32) {
+// v[i] = accumulator of (row, token t0 + i); for GEMM_CROSS_KV token t0 + i is position pos0 + i of sequence b (pos0 a
+// multiple of 32).  Rows g and g+8 of a 16-row block, which the fused epilogues combine, are 8 lanes apart.
+//
+// Every thread (one row) has 32 tokens of one column of the output: stored directly, a warp's store instruction would
+// write 2-byte pieces.  Instead the warp turns its 32 x 32 block round through its own 2.5 KB of shared memory and
+// writes whole runs.  One instantiation per epilogue: with all of them in one kernel behind run-time branches, four
+// epilogue warps and direct 2-byte stores a 256 x 256 tile took 41 us to drain (53 with GELU) and every product whose K
+// was below a few thousand waited for it: 12000 tokens x 512 rows, K 512, took 82 us.
+template <int EPI>
+__device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32], int row, int t0, int t_end, int b, int pos0, unsigned char* stage) {
+  const int lane = threadIdx.x & 31, n_tok = min(32, t_end - t0);
+  __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
+  const int row0 = row & ~31;                          // the warp's first row: rows row0 .. row0 + 31 (a multiple of 32)
+  if (EPI == GEMM_STORE_F32) {
     if (row < p.rows) {
+      float* out = p.out + (int64_t)t0 * p.ldo + row;
 #pragma unroll
       for (int i = 0; i < 32; ++i)
-        if (t0 + i < t_end) p.out[(int64_t)(t0 + i) * p.ldo + row] = v[i];
+        if (i < n_tok) out[(int64_t)i * p.ldo] = v[i];
     }
     return;
   }
-  if (p.epi == GEMM_AFFINE || p.epi == GEMM_CROSS_KV) {
-    if (row >= p.rows) return;
-    const float bias = p.bias ? p.bias[row] : 0.f;
-    const int h = p.epi == GEMM_CROSS_KV ? row / p.D : 0, d = p.epi == GEMM_CROSS_KV ? row - h * p.D : 0;
+  if (EPI == GEMM_AFFINE || EPI == GEMM_CROSS_KV) {
+    const float bias = p.bias && row < p.rows ? p.bias[row] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const int t = t0 + i;
-      if (t >= t_end) continue;
-      float y = v[i] + bias;
-      if (p.gelu) y = gelu_ref(y);
-      y *= p.out_scale;
-      if (p.epi == GEMM_CROSS_KV) {
-        const int b = t / p.n_seq, pos = t - b * p.n_seq;
-        p.kv_layer[b * p.kv_batch_stride + h * p.kv_head_stride + (p.is_v ? vcache_offset(pos, d, p.D) : kcache_offset(pos, d, p.D))] =
-            __float2bfloat16_rn(y);
-      } else if (p.out_bf16) {
-        reinterpret_cast<__nv_bfloat16*>(p.out_any)[(int64_t)t * p.ldo + row] = __float2bfloat16_rn(y);
-      } else {
-        reinterpret_cast<float*>(p.out_any)[(int64_t)t * p.ldo + row] = y;
+    for (int i = 0; i < 32; ++i) v[i] += bias;
+    if (p.gelu) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = gelu_ref(v[i]);
+    }
+    if (p.out_scale != 1.0f) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] *= p.out_scale;
+    }
+    if (EPI == GEMM_AFFINE && !p.out_bf16) {
+      if (row < p.rows) {
+        float* out = reinterpret_cast<float*>(p.out_any) + (int64_t)t0 * p.ldo + row;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i < n_tok) out[(int64_t)i * p.ldo] = v[i];
       }
+      return;
     }
-    return;
-  }
-  if (p.epi == GEMM_SEGMENTS) {
-    segment_epilogue(p, v, row, t0, t_end, stage);
-    return;
-  }
-  // The fused epilogues below give every thread (one row) 32 tokens of one column of the output: stored directly,
-  // a warp's store instruction would write 16-byte pieces of 32 different token rows.  Instead the warp turns its
-  // 32 x 32 block round through its own 2.5 KB of shared memory (rows of 80 bytes: conflict-free both ways), after
-  // which lane L holds token t0 + L's 32 outputs and writes them as 16-byte vectors.
-  float w[32];
+    if (row0 >= p.rows) return;                        // uniform over the warp
+    if (EPI == GEMM_AFFINE) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) w[i] = __shfl_xor_sync(0xffffffffu, v[i], 8);
-  const int lane = threadIdx.x & 31;
-  const int rbl = (row >> 4) & 1;                      // which of the warp's two 16-row blocks
-  const int row0 = row & ~31;                          // the warp's first row: rows row0 .. row0 + 31 (a multiple of 32)
-  __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
-  constexpr int kPitch = 40;                           // bf16 elements per staged token row (80 bytes)
-  const int tL = t0 + lane;                            // the token this lane stores after the turn
-  if (p.epi == GEMM_SILU_GATE) {
-    // column of (rb, g): rbl * 8 + g, 16 outputs per token = act[t, (row0 / 16) * 8 .. + 16)
-    if (hi == 0) {
-      const int col = rbl * 8 + g;
+      for (int i = 0; i < 32; ++i) st[i * kEpiPitch + lane] = __float2bfloat16_rn(v[i]);
+      __syncwarp();
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out_any) + (int64_t)t0 * p.ldo + row0;
+      if (row0 + 32 <= p.rows && vector_rows(dst, p.ldo)) store_block<4>(dst, p.ldo, st, n_tok);
+      else store_block_ragged(dst, p.ldo, st, n_tok, min(32, p.rows - row0));
+      __syncwarp();
+      return;
+    }
+    // two 16-key blocks x two 16-feature units of the cache (kcache_offset / vcache_offset): lane (g, t) assembles the 16
+    // bytes it owns of each unit.  Keys past the sequence are written as zeros: the cache holds whole blocks.
+    const int h = row0 / p.D, d0 = row0 - h * p.D;
+    const int g = lane >> 2, t = lane & 3;
+    __nv_bfloat16* base = p.kv_layer + b * p.kv_batch_stride + h * p.kv_head_stride;
+    if (p.is_v) {                                      // staged as st[feature][key]
+      uint32_t w[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float a = v[i], u = w[i];
-        const float ex = exp2f((a * -1.0f) * kInvLn2);          // src/HighLevelOps.jl:153-160
-        const float sg = 1.0f / (1.0f + ex);
-        st[i * kPitch + col] = __float2bfloat16_rn((a * sg) * u);
+      for (int i = 0; i < 16; ++i) {
+        const __nv_bfloat162 pr = __floats2bfloat162_rn(2 * i < n_tok ? v[2 * i] : 0.f, 2 * i + 1 < n_tok ? v[2 * i + 1] : 0.f);
+        w[i] = *reinterpret_cast<const uint32_t*>(&pr);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(st + lane * kEpiPitch)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+    } else {                                           // staged as st[key][feature]
+#pragma unroll
+      for (int i = 0; i < 32; ++i) st[i * kEpiPitch + lane] = __float2bfloat16_rn(i < n_tok ? v[i] : 0.f);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kb = u >> 1, du = u & 1;               // key block, feature unit
+      const int r0 = p.is_v ? 16 * du : 16 * kb, c0 = p.is_v ? 16 * kb : 16 * du;      // unit rows g / g + 8, columns 2 t / 2 t + 8
+      const __nv_bfloat16* s0 = st + (r0 + g) * kEpiPitch + c0 + 2 * t;
+      uint4 o;
+      o.x = *reinterpret_cast<const uint32_t*>(s0);
+      o.y = *reinterpret_cast<const uint32_t*>(s0 + 8 * kEpiPitch);
+      o.z = *reinterpret_cast<const uint32_t*>(s0 + 8);
+      o.w = *reinterpret_cast<const uint32_t*>(s0 + 8 * kEpiPitch + 8);
+      if (16 * kb < n_tok) {
+        const int64_t at = p.is_v ? vcache_offset(pos0 + 16 * kb, d0 + 16 * du, p.D) : kcache_offset(pos0 + 16 * kb, d0 + 16 * du, p.D);
+        *reinterpret_cast<uint4*>(base + at + lane * 8) = o;
       }
     }
     __syncwarp();
+    return;
+  }
+  if (EPI == GEMM_SEGMENTS) {
+    segment_epilogue(p, v, row, t0, t_end, st);
+    return;
+  }
+  const int rb = row >> 4, rr = row & 15, g = rr & 7, hi = rr >> 3;
+  const int rbl = rb & 1;                              // which of the warp's two 16-row blocks
+  if (EPI == GEMM_SILU_GATE) {
+    // column of (rb, g): rbl * 8 + g, 16 outputs per token = act[t, (row0 / 16) * 8 .. + 16).  The gate row's lane takes tokens
+    // 0 .. 15, the up row's lane 16 .. 31: each sends the other half of its row.
+    const int col = rbl * 8 + g;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float got = __shfl_xor_sync(0xffffffffu, hi ? v[i] : v[i + 16], 8);
+      const float a = hi ? got : v[i], u = hi ? v[i + 16] : got;
+      const float ex = exp2f((a * -1.0f) * kInvLn2);            // src/HighLevelOps.jl:153-160
+      const float sg = __fdividef(1.0f, 1.0f + ex);
+      st[(i + 16 * hi) * kEpiPitch + col] = __float2bfloat16_rn((a * sg) * u);
+    }
+    __syncwarp();
     const int o0 = (row0 >> 4) * 8;
-    if (tL < t_end && o0 < p.n_act) {
-      __nv_bfloat16* dst = p.act + (int64_t)tL * p.ld_act + o0;
-      const uint4* src = reinterpret_cast<const uint4*>(st + lane * kPitch);
-      if (o0 + 16 <= p.n_act && (p.ld_act & 7) == 0) {
-        reinterpret_cast<uint4*>(dst)[0] = src[0];
-        reinterpret_cast<uint4*>(dst)[1] = src[1];
-      } else {
-        for (int c = 0; c < 16 && o0 + c < p.n_act; ++c) dst[c] = st[lane * kPitch + c];
-      }
+    if (o0 < p.n_act) {
+      __nv_bfloat16* dst = p.act + (int64_t)t0 * p.ld_act + o0;
+      if (o0 + 16 <= p.n_act && vector_rows(dst, p.ld_act)) store_block<2>(dst, p.ld_act, st, n_tok);
+      else store_block_ragged(dst, p.ld_act, st, n_tok, min(16, p.n_act - o0));
     }
     __syncwarp();
     return;
@@ -246,50 +303,38 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32
   const int D = p.D, tiles_per_head = D >> 4, half = D >> 1;
   const int hs = rb / tiles_per_head, jj = rb - hs * tiles_per_head;
   const int jj0 = jj - rbl;                            // the warp's first 16-row block inside the head (even)
-  const bool live = row0 < p.rows;                     // uniform over the warp (rows is a multiple of 32 here)
+  if (row0 >= p.rows) return;                          // uniform over the warp (rows is a multiple of 32 here)
   if (hs < p.Hl + p.KVl) {
     const int d0 = 8 * jj + g;                         // rows g / g+8 are the pair (d0, d0 + D/2), src/NN.jl:253-303
     // staged columns: [0, 16) = d 8*jj0 .. + 15, [16, 32) = D/2 + the same
     const int col = rbl * 8 + g + (hi ? 16 : 0);
-    if (live) {
-      // all table reads of the chunk first: between stores the compiler could not move them
-      float2 sc[32];
-      int sq = t0 % p.n_seq;
+    // all table reads of the chunk first: between stores the compiler could not move them
+    float2 sc[32];
+    int sq = t0 % p.n_seq;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        sc[i] = (t0 + i < t_end) ? __ldg(p.rope + (int64_t)sq * half + d0) : make_float2(0.f, 1.f);
-        if (++sq == p.n_seq) sq = 0;
-      }
+    for (int i = 0; i < 32; ++i) {
+      sc[i] = i < n_tok ? __ldg(p.rope + (int64_t)sq * half + d0) : make_float2(0.f, 1.f);
+      if (++sq == p.n_seq) sq = 0;
+    }
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float sn = sc[i].x, cs = sc[i].y;
-        const float o = hi ? (w[i] * sn + v[i] * cs) : (v[i] * cs + (w[i] * sn) * -1.0f);
-        st[i * kPitch + col] = __float2bfloat16_rn(o);
-      }
+    for (int i = 0; i < 32; ++i) {
+      const float sn = sc[i].x, cs = sc[i].y;
+      const float w = __shfl_xor_sync(0xffffffffu, v[i], 8);
+      const float o = hi ? (w * sn + v[i] * cs) : (v[i] * cs + (w * sn) * -1.0f);
+      st[i * kEpiPitch + col] = __float2bfloat16_rn(o);
     }
     __syncwarp();
-    if (live && tL < t_end) {
-      __nv_bfloat16* base = hs < p.Hl ? p.q + (int64_t)tL * p.ldq + hs * D : p.kbuf + (int64_t)tL * p.ldkv + (hs - p.Hl) * D;
-      const uint4* src = reinterpret_cast<const uint4*>(st + lane * kPitch);
-      uint4* lo = reinterpret_cast<uint4*>(base + 8 * jj0);
-      uint4* up = reinterpret_cast<uint4*>(base + half + 8 * jj0);
-      lo[0] = src[0]; lo[1] = src[1];
-      up[0] = src[2]; up[1] = src[3];
-    }
+    const int64_t pitch = hs < p.Hl ? p.ldq : p.ldkv;
+    __nv_bfloat16* base = (hs < p.Hl ? p.q + hs * D : p.kbuf + (hs - p.Hl) * D) + (int64_t)t0 * pitch + 8 * jj0;
+    store_block<2>(base, pitch, st, n_tok);
+    store_block<2>(base + half, pitch, st + 16, n_tok);
   } else {
     const int kvh = hs - p.Hl - p.KVl;
     const int col = rbl * 16 + rr;                     // d = 16 * jj0 + col
-    if (live) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) st[i * kPitch + col] = __float2bfloat16_rn(v[i]);
-    }
+    for (int i = 0; i < 32; ++i) st[i * kEpiPitch + col] = __float2bfloat16_rn(v[i]);
     __syncwarp();
-    if (live && tL < t_end) {
-      uint4* dst = reinterpret_cast<uint4*>(p.vbuf + (int64_t)tL * p.ldkv + kvh * D + 16 * jj0);
-      const uint4* src = reinterpret_cast<const uint4*>(st + lane * kPitch);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) dst[c] = src[c];
-    }
+    store_block<4>(p.vbuf + (int64_t)t0 * p.ldkv + kvh * D + 16 * jj0, p.ldkv, st, n_tok);
   }
   __syncwarp();
 }
@@ -319,15 +364,15 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
-// BN tokens per tile (128 or 256).  256 halves the number of MMA instructions and barrier round trips
+// BN tokens per tile (64, 128 or 256; gemm_launch chooses).  256 halves the number of MMA instructions and barrier round trips
 // per flop and doubles the reuse of each weight byte read from shared memory; its two accumulators
 // take all 512 TMEM columns.
-template <int BN>
+template <int BN, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap,
                                                                   int* err) {
   using namespace tc;
   constexpr int kGemmBN = BN;
-  constexpr int kGemmStages = BN == 256 ? 4 : 6;
+  constexpr int kGemmStages = BN == 256 ? 4 : BN == 128 ? 6 : 8;
   constexpr int kABytes = kUnitBytes / 2;                 // 128 rows x 64 k: half a weight unit (its first / last 8 k-groups)
   constexpr int kBBytes = kGemmBN * 128;                  // BN tokens x 64 k, bf16: one 128-byte swizzled row per token
   constexpr int kStage = kABytes + kBBytes;
@@ -339,29 +384,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
   const int NS = (p.K + 63) >> 6;                         // pipeline steps of 64 k per tile
   // Persistent CTAs walk the tiles with the token tile as the fast index: the CTAs running at one
   // time share a few weight row groups (L2 hits) and the activations fit L2 as a whole.
+  // Token tiles never cross a sequence in a convolution and for GEMM_CROSS_KV (whole 16-key blocks of the cache are written).
   const bool conv = p.conv_taps > 0;
-  const int tpb = conv ? (p.conv_Lout + kGemmBN - 1) / kGemmBN : 0;      // convolution: token tiles per batch element
-  const int n_tt = conv ? p.conv_B * tpb : (p.T + kGemmBN - 1) / kGemmBN, n_rg = (p.rows + 127) >> 7;
+  const int n_own = conv ? p.conv_Lout : EPI == GEMM_CROSS_KV ? p.n_seq : p.T;
+  const int tpb = (n_own + kGemmBN - 1) / kGemmBN;                       // token tiles per sequence
+  const int n_tt = tpb * (conv ? p.conv_B : EPI == GEMM_CROSS_KV ? p.T / p.n_seq : 1), n_rg = (p.rows + 127) >> 7;
   const int n_tiles = n_tt * n_rg;
   TileOrder order;
   order.n_tt = n_tt; order.n_rg = n_rg;
   order.gt = max(8, min(n_tt, (64 << 20) / (kGemmBN * p.K * 2)));
   if (tid == 0) {
     for (int s = 0; s < kGemmStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpiWarps); }
     mbar_init_fence();
   }
-  if (warp == 4) tmem_alloc(&tmem_slot, 2 * kGemmBN);
+  if (warp == kMmaWarp) tmem_alloc(&tmem_slot, 2 * kGemmBN);
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
   bool dead = false;
 
-  if (warp == 5) {
+  if (warp == kLoadWarp) {
     // producer: per step half a weight unit (bulk copy, already in the tensor core's layout) and the
-    // activations of BN tokens x 64 k through a 2-D tensor map over the row-major [T, K] matrix: the box
-    // {64, BN} lands as BN rows of 128 bytes in the 128-byte swizzle (one request per row instead of one
+    // activations of BN tokens x 64 k through a 3-D tensor map over the row-major [sequence, token, K] tensor: the box
+    // {64, BN, 1} lands as BN rows of 128 bytes in the 128-byte swizzle (one request per row instead of one
     // per 16 bytes); rows past T and columns past K arrive as zeros
     int g = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -387,16 +434,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
         } else if (lane == 0) {
           mbar_expect_tx(&full[s], (uint32_t)kStage);
           bulk_g2s(smem + s * kStage, p.W + ((int64_t)rg * KS + (st >> 1)) * 16384 + (st & 1) * 8192, (uint32_t)kABytes, &full[s]);
+          const int b = tt_ / tpb;
           asm volatile(
-              "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
+              "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(
                   smem_u32(smem + s * kStage + kABytes)),
-              "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(st * 64), "r"(tt_ * kGemmBN), "r"(smem_u32(&full[s]))
+              "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(st * 64), "r"((tt_ - b * tpb) * kGemmBN), "r"(b), "r"(smem_u32(&full[s]))
               : "memory");
         }
         __syncwarp();
       }
     }
-  } else if (warp == 4) {
+  } else if (warp == kMmaWarp) {
     constexpr uint32_t kIdesc = idesc_bf16(128, kGemmBN, false, false);
     int g = 0, n = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
@@ -423,37 +471,36 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
     }
   } else {
     // epilogue of tile n while the MMAs of tile n + 1 fill the other accumulator
-    const uint32_t lane_base = (uint32_t)(32 * warp) << 16;
+    const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
+    constexpr int kHalf = kGemmBN / 2;                   // the tokens one warp drains: warps 4 .. 7 the tile's second half
+    const int c0 = (warp >> 2) * kHalf;
     int n = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
       const int buf = n & 1;
       int rg_, tt_;
       order.decode(tile, &rg_, &tt_);
-      int t0 = tt_ * kGemmBN, t_end = p.T;
-      if (conv) {
-        const int b = tt_ / tpb, o0 = (tt_ - b * tpb) * kGemmBN;
-        t0 = b * p.conv_out_rpb + o0;
-        t_end = b * p.conv_out_rpb + p.conv_Lout;
-      }
-      const int row = rg_ * 128 + 32 * warp + lane;
+      const int b = tt_ / tpb, o0 = (tt_ - b * tpb) * kGemmBN, rpb = conv ? p.conv_out_rpb : n_own;
+      const int t0 = b * rpb + o0, t_end = b * rpb + n_own;
+      const int row = rg_ * 128 + 32 * (warp & 3) + lane;
       mbar_wait(&acc_full[buf], (n >> 1) & 1, dead, err);
       fence_after();
 #pragma unroll 1
-      for (int ch = 0; ch < kGemmBN / 32; ++ch) {
+      for (int ch = 0; ch < kHalf; ch += 32) {
         float v[32];
-        tmem_ld32(v, tmem + lane_base + buf * kGemmBN + ch * 32);
-        if (ch == kGemmBN / 32 - 1) {                  // the whole accumulator is in registers or done with
+        tmem_ld32(v, tmem + lane_base + buf * kGemmBN + c0 + ch);
+        if (ch == kHalf - 32) {                        // the whole share is in registers or done with
           fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
-        gemm_epilogue(p, v, row, t0 + ch * 32, t_end, smem + kGemmStages * kStage + warp * kEpiStageBytes);
+        if (t0 + c0 + ch < t_end)
+          gemm_epilogue<EPI>(p, v, row, t0 + c0 + ch, t_end, b, o0 + c0 + ch, smem + kGemmStages * kStage + warp * kEpiStageBytes);
       }
     }
   }
   fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     fence_after();
     tmem_dealloc(tmem, 2 * kGemmBN);
   }
@@ -503,6 +550,12 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {
 
 // TMA tile load whose completion is counted on a barrier given by its shared::cluster address: with cta_group::2 that
 // may be the partner CTA's barrier
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar_cluster_addr) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar_cluster_addr)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster_addr) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
@@ -513,6 +566,7 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 constexpr int kPairStages = 6;
 constexpr int kPairStage = 32768;       // 128 rows x 64 k of weights + 128 tokens x 64 k of activations
 
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     gemm_tc2_kernel(const GemmParams p, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, int* err) {
   using namespace tc;
@@ -523,7 +577,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = cluster_rank();
   const int KS = (p.K + 127) >> 7, NS = (p.K + 63) >> 6;
-  const int n_tt = (p.T + kBN - 1) / kBN, n_rgp = (p.rows + 255) >> 8;
+  const int n_own = EPI == GEMM_CROSS_KV ? p.n_seq : p.T;
+  const int tpb = (n_own + kBN - 1) / kBN;               // token tiles per sequence (GEMM_CROSS_KV: no tile crosses one)
+  const int n_tt = tpb * (EPI == GEMM_CROSS_KV ? p.T / p.n_seq : 1), n_rgp = (p.rows + 255) >> 8;
   const int n_tiles = n_tt * n_rgp;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   TileOrder order;
@@ -531,10 +587,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   order.gt = max(8, min(n_tt, (64 << 20) / (kBN * p.K * 2)));
   if (tid == 0) {
     for (int s = 0; s < kPairStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 2 * kEpiWarps); }
     mbar_init_fence();
   }
-  if (warp == 4) tmem_alloc(&tmem_slot, 512);          // all columns in both CTAs: the same base address in both
+  if (warp == kMmaWarp) tmem_alloc(&tmem_slot, 512);          // all columns in both CTAs: the same base address in both
   fence_before();
   __syncthreads();
   cluster_barrier();                                     // both CTAs' barriers exist before anything arrives on them
@@ -542,7 +598,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   const uint32_t tmem = tmem_slot;
   bool dead = false;
 
-  if (warp == 5) {
+  if (warp == kLoadWarp) {
     int g = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs) {
       int rgp, tt_;
@@ -557,14 +613,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           const uint32_t bar0 = map_to_cta(smem_u32(&full[s]), 0);
           if (rank == 0) mbar_expect_tx(&full[s], 2u * (uint32_t)kPairStage);
           tma_load_2d_pair(smem_u32(smem + s * kPairStage), &wmap, 0, (int)((((int64_t)rg * KS + (st >> 1)) * 2 + (st & 1)) * 128), bar0);
-          tma_load_2d_pair(smem_u32(smem + s * kPairStage + kABytes), &xmap, st * 64, tt_ * kBN + (int)rank * 128, bar0);
+          const int b = tt_ / tpb;
+          tma_load_3d_pair(smem_u32(smem + s * kPairStage + kABytes), &xmap, st * 64, (tt_ - b * tpb) * kBN + (int)rank * 128, b, bar0);
         }
         __syncwarp();
       }
     }
-  } else if (warp == 4 && rank == 1) {
+  } else if (warp == kMmaWarp && rank == 1) {
     // CTA 1 issues no MMAs: CTA 0's thread drives both tensor cores
-  } else if (warp == 4) {
+  } else if (warp == kMmaWarp) {
     constexpr uint32_t kIdesc = idesc_bf16(256, kBN, false, false);
     int g = 0, n = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++n) {
@@ -590,21 +647,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       }
     }
   } else {
-    const uint32_t lane_base = (uint32_t)(32 * warp) << 16;
+    const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t acc_empty_remote[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
+    constexpr int kHalf = kBN / 2;
+    const int c0 = (warp >> 2) * kHalf;
     int n = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++n) {
       const int buf = n & 1;
       int rgp, tt_;
       order.decode(tile, &rgp, &tt_);
-      const int t0 = tt_ * kBN, row = (2 * rgp + (int)rank) * 128 + 32 * warp + lane;
+      const int b = tt_ / tpb, o0 = (tt_ - b * tpb) * kBN, t0 = b * n_own + o0, t_end = (b + 1) * n_own;
+      const int row = (2 * rgp + (int)rank) * 128 + 32 * (warp & 3) + lane;
       mbar_wait(&acc_full[buf], (n >> 1) & 1, dead, err);
       fence_after();
 #pragma unroll 1
-      for (int ch = 0; ch < kBN / 32; ++ch) {
+      for (int ch = 0; ch < kHalf; ch += 32) {
         float v[32];
-        tmem_ld32(v, tmem + lane_base + buf * kBN + ch * 32);
-        if (ch == kBN / 32 - 1) {
+        tmem_ld32(v, tmem + lane_base + buf * kBN + c0 + ch);
+        if (ch == kHalf - 32) {
           fence_before();
           __syncwarp();
           if (lane == 0) {
@@ -612,23 +672,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
             else mbar_arrive_cluster(acc_empty_remote[buf]);
           }
         }
-        gemm_epilogue(p, v, row, t0 + ch * 32, p.T, smem + kPairStages * kPairStage + warp * kEpiStageBytes);
+        if (t0 + c0 + ch < t_end)
+          gemm_epilogue<EPI>(p, v, row, t0 + c0 + ch, t_end, b, o0 + c0 + ch, smem + kPairStages * kPairStage + warp * kEpiStageBytes);
       }
     }
   }
   fence_before();
   __syncthreads();
   cluster_barrier();            // no CTA leaves while its partner may still arrive on its barriers or read its shared memory
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     fence_after();
     tmem_dealloc(tmem, 512);
   }
 }
 
-constexpr size_t gemm_pair_smem() { return (size_t)kPairStages * kPairStage + 4 * kEpiStageBytes + 1024; }
+constexpr size_t gemm_pair_smem() { return (size_t)kPairStages * kPairStage + kEpiWarps * kEpiStageBytes + 1024; }
 
 template <int BN>
-constexpr size_t gemm_smem() { return (size_t)(BN == 256 ? 4 : 6) * (kUnitBytes / 2 + BN * 128) + 4 * kEpiStageBytes + 1024; }
+constexpr size_t gemm_smem() { return (size_t)(BN == 256 ? 4 : BN == 128 ? 6 : 8) * (kUnitBytes / 2 + BN * 128) + kEpiWarps * kEpiStageBytes + 1024; }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -649,15 +710,45 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-int32_t gemm_launch(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
+template <int EPI>
+int32_t gemm_launch_epi(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
   LMB_REQUIRE(p.ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(p.X) & 15) == 0, "prefill gemm: K %d, row pitch %d", p.K, p.ldx);
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return fail(LMB200_ECUDA, "prefill gemm: cuTensorMapEncodeTiled is not available");
-  // 256-token tiles once there are enough tokens to fill them (LMB200_GEMM_BN=128 keeps the narrow tile for A/B runs)
-  static const int forced_bn = [] { const char* e = getenv("LMB200_GEMM_BN"); return e ? atoi(e) : 0; }();
   const bool conv = p.conv_taps > 0;
-  const int n_tok = conv ? p.conv_Lout : p.T;
-  const int BN = forced_bn == 128 || forced_bn == 256 ? forced_bn : (n_tok >= 256 ? 256 : 128);
+  const int n_own = conv ? p.conv_Lout : EPI == GEMM_CROSS_KV ? p.n_seq : p.T;      // tokens a tile may cover
+  const int64_t seqs = conv ? p.conv_B : EPI == GEMM_CROSS_KV ? p.T / p.n_seq : 1;
+  // a persistent grid: as many CTA pairs as can be resident at once (SMs whose TPC partner is fused off take none)
+  static int max_pairs = 0;
+  if (!max_pairs) {
+    cudaLaunchConfig_t qc = {};
+    qc.gridDim = dim3((unsigned)(ctx->sm_count / 2 * 2));
+    qc.blockDim = dim3(kGemmThreads);
+    qc.dynamicSmemBytes = gemm_pair_smem();
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tc2_kernel<EPI>, &qc) != cudaSuccess || n < 1) { cudaGetLastError(); n = ctx->sm_count / 2; }
+    max_pairs = n;
+    if (getenv("LMB200_DEBUG_GEMM")) fprintf(stderr, "gemm_tc2_kernel: %d pairs resident on %d SMs\n", n, ctx->sm_count);
+  }
+  // The tile: waves x clocks of a tile.  A 64-k step costs what its operands take to arrive (64 bytes a clock and SM) or the MMA,
+  // whichever is longer -- 512 clocks for a CTA pair's 256 x 256, 768 / 512 / 384 for 128 rows x 256 / 128 / 64 tokens -- and the last
+  // tile's epilogue, which nothing overlaps, about 12 clocks a token.  Large products take CTA pairs; few tokens or few rows take the
+  // tile that still fills the SMs (128 rows x 2096 tokens, K 2048: 9 CTAs of 256 tokens took 124 us).
+  // LMB200_GEMM_BN=64|128|256 and LMB200_GEMM_PAIR=0 force a choice for A/B runs.
+  static const int forced_bn = [] { const char* e = getenv("LMB200_GEMM_BN"); return e ? atoi(e) : 0; }();
+  static const bool pair_on = [] { const char* e = getenv("LMB200_GEMM_PAIR"); return !(e && atoi(e) == 0); }();
+  const int64_t n_rg = ceil_div(p.rows, 128), steps = ceil_div(p.K, 64);
+  int BN = 0;
+  int64_t best = -1;
+  auto offer = [&](int bn, int64_t clocks, int64_t tiles, int64_t resident) {
+    const int64_t cost = ceil_div(tiles, resident) * steps * clocks + 12 * std::min(bn, 256);
+    if (best < 0 || cost < best) { best = cost; BN = bn; }
+  };
+  if (pair_on && !conv && p.rows % 256 == 0 && (!forced_bn || forced_bn == 256)) offer(512, 512, n_rg / 2 * seqs * ceil_div(n_own, 256), max_pairs);
+  if (forced_bn == 0 || forced_bn == 256) offer(256, 768, n_rg * seqs * ceil_div(n_own, 256), ctx->sm_count);
+  if (forced_bn == 0 || forced_bn == 128) offer(128, 512, n_rg * seqs * ceil_div(n_own, 128), ctx->sm_count);
+  if (forced_bn == 0 || forced_bn == 64) offer(64, 384, n_rg * seqs * ceil_div(n_own, 64), ctx->sm_count);
+  const bool pair = BN == 512;
   CUtensorMap xmap;
   CUresult r;
   if (conv) {
@@ -674,61 +765,58 @@ int32_t gemm_launch(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   } else {
-    const cuuint64_t dims[2] = {(cuuint64_t)p.K, (cuuint64_t)p.T};
-    const cuuint64_t strides[1] = {(cuuint64_t)p.ldx * 2};               // bytes, dim 1
-    const cuuint32_t box[2] = {64, (cuuint32_t)BN};
-    const cuuint32_t estr[2] = {1, 1};
-    r = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.X), dims, strides, box, estr,
+    // a CTA of a pair stages its half of the 256 tokens
+    const cuuint64_t dims[3] = {(cuuint64_t)p.K, (cuuint64_t)n_own, (cuuint64_t)seqs};
+    const cuuint64_t strides[2] = {(cuuint64_t)p.ldx * 2, (cuuint64_t)n_own * p.ldx * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)(pair ? 128 : BN), 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    r = enc(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(p.X), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
   if (r != CUDA_SUCCESS) return fail(LMB200_ECUDA, "prefill gemm: cuTensorMapEncodeTiled failed (%d)", (int)r);
-  // CTA pairs where the tile grid allows them (LMB200_GEMM_PAIR=0 keeps the single-CTA kernel for A/B runs)
-  static const bool pair_on = [] { const char* e = getenv("LMB200_GEMM_PAIR"); return !(e && atoi(e) == 0); }();
-  if (pair_on && !conv && BN == 256 && p.rows % 256 == 0) {
-    CUtensorMap hmap;                                       // each CTA's half of a token tile: a box of 128 tokens
-    const cuuint64_t dims[2] = {(cuuint64_t)p.K, (cuuint64_t)p.T};
-    const cuuint64_t strides[1] = {(cuuint64_t)p.ldx * 2};
-    const cuuint32_t box[2] = {64, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    r = enc(&hmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.X), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(LMB200_ECUDA, "prefill gemm: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  if (pair) {
     // the weights as rows of 128 bytes: half a canonical unit (128 rows x 64 k) is 128 consecutive rows, copied as it lies
     CUtensorMap wmap;
     const int64_t w_rows = (int64_t)(p.rows / 128) * ceil_div(p.K, 128) * 2 * 128;
     const cuuint64_t wdims[2] = {64, (cuuint64_t)w_rows};
     const cuuint64_t wstrides[1] = {128};
-    r = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.W), wdims, wstrides, box, estr,
+    const cuuint32_t wbox[2] = {64, 128};
+    const cuuint32_t westr[2] = {1, 1};
+    r = enc(&wmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.W), wdims, wstrides, wbox, westr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(LMB200_ECUDA, "prefill gemm: cuTensorMapEncodeTiled (weights) failed (%d)", (int)r);
-    const int64_t pair_tiles = (int64_t)(p.rows / 256) * ceil_div(p.T, 256);
-    // a persistent grid: as many pairs as can be resident at once (SMs whose TPC partner is fused off take none)
-    static int max_pairs = 0;
-    if (!max_pairs) {
-      cudaLaunchConfig_t qc = {};
-      qc.gridDim = dim3((unsigned)(ctx->sm_count / 2 * 2));
-      qc.blockDim = dim3(kGemmThreads);
-      qc.dynamicSmemBytes = gemm_pair_smem();
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm_tc2_kernel, &qc) != cudaSuccess || n < 1) { cudaGetLastError(); n = ctx->sm_count / 2; }
-      max_pairs = n;
-      if (getenv("LMB200_DEBUG_GEMM")) fprintf(stderr, "gemm_tc2_kernel: %d pairs resident on %d SMs\n", n, ctx->sm_count);
-    }
-    const unsigned pairs = (unsigned)std::min<int64_t>(pair_tiles, max_pairs);
-    gemm_tc2_kernel<<<2 * pairs, kGemmThreads, gemm_pair_smem(), st>>>(p, wmap, hmap, ctx->dev_err);
-    ctx->launches++;
-    LMB_CUDA(cudaGetLastError());
-    return LMB200_OK;
+    const unsigned pairs = (unsigned)std::min<int64_t>(n_rg / 2 * seqs * ceil_div(n_own, 256), max_pairs);
+    gemm_tc2_kernel<EPI><<<2 * pairs, kGemmThreads, gemm_pair_smem(), st>>>(p, wmap, xmap, ctx->dev_err);
+  } else {
+    const unsigned grid = (unsigned)std::min<int64_t>(n_rg * seqs * ceil_div(n_own, BN), ctx->sm_count);
+    if (BN == 256) gemm_tc_kernel<256, EPI><<<grid, kGemmThreads, gemm_smem<256>(), st>>>(p, xmap, ctx->dev_err);
+    else if (BN == 128) gemm_tc_kernel<128, EPI><<<grid, kGemmThreads, gemm_smem<128>(), st>>>(p, xmap, ctx->dev_err);
+    else gemm_tc_kernel<64, EPI><<<grid, kGemmThreads, gemm_smem<64>(), st>>>(p, xmap, ctx->dev_err);
   }
-  const int64_t tiles = ceil_div(p.rows, 128) * (conv ? (int64_t)p.conv_B * ceil_div(p.conv_Lout, BN) : ceil_div(p.T, BN));
-  const unsigned grid = (unsigned)std::min<int64_t>(tiles, ctx->sm_count);
-  if (BN == 256) gemm_tc_kernel<256><<<grid, kGemmThreads, gemm_smem<256>(), st>>>(p, xmap, ctx->dev_err);
-  else gemm_tc_kernel<128><<<grid, kGemmThreads, gemm_smem<128>(), st>>>(p, xmap, ctx->dev_err);
   ctx->launches++;
   LMB_CUDA(cudaGetLastError());
+  return LMB200_OK;
+}
+
+int32_t gemm_launch(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
+  switch (p.epi) {
+    case GEMM_STORE_F32: return gemm_launch_epi<GEMM_STORE_F32>(ctx, p, st);
+    case GEMM_SILU_GATE: return gemm_launch_epi<GEMM_SILU_GATE>(ctx, p, st);
+    case GEMM_QKV_ROPE: return gemm_launch_epi<GEMM_QKV_ROPE>(ctx, p, st);
+    case GEMM_AFFINE: return gemm_launch_epi<GEMM_AFFINE>(ctx, p, st);
+    case GEMM_CROSS_KV: return gemm_launch_epi<GEMM_CROSS_KV>(ctx, p, st);
+    default: return gemm_launch_epi<GEMM_SEGMENTS>(ctx, p, st);
+  }
+}
+
+template <int EPI>
+int32_t gemm_configure() {
+  LMB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<64, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<64>()));
+  LMB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<128, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<128>()));
+  LMB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<256, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<256>()));
+  LMB_CUDA(cudaFuncSetAttribute(gemm_tc2_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_pair_smem()));
   return LMB200_OK;
 }
 
@@ -899,10 +987,12 @@ int32_t gemm_cross_kv(Ctx* ctx, const void* W, const __nv_bfloat16* X, int ldx, 
 }
 
 int32_t prefill_configure() {
-  LMB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<128>()));
-  LMB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<256>()));
-  LMB_CUDA(cudaFuncSetAttribute(gemm_tc2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_pair_smem()));
-  return LMB200_OK;
+  LMB_TRY(gemm_configure<GEMM_STORE_F32>());
+  LMB_TRY(gemm_configure<GEMM_SILU_GATE>());
+  LMB_TRY(gemm_configure<GEMM_QKV_ROPE>());
+  LMB_TRY(gemm_configure<GEMM_AFFINE>());
+  LMB_TRY(gemm_configure<GEMM_CROSS_KV>());
+  return gemm_configure<GEMM_SEGMENTS>();
 }
 
 bool prefill_gemm_ok(const Session* S, int n) {

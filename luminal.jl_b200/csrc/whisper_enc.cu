@@ -17,6 +17,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -136,41 +137,54 @@ __global__ void add_sinusoids_kernel(float* __restrict__ x, const float* __restr
   }
 }
 
-// x[t, :] += delta[t, :] (if given); y = LayerNorm(x) * w + b with mean-centering (src/NN.jl:138-173)
+// x[t, :] += delta[t, :] (if given); y = LayerNorm(x) * w + b with mean-centering (src/NN.jl:138-173).  One warp per row: a lane
+// keeps its own float4 pieces of the row in shared memory between the passes and the sums cross lanes by shuffles only.
+// Memory bound; a block per 512-wide row (three block barriers around four loads) took 36 us for 12000 rows.
 __global__ void __launch_bounds__(256) layernorm_rows_kernel(float* __restrict__ x, const float* __restrict__ delta,
                                                              const float* __restrict__ w, const float* __restrict__ bias,
-                                                             __nv_bfloat16* __restrict__ yb, float* __restrict__ yf, int n, float eps) {
-  extern __shared__ float row[];
-  __shared__ float red[8];
-  const int t = blockIdx.x, tid = threadIdx.x;
-  float* xr = x + (int64_t)t * n;
-  auto block_sum = [&](float v) -> float {
+                                                             __nv_bfloat16* __restrict__ yb, float* __restrict__ yf, int T, int n, float eps) {
+  extern __shared__ float4 rows[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n4 = n >> 2;
+  const int t = blockIdx.x * (blockDim.x >> 5) + warp;
+  if (t >= T) return;
+  float4* row = rows + warp * n4;
+  float4* xr = reinterpret_cast<float4*>(x + (int64_t)t * n);
+  const float4* dr = reinterpret_cast<const float4*>(delta + (delta ? (int64_t)t * n : 0));
+  auto warp_sum = [](float v) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    __syncthreads();
-    if ((tid & 31) == 0) red[tid >> 5] = v;
-    __syncthreads();
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += red[i];
-    return s;
+    return v;
   };
   float s1 = 0.f;
-  for (int i = tid; i < n; i += 256) {
-    float v = xr[i];
-    if (delta) { v += delta[(int64_t)t * n + i]; xr[i] = v; }
+#pragma unroll 4
+  for (int i = lane; i < n4; i += 32) {
+    float4 v = xr[i];
+    if (delta) {
+      const float4 d = dr[i];
+      v.x += d.x; v.y += d.y; v.z += d.z; v.w += d.w;
+      xr[i] = v;
+    }
     row[i] = v;
-    s1 += v;
+    s1 += (v.x + v.y) + (v.z + v.w);
   }
-  const float mean = block_sum(s1) * (1.0f / (float)n);
+  const float mean = warp_sum(s1) * (1.0f / (float)n);
   float s2 = 0.f;
-  for (int i = tid; i < n; i += 256) { const float c = row[i] + mean * -1.0f; row[i] = c; s2 += c * c; }
-  const float var = block_sum(s2) * (1.0f / (float)n);
-  const float inv = 1.0f / sqrtf(var + eps);
-  for (int i = tid; i < n; i += 256) {
-    const float y = (row[i] * inv) * w[i] + bias[i];
-    if (yb) yb[(int64_t)t * n + i] = __float2bfloat16_rn(y);
-    if (yf) yf[(int64_t)t * n + i] = y;
+  for (int i = lane; i < n4; i += 32) {
+    float4 c = row[i];
+    c.x -= mean; c.y -= mean; c.z -= mean; c.w -= mean;
+    row[i] = c;
+    s2 += (c.x * c.x + c.y * c.y) + (c.z * c.z + c.w * c.w);
+  }
+  const float inv = 1.0f / sqrtf(warp_sum(s2) * (1.0f / (float)n) + eps);
+#pragma unroll 4
+  for (int i = lane; i < n4; i += 32) {
+    const float4 c = row[i], g = reinterpret_cast<const float4*>(w)[i], b = reinterpret_cast<const float4*>(bias)[i];
+    const float4 y = make_float4((c.x * inv) * g.x + b.x, (c.y * inv) * g.y + b.y, (c.z * inv) * g.z + b.z, (c.w * inv) * g.w + b.w);
+    if (yb) {
+      __nv_bfloat162 h[2] = {__floats2bfloat162_rn(y.x, y.y), __floats2bfloat162_rn(y.z, y.w)};
+      reinterpret_cast<uint2*>(yb + (int64_t)t * n)[i] = *reinterpret_cast<const uint2*>(h);
+    }
+    if (yf) reinterpret_cast<float4*>(yf + (int64_t)t * n)[i] = y;
   }
 }
 
@@ -427,25 +441,28 @@ extern "C" int32_t lmb200_whisper_encoder_run(uint64_t h, const float* mel_host,
   add_sinusoids_kernel<<<grid_for(T * d), 256, 0, st>>>(x, E->inv_ts, S, d, T * d);
   ctx->launches++;
   const float scale = powf((float)d / (float)H, -0.25f);          // on q and k (src/Whisper.jl:257-260)
-  const size_t ln_smem = (size_t)d * sizeof(float);
+  // rows per block: eight, fewer where their rows would not fit the 48 KB every launch may use
+  const int ln_rows = std::max(1, std::min<int>(8, 49152 / (d * (int)sizeof(float))));
+  const size_t ln_smem = (size_t)ln_rows * d * sizeof(float);
+  const unsigned ln_grid = (unsigned)ceil_div(T, ln_rows);
   FlashView fv;
   fv.H = H; fv.G = 1;
   fv.q_b = fv.k_b = (int64_t)S * d; fv.q_h = fv.k_h = D; fv.q_s = fv.k_s = d;
   for (int i = 0; i < E->L; ++i) {
     EncLayer& l = E->layers[i];
-    layernorm_rows_kernel<<<(unsigned)T, 256, ln_smem, st>>>(x, i == 0 ? nullptr : delta, l.ln1_w, l.ln1_b, xn, nullptr, d, 1e-5f);
+    layernorm_rows_kernel<<<ln_grid, 32 * ln_rows, ln_smem, st>>>(x, i == 0 ? nullptr : delta, l.ln1_w, l.ln1_b, xn, nullptr, (int)T, d, 1e-5f);
     ctx->launches++;
     LMB_TRY(gemm_affine(ctx, l.q.W, xn, d, (int)T, d, d, l.q.bias, scale, 0, qb, d, 1, st));
     LMB_TRY(gemm_affine(ctx, l.k.W, xn, d, (int)T, d, d, l.k.bias, scale, 0, kb, d, 1, st));
     LMB_TRY(gemm_affine(ctx, l.v.W, xn, d, (int)T, d, d, l.v.bias, 1.0f, 0, vb, d, 1, st));
     LMB_TRY(flash_tc_launch_view(ctx, attn, qb, kb, vb, fv, batch, S, D, 1.0f, 0, st));
     LMB_TRY(gemm_affine(ctx, l.o.W, attn, d, (int)T, d, d, l.o.bias, 1.0f, 0, delta, d, 0, st));
-    layernorm_rows_kernel<<<(unsigned)T, 256, ln_smem, st>>>(x, delta, l.ln2_w, l.ln2_b, xn, nullptr, d, 1e-5f);
+    layernorm_rows_kernel<<<ln_grid, 32 * ln_rows, ln_smem, st>>>(x, delta, l.ln2_w, l.ln2_b, xn, nullptr, (int)T, d, 1e-5f);
     ctx->launches++;
     LMB_TRY(gemm_affine(ctx, l.fc1.W, xn, d, (int)T, E->ffn, d, l.fc1.bias, 1.0f, 1, act, E->ffn, 1, st));
     LMB_TRY(gemm_affine(ctx, l.fc2.W, act, E->ffn, (int)T, d, E->ffn, l.fc2.bias, 1.0f, 0, delta, d, 0, st));
   }
-  layernorm_rows_kernel<<<(unsigned)T, 256, ln_smem, st>>>(x, delta, E->post_w, E->post_b, E->enc_b, E->enc_f, d, 1e-5f);
+  layernorm_rows_kernel<<<ln_grid, 32 * ln_rows, ln_smem, st>>>(x, delta, E->post_w, E->post_b, E->enc_b, E->enc_f, (int)T, d, 1e-5f);
   ctx->launches++;
   LMB_CUDA(cudaGetLastError());
   if (out_host) LMB_CUDA(cudaMemcpyAsync(out_host, E->enc_f, (size_t)T * d * 4, cudaMemcpyDeviceToHost, st));

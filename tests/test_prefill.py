@@ -80,7 +80,9 @@ def test_gemm_prefill_phi3_width(lib_built, device):
 
 
 @pytest.mark.parametrize("rows,K,tokens", [(128, 128, 128), (100, 72, 37), (384, 1024, 300), (1000, 2816, 129), (4608, 3072, 512),
-                                            (256, 256, 256), (512, 4096, 1000), (768, 64, 257)])
+                                            (256, 256, 256), (512, 4096, 1000), (768, 64, 257),
+                                            # one case per tile: 64 tokens (few rows), 128, 256, CTA pairs, each with a ragged last tile
+                                            (128, 2048, 2095), (1152, 640, 1025), (19072, 72, 385), (9472, 192, 513), (32, 8, 1)])
 def test_prefill_gemm_matches_float64(lib_built, device, rows, K, tokens):
     L = lib_built
     rng = np.random.default_rng(rows + tokens)
