@@ -9,8 +9,12 @@
 //
 // One CTA = one tile of 128 query rows of one (batch, head); keys in tiles of 64, two stages of
 // (K_hi, K_lo, V_hi, V_lo) in flight through TMA (swizzled sub-tiles, as in flash_tc.cu); one MMA warp;
-// four softmax warps, one query row per thread; S double-buffered in TMEM, P single-buffered in shared
-// memory; the running maximum is raised lazily as in the bf16 kernel.
+// four softmax warps, one query row per thread; S double-buffered in TMEM; the running maximum is raised lazily
+// as in the bf16 kernel.  A tile is a chain -- scores, exponentials, the split, P V -- that neither the tensor core
+// (768 clocks a tile at D = 64) nor the exp2 unit (512) fills: P_hi / P_lo go to TMEM as the A operand of P V, which
+// leaves two CTAs room on an SM at D = 64, and a thread has its weights in registers before it waits for the
+// previous P V.  Q is split where it is loaded, K and V by one launch.
+// [2, 16, 1531, 64] causal: 114 us with P through shared memory, one CTA per SM and three split launches.
 #include <cuda.h>
 #include <math_constants.h>
 
@@ -32,12 +36,18 @@ template <int D>
 struct SmemF {
   static constexpr int kQ = kBM * D * 2;          // one of Q_hi / Q_lo
   static constexpr int kKV = kBN * D * 2;         // one of K_hi / K_lo / V_hi / V_lo
-  static constexpr int kP = kBM * kBN * 2;        // one of P_hi / P_lo
   static constexpr int offQ = 0;                  // [hi, lo]
   static constexpr int offKV = offQ + 2 * kQ;     // [stage][K_hi, K_lo, V_hi, V_lo]
-  static constexpr int offP = offKV + kStages * 4 * kKV;
-  static constexpr int total = offP + 2 * kP;
+  static constexpr int total = offKV + kStages * 4 * kKV;
+  static constexpr int kCtas = 2 * (total + 2048) <= 227 * 1024 ? 2 : 1;      // resident per SM; their TMEM columns add up to 512 at most
 };
+
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -66,22 +76,24 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t* hi, uint32_t*
   *lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-// x (float32) -> hl[0][i] = bf16(x), hl[1][i] = bf16(x - hl[0][i]);  n a multiple of 4
-__global__ void split_hi_lo_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hl, int64_t n) {
+// k, v (float32) -> hl[0][i] = bf16(x), hl[n + i] = bf16(x - hl[i]) of each, v's halves behind k's;  n a multiple of 4
+__global__ void split_hi_lo_kernel(const float* __restrict__ k, const float* __restrict__ v, __nv_bfloat16* __restrict__ khl, int64_t n) {
+  const float* x = blockIdx.y ? v : k;
+  __nv_bfloat16* hl = khl + blockIdx.y * 2 * n;
   for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(x + i);
+    const float4 f = *reinterpret_cast<const float4*>(x + i);
     uint2 h, l;
-    split2(v.x, v.y, &h.x, &l.x);
-    split2(v.z, v.w, &h.y, &l.y);
+    split2(f.x, f.y, &h.x, &l.x);
+    split2(f.z, f.w, &h.y, &l.y);
     *reinterpret_cast<uint2*>(hl + i) = h;
     *reinterpret_cast<uint2*>(hl + n + i) = l;
   }
 }
 
-// qhl: [2][BH][S][D] bf16 (hi, lo); kmap / vmap: 4-D maps over [2][BH][S][D] (d, key, batch-head, hi/lo)
+// q: float32 [BH][S][D]; kmap / vmap: 4-D maps over bf16 [2][BH][S][D] (d, key, batch-head, hi/lo)
 template <int D>
-__global__ void __launch_bounds__(kThreads, 1)
-flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ qhl, const __grid_constant__ CUtensorMap kmap,
+__global__ void __launch_bounds__(kThreads, SmemF<D>::kCtas)
+flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const __grid_constant__ CUtensorMap kmap,
                     const __grid_constant__ CUtensorMap vmap, int64_t BH, int S, float scale, int causal, int* err) {
   using namespace tc;
   typedef SmemF<D> SM;
@@ -91,8 +103,9 @@ flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ q
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t q_full, kv_full[kStages], kv_empty[kStages], s_full[2], s_empty[2], p_full, p_empty;
   __shared__ uint32_t tmem_slot;
-  constexpr uint32_t kTmemCols = 256;
-  constexpr uint32_t kColS = 0, kColO = 128;                  // S: two buffers of 64 columns; O: D columns
+  constexpr uint32_t kTmemCols = D <= 64 ? 256 : 512;
+  constexpr uint32_t kColS = 0, kColP = 128, kColO = 192;     // S: two buffers of 64 columns; P: hi, lo as bf16 pairs; O: D columns
+  static_assert(kColO + D <= kTmemCols && SM::kCtas * kTmemCols <= 512, "tensor memory");
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int qp = (int)gridDim.x - 1 - (int)blockIdx.x;         // heavy (late) causal tiles first
@@ -119,16 +132,20 @@ flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ q
   if (warp >= 5) {
     // ------------------------------ loaders ------------------------------
     const int lw = warp - 5, lt = tid - 5 * 32;
-    const uint32_t sQ = smem_u32(smem + SM::offQ);
-    for (int i = lt; i < 2 * kBM * (D / 8); i += kLoaders) {
-      const int part = i / (kBM * (D / 8)), rem = i - part * (kBM * (D / 8));      // 0: hi, 1: lo
-      const int row = rem / (D / 8), c8 = rem - row * (D / 8);
-      const int qi = q0 + row;
-      const __nv_bfloat16* src = qhl + ((int64_t)part * BH + bh) * (int64_t)S * D + (int64_t)min(qi, S - 1) * D + c8 * 8;
-      cp_async16(sQ + part * SM::kQ + canon(row, c8, kBM), src, qi < S ? 16u : 0u);
+#pragma unroll 4
+    for (int i = lt; i < kBM * (D / 8); i += kLoaders) {
+      const int row = i / (D / 8), c8 = i - row * (D / 8), qi = q0 + row;
+      float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
+      if (qi < S) {
+        const float4* src = reinterpret_cast<const float4*>(q + ((int64_t)bh * S + qi) * D + c8 * 8);
+        f0 = src[0]; f1 = src[1];
+      }
+      uint4 h, l;
+      split2(f0.x, f0.y, &h.x, &l.x); split2(f0.z, f0.w, &h.y, &l.y);
+      split2(f1.x, f1.y, &h.z, &l.z); split2(f1.z, f1.w, &h.w, &l.w);
+      *reinterpret_cast<uint4*>(smem + SM::offQ + canon(row, c8, kBM)) = h;
+      *reinterpret_cast<uint4*>(smem + SM::offQ + SM::kQ + canon(row, c8, kBM)) = l;
     }
-    cp_async_commit();
-    cp_async_wait<0>();
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(&q_full);
@@ -166,12 +183,10 @@ flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ q
         unsigned char* st = smem + SM::offKV + s * 4 * SM::kKV;
 #pragma unroll
         for (int t3 = 0; t3 < 3; ++t3) {
-          const uint64_t adesc = smem_desc(smem_u32(smem + SM::offP + a_part[t3] * SM::kP), kBM * 16, 128);
           const uint64_t bdesc = smem_desc_swz(smem_u32(st + (2 + b_part[t3]) * SM::kKV), kSub, 16 * W, kSwz);
 #pragma unroll
           for (int ks = 0; ks < kBN / 16; ++ks)
-            mma_f16(tmem + kColO, adesc + (uint64_t)(ks * ((2 * kBM * 16) >> 4)), bdesc + (uint64_t)(ks * ((32 * W) >> 4)),
-                    kIdescPV, (j > 0 || ks > 0 || t3 > 0) ? 1u : 0u);
+            mma_f16_ts(tmem + kColO, tmem + kColP + a_part[t3] * 32 + ks * 8, bdesc + (uint64_t)(ks * ((32 * W) >> 4)), kIdescPV, (j > 0 || ks > 0 || t3 > 0) ? 1u : 0u);
         }
         commit(&p_empty);
         commit(&kv_empty[s]);
@@ -234,14 +249,34 @@ flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ q
       mx *= c;
       const bool first = m == -CUDART_INF_F && mx > -CUDART_INF_F;
       const bool raise = m > -CUDART_INF_F && mx > m + kRescaleStep;
+      const float alpha = raise ? exp2f(m - mx) : 1.0f;
+      if (raise) { l *= alpha; m = mx; }
+      if (first) m = mx;
+      const float neg_m = m == -CUDART_INF_F ? 0.f : -m;
+      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t hi[kBN / 2], lo[kBN / 2];
+#pragma unroll
+      for (int i = 0; i < kBN / 2; ++i) {
+        const float p0 = ex2_approx(fmaf(sv[2 * i], c, neg_m)), p1 = ex2_approx(fmaf(sv[2 * i + 1], c, neg_m));
+        sum4[i & 3] += p0 + p1;
+        split2(p0, p1, &hi[i], &lo[i]);
+      }
+      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       // P V of the previous key tile has landed: the single P buffer is free again and O may be rescaled.  This
       // thread waits every phase of the barrier in turn, so the parity is never that of an older phase.
       if (j > 0) {
         mbar_wait(&p_empty, (j - 1) & 1, dead, err);
         fence_after();
       }
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t ph[16], pl[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { ph[i] = hi[16 * hf + i]; pl[i] = lo[16 * hf + i]; }
+        tmem_st16_nowait(tmem + lane_base + kColP + 16 * hf, ph);
+        tmem_st16_nowait(tmem + lane_base + kColP + 32 + 16 * hf, pl);
+      }
       if (__any_sync(0xffffffffu, raise) && j > 0) {
-        const float alpha = raise ? exp2f(m - mx) : 1.0f;
 #pragma unroll
         for (int ch = 0; ch < D / 32; ++ch) {
           float o[32];
@@ -250,30 +285,9 @@ flash_tc_f32_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ q
           for (int i = 0; i < 32; ++i) o[i] *= alpha;
           tmem_st32(tmem + lane_base + kColO + ch * 32, o);
         }
-        fence_before();
       }
-      if (raise) { l *= exp2f(m - mx); m = mx; }
-      if (first) m = mx;
-      const float neg_m = m == -CUDART_INF_F ? 0.f : -m;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      unsigned char* ph = smem + SM::offP;
-      unsigned char* pl = ph + SM::kP;
-#pragma unroll
-      for (int c8 = 0; c8 < kBN / 8; ++c8) {
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = 8 * c8 + 2 * e;
-          const float p0 = ex2_approx(fmaf(sv[i], c, neg_m)), p1 = ex2_approx(fmaf(sv[i + 1], c, neg_m));
-          sum4[e] += p0 + p1;
-          split2(p0, p1, &hi[e], &lo[e]);
-        }
-        *reinterpret_cast<uint4*>(ph + canon(r, c8, kBM)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(pl + canon(r, c8, kBM)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-      }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      fence_async_smem();
-      fence_before();
+      tmem_st_wait();
+      fence_before();                    // orders the stores (P, a rescaled O) before the MMA that the arrive releases
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full);
     }
@@ -345,13 +359,13 @@ int32_t flash_tc_f32_configure() {
   return LMB200_OK;
 }
 
-// out, q, k, v: float32 [BH, S, D] contiguous on the device.  Scratch: the six bf16 halves (3 x 2 x BH x S x D x 2 bytes),
+// out, q, k, v: float32 [BH, S, D] contiguous on the device.  Scratch: the bf16 halves of k and v (2 x 2 x BH x S x D x 2 bytes),
 // kept in the context between calls.  Asynchronous on the context's stream like the bf16 kernel.
 int32_t flash_tc_f32_launch(Ctx* ctx, float* out, const float* q, const float* k, const float* v, int64_t BH, int64_t S, int64_t D,
                             float scale, int causal) {
   const int64_t n = BH * S * D;
   LMB_REQUIRE(n % 4 == 0, "flash attention: element count must be a multiple of 4");
-  const size_t need = (size_t)n * 2 * 3 * sizeof(__nv_bfloat16);
+  const size_t need = (size_t)n * 2 * 2 * sizeof(__nv_bfloat16);
   if (ctx->scratch_bytes < need) {
     if (ctx->capturing)
       return fail(LMB200_ESTATE, "flash attention: the scratch must grow to %lld bytes, which a capture cannot record: run the call once before capture_begin",
@@ -373,20 +387,17 @@ int32_t flash_tc_f32_launch(Ctx* ctx, float* out, const float* q, const float* k
     ctx->scratch_bytes = need;
   }
   if (ctx->capturing) ctx->scratch_in_graph = true;
-  __nv_bfloat16* hl = reinterpret_cast<__nv_bfloat16*>(ctx->scratch);
-  __nv_bfloat16 *qhl = hl, *khl = hl + 2 * n, *vhl = hl + 4 * n;
-  const unsigned grid1 = (unsigned)std::min<int64_t>(ceil_div(n / 4, 256), 148 * 16);
-  split_hi_lo_kernel<<<grid1, 256, 0, ctx->stream>>>(q, qhl, n);
-  split_hi_lo_kernel<<<grid1, 256, 0, ctx->stream>>>(k, khl, n);
-  split_hi_lo_kernel<<<grid1, 256, 0, ctx->stream>>>(v, vhl, n);
-  ctx->launches += 3;
+  __nv_bfloat16 *khl = reinterpret_cast<__nv_bfloat16*>(ctx->scratch), *vhl = khl + 2 * n;
+  const unsigned grid1 = (unsigned)std::min<int64_t>(ceil_div(n / 4, 256), 148 * 8);
+  split_hi_lo_kernel<<<dim3(grid1, 2), 256, 0, ctx->stream>>>(k, v, khl, n);
+  ctx->launches++;
   CUtensorMap kmap, vmap;
   int32_t rc = hl_tensor_map(&kmap, khl, BH, S, D);
   if (rc == LMB200_OK) rc = hl_tensor_map(&vmap, vhl, BH, S, D);
   if (rc == LMB200_OK) {
     dim3 grid((unsigned)ceil_div(S, kBM), (unsigned)BH);
 #define LMB_FLASH(DD) \
-  flash_tc_f32_kernel<DD><<<grid, kThreads, SmemF<DD>::total + 1024, ctx->stream>>>(out, qhl, kmap, vmap, BH, (int)S, scale, causal, ctx->dev_err)
+  flash_tc_f32_kernel<DD><<<grid, kThreads, SmemF<DD>::total + 1024, ctx->stream>>>(out, q, kmap, vmap, BH, (int)S, scale, causal, ctx->dev_err)
     if (D == 128) LMB_FLASH(128);
     else if (D == 96) LMB_FLASH(96);
     else if (D == 64) LMB_FLASH(64);
