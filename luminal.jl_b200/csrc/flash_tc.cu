@@ -135,6 +135,8 @@ struct FlashExtra {
   int64_t o_b = 0, o_h = 0, o_s = 0;
   const float* gate = nullptr;
   int gate_pitch = 0;
+  const int* cu = nullptr;          // [B + 1]: sequence b is rows cu[b] .. cu[b + 1] - 1 of packed tensors (one batch element); causal only:
+                                    // the keys behind a sequence's end belong to the next one and are masked
   int window = 0;                   // a query sees the last `window` positions (0: all)
   float cap = 0.f;                  // scores pass cap tanh(. / cap) (0: not)
   float poly[4] = {0.f, 0.f, 0.f, 0.f};      // WIN 2: cap tanh(z) log2(e) = z (poly[0] + poly[1] z^2 + ...) for every z that occurs
@@ -151,7 +153,7 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
 template <int DN, int DR, int DV, int WIN>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q, const __grid_constant__ CUtensorMap kmap,
-                   const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap rmap, const FlashView fv, const FlashExtra ex, int S,
+                   const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap rmap, const FlashView fv, const FlashExtra ex, int S_all,
                    float scale, int causal, int* err) {
   constexpr int D = DN + DR;
   constexpr int W = DN % 64 == 0 ? 64 : 32;           // head dims per swizzled sub-tile
@@ -163,7 +165,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   constexpr int kStages = SM::kStages, vStages = SM::vStages;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[vStages], v_empty[vStages];
-  __shared__ __align__(8) uint64_t s_full[2], p_full[2], o_done[2];
+  __shared__ __align__(8) uint64_t s_full[2], p_full[2], o_done[2], v_tail;
   __shared__ float xch[2][2][kBM];                    // [tile][column half][row]: the halves' row maxima, later their sums
   __shared__ uint32_t tmem_slot;
   constexpr uint32_t kTmemCols = 512;
@@ -173,11 +175,14 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   const int qp = (int)gridDim.x - 1 - (int)blockIdx.x;        // heavy (late) causal tiles first
   const int q0 = qp * 2 * kBM;
   const int bi = (int)blockIdx.y / fv.H, hi = (int)blockIdx.y - bi * fv.H;
-  const __nv_bfloat16* qb = q + bi * fv.q_b + hi * fv.q_h;
+  const int row0 = ex.cu ? ex.cu[bi] : 0, S = ex.cu ? ex.cu[bi + 1] - row0 : S_all;
+  if (q0 >= S) return;                                // a packed sequence shorter than the longest
+  const int kv_b = ex.cu ? 0 : bi;
+  const __nv_bfloat16* qb = q + (ex.cu ? row0 * fv.q_s : bi * fv.q_b) + hi * fv.q_h;
   const int kvh = hi / fv.G;
-  __nv_bfloat16* ob_base = out + bi * ex.o_b + hi * ex.o_h;
+  __nv_bfloat16* ob_base = out + (ex.cu ? row0 * ex.o_s : bi * ex.o_b) + hi * ex.o_h;
   const int64_t q_s = fv.q_s;
-  const int Sk = ex.Sk, q_off = ex.q_off;
+  const int Sk = ex.cu ? S : ex.Sk, q_off = ex.q_off;
   int n_tiles[2], first[2];                           // key tiles first[t] .. n_tiles[t] - 1
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
@@ -194,6 +199,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
     for (int s = 0; s < kStages; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
     for (int s = 0; s < vStages; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 8); mbar_init(&o_done[t], 1); }
+    mbar_init(&v_tail, 1);
     mbar_init_fence();
   }
   if (warp == kMmaWarp) tmem_alloc(&tmem_slot, kTmemCols);
@@ -228,14 +234,26 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
     for (int j = jb; j < n_max; ++j) {
       const int s = (j - jb) % stages;
       mbar_wait(&empty[s], (((j - jb) / stages) & 1) ^ 1, dead, err);
+      const bool tail = ex.cu && lw == 1 && (j + 1) * kBN > Sk;
+      unsigned char* at = smem + off + s * stage_bytes;
       if (lane == 0) {
-        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
-        unsigned char* at = smem + off + s * stage_bytes;
-        for (int sub = 0; sub < subs; ++sub) tma_load_4d(at + sub * kSub, map, sub * W, j * kBN, kvh, bi, &full[s]);
+        uint64_t* bar = tail ? &v_tail : &full[s];
+        mbar_expect_tx(bar, (uint32_t)stage_bytes);
+        for (int sub = 0; sub < subs; ++sub) tma_load_4d(at + sub * kSub, map, sub * W, row0 + j * kBN, kvh, kv_b, bar);
         if (DR > 0 && lw == 0)
-          for (int sub = 0; sub < DR / W; ++sub) tma_load_4d(at + (DN / W + sub) * kSub, &rmap, sub * W, j * kBN, 0, bi, &full[s]);
+          for (int sub = 0; sub < DR / W; ++sub) tma_load_4d(at + (DN / W + sub) * kSub, &rmap, sub * W, row0 + j * kBN, 0, kv_b, &full[s]);
       }
       __syncwarp();
+      if (tail) {
+        // rows behind a packed sequence's end are the next one's: their weight is 0, but 0 times an infinity or NaN over there
+        // would reach this sequence.  Whole rows are cleared, so the swizzle does not matter
+        mbar_wait(&v_tail, 0, dead, err);
+        for (int sub = 0; sub < subs; ++sub)
+          for (int i = (Sk - j * kBN) * (W / 8) + lane; i < kBN * (W / 8); i += 32) reinterpret_cast<uint4*>(at + sub * kSub)[i] = make_uint4(0, 0, 0, 0);
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[s]);
+      }
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------ MMA issue ------------------------------
@@ -548,16 +566,20 @@ int32_t kv_tensor_map(CUtensorMap* map, const void* base, int64_t n_kv, int64_t 
 }
 }  // namespace
 
-// q, out: element (b, h, s, d) at b * q_b + h * q_h + s * q_s + d; k, v likewise with the k strides
+// q, out: element (b, h, s, d) at b * q_b + h * q_h + s * q_s + d; k, v likewise with the k strides.  cu (NULL or device [B + 1], causal
+// only): sequence b is rows cu[b] .. cu[b + 1] - 1 of tensors of `total` rows, none longer than S; the batch strides are not used
 int32_t flash_tc_launch_view(Ctx* ctx, void* out, const void* q, const void* k, const void* v, const FlashView& fv, int64_t B,
-                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream) {
+                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream, const int* cu, int64_t total) {
+  LMB_REQUIRE(!cu || causal, "flash attention: packed sequences are causal");
   dim3 grid((unsigned)ceil_div(S, 2 * kBM), (unsigned)(B * fv.H));
   CUtensorMap kmap, vmap;
   const int W = D % 64 == 0 ? 64 : 32;
   const int64_t n_kv = fv.H / fv.G;
-  LMB_TRY(kv_tensor_map(&kmap, k, n_kv, B, S, D, fv.k_s, fv.k_h, fv.k_b, W));
-  LMB_TRY(kv_tensor_map(&vmap, v, n_kv, B, S, D, fv.k_s, fv.k_h, fv.k_b, W));
+  const int64_t map_B = cu ? 1 : B, map_S = cu ? total : S;
+  LMB_TRY(kv_tensor_map(&kmap, k, n_kv, map_B, map_S, D, fv.k_s, fv.k_h, fv.k_b, W));
+  LMB_TRY(kv_tensor_map(&vmap, v, n_kv, map_B, map_S, D, fv.k_s, fv.k_h, fv.k_b, W));
   FlashExtra ex;
+  ex.cu = cu;
   ex.Sk = (int)S; ex.dn = ex.dv = (int)D;
   ex.o_b = fv.q_b; ex.o_h = fv.q_h; ex.o_s = fv.q_s;
 #define LMB_FLASH(DD)                                                                                                   \
@@ -674,7 +696,7 @@ int32_t flash_tc_launch(Ctx* ctx, void* out, const void* q, const void* k, const
   FlashView fv;                       // [B*H, S, D] contiguous, as the op's tensors are
   fv.H = 1; fv.G = 1;
   fv.q_b = fv.k_b = S * D; fv.q_h = fv.k_h = 0; fv.q_s = fv.k_s = D;
-  return flash_tc_launch_view(ctx, out, q, k, v, fv, BH, S, D, scale, causal, ctx->stream);
+  return flash_tc_launch_view(ctx, out, q, k, v, fv, BH, S, D, scale, causal, ctx->stream, nullptr, 0);
 }
 
 }  // namespace lmb

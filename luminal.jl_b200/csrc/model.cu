@@ -2267,7 +2267,7 @@ extern "C" int32_t lmb200_prefill(lmb200_session h, const int32_t* tokens, int32
   if (prefill_gemm_ok(S, n)) {
     // every position at once: GEMMs + flash attention, then the head on the last position
     LMB_CUDA(cudaMemcpyAsync(S->prompt, tokens, (size_t)n * B * 4, cudaMemcpyHostToDevice, ctx->stream));
-    LMB_TRY(prefill_gemm(S, S->prompt, n, nullptr, ctx->stream));
+    LMB_TRY(prefill_gemm(S, S->prompt, n, RaggedRows(), ctx->stream));
     LMB_CUDA(cudaMemsetAsync(S->step_ctr, 0, 4, ctx->stream));
     LMB_TRY(enqueue_head_bf16(S, ctx->stream));
     LMB_TRY(set_all_positions(S, S->host_pos + n));
@@ -2293,8 +2293,8 @@ extern "C" int32_t lmb200_prefill(lmb200_session h, const int32_t* tokens, int32
 // length; a batch of real prompts does not).  tokens: [batch, n_max] row-major, sequence b uses its first lengths[b]
 // ids.  logits_out (NULL or [batch, vocab]): for every sequence the logits of ITS last prompt position.  Afterwards
 // sequence b stands at its old position + lengths[b] and decoding goes on with one position per sequence.
-// A fresh bf16 Llama / Phi-3 session runs all positions at once through the prompt GEMMs (the padding behind a short
-// prompt is computed and never read: attention is causal and later steps overwrite those cache slots); otherwise
+// A fresh bf16 Llama / Phi-3 session runs all positions at once through the prompt GEMMs, the prompts packed one after the
+// other (no padding is computed); otherwise
 // the prompt goes through the decode step, a finished sequence standing still while the longer ones go on.
 extern "C" int32_t lmb200_prefill_ragged(lmb200_session h, const int32_t* tokens, const int32_t* lengths, int32_t n_max,
                                          float* logits_out) {
@@ -2318,28 +2318,33 @@ extern "C" int32_t lmb200_prefill_ragged(lmb200_session h, const int32_t* tokens
     for (int b = 0; b < B; ++b) packed.insert(packed.end(), tokens + (size_t)b * n_max, tokens + (size_t)b * n_max + lengths[b]);
     return extend_last(S, packed.data(), std::vector<int32_t>(lengths, lengths + B), logits_out);
   }
-  if ((int64_t)longest * B > S->prompt_cap) {
+  const bool packed = !S->ragged && prefill_gemm_ok(S, longest);
+  int64_t total = 0;
+  for (int b = 0; b < B; ++b) total += lengths[b];
+  LMB_REQUIRE(total <= 0x3fffffff, "prefill_ragged: %lld tokens", (long long)total);
+  const int64_t need = packed ? 2 * total + B + 1 : (int64_t)longest * B;         // packed: tokens, their positions, the prompts' starts
+  if (need > S->prompt_cap) {
     cudaFree(S->prompt);
     S->prompt = nullptr;
     S->prompt_cap = 0;
-    LMB_TRY(dmalloc((void**)&S->prompt, (int64_t)longest * B * 4, false, ctx->stream));
-    S->prompt_cap = (int64_t)longest * B;
+    LMB_TRY(dmalloc((void**)&S->prompt, need * 4, false, ctx->stream));
+    S->prompt_cap = need;
   }
   std::vector<int> new_pos(B), limits(B);
   for (int b = 0; b < B; ++b) new_pos[b] = limits[b] = S->host_pos_v[b] + lengths[b];
-  if (!S->ragged && prefill_gemm_ok(S, longest)) {
-    std::vector<int32_t> tk((size_t)longest * B, 0);            // [B, longest]
-    for (int b = 0; b < B; ++b)
-      for (int i = 0; i < lengths[b]; ++i) tk[(size_t)b * longest + i] = tokens[(size_t)b * n_max + i];
-    int* lens_dev = nullptr;
-    LMB_TRY(dmalloc((void**)&lens_dev, (int64_t)B * 4, false, ctx->stream));
-    int32_t rc = LMB200_OK;
-    if (cudaMemcpyAsync(S->prompt, tk.data(), tk.size() * 4, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
-        cudaMemcpyAsync(lens_dev, lengths, (size_t)B * 4, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-      rc = fail(LMB200_ECUDA, "prefill_ragged: upload failed");
-    if (rc == LMB200_OK) rc = prefill_gemm(S, S->prompt, longest, lens_dev, ctx->stream);
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(lens_dev);
+  if (packed) {
+    std::vector<int32_t> tk((size_t)need);
+    for (int64_t b = 0, at = 0; b < B; at += lengths[b], ++b) {
+      memcpy(tk.data() + at, tokens + (size_t)b * n_max, (size_t)lengths[b] * 4);
+      for (int i = 0; i < lengths[b]; ++i) tk[total + at + i] = i;
+      tk[2 * total + b] = (int32_t)at;
+    }
+    tk[2 * total + B] = (int32_t)total;
+    LMB_CUDA(cudaMemcpyAsync(S->prompt, tk.data(), tk.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    RaggedRows rows;
+    rows.total = (int)total; rows.pos = S->prompt + total; rows.cu = S->prompt + 2 * total;
+    const int32_t rc = prefill_gemm(S, S->prompt, longest, rows, ctx->stream);
+    cudaStreamSynchronize(ctx->stream);                           // the staging array goes
     LMB_TRY(rc);
     LMB_CUDA(cudaMemsetAsync(S->step_ctr, 0, 4, ctx->stream));
     LMB_TRY(enqueue_head_bf16(S, ctx->stream));

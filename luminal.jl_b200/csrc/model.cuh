@@ -311,8 +311,13 @@ int32_t gemm_silu_gate_bf16(Ctx* ctx, const void* W, const void* X, int ldx, int
 // prompt phase as GEMMs + flash attention (csrc/prefill.cu)
 int32_t prefill_configure();
 bool prefill_gemm_ok(const Session* S, int n);
-// lens_dev: NULL (every sequence has n tokens) or device [B] prompt lengths <= n (the last-position rows are taken per sequence)
-int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const int* lens_dev, cudaStream_t st);
+// prompts of unequal length packed one after the other: device arrays; total 0: every sequence has n tokens
+struct RaggedRows {
+  int total = 0;
+  const int* pos = nullptr;             // [total]: each token's position in its prompt
+  const int* cu = nullptr;              // [B + 1]: where the prompts begin, and the total
+};
+int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows& ragged, cudaStream_t st);
 int32_t prefill_linear(Ctx* ctx, const void* W, const float* x_dev, int T, int rows, int K, float* out_dev, cudaStream_t st);
 Model* model_from(lmb200_model h);
 Session* session_from(lmb200_session h);

@@ -28,7 +28,7 @@
 namespace lmb {
 
 int32_t flash_tc_launch_view(Ctx* ctx, void* out, const void* q, const void* k, const void* v, const FlashView& fv, int64_t B,
-                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream);
+                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream, const int* cu = nullptr, int64_t total = 0);
 bool flash_tc_supported(int64_t D);
 
 namespace {
@@ -67,6 +67,7 @@ struct GemmParams {
   void* out_any = nullptr;
   RowSegs segs;                         // GEMM_SEGMENTS
   const float2* rope = nullptr;         // [n_seq, D/2]: (sin, cos) of position pos0 + s times inv_freq[d0]
+  const int* tok_pos = nullptr;         // packed prompts of unequal length: [T], the row of `rope` for each token
   int pos0 = 0, n_seq = 1, Hl = 0, KVl = 0, D = 0;
   // Implicit 1-D convolution (conv_taps > 0; src/NN.jl:55-104 without the unfolded buffer): X is the token-major input
   // [conv_B][conv_rows_in][ldx] (channels contiguous, conv_rows_in a multiple of the stride conv_P, rows past the valid
@@ -310,11 +311,11 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32
     const int col = rbl * 8 + g + (hi ? 16 : 0);
     // all table reads of the chunk first: between stores the compiler could not move them
     float2 sc[32];
-    int sq = t0 % p.n_seq;
+    const int own = p.tok_pos ? (lane < n_tok ? __ldg(p.tok_pos + t0 + lane) : 0) : (t0 + lane) % p.n_seq;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
+      const int sq = __shfl_sync(0xffffffffu, own, i);
       sc[i] = i < n_tok ? __ldg(p.rope + (int64_t)sq * half + d0) : make_float2(0.f, 1.f);
-      if (++sq == p.n_seq) sq = 0;
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -825,15 +826,17 @@ int32_t gemm_configure() {
 // contiguous elements (K units then V units, the layout of kcache_offset / vcache_offset).
 __global__ void __launch_bounds__(256) cache_fill_kernel(__nv_bfloat16* __restrict__ kv_layer, int64_t batch_stride, int64_t head_stride,
                                                          const __nv_bfloat16* __restrict__ kbuf, const __nv_bfloat16* __restrict__ vbuf,
-                                                         int ldkv, int n_seq, int pos0, int KVl, int D) {
+                                                         int ldkv, int n_seq, int pos0, int KVl, int D, const int* __restrict__ cu) {
   const int blk = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  int64_t row0 = (int64_t)b * n_seq;
+  if (cu) { row0 = cu[b]; n_seq = cu[b + 1] - cu[b]; }            // packed prompts of unequal length
   __nv_bfloat16* base = kv_layer + b * batch_stride + kvh * head_stride;
   for (int i = threadIdx.x; i < 16 * D; i += 256) {
     const int key = i / D, d = i - key * D;
     const int sq = blk * 16 + key - (pos0 & 15);                 // position pos0 + sq sits in block (pos0 >> 4) + blk
     if (sq < 0 || sq >= n_seq) continue;
     const int pos = pos0 + sq;
-    const int64_t src = ((int64_t)b * n_seq + sq) * ldkv + kvh * D + d;
+    const int64_t src = (row0 + sq) * ldkv + kvh * D + d;
     base[kcache_offset(pos, d, D)] = kbuf[src];
     base[vcache_offset(pos, d, D)] = vbuf[src];
   }
@@ -887,9 +890,9 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(float* __restrict__ x
 
 // the residual rows of each sequence's last prompt position -> the decode step's [B, n] buffer
 __global__ void last_rows_kernel(float* __restrict__ dst, const float* __restrict__ x, const float* __restrict__ delta, int n_seq,
-                                 int n, const int* __restrict__ lens) {
+                                 int n, const int* __restrict__ cu) {
   const int b = blockIdx.x;
-  const int64_t t = (int64_t)b * n_seq + (lens ? lens[b] : n_seq) - 1;
+  const int64_t t = cu ? cu[b + 1] - 1 : (int64_t)(b + 1) * n_seq - 1;
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[(int64_t)b * n + i] = x[t * n + i] + (delta ? delta[t * n + i] : 0.f);
 }
 
@@ -1004,14 +1007,15 @@ bool prefill_gemm_ok(const Session* S, int n) {
          c.hidden % 8 == 0 && M->inter_l % 8 == 0;
 }
 
-// tokens_dev: [B, n] int32, sequence-major.  On return the cache holds positions 0..n-1 of every
-// sequence and S->x the residual rows of the last position (the caller runs the final norm + head).
-int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const int* lens_dev, cudaStream_t st) {
+// tokens_dev: [B, n] int32, sequence-major -- or, with ragged.total > 0, the prompts of unequal length one after the other (none
+// longer than n).  On return the cache holds every sequence's prompt and S->x the residual rows of its last position (the caller
+// runs the final norm + head).  Unequal prompts are packed, not padded: five prompts of 97 to 777 tokens have 56 % of the padded rows.
+int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows& ragged, cudaStream_t st) {
   Model* M = S->m;
   Ctx* ctx = M->ctx;
   const lmb200_model_config& c = M->cfg;
   const int B = S->B, hid = c.hidden, L = c.n_layers, D = M->D;
-  const int T = B * n;
+  const int T = ragged.total > 0 ? ragged.total : B * n;
   const int qw = M->Hl * D, kvw = M->KVl * D;
   // one scratch block per session, kept for the next prompt of the same or a smaller size
   const int64_t sizes[9] = {(int64_t)T * hid * 4, (int64_t)T * hid * 4, (int64_t)T * hid * 2, (int64_t)T * qw * 2, (int64_t)T * kvw * 2,
@@ -1062,13 +1066,13 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const int* lens_d
       p.q = q; p.kbuf = kb; p.vbuf = vb; p.ldq = qw; p.ldkv = kvw;
       p.kv_layer = reinterpret_cast<__nv_bfloat16*>(S->kv) + (int64_t)l * S->kv_layer_stride;
       p.kv_batch_stride = S->kv_batch_stride; p.kv_head_stride = S->kv_head_stride;
-      p.rope = rope; p.pos0 = 0; p.n_seq = n; p.Hl = M->Hl; p.KVl = M->KVl; p.D = D;
+      p.rope = rope; p.pos0 = 0; p.n_seq = n; p.tok_pos = ragged.pos; p.Hl = M->Hl; p.KVl = M->KVl; p.D = D;
       LMB_TRY(gemm_launch(ctx, p, st));
       cache_fill_kernel<<<dim3((unsigned)ceil_div(n, 16), (unsigned)M->KVl, (unsigned)B), 256, 0, st>>>(
-          p.kv_layer, p.kv_batch_stride, p.kv_head_stride, kb, vb, kvw, n, 0, M->KVl, D);
+          p.kv_layer, p.kv_batch_stride, p.kv_head_stride, kb, vb, kvw, n, 0, M->KVl, D, ragged.cu);
       ctx->launches++;
     }
-    LMB_TRY(flash_tc_launch_view(ctx, attn, q, kb, vb, fv, B, n, D, 1.0f / sqrtf((float)D), 1, st));
+    LMB_TRY(flash_tc_launch_view(ctx, attn, q, kb, vb, fv, B, n, D, 1.0f / sqrtf((float)D), 1, st, ragged.cu, T));
     {
       GemmParams p;
       p.W = reinterpret_cast<const __nv_bfloat16*>(W.wo); p.X = attn; p.ldx = qw; p.T = T; p.rows = hid; p.K = qw;
@@ -1092,7 +1096,7 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const int* lens_d
       LMB_TRY(reduce(delta));
     }
   }
-  last_rows_kernel<<<B, 256, 0, st>>>(S->x, x, delta, n, hid, lens_dev);
+  last_rows_kernel<<<B, 256, 0, st>>>(S->x, x, delta, n, hid, ragged.cu);
   ctx->launches++;
   LMB_CUDA(cudaGetLastError());
   LMB_CUDA(cudaStreamSynchronize(st));

@@ -33,7 +33,7 @@ int32_t gemm_conv1d(Ctx* ctx, const void* W, const __nv_bfloat16* X, int ldx, in
 int32_t gemm_cross_kv(Ctx* ctx, const void* W, const __nv_bfloat16* X, int ldx, int T, int rows, int K, const float* bias, float scale,
                       void* kv_layer, int64_t batch_stride, int64_t head_stride, int n_seq, int D, int is_v, cudaStream_t st);
 int32_t flash_tc_launch_view(Ctx* ctx, void* out, const void* q, const void* k, const void* v, const FlashView& fv, int64_t B,
-                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream);
+                             int64_t S, int64_t D, float scale, int causal, cudaStream_t stream, const int* cu = nullptr, int64_t total = 0);
 bool flash_tc_supported(int64_t D);
 
 namespace {

@@ -120,3 +120,32 @@ def test_extend_mixes_portions_and_single_tokens(lib_built, device):
 def _step_logits(w, cfg, toks):
     m = O.CachedLlama(w, cfg, 1, 64)
     return [m.forward(np.asarray([[t]])) for t in toks]
+
+
+def test_packed_prompts_keep_to_themselves(lib_built, device):
+    """Unequal bf16 prompts are packed row behind row: lengths around the 128-key and 256-query tiles give each sequence the logits
+    it has alone, and a sequence of infinities leaves its neighbours untouched, bit for bit."""
+    L = lib_built
+    cfg = dict(O.CONFIGS["mid_gqa"], vocab=512)
+    w = O.synth_llama_weights(cfg, seed=23)
+    w["model.embed_tokens.weight"][511] = np.inf
+    lens = [129, 8, 300, 127, 256, 1]
+    prompts = [O.synth_tokens(23, 700 + b, (n,), 511) for b, n in enumerate(lens)]
+    model = make_model(L, device, cfg, w, "bf16")
+    sess = L.Session(model, len(lens), 320)
+    clean = sess.prefill_ragged(prompts)
+    alone = L.Session(model, 1, 320)
+    for b, p in enumerate(prompts):
+        if len(p) < 8:
+            continue                                    # shorter prompts alone go through the decode step
+        alone.reset()
+        ref = alone.prefill(np.asarray(p, np.int32)[None])[0]
+        # the same kernels on other rows of a tile: bf16 roundings may flip, nothing else
+        assert np.linalg.norm(clean[b] - ref) <= 5e-3 * np.linalg.norm(ref), b
+    bad = list(prompts)
+    bad[3] = np.full(lens[3], 511)
+    sess.reset()
+    got = sess.prefill_ragged(bad)
+    keep = [b for b in range(len(lens)) if b != 3]
+    assert np.array_equal(got[keep], clean[keep]) and not np.isfinite(got[3]).all()
+    alone.close(); sess.close(); model.close()
