@@ -16,6 +16,7 @@
 //
 // float32 ("ring") kernel: weights streamed by plain loads through a register ring, fp32 FMAs --
 // the parity path.
+#include <algorithm>
 #include <type_traits>
 
 #include "gemv.cuh"
@@ -516,6 +517,22 @@ __device__ __forceinline__ void tmem_load_row<16>(float (&v)[16], uint32_t taddr
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// What a row's epilogue reads besides the accumulators; the chain kernel fetches it while the weights stream.
+struct RowConst { float wg, bias, inv_freq; int pos; };
+__device__ __forceinline__ RowConst row_const(const GemvParams& p, int row) {
+  RowConst rc = {0.f, 0.f, 0.f, 0};
+  if (row < p.rows) {
+    if (p.ln_wg) rc.wg = p.ln_wg[row];
+    if (p.bias) rc.bias = p.bias[row];
+  }
+  if (p.epi == EPI_QKV_ROPE) {
+    rc.pos = p.pos[0];
+    const int rb = row >> 4, tiles_per_head = p.D >> 4;
+    if (p.rope && rb / tiles_per_head < p.Hl + p.KVl) rc.inv_freq = p.inv_freq[8 * (rb % tiles_per_head) + (row & 7)];
+  }
+  return rc;
+}
+
 // Epilogue of one accumulator row held by one thread (v[b], b < N).  Rows g and g+8 of a 16-row
 // block -- the pairs the fused epilogues combine -- are 8 lanes apart in the same warp.
 // The thread holds batch columns b0 .. b0+NV-1 of the row (the whole row when NV == BP); BP is the
@@ -523,7 +540,7 @@ __device__ __forceinline__ void tmem_load_row<16>(float (&v)[16], uint32_t taddr
 // X: the epilogues of decoders described layer by layer (softcap, EPI_STORE_RELU2) are compiled in.  They have instantiations of their
 // own: the other models' kernels carry no code of them.
 template <int NV, int BP, bool X>
-__device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV], int row, int b0, const float* s_inv) {
+__device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV], int row, int b0, const float* s_inv, const RowConst& rc) {
   typedef Layout<__nv_bfloat16> LY;
   constexpr int N = NV;
   const int rb = row >> 4, rr = row & 15, g = rr & 7, hi = rr >> 3;
@@ -531,15 +548,13 @@ __device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV]
 #pragma unroll
     for (int b = 0; b < N; ++b) v[b] *= s_inv[b0 + b];
     if (p.ln_wg) {                               // LayerNorm: the mean's share, inv * mu * (W g)[row]
-      const float wg = row < p.rows ? p.ln_wg[row] : 0.f;
 #pragma unroll
-      for (int b = 0; b < N; ++b) v[b] -= s_inv[32 + b0 + b] * wg;
+      for (int b = 0; b < N; ++b) v[b] -= s_inv[32 + b0 + b] * rc.wg;
     }
   }
   if (p.bias) {
-    const float bias = row < p.rows ? p.bias[row] : 0.f;
 #pragma unroll
-    for (int b = 0; b < N; ++b) v[b] += bias;
+    for (int b = 0; b < N; ++b) v[b] += rc.bias;
   }
   if (p.epi == EPI_STORE_F32) {
     if (row < p.rows) {
@@ -617,13 +632,13 @@ __device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV]
   const int D = p.D, tiles_per_head = D >> 4, half = D >> 1;
   // One position per sequence.  When the host knows they are all equal (pos_uniform) the rotation's sine and
   // cosine are computed once per row; otherwise once per batch column.
-  int pos = p.pos[0];
+  int pos = rc.pos;
   const int hs = rb / tiles_per_head, jj = rb - hs * tiles_per_head;
   if (hs < p.Hl + p.KVl) {
     // rows g / g+8 of the block are the RoPE pair (d0, d0 + D/2)      src/NN.jl:253-303
     const int d0 = 8 * jj + g;
     float sn = 0.f, cs = p.qk_scale;                // no rotation: q and k rows are only scaled
-    const float inv_f = p.rope ? p.inv_freq[d0] : 0.f;
+    const float inv_f = rc.inv_freq;
     if (p.rope) {
       const float ang = (float)pos * inv_f;
       sn = sinf(ang);
@@ -682,18 +697,24 @@ namespace {
 // per-sequence scale 1 / sqrt(mean(x*x) + eps) (src/HighLevelOps.jl:299-304).  Four lanes share a
 // sequence; each adds every fourth slot in ascending order and the four are combined pairwise, the
 // same arithmetic in every CTA and on every rank.
+// Slots part, part + 4, ... added in ascending order, 16 loads in flight: one load after the other took 9 us for 128 slots.
+__device__ __forceinline__ float sum_slots(const float* slots, int tiles, int part, int b) {
+  float s = 0.f;
+  for (int t0 = part; t0 < tiles; t0 += 64) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = t0 + 4 * i < tiles ? __ldcg(slots + (t0 + 4 * i) * 32 + b) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s += v[i];
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s;
+}
 __device__ __forceinline__ void compute_inv_scale(const InvScale& iv, float* s_inv, int e) {
   if (!iv.ssq) return;
   const int b = e >> 2, part = e & 3;
-  float s = 0.f, sx = 0.f;
-  for (int t = part; t < iv.tiles; t += 4) s += __ldcg(iv.ssq + t * 32 + b);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  if (iv.sum) {
-    for (int t = part; t < iv.tiles; t += 4) sx += __ldcg(iv.sum + t * 32 + b);
-    sx += __shfl_xor_sync(0xffffffffu, sx, 1);
-    sx += __shfl_xor_sync(0xffffffffu, sx, 2);
-  }
+  const float s = sum_slots(iv.ssq, iv.tiles, part, b), sx = iv.sum ? sum_slots(iv.sum, iv.tiles, part, b) : 0.f;
   if (part == 0) {
     const float rn = 1.0f / (float)iv.n;
     const float mu = sx * rn;                                   // 0 for RMSNorm
@@ -1138,7 +1159,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_tc_kernel(const GemvParams
       int c_first, n;
       contributors(ur, r, &c_first, &n);
       if (n == 1) {
-        row_epilogue<N, N, X>(p, v, r * 128 + row_in_group, 0, s_inv);
+        row_epilogue<N, N, X>(p, v, r * 128 + row_in_group, 0, s_inv, row_const(p, r * 128 + row_in_group));
         continue;
       }
       float4* part = reinterpret_cast<float4*>(p.partials) + (int64_t)r * p.ksplit * (128 * N / 4);
@@ -1207,7 +1228,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_tc_kernel(const GemvParams
             const float4 t = lds4(slot);
             v4[0] += t.x; v4[1] += t.y; v4[2] += t.z; v4[3] += t.w;
           }
-          row_epilogue<4, N, X>(p, v4, pend_r[ip] * 128 + 16 * (ci_[ip] + jj * n_[ip]) + row16, 4 * cg, s_inv);
+          const int row = pend_r[ip] * 128 + 16 * (ci_[ip] + jj * n_[ip]) + row16;
+          row_epilogue<4, N, X>(p, v4, row, 4 * cg, s_inv, row_const(p, row));
         }
         return slot;
       };
@@ -1239,7 +1261,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_tc_kernel(const GemvParams
               v4[0] += t.x; v4[1] += t.y; v4[2] += t.z; v4[3] += t.w;
             }
           }
-          row_epilogue<4, N, X>(p, v4, pend_r[ip] * 128 + 16 * ci_[ip] + row16, 4 * cg, s_inv);
+          const int row = pend_r[ip] * 128 + 16 * ci_[ip] + row16;
+          row_epilogue<4, N, X>(p, v4, row, 4 * cg, s_inv, row_const(p, row));
         }
       }
       if (tid == 64) LMB_TRACE(13);
@@ -1442,7 +1465,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
           const float4 t = recv[((src * rows_per + 16 * j + row16) * N) / 4 + cg];
           v4[0] += t.x; v4[1] += t.y; v4[2] += t.z; v4[3] += t.w;
         }
-        row_epilogue<4, N, X>(p, v4, r * 128 + c * rows_per + 16 * j + row16, 4 * cg, s_inv);
+        const int row = r * 128 + c * rows_per + 16 * j + row16;
+        row_epilogue<4, N, X>(p, v4, row, 4 * cg, s_inv, row_const(p, row));
       }
     }
   }
@@ -1454,6 +1478,378 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
   if (tid == 0) { LMB_TRACE(9); LMB_TRACE_NS(11); }
+}
+
+// =============================================================================================
+// Chain kernel: several dependent GEMVs of a step in one launch.
+//
+// A decode step is a chain of short GEMVs, and one launch each leaves HBM idle between the last MMA of one and the
+// first bytes of the next: fold, epilogue, drain, launch, set-up and ring fill, about 8 us of which a 34 to 50 MB matrix streams
+// for 5 to 8.  Here one persistent grid (clusters of 4 CTAs, one CTA per SM) runs them all.  Weights depend on nothing, so the
+// weight producer walks straight through the list and has its ring full of the next GEMV's units when that one may start.
+//   Work: cluster i takes row groups i, i + n, ...; CTA c of it the c-th quarter of the k range.  A warp's 32 accumulator rows
+//   are exactly the rows one CTA of the cluster finalises: it sends them there with st.async (the receiver's mbarrier
+//   counts the bytes; no fence, no cluster barrier), and the receiver adds the four parts in CTA order.
+//   Dependency: every CTA counts itself into done[op] once its epilogues are written; the activation producer and
+//   the epilogue warps of the next GEMV wait for that count.  Counting all CTAs is enough for the buffers that are written again
+//   (xg, ssq, act) as well: whoever writes them has waited for all readers.
+//   warp 0 weights, 1 MMA, 2..5 epilogue, 6 activations.
+// =============================================================================================
+constexpr int kChainThreads = 7 * 32;
+constexpr int kChainLine = 32;               // counters are a 128-byte line apart
+
+struct ChainParams {
+  GemvParams op[kChainMax];
+  int n_ops = 0;
+  unsigned* done = nullptr;                  // [kChainMax + 1] lines, zero between launches; the last one counts exits
+};
+
+template <int N> constexpr int kChainStages = N == 16 ? 6 : 5;
+template <int N> constexpr size_t chain_smem() { return (size_t)kChainStages<N> * (kWStage + N * 256) + 128 * N * 4 + 1024; }
+
+__device__ __forceinline__ void dsmem_store4_async(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1,%2,%3,%4}, [%5];\n" ::"r"(addr), "f"(a), "f"(b),
+               "f"(c), "f"(d), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity, bool& dead, int* err) {
+  if (dead) return;
+  const long long t0 = clock64();
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return;
+    if (clock64() - t0 > kWaitLimit) {
+      dead = true;
+      if (err) atomicExch(err, 1);
+      return;
+    }
+  }
+}
+// the CTAs that take part in op o
+__device__ __forceinline__ unsigned chain_ctas(const ChainParams& P, int o, int ncl) {
+  return (unsigned)(min(ncl, (P.op[o].rows + 127) >> 7) * kChainC);
+}
+__device__ __forceinline__ void chain_wait_done(const unsigned* done, unsigned want, bool& dead, int* err) {
+  if (dead) return;
+  const long long t0 = clock64();
+  for (;;) {
+    unsigned seen;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(done) : "memory");
+    if (seen >= want) return;
+    if (clock64() - t0 > kWaitLimit) {
+      dead = true;
+      if (err) atomicExch(err, 1);
+      return;
+    }
+  }
+}
+
+// a row of N floats in the receive buffer: its 16-byte pieces are rotated so that a warp's rows meet different banks
+template <int N>
+__device__ __forceinline__ int chain_piece(int row, int piece) {
+  return N == 32 ? piece ^ (row & 7) : piece ^ ((row >> 1) & 3);
+}
+
+// EPI_RESID_NORM for the 32 rows this CTA finalises, one rank; arithmetic and order as in resid_norm_tile.
+// Thread e holds row e >> 2 and batch columns 8 (e & 3) .. + 7; the residual row is fetched while the weights stream.
+struct ChainResid { float4 x0, x1; float gain, bias; };
+template <int N>
+__device__ __forceinline__ void chain_resid_load(const GemvParams& p, int row0, int e, ChainResid& h) {
+  const int bg = e & 3, grow = row0 + (e >> 2);
+  if (bg >= N / 8 || grow >= p.rows) return;
+  const float4* xr = reinterpret_cast<const float4*>(p.rn.x + (size_t)grow * N + 8 * bg);
+  h.x0 = xr[0]; h.x1 = xr[1];
+  h.bias = p.bias ? p.bias[grow] : 0.f;
+  h.gain = p.rn.gain[grow];
+}
+template <int N>
+__device__ __forceinline__ void chain_resid_tile(const GemvParams& p, const ChainResid& h, const float4* recv, int row0, int slot, int e, float* s_red) {
+  constexpr int BG = N / 8;
+  const int lane = e & 31, we = e >> 5, bg = e & 3, rl = e >> 2, grow = row0 + rl;
+  const bool valid = bg < BG && grow < p.rows;
+  float ssq[8], sxv[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ssq[i] = sxv[i] = 0.f;
+  if (valid) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int src = 0; src < kChainC; ++src) {
+      const float4 t0 = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, 2 * bg)], t1 = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, 2 * bg + 1)];
+      acc[0] += t0.x; acc[1] += t0.y; acc[2] += t0.z; acc[3] += t0.w;
+      acc[4] += t1.x; acc[5] += t1.y; acc[6] += t1.z; acc[7] += t1.w;
+    }
+    const float xv[8] = {h.x0.x + (acc[0] + h.bias), h.x0.y + (acc[1] + h.bias), h.x0.z + (acc[2] + h.bias), h.x0.w + (acc[3] + h.bias),
+                         h.x1.x + (acc[4] + h.bias), h.x1.y + (acc[5] + h.bias), h.x1.z + (acc[6] + h.bias), h.x1.w + (acc[7] + h.bias)};
+    float4* xr = reinterpret_cast<float4*>(p.rn.x + (size_t)grow * N + 8 * bg);
+    xr[0] = make_float4(xv[0], xv[1], xv[2], xv[3]);
+    xr[1] = make_float4(xv[4], xv[5], xv[6], xv[7]);
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.rn.xg) + (size_t)(grow >> 3) * (N * 8) + bg * 64 + (grow & 7);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o[8 * i] = __float2bfloat16_rn(xv[i] * h.gain);
+      ssq[i] = xv[i] * xv[i];
+      sxv[i] = xv[i];
+    }
+    if (p.rn.capture) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (8 * bg + i < p.B) p.rn.capture[(size_t)(8 * bg + i) * p.rows + grow] = xv[i];
+    }
+  }
+  auto fold = [&](float (&v)[8], float* out) {                 // over the tile's 32 rows, in a fixed order
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 4);
+      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 8);
+      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
+    }
+    if (lane < 4) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s_red[we * 32 + 8 * lane + i] = v[i];
+    }
+    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+    if (e < 32) out[(size_t)slot * 32 + e] = ((s_red[e] + s_red[32 + e]) + s_red[64 + e]) + s_red[96 + e];
+  };
+  fold(ssq, p.rn.ssq);
+  if (p.rn.sum) {
+    asm volatile("bar.sync 1, 128;\n" ::: "memory");           // s_red has been read
+    fold(sxv, p.rn.sum);
+  }
+}
+
+template <int N, bool X>
+__global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __grid_constant__ ChainParams P, int* err) {
+  constexpr int ST = kChainStages<N>;
+  constexpr int kXStage = N * 256;
+  constexpr int kStage = kWStage + kXStage;
+  constexpr uint32_t kTmemCols = 2 * N;                          // two accumulators
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
+  extern __shared__ __align__(1024) unsigned char smem[];        // ST stages, then recv[4][32][N] floats
+  __shared__ __align__(8) uint64_t full_bar[ST];                 // two arrivals: weights, activations
+  __shared__ __align__(8) uint64_t empty_bar[ST];
+  __shared__ __align__(8) uint64_t acc_full[2];
+  __shared__ __align__(8) uint64_t acc_empty[2];
+  __shared__ __align__(8) uint64_t recv_full;                    // the four parts of this CTA's rows have arrived
+  __shared__ __align__(8) uint64_t send_ok;                      // every CTA of the cluster has read its receive buffer
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ float s_inv_buf[64];
+  __shared__ float s_red[128];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c = (int)cluster_ctarank(), cid = (int)blockIdx.x / kChainC, ncl = (int)gridDim.x / kChainC;
+  if (tid == 0) {
+#pragma unroll
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(&full_bar[s], 2);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_full[0], 1); mbar_init(&acc_full[1], 1);
+    mbar_init(&acc_empty[0], 4); mbar_init(&acc_empty[1], 4);
+    mbar_init(&recv_full, 1);
+    mbar_init(&send_ok, kChainC);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base_slot)), "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+  bool dead = false;
+  pdl_launch_dependents();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");      // the peers' barriers are initialised: waited for before the first send
+
+  if (warp == 0) {
+    // ---------------- weights ----------------
+    if (lane == 0) {
+      uint64_t pol_w;
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(pol_w));
+      int it = 0;
+      for (int o = 0; o < P.n_ops; ++o) {
+        const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
+        const int ks0 = c * KS / kChainC, ks1 = (c + 1) * KS / kChainC;
+        const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(P.op[o].W);
+        for (int r = cid; r < nrbg; r += ncl)
+          for (int ks = ks0; ks < ks1; ++ks, ++it) {
+            const int s = it % ST, k = it / ST;
+            mbar_wait(&empty_bar[s], (k & 1) ^ 1, dead, err);
+            mbar_expect_tx(&full_bar[s], (uint32_t)kWStage);
+            bulk_g2s(smem + s * kStage, W + ((int64_t)r * KS + ks) * 16384, (uint32_t)kWStage, &full_bar[s], pol_w);
+          }
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  } else if (warp == 6) {
+    // ---------------- activations ----------------
+    pdl_wait();
+    if (lane == 0) {
+      uint64_t pol_x;
+      asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(pol_x));
+      int it = 0;
+      for (int o = 0; o < P.n_ops; ++o) {
+        const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
+        const int ks0 = c * KS / kChainC, ks1 = (c + 1) * KS / kChainC;
+        if (cid >= nrbg || ks0 >= ks1) continue;
+        if (o > 0) {
+          chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P, o - 1, ncl), dead, err);
+          asm volatile("fence.proxy.async;\n" ::: "memory");      // the bulk copies read what the epilogues stored
+        }
+        const __nv_bfloat16* xsrc = reinterpret_cast<const __nv_bfloat16*>(P.op[o].x);
+        for (int r = cid; r < nrbg; r += ncl)
+          for (int ks = ks0; ks < ks1; ++ks, ++it) {
+            const int s = it % ST, k = it / ST;
+            mbar_wait(&empty_bar[s], (k & 1) ^ 1, dead, err);
+            mbar_expect_tx(&full_bar[s], (uint32_t)kXStage);
+            bulk_g2s(smem + s * kStage + kWStage, xsrc + (int64_t)ks * (128 * N), (uint32_t)kXStage, &full_bar[s], pol_x);
+          }
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  } else if (warp == 1) {
+    // ---------------- MMA issue ----------------
+    int it = 0, seg = 0;
+    for (int o = 0; o < P.n_ops; ++o) {
+      const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
+      const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
+      if (n_steps == 0) continue;
+      for (int r = cid; r < nrbg; r += ncl, ++seg) {
+        const int buf = seg & 1;
+        mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, dead, err);
+        tc_fence_after();
+        for (int i = 0; i < n_steps; ++i, ++it) {
+          const int s = it % ST, k = it / ST;
+          mbar_wait(&full_bar[s], k & 1, dead, err);
+          tc_fence_after();
+          if (lane == 0) {
+            const uint32_t sa = smem_u32(smem + s * kStage);
+            const uint64_t adesc = smem_desc(sa, 2048, 128);
+            const uint64_t bdesc = smem_desc(sa + kWStage, N * 16, 128);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              tc_mma_f16(tmem_base + buf * N, adesc + (uint64_t)(j * (4096 >> 4)), bdesc + (uint64_t)(j * ((2 * N * 16) >> 4)), kIdesc,
+                         (i == 0 && j == 0) ? 0u : 1u);
+            tc_commit(&empty_bar[s]);
+            if (i == n_steps - 1) tc_commit(&acc_full[buf]);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  } else {
+    // ---------------- epilogue ----------------
+    pdl_wait();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    const int q = warp & 3, e = tid - 64;
+    const float4* recv = reinterpret_cast<const float4*>(smem + ST * kStage);
+    const uint32_t to = dsmem_addr(smem_u32(recv) + (uint32_t)((c * 32 + lane) * N * 4), (uint32_t)q);
+    const uint32_t to_bar = dsmem_addr(smem_u32(&recv_full), (uint32_t)q);
+    int seg = 0, g = 0;                        // accumulators drained, tiles exchanged
+    for (int o = 0; o < P.n_ops; ++o) {
+      const GemvParams& p = P.op[o];
+      const int KS = (p.K + 127) >> 7, nrbg = (p.rows + 127) >> 7;
+      const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
+      if (cid >= nrbg) continue;
+      const float* s_inv = p.inv.ssq ? s_inv_buf : nullptr;
+      if (o > 0) {
+        if (e == 0) chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P, o - 1, ncl), dead, err);
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+      }
+      compute_inv_scale(p.inv, s_inv_buf, e);
+      for (int r = cid; r < nrbg; r += ncl, ++g) {
+        const int row0 = r * 128 + c * 32;
+        // what the epilogue reads besides the accumulators, fetched while the weights stream
+        ChainResid h;
+        RowConst rc[2];
+        if (p.epi == EPI_RESID_NORM) {
+          chain_resid_load<N>(p, row0, e, h);
+        } else {
+          rc[0] = row_const(p, row0 + (lane & 15));
+          rc[1] = row_const(p, row0 + 16 + (lane & 15));
+        }
+        float v[N];
+        if (n_steps > 0) {
+          const int buf = seg & 1;
+          mbar_wait(&acc_full[buf], (seg >> 1) & 1, dead, err);
+          tc_fence_after();
+          tmem_load_row<N>(v, tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * N));
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[buf]);
+          ++seg;
+        } else {
+#pragma unroll
+          for (int i = 0; i < N; ++i) v[i] = 0.f;
+        }
+        if (e == 0) mbar_expect_tx(&recv_full, 128u * N * 4u);
+        if (g > 0) mbar_wait_cluster(&send_ok, (g - 1) & 1, dead, err);
+#pragma unroll
+        for (int i = 0; i < N / 4; ++i)
+          dsmem_store4_async(to + 16u * chain_piece<N>(lane, i), to_bar, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        mbar_wait_cluster(&recv_full, g & 1, dead, err);
+        if (p.epi == EPI_RESID_NORM) {
+          chain_resid_tile<N>(p, h, recv, row0, r * kChainC + c, e, s_red);
+        } else {
+          const int row16 = lane & 15, cg = e >> 4;
+          if (cg < N / 4) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              float v4[4] = {0.f, 0.f, 0.f, 0.f};
+              const int rl = 16 * j + row16;
+#pragma unroll
+              for (int src = 0; src < kChainC; ++src) {
+                const float4 t = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, cg)];
+                v4[0] += t.x; v4[1] += t.y; v4[2] += t.z; v4[3] += t.w;
+              }
+              row_epilogue<4, N, X>(p, v4, row0 + rl, 4 * cg, s_inv, rc[j]);
+            }
+          }
+        }
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");         // the receive buffer has been read
+        if (e < kChainC) mbar_arrive_remote(dsmem_addr(smem_u32(&send_ok), (uint32_t)e));
+      }
+      if (o + 1 < P.n_ops) {
+        // the barrier puts every thread's stores before thread 0's release, which covers them
+        asm volatile("fence.proxy.async;\n" ::: "memory");
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        if (e == 0) asm volatile("fence.acq_rel.gpu;\nred.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
+      }
+    }
+  }
+  if (dead) {                                  // copies may still be on their way into this shared memory
+    const long long t0 = clock64();
+    while (clock64() - t0 < kWaitLimit / 100) {}
+  }
+  tc_fence_before();
+  __syncwarp();
+  cluster_sync_all();                          // no peer sends into a CTA that has gone
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+  }
+  if (tid == 0) {                              // the last CTA out leaves the counters empty
+    unsigned* gone = P.done + kChainMax * kChainLine;
+    __threadfence();
+    if (atomicAdd(gone, 1u) == gridDim.x - 1u) {
+      for (int o = 0; o < kChainMax; ++o) P.done[o * kChainLine] = 0u;
+      *gone = 0u;
+    }
+  }
 }
 
 bool layered_epilogue(const GemvParams& p) {
@@ -1537,6 +1933,49 @@ int32_t launch_bf16(Ctx* ctx, const GemvParams& p, cudaStream_t stream) {
   if (p.cluster >= 1) return launch_cluster<Bp>(ctx, p, stream);
   LMB_REQUIRE(p.epi != EPI_RESID_NORM && p.epi != EPI_POST_NORM, "gemv: this epilogue needs a plan of gemv_plan_resid");
   LMB_CUDA(launch_k(layered_epilogue(p) ? gemv_tc_kernel<Bp, true> : gemv_tc_kernel<Bp, false>, dim3(p.grid), dim3(kTcThreads), stream_smem<Bp>(), stream, p, ctx->dev_err));
+  ctx->launches++;
+  return LMB200_OK;
+}
+
+template <int N>
+cudaLaunchConfig_t chain_config(cudaLaunchAttribute* attr, int clusters, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(clusters * kChainC));
+  cfg.blockDim = dim3(kChainThreads);
+  cfg.dynamicSmemBytes = chain_smem<N>();
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kChainC;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cfg;
+}
+
+template <int N>
+int chain_clusters() {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = chain_config<N>(attr, 1, 0);
+  cfg.numAttrs = 1;
+  int n = 0, m = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, gemv_chain_kernel<N, false>, &cfg) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&m, gemv_chain_kernel<N, true>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return std::min(n, m);
+}
+
+template <int N>
+int32_t launch_chain(Ctx* ctx, const ChainParams& P, int clusters, cudaStream_t stream) {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = chain_config<N>(attr, clusters, stream);
+  bool x = false;
+  for (int i = 0; i < P.n_ops; ++i) x = x || layered_epilogue(P.op[i]);
+  LMB_CUDA(cudaLaunchKernelEx(&cfg, x ? gemv_chain_kernel<N, true> : gemv_chain_kernel<N, false>, P, ctx->dev_err));
   ctx->launches++;
   return LMB200_OK;
 }
@@ -1632,6 +2071,38 @@ int gemv_plan_ctas(const GemvPlan& pl, int rows) {
   return pl.cluster >= 1 ? (int)ceil_div(rows, 128) * pl.cluster : pl.grid;
 }
 
+int gemv_chain_max_clusters(const Ctx* ctx, int B) {
+  (void)ctx;
+  const char* e = getenv("LMB200_GEMV_CHAIN");                  // 0: one launch per GEMV (A/B runs)
+  if ((e && atoi(e) == 0) || g_variant != GEMV_TCGEN05) return 0;
+  return Layout<__nv_bfloat16>::batch_pad(B) == 16 ? chain_clusters<16>() : chain_clusters<32>();
+}
+int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMax + 1) * kChainLine * 4; }
+
+int32_t GemvChain::add(const GemvParams& p) {
+  if (clusters == 0) return gemv_launch(ctx, LMB200_BF16, p, stream);
+  if (n == kChainMax) LMB_TRY(flush());
+  op[n++] = p;
+  return LMB200_OK;
+}
+int32_t GemvChain::flush() {
+  const int count = n;
+  n = 0;
+  if (count == 0) return LMB200_OK;
+  if (count == 1 && op[0].epi != EPI_RESID_NORM) return gemv_launch(ctx, LMB200_BF16, op[0], stream);
+  ChainParams P;
+  int most = 1;
+  for (int i = 0; i < count; ++i) {
+    LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1 && op[i].epi != EPI_POST_NORM, "gemv chain: op %d cannot run here", i);
+    P.op[i] = op[i];
+    most = std::max(most, (int)ceil_div(op[i].rows, 128));
+  }
+  P.n_ops = count;
+  P.done = done;
+  const int g = std::min(most, clusters);
+  return Layout<__nv_bfloat16>::batch_pad(op[0].B) == 16 ? launch_chain<16>(ctx, P, g, stream) : launch_chain<32>(ctx, P, g, stream);
+}
+
 // Raise the dynamic shared-memory limit of every instantiation once per device, outside any
 // stream capture.
 int32_t gemv_configure() {
@@ -1648,6 +2119,10 @@ int32_t gemv_configure() {
   LMB_CFG((gemv_cl_kernel<16, true>), cluster_smem<16>());
   LMB_CFG((gemv_cl_kernel<32, false>), cluster_smem<32>());
   LMB_CFG((gemv_cl_kernel<32, true>), cluster_smem<32>());
+  LMB_CFG((gemv_chain_kernel<16, false>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<16, true>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<32, false>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<32, true>), chain_smem<32>());
 #undef LMB_CFG
   return LMB200_OK;
 }

@@ -173,4 +173,23 @@ void gemv_prefetch_next(GemvParams& p, const Ctx* ctx, int dtype, const void* ne
 // dtype: LMB200_F32 or LMB200_BF16
 int32_t gemv_launch(Ctx* ctx, int dtype, GemvParams p, cudaStream_t stream);
 
+// A run of bf16 GEMVs, each reading what the one before it wrote, as one launch (gemv_chain_kernel).  `clusters` is
+// gemv_chain_max_clusters for the batch; 0 launches every GEMV by itself.  One rank only.
+constexpr int kChainMax = 4;                 // GEMVs per launch
+constexpr int kChainC = 4;                   // CTAs per cluster
+struct GemvChain {
+  Ctx* ctx = nullptr;
+  cudaStream_t stream = nullptr;
+  int clusters = 0;
+  unsigned* done = nullptr;                  // gemv_chain_scratch_bytes(), zero before the first launch
+  GemvParams op[kChainMax];
+  int n = 0;
+  int32_t add(const GemvParams& p);
+  int32_t flush();                           // before anything that reads the last GEMV's output
+  // ssq slots an EPI_RESID_NORM of these rows leaves
+  int slots(const GemvPlan& pl, int rows) const { return clusters ? (int)ceil_div(rows, 128) * kChainC : gemv_plan_ctas(pl, rows); }
+};
+int gemv_chain_max_clusters(const Ctx* ctx, int B);
+int64_t gemv_chain_scratch_bytes();
+
 }  // namespace lmb

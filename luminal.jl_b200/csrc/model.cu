@@ -1272,6 +1272,12 @@ GemvParams gemv_params(Session* S, const void* W, const WMap& m, const GemvPlan&
 
 namespace {
 
+GemvChain gemv_chain(Session* S, cudaStream_t st) {
+  GemvChain ch;
+  ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done;
+  return ch;
+}
+
 // Partial-sum exchange of the two row-parallel projections of a layer (index 2l: o_proj, 2l + 1:
 // down_proj).  With the peer regions mapped, the projection writes this rank's partial into its
 // region (buffers alternate, so a buffer is rewritten only after every peer has passed the next
@@ -1478,6 +1484,7 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
   const lmb200_model_config& c = M->cfg;
   const int dt = LMB200_BF16;
   const int B = S->B, hid = c.hidden, L = c.n_layers;
+  GemvChain chain = gemv_chain(S, st);
   LMB_TRY(embed_prep_launch(S, M->layers[0].attn_norm, st));
   int tiles = (int)ceil_div(hid, S->embed_rows_per_cta);        // slots of S->ssq the last producer wrote
   auto inv_scale = [&]() { InvScale iv; iv.ssq = S->ssq; iv.tiles = tiles; iv.n = hid; iv.eps = c.rms_eps; return iv; };
@@ -1490,7 +1497,8 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
       p.q_out = S->qbuf; p.q_pitch = S->q_pitch;
       p.kv_layer = kv_layer; p.kv_batch_stride = S->kv_batch_stride; p.kv_head_stride = S->kv_head_stride;
       p.inv_freq = M->inv_freq; p.pos = S->pos; p.pos_uniform = S->ragged ? 0 : 1; p.Hl = M->Hl; p.KVl = M->KVl; p.D = M->D;
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
+      LMB_TRY(chain.add(p));
+      LMB_TRY(chain.flush());
     }
     {
       AttnParams a;
@@ -1509,14 +1517,14 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
       p.rn.x = S->xT; p.rn.gain = W.ffn_norm; p.rn.xg = S->xn; p.rn.ssq = S->ssq;
       p.push = peer_push(S, 2 * l);
       gemv_prefetch_next(p, ctx, dt, W.wgu, M->m_gu.rows, M->m_gu.K, S->p_gu);
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
-      tiles = gemv_plan_ctas(S->p_o, M->m_o.rows);
+      LMB_TRY(chain.add(p));
+      tiles = chain.slots(S->p_o, M->m_o.rows);
     }
     {  // gate/up (norm scale on the accumulators) + SiLU gate
       GemvParams p = gemv_params(S, W.wgu, M->m_gu, S->p_gu, S->xn);
       p.epi = EPI_SILU_GATE; p.inv = inv_scale(); p.act = S->act; p.n_act = M->inter_l;
       gemv_prefetch_next(p, ctx, dt, W.wdown, M->m_down.rows, M->m_down.K, S->p_down);
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
+      LMB_TRY(chain.add(p));
     }
     {  // down_proj + all-reduce + residual add + what the next norm (next layer's, or the final one) needs
       GemvParams p = gemv_params(S, W.wdown, M->m_down, S->p_down, S->act);
@@ -1526,10 +1534,11 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
       p.push = peer_push(S, 2 * l + 1);
       if (l + 1 < L) gemv_prefetch_next(p, ctx, dt, M->layers[l + 1].wqkv, M->m_qkv.rows, M->m_qkv.K, S->p_qkv);
       else if (with_head) gemv_prefetch_next(p, ctx, dt, M->lm_head, M->m_head.rows, M->m_head.K, S->p_head);
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
-      tiles = gemv_plan_ctas(S->p_down, M->m_down.rows);
+      LMB_TRY(chain.add(p));
+      tiles = chain.slots(S->p_down, M->m_down.rows);
     }
   }
+  if (S->head_sliced || !with_head) LMB_TRY(chain.flush());
   if (with_head && S->head_sliced) {
     // this rank's rows of the head, its best (logit, id) per sequence, the exchange; the full logits only on request
     {
@@ -1556,7 +1565,8 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
   } else if (with_head) {
     GemvParams p = gemv_params(S, M->lm_head, M->m_head, S->p_head, S->xn);
     p.epi = EPI_STORE_F32; p.inv = inv_scale(); p.out = S->logits; p.out_pitch = S->logits_pitch;
-    LMB_TRY(gemv_launch(ctx, dt, p, st));
+    LMB_TRY(chain.add(p));
+    LMB_TRY(chain.flush());
     LMB_CUDA(launch_k(argmax_step_kernel, dim3(B), dim3(kArgmaxThreads), 0, st, (const float*)S->logits, S->logits_pitch, c.vocab,
                       S->tokens, S->tok_hist, (const int*)S->step_ctr, B, S->stop));
     ctx->launches++;
@@ -1972,6 +1982,8 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
       else fused = false;
     }
     S->fused = fused;
+    // ssq has 256 slots, of which a chained projection fills 4 per row group
+    if (fused && c.tp_size == 1 && ceil_div(c.hidden, 128) * kChainC <= 256 && !whisper) S->chain_clusters = gemv_chain_max_clusters(ctx, batch);
     S->embed_rows_per_cta = 32 * (int)ceil_div(c.hidden, 32 * 256);
     // The head is replicated; under tensor parallelism every rank multiplies only its share of the rows and the ranks
     // exchange their best (logit, id) pairs (LMB200_TP_HEAD=replicated keeps every rank on the whole head, A/B runs).
@@ -2035,6 +2047,7 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
   if (S->fused) {
     alloc((void**)&S->xT, (int64_t)round_up(c.hidden, 128) * S->Bp * 4);
     alloc((void**)&S->ssq, (int64_t)256 * 32 * 4);
+    if (S->chain_clusters) alloc((void**)&S->chain_done, gemv_chain_scratch_bytes());
     if (whisper) alloc((void**)&S->sum_slots, (int64_t)256 * 32 * 4);
   }
   if (S->head_sliced) alloc((void**)&S->logits_slice, (int64_t)batch * S->head_pitch * 4);
@@ -2061,7 +2074,7 @@ extern "C" int32_t lmb200_session_destroy(lmb200_session h) {
   cudaFree(S->cross_kv);
   cudaFree(S->kv); cudaFree(S->x); cudaFree(S->delta); cudaFree(S->logits); cudaFree(S->xn); cudaFree(S->qbuf);
   cudaFree(S->attn_out); cudaFree(S->act); cudaFree(S->tokens); cudaFree(S->pos); cudaFree(S->limit); cudaFree(S->step_ctr); cudaFree(S->ragged_logits);
-  cudaFree(S->tok_hist); cudaFree(S->prompt); cudaFree(S->gemv_partials); cudaFree(S->gemv_counters);
+  cudaFree(S->tok_hist); cudaFree(S->prompt); cudaFree(S->gemv_partials); cudaFree(S->gemv_counters); cudaFree(S->chain_done);
   cudaFree(S->part_o); cudaFree(S->part_ml); cudaFree(S->attn_counters); cudaFree(S->prefill_buf); cudaFree(S->capture);
   cudaFree(S->xT); cudaFree(S->ssq); cudaFree(S->sum_slots); cudaFree(S->logits_slice); cudaFree(S->stop);
   S->magic = 0;

@@ -162,6 +162,8 @@ struct Session {
   // scratch
   float* gemv_partials = nullptr;
   unsigned* gemv_counters = nullptr;
+  unsigned* chain_done = nullptr;      // GemvChain::done
+  int chain_clusters = 0;              // > 0: the fused step runs its GEMVs in chains
   float* part_o = nullptr;
   float* part_ml = nullptr;
   unsigned* attn_counters = nullptr;   // [B*KVl], zero between launches
