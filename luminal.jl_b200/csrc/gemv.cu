@@ -1627,6 +1627,116 @@ __device__ __forceinline__ void chain_resid_tile(const GemvParams& p, const Chai
   }
 }
 
+// EPI_POST_NORM for the 32 rows this CTA finalises; protocol, arithmetic and order as in post_norm_tile.  The op's CTAs (n of
+// them, one tile each) wait for one another's sums of squares; rows and columns of a thread as in chain_resid_tile.
+template <int N>
+__device__ __forceinline__ void chain_post_load(const GemvParams& p, int row0, int e, ChainResid& h) {
+  const int bg = e & 3, grow = row0 + (e >> 2);
+  if (bg >= N / 8 || grow >= p.rows) return;
+  const float4* xr = reinterpret_cast<const float4*>(p.pn.x + (size_t)grow * N + 8 * bg);
+  h.x0 = xr[0]; h.x1 = xr[1];
+  h.bias = p.pn.w[grow];
+  h.gain = p.pn.gain ? p.pn.gain[grow] : 1.0f;
+}
+template <int N>
+__device__ __forceinline__ void chain_post_tile(const GemvParams& p, const ChainResid& h, const float4* recv, int row0, int slot, int n, int e,
+                                                float* s_red, float* s_scale, const float* s_inv, int* err) {
+  constexpr int BG = N / 8;
+  const int lane = e & 31, we = e >> 5, bg = e & 3, rl = e >> 2, grow = row0 + rl;
+  const bool valid = bg < BG && grow < p.rows;
+  float acc[8], ss[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = ss[i] = 0.f;
+  if (valid) {
+#pragma unroll
+    for (int src = 0; src < kChainC; ++src) {
+      const float4 t0 = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, 2 * bg)], t1 = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, 2 * bg + 1)];
+      acc[0] += t0.x; acc[1] += t0.y; acc[2] += t0.z; acc[3] += t0.w;
+      acc[4] += t1.x; acc[5] += t1.y; acc[6] += t1.z; acc[7] += t1.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (s_inv) acc[i] *= s_inv[8 * bg + i];
+      ss[i] = acc[i] * acc[i];
+    }
+  }
+  auto publish = [&](float* slots, bool flagged) {             // this tile's sums of ss over the rows
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 4);
+      ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 8);
+      ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 16);
+    }
+    if (lane < 4) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s_red[we * 32 + 8 * lane + i] = ss[i];
+    }
+    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+    if (e < 32) {
+      const float t = ((s_red[e] + s_red[32 + e]) + s_red[64 + e]) + s_red[96 + e];
+      unsigned u = __float_as_uint(t);
+      if (flagged && u == kSlotEmpty) u = 0x7FC00000u;
+      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;\n" ::"l"(slots + (size_t)slot * 32 + e), "r"(u) : "memory");
+    }
+  };
+  publish(p.pn.slots, true);
+  // the set of the next output norm: its last readers have counted themselves into done[] before this op began
+  if (p.pn.clear && e < 32)
+    for (int i = slot * 32 + e; i < kPushMaxCtas * 32; i += n * 32) p.pn.clear[i] = __uint_as_float(kSlotEmpty);
+  {                                                            // four lanes per sequence, the same sums in every CTA
+    const int b = e >> 2, part = e & 3;
+    float s = 0.f;
+    const long long t0 = clock64();
+    bool late = false;
+    for (int first = part; first < n; first += 64) {           // sixteen slots in flight
+      unsigned u[16];
+      bool wait = true;
+      while (wait) {
+        wait = false;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          u[i] = 0u;
+          if (first + 4 * i < n) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(u[i]) : "l"(p.pn.slots + (first + 4 * i) * 32 + b) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) wait = wait || u[i] == kSlotEmpty;
+        if (wait && (late || clock64() - t0 > kWaitLimit)) {
+          if (!late && err) atomicExch(err, 1);
+          late = true;
+          wait = false;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) s += __uint_as_float(u[i]);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (part == 0) s_scale[b] = 1.0f / sqrtf(s / (float)p.rows + p.pn.eps);
+  }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ss[i] = 0.f;
+  if (valid) {
+    float xv[8] = {h.x0.x, h.x0.y, h.x0.z, h.x0.w, h.x1.x, h.x1.y, h.x1.z, h.x1.w};
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.pn.xg) + (size_t)(grow >> 3) * (N * 8) + bg * 64 + (grow & 7);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      xv[i] += acc[i] * s_scale[8 * bg + i] * h.bias;
+      o[8 * i] = __float2bfloat16_rn(xv[i] * h.gain);
+      ss[i] = xv[i] * xv[i];
+    }
+    float4* xr = reinterpret_cast<float4*>(p.pn.x + (size_t)grow * N + 8 * bg);
+    xr[0] = make_float4(xv[0], xv[1], xv[2], xv[3]);
+    xr[1] = make_float4(xv[4], xv[5], xv[6], xv[7]);
+    if (p.pn.capture) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (8 * bg + i < p.B) p.pn.capture[(size_t)(8 * bg + i) * p.rows + grow] = xv[i];
+    }
+  }
+  if (p.pn.ssq) publish(p.pn.ssq, false);
+}
+
 template <int N, bool X>
 __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __grid_constant__ ChainParams P, int* err) {
   constexpr int ST = kChainStages<N>;
@@ -1644,6 +1754,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
   __shared__ uint32_t tmem_base_slot;
   __shared__ float s_inv_buf[64];
   __shared__ float s_red[128];
+  __shared__ float s_scale[X ? 32 : 1];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c = (int)cluster_ctarank(), cid = (int)blockIdx.x / kChainC, ncl = (int)gridDim.x / kChainC;
@@ -1778,6 +1889,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
         RowConst rc[2];
         if (p.epi == EPI_RESID_NORM) {
           chain_resid_load<N>(p, row0, e, h);
+        } else if (X && p.epi == EPI_POST_NORM) {
+          chain_post_load<N>(p, row0, e, h);
         } else {
           rc[0] = row_const(p, row0 + (lane & 15));
           rc[1] = row_const(p, row0 + 16 + (lane & 15));
@@ -1804,6 +1917,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
         mbar_wait_cluster(&recv_full, g & 1, dead, err);
         if (p.epi == EPI_RESID_NORM) {
           chain_resid_tile<N>(p, h, recv, row0, r * kChainC + c, e, s_red);
+        } else if (X && p.epi == EPI_POST_NORM) {
+          chain_post_tile<N>(p, h, recv, row0, r * kChainC + c, nrbg * kChainC, e, s_red, s_scale, s_inv, err);
         } else {
           const int row16 = lane & 15, cg = e >> 4;
           if (cg < N / 4) {
@@ -2081,6 +2196,12 @@ int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMax + 1) * kChainLin
 
 int32_t GemvChain::add(const GemvParams& p) {
   if (clusters == 0) return gemv_launch(ctx, LMB200_BF16, p, stream);
+  // Every tile costs an exchange inside the cluster, about 2.4 us.  A GEMV of several tiles per cluster whose tiles stream for less than
+  // that (a unit is 0.57 us) is better off alone: 51865 x 512 takes 12 us by itself and 31 us here.
+  if (ceil_div(p.rows, 128) > clusters && p.K <= 3 * 128 * kChainC) {
+    LMB_TRY(flush());
+    return gemv_launch(ctx, LMB200_BF16, p, stream);
+  }
   if (n == kChainMax) LMB_TRY(flush());
   op[n++] = p;
   return LMB200_OK;
@@ -2089,11 +2210,13 @@ int32_t GemvChain::flush() {
   const int count = n;
   n = 0;
   if (count == 0) return LMB200_OK;
-  if (count == 1 && op[0].epi != EPI_RESID_NORM) return gemv_launch(ctx, LMB200_BF16, op[0], stream);
+  if (count == 1 && op[0].epi != EPI_RESID_NORM && op[0].epi != EPI_POST_NORM) return gemv_launch(ctx, LMB200_BF16, op[0], stream);
   ChainParams P;
   int most = 1;
   for (int i = 0; i < count; ++i) {
-    LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1 && op[i].epi != EPI_POST_NORM, "gemv chain: op %d cannot run here", i);
+    LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1, "gemv chain: op %d cannot run here", i);
+    LMB_REQUIRE(op[i].epi != EPI_POST_NORM || ceil_div(op[i].rows, 128) <= std::min(clusters, kPushMaxCtas / kChainC),
+                "gemv chain: %d rows are more than one wave", op[i].rows);
     P.op[i] = op[i];
     most = std::max(most, (int)ceil_div(op[i].rows, 128));
   }

@@ -175,7 +175,7 @@ int32_t gemv_launch(Ctx* ctx, int dtype, GemvParams p, cudaStream_t stream);
 
 // A run of bf16 GEMVs, each reading what the one before it wrote, as one launch (gemv_chain_kernel).  `clusters` is
 // gemv_chain_max_clusters for the batch; 0 launches every GEMV by itself.  One rank only.
-constexpr int kChainMax = 4;                 // GEMVs per launch
+constexpr int kChainMax = 8;                 // GEMVs per launch
 constexpr int kChainC = 4;                   // CTAs per cluster
 struct GemvChain {
   Ctx* ctx = nullptr;

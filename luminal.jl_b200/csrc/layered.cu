@@ -1209,9 +1209,10 @@ int32_t fused_post_step(Session* S, cudaStream_t st, bool with_head) {
   auto slots = [&](int i) { return Z.post_slots + (int64_t)(n_post % 2 && i == n_post - 1 ? 2 : i & 1) * kPushMaxCtas * 32; };
   // the matrix that follows: its weights are drawn into L2 while this one drains
   struct Next { const void* W = nullptr; const WMap* m = nullptr; const GemvPlan* pl = nullptr; };
+  GemvChain chain = gemv_chain(S, st);                       // the GEMVs from one mixer to the next
   auto launch = [&](GemvParams& p, const Next& nx) -> int32_t {
     if (nx.W) gemv_prefetch_next(p, ctx, dt, nx.W, nx.m->rows, nx.m->K, *nx.pl);
-    return gemv_launch(ctx, dt, p, st);
+    return chain.add(p);
   };
   auto head_next = [&]() { Next n; if (with_head) { n.W = M->lm_head; n.m = &M->m_head; n.pl = &S->p_head; } return n; };
   auto after = [&](int l) { Next n; if (l + 1 == L) return head_next(); n.W = M->lw[l + 1].w_in; n.m = &M->specs[l + 1].m_in; n.pl = &Z.p_in[l + 1]; return n; };
@@ -1225,7 +1226,7 @@ int32_t fused_post_step(Session* S, cudaStream_t st, bool with_head) {
     ++at_post;
     if (layer_end && S->capture_on) p.pn.capture = S->capture + (int64_t)l * B * hid;
     if (layer_end && l + 1 == L) { p.pn.gain = M->final_norm; p.pn.ssq = S->ssq; }
-    tiles = gemv_plan_ctas(pl, m.rows);
+    tiles = chain.slots(pl, m.rows);
     return launch(p, nx);
   };
   LMB_TRY(embed_prep_launch(S, nullptr, st, M->embed_scale));
@@ -1242,6 +1243,12 @@ int32_t fused_post_step(Session* S, cudaStream_t st, bool with_head) {
       LMB_TRY(launch(p, delta ? lr : out));
     }
     InvScale iv;
+    if (delta) {
+      GemvParams p = gemv_params(S, w.w_lr, s.m_lr, Z.p_lr[l], Z.lr_in);
+      p.epi = EPI_STORE_F32; p.out = Z.lr; p.out_pitch = s.m_lr.rows;
+      LMB_TRY(launch(p, out));
+    }
+    LMB_TRY(chain.flush());
     if (is_attention(s)) {
       WindowView v = window_view(S, l);
       v.T = B; v.seq = Z.iota; v.pos = S->pos;
@@ -1257,9 +1264,6 @@ int32_t fused_post_step(Session* S, cudaStream_t st, bool with_head) {
       }
       LMB_TRY(window_attend(ctx, dt, v, in, Z.win[l], Z.attn_part, Z.win_cnt, S->act, 0, S->Bp, st));
     } else if (delta) {
-      GemvParams p = gemv_params(S, w.w_lr, s.m_lr, Z.p_lr[l], Z.lr_in);
-      p.epi = EPI_STORE_F32; p.out = Z.lr; p.out_pitch = s.m_lr.rows;
-      LMB_TRY(launch(p, out));
       DeltaView v = delta_view(S, l);
       v.start = Z.iota; v.len = Z.ones; v.pos0 = S->pos; v.total = B; v.raw = 1;
       v.q = Z.proj + s.row0[D_Q]; v.k = Z.proj + s.row0[D_K]; v.v = Z.proj + s.row0[D_V];
@@ -1299,9 +1303,9 @@ int32_t fused_post_step(Session* S, cudaStream_t st, bool with_head) {
     GemvParams p = gemv_params(S, M->lm_head, M->m_head, S->p_head, S->xn);
     p.epi = EPI_STORE_F32; p.out = S->logits; p.out_pitch = S->logits_pitch; p.softcap = M->softcap;
     p.inv.ssq = S->ssq; p.inv.tiles = tiles; p.inv.n = hid; p.inv.eps = M->cfg.rms_eps;
-    LMB_TRY(gemv_launch(ctx, dt, p, st));
+    LMB_TRY(chain.add(p));
   }
-  return LMB200_OK;
+  return chain.flush();
 }
 
 // bf16, one token per sequence
@@ -1310,6 +1314,7 @@ int32_t fused_step(Session* S, cudaStream_t st, bool with_head) {
   Ctx* ctx = M->ctx;
   LayeredScratch& Z = *S->lay;
   const int B = S->B, hid = M->cfg.hidden, L = M->cfg.n_layers, dt = LMB200_BF16;
+  GemvChain chain = gemv_chain(S, st);
   LMB_TRY(embed_prep_launch(S, M->lw[0].norm, st));
   int tiles = (int)ceil_div(hid, S->embed_rows_per_cta);
   auto inv_scale = [&]() { InvScale iv; iv.ssq = S->ssq; iv.tiles = tiles; iv.n = hid; iv.eps = M->cfg.rms_eps; return iv; };
@@ -1322,7 +1327,8 @@ int32_t fused_step(Session* S, cudaStream_t st, bool with_head) {
       p.out = Z.proj; p.out_pitch = s.n_store; p.act_row0 = s.n_store; p.act = S->act; p.act_col0 = s.cat0; p.n_act = s.c.ff;
       if (is_latent(s)) gemv_prefetch_next(p, ctx, dt, w.w_uq, s.m_uq.rows, s.m_uq.K, Z.p_uq[l]);
       else gemv_prefetch_next(p, ctx, dt, w.w_out, s.m_out.rows, s.m_out.K, Z.p_out[l]);
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
+      LMB_TRY(chain.add(p));
+      LMB_TRY(chain.flush());
     }
     if (is_latent(s)) {
       const bool own = s.c.kv_from < 0;
@@ -1354,16 +1360,16 @@ int32_t fused_step(Session* S, cudaStream_t st, bool with_head) {
       p.rn.capture = S->capture_on ? S->capture + (int64_t)l * B * hid : nullptr;
       if (l + 1 < L) gemv_prefetch_next(p, ctx, dt, M->lw[l + 1].w_in, M->specs[l + 1].m_in.rows, M->specs[l + 1].m_in.K, Z.p_in[l + 1]);
       else if (with_head) gemv_prefetch_next(p, ctx, dt, M->lm_head, M->m_head.rows, M->m_head.K, S->p_head);
-      LMB_TRY(gemv_launch(ctx, dt, p, st));
-      tiles = gemv_plan_ctas(Z.p_out[l], s.m_out.rows);
+      LMB_TRY(chain.add(p));
+      tiles = chain.slots(Z.p_out[l], s.m_out.rows);
     }
   }
   if (with_head) {
     GemvParams p = gemv_params(S, M->lm_head, M->m_head, S->p_head, S->xn);
     p.epi = EPI_STORE_F32; p.inv = inv_scale(); p.out = S->logits; p.out_pitch = S->logits_pitch; p.softcap = M->softcap;
-    LMB_TRY(gemv_launch(ctx, dt, p, st));
+    LMB_TRY(chain.add(p));
   }
-  return LMB200_OK;
+  return chain.flush();
 }
 
 RowsRun decode_run(const Session* S) {
@@ -1465,6 +1471,9 @@ int32_t layered_session_create(Model* M, int batch, int max_ctx, lmb200_session*
     }
     S->p_head = take(gemv_plan(ctx, c.dtype, batch, M->m_head.rows, M->m_head.K));
     S->embed_rows_per_cta = 32 * (int)ceil_div(c.hidden, 32 * 256);
+    // A chained projection fills 4 of the 256 slots per row group, and an output norm needs every row group resident at once.
+    if (const int n = gemv_chain_max_clusters(ctx, batch); ceil_div(c.hidden, 128) <= std::min(post_norm(M) ? n : 64, 64)) S->chain_clusters = n;
+    if (S->chain_clusters) alloc((void**)&S->chain_done, gemv_chain_scratch_bytes());
     auto x_bytes = [&](int64_t K) { return Layout<__nv_bfloat16>::x_elems((int)K, S->Bp) * 2; };
     alloc(&S->xn, x_bytes(c.hidden));
     alloc(&S->act, x_bytes(max_over(M, [](const LayerSpec& s) { return s.m_out.K; })));

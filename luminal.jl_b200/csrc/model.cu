@@ -1270,13 +1270,13 @@ GemvParams gemv_params(Session* S, const void* W, const WMap& m, const GemvPlan&
   return p;
 }
 
-namespace {
-
 GemvChain gemv_chain(Session* S, cudaStream_t st) {
   GemvChain ch;
   ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done;
   return ch;
 }
+
+namespace {
 
 // Partial-sum exchange of the two row-parallel projections of a layer (index 2l: o_proj, 2l + 1:
 // down_proj).  With the peer regions mapped, the projection writes this rank's partial into its

@@ -268,6 +268,7 @@ int64_t tiled_elems(const WMap& m, int dtype);
 void finish_map(WMap& m);
 int32_t dmalloc(void** p, int64_t bytes, bool zero, cudaStream_t st);
 int32_t push_positions(Session* S);
+GemvChain gemv_chain(Session* S, cudaStream_t st);
 int32_t embed_prep_launch(Session* S, const float* gain, cudaStream_t st, float scale = 1.0f);
 GemvParams gemv_params(Session* S, const void* W, const WMap& m, const GemvPlan& pl, const void* x);
 int32_t argmax_launch(Session* S, cudaStream_t st);       // greedy tokens of S->logits into S->tokens
