@@ -533,6 +533,12 @@ __device__ __forceinline__ RowConst row_const(const GemvParams& p, int row) {
   return rc;
 }
 
+// EPI_GELU_TOKEN: the entry of sequence b's token (two dependent loads from anywhere in a table of hundreds of MB)
+__device__ __forceinline__ float token_factor(const GemvParams& p, int b, int row) {
+  const int tok = p.tokens[b];
+  return tok >= 0 && tok < p.token_rows ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.token_table)[(int64_t)tok * p.token_pitch + row]) : 0.f;
+}
+
 // Epilogue of one accumulator row held by one thread (v[b], b < N).  Rows g and g+8 of a 16-row
 // block -- the pairs the fused epilogues combine -- are 8 lanes apart in the same warp.
 // The thread holds batch columns b0 .. b0+NV-1 of the row (the whole row when NV == BP); BP is the
@@ -540,7 +546,8 @@ __device__ __forceinline__ RowConst row_const(const GemvParams& p, int row) {
 // X: the epilogues of decoders described layer by layer (softcap, EPI_STORE_RELU2) are compiled in.  They have instantiations of their
 // own: the other models' kernels carry no code of them.
 template <int NV, int BP, bool X>
-__device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV], int row, int b0, const float* s_inv, const RowConst& rc) {
+__device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV], int row, int b0, const float* s_inv, const RowConst& rc,
+                                             const float* factor = nullptr) {
   typedef Layout<__nv_bfloat16> LY;
   constexpr int N = NV;
   const int rb = row >> 4, rr = row & 15, g = rr & 7, hi = rr >> 3;
@@ -586,12 +593,10 @@ __device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV]
   if (X && p.epi == EPI_GELU_TOKEN) {
     if (row < p.rows) {
       __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(p.act);
-      const __nv_bfloat16* table = reinterpret_cast<const __nv_bfloat16*>(p.token_table);
 #pragma unroll
       for (int b = 0; b < N; ++b) {
         if (b0 + b >= p.B) continue;
-        const int tok = p.tokens[b0 + b];
-        const float e = tok >= 0 && tok < p.token_rows ? __bfloat162float(table[(int64_t)tok * p.token_pitch + row]) : 0.f;
+        const float e = factor ? factor[b] : token_factor(p, b0 + b, row);
         act[LY::x_offset(b0 + b, row, BP)] = __float2bfloat16_rn(gelu_ref(v[b]) * e);
       }
     }
@@ -1887,6 +1892,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
         // what the epilogue reads besides the accumulators, fetched while the weights stream
         ChainResid h;
         RowConst rc[2];
+        float factor[2][4];
         if (p.epi == EPI_RESID_NORM) {
           chain_resid_load<N>(p, row0, e, h);
         } else if (X && p.epi == EPI_POST_NORM) {
@@ -1894,6 +1900,13 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
         } else {
           rc[0] = row_const(p, row0 + (lane & 15));
           rc[1] = row_const(p, row0 + 16 + (lane & 15));
+          if (X && p.epi == EPI_GELU_TOKEN) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int b = 4 * (e >> 4) + (i & 3), row = row0 + 16 * (i >> 2) + (lane & 15);
+              factor[i >> 2][i & 3] = b < p.B && row < p.rows ? token_factor(p, b, row) : 0.f;
+            }
+          }
         }
         float v[N];
         if (n_steps > 0) {
@@ -1931,7 +1944,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
                 const float4 t = recv[(src * 32 + rl) * (N / 4) + chain_piece<N>(rl, cg)];
                 v4[0] += t.x; v4[1] += t.y; v4[2] += t.z; v4[3] += t.w;
               }
-              row_epilogue<4, N, X>(p, v4, row0 + rl, 4 * cg, s_inv, rc[j]);
+              row_epilogue<4, N, X>(p, v4, row0 + rl, 4 * cg, s_inv, rc[j], factor[j]);
             }
           }
         }
