@@ -5,10 +5,15 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace lmb {
 namespace {
 
+// A traced graph is a chain of hundreds of these, most of a microsecond's work, so what counts is the time from one to the next:
+// all are launched programmatically (each waits for its predecessor before it touches memory), and index arithmetic is 32-bit
+// (I = uint32_t) wherever the element counts allow: a 64-bit division is a subroutine of about a hundred instructions.
+// The small Llama's 32-token graph (404 kernels): 1522 -> 1343 us a call.
 constexpr int kMaxRank = 8;
 constexpr float kInvLn2 = 1.4426950408889634f;
 constexpr float kHalfPi = 1.5707963267948966f;
@@ -40,12 +45,16 @@ __device__ __forceinline__ float apply_op(int op, float a, float b, float c) {
   return 0.f;
 }
 
+template <typename I>
 __global__ void ew_kernel(int op, float* out, const float* a, const float* b, const float* c, Idx ix, int64_t total) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = o, oa = 0, ob = 0, oc = 0;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (I o = blockIdx.x * (I)blockDim.x + threadIdx.x; o < (I)total; o += (I)gridDim.x * blockDim.x) {
+    I rem = o;
+    int64_t oa = 0, ob = 0, oc = 0;
     for (int k = ix.rank - 1; k >= 0; --k) {
-      const int64_t i = rem % ix.out_d[k];
-      rem /= ix.out_d[k];
+      const I d = (I)ix.out_d[k], nx = rem / d, i = rem - nx * d;
+      rem = nx;
       oa += i * ix.sa[k]; ob += i * ix.sb[k]; oc += i * ix.sc[k];
     }
     out[o] = apply_op(op, a ? a[oa] : 0.f, b ? b[ob] : 0.f, c ? c[oc] : 0.f);
@@ -67,15 +76,18 @@ struct FusedProgram {
   int op[kFusedMaxInstr];
   float arg[kFusedMaxInstr];                  // PUSH_IN: input index; PUSH_CONST: the value
 };
+template <typename I>
 __global__ void fused_ew_kernel(float* out, const FusedProgram pg, int64_t total) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (I o = blockIdx.x * (I)blockDim.x + threadIdx.x; o < (I)total; o += (I)gridDim.x * blockDim.x) {
     int64_t off[kFusedMaxInputs];
 #pragma unroll
     for (int i = 0; i < kFusedMaxInputs; ++i) off[i] = 0;
-    int64_t rem = o;
+    I rem = o;
     for (int k = pg.rank - 1; k >= 0; --k) {
-      const int64_t idx = rem % pg.out_d[k];
-      rem /= pg.out_d[k];
+      const I d = (I)pg.out_d[k], nx = rem / d, idx = rem - nx * d;
+      rem = nx;
 #pragma unroll
       for (int i = 0; i < kFusedMaxInputs; ++i)
         if (i < pg.n_in) off[i] += idx * pg.st[i][k];
@@ -129,12 +141,16 @@ struct Gather {
   int64_t st[kMaxRank];
   int64_t offset;
 };
+template <typename I>
 __global__ void strided_copy_kernel(float* out, const float* in, Gather gt, int64_t total) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = o, src = gt.offset;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (I o = blockIdx.x * (I)blockDim.x + threadIdx.x; o < (I)total; o += (I)gridDim.x * blockDim.x) {
+    I rem = o;
+    int64_t src = gt.offset;
     for (int k = gt.rank - 1; k >= 0; --k) {
-      const int64_t i = rem % gt.out_d[k];
-      rem /= gt.out_d[k];
+      const I d = (I)gt.out_d[k], nx = rem / d, i = rem - nx * d;
+      rem = nx;
       src += i * gt.st[k];
     }
     out[o] = in[src];
@@ -145,13 +161,18 @@ struct Pad {
   int rank;
   int64_t out_d[kMaxRank], in_d[kMaxRank], left[kMaxRank];
 };
+template <typename I>
 __global__ void pad_kernel(float* out, const float* in, Pad pd, int64_t total) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rem = o, src = 0, mul = 1;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (I o = blockIdx.x * (I)blockDim.x + threadIdx.x; o < (I)total; o += (I)gridDim.x * blockDim.x) {
+    I rem = o;
+    int64_t src = 0, mul = 1;
     bool inside = true;
     for (int k = pd.rank - 1; k >= 0; --k) {
-      const int64_t i = rem % pd.out_d[k] - pd.left[k];
-      rem /= pd.out_d[k];
+      const I d = (I)pd.out_d[k], nx = rem / d;
+      const int64_t i = (int64_t)(rem - nx * d) - pd.left[k];
+      rem = nx;
       if (i < 0 || i >= pd.in_d[k]) inside = false;
       src += i * mul;
       mul *= pd.in_d[k];
@@ -165,30 +186,43 @@ struct Reshape {
   int in_rank, out_rank;
   int64_t in_d[kMaxRank], out_d[kMaxRank];
 };
+template <typename I>
 __global__ void reshape_cm_kernel(float* out, const float* in, Reshape rs, int64_t total) {
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (I o = blockIdx.x * (I)blockDim.x + threadIdx.x; o < (I)total; o += (I)gridDim.x * blockDim.x) {
     // row-major index of out -> multi-index -> column-major linear index
-    int64_t rem = o, lin = 0;
-    int64_t idx[kMaxRank];
-    for (int k = rs.out_rank - 1; k >= 0; --k) { idx[k] = rem % rs.out_d[k]; rem /= rs.out_d[k]; }
-    int64_t mul = 1;
-    for (int k = 0; k < rs.out_rank; ++k) { lin += idx[k] * mul; mul *= rs.out_d[k]; }
+    I rem = o, lin = 0;
+    I idx[kMaxRank];
+    for (int k = rs.out_rank - 1; k >= 0; --k) { const I d = (I)rs.out_d[k], nx = rem / d; idx[k] = rem - nx * d; rem = nx; }
+    I mul = 1;
+    for (int k = 0; k < rs.out_rank; ++k) { lin += idx[k] * mul; mul *= (I)rs.out_d[k]; }
     // column-major linear index -> multi-index of in -> row-major offset
-    int64_t src = 0;
-    for (int k = 0; k < rs.in_rank; ++k) { idx[k] = lin % rs.in_d[k]; lin /= rs.in_d[k]; }
-    for (int k = 0; k < rs.in_rank; ++k) src = src * rs.in_d[k] + idx[k];
+    I src = 0;
+    for (int k = 0; k < rs.in_rank; ++k) { const I d = (I)rs.in_d[k], nx = lin / d; idx[k] = lin - nx * d; lin = nx; }
+    for (int k = 0; k < rs.in_rank; ++k) src = src * (I)rs.in_d[k] + idx[k];
     out[o] = in[src];
   }
 }
 
 // reduce over one axis: in viewed as [outer, n, inner]
 __global__ void reduce_kernel(int kind, float* out, const float* in, int64_t outer, int64_t n, int64_t inner) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t total = outer * inner;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     const int64_t a = o / inner, c = o - a * inner;
     const float* p = in + a * n * inner + c;
     float acc = kind == LMB200_REDUCE_SUM ? 0.f : -INFINITY;
-    for (int64_t i = 0; i < n; ++i) {
+    int64_t i = 0;
+    for (; i + 16 <= n; i += 16) {                  // same order, 16 loads in flight
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = p[(i + j) * inner];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) acc = kind == LMB200_REDUCE_SUM ? acc + v[j] : fmaxf(acc, v[j]);
+    }
+    for (; i < n; ++i) {
       const float v = p[i * inner];
       acc = kind == LMB200_REDUCE_SUM ? acc + v : fmaxf(acc, v);
     }
@@ -196,29 +230,58 @@ __global__ void reduce_kernel(int kind, float* out, const float* in, int64_t out
   }
 }
 
-// C[bt] = A[bt] (MxK) * B[bt] (KxN), 32x32 tiles, plain fp32 FMAs
-__global__ void __launch_bounds__(1024) matmul_kernel(float* C, const float* A, const float* Bm, int M, int N, int K,
-                                                      int64_t sA, int64_t sB, int64_t sC) {
-  __shared__ float As[32][33], Bs[32][33];
+// C[bt] = A[bt] (MxK) * B[bt] (KxN), 32x32 tiles, plain fp32 FMAs in ascending k.  With one output per thread the two
+// shared-memory reads per FMA bound it (64 wavefronts per k); a thread has four rows of one column now and reads its A values four k at
+// a time (16 wavefronts), and the next tile is on its way from global memory while this one is multiplied.
+constexpr int kMatmulThreads = 256;
+__global__ void __launch_bounds__(kMatmulThreads) matmul_kernel(float* C, const float* A, const float* Bm, int M, int N, int K,
+                                                                int64_t sA, int64_t sB, int64_t sC) {
+  __shared__ __align__(16) float As[32][36], Bs[32][33];
+  pdl_launch_dependents();
+  pdl_wait();
   const int bt = blockIdx.z;
   const float* a = A + bt * sA;
   const float* b = Bm + bt * sB;
   float* c = C + bt * sC;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int row = blockIdx.y * 32 + ty, col = blockIdx.x * 32 + tx;
-  float acc = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    As[ty][tx] = (row < M && k0 + tx < K) ? a[(int64_t)row * K + k0 + tx] : 0.f;
-    Bs[ty][tx] = (k0 + ty < K && col < N) ? b[(int64_t)(k0 + ty) * N + col] : 0.f;
-    __syncthreads();
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;        // rows ty, ty + 8, ty + 16, ty + 24
+  const int row0 = blockIdx.y * 32, col = blockIdx.x * 32 + tx;
+  float an[4], bn[4], acc[4] = {0.f, 0.f, 0.f, 0.f};
+  auto fetch = [&](int k0) {
 #pragma unroll
-    for (int k = 0; k < 32; ++k) acc = fmaf(As[ty][k], Bs[k][tx], acc);
+    for (int j = 0; j < 4; ++j) {
+      const int r = ty + 8 * j;
+      an[j] = (row0 + r < M && k0 + tx < K) ? a[(int64_t)(row0 + r) * K + k0 + tx] : 0.f;
+      bn[j] = (k0 + r < K && col < N) ? b[(int64_t)(k0 + r) * N + col] : 0.f;
+    }
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += 32) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { As[ty + 8 * j][tx] = an[j]; Bs[ty + 8 * j][tx] = bn[j]; }
+    __syncthreads();
+    if (k0 + 32 < K) fetch(k0 + 32);
+#pragma unroll
+    for (int k = 0; k < 32; k += 4) {
+      const float b0 = Bs[k][tx], b1 = Bs[k + 1][tx], b2 = Bs[k + 2][tx], b3 = Bs[k + 3][tx];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 av = *reinterpret_cast<const float4*>(&As[ty + 8 * j][k]);
+        acc[j] = fmaf(av.x, b0, acc[j]);
+        acc[j] = fmaf(av.y, b1, acc[j]);
+        acc[j] = fmaf(av.z, b2, acc[j]);
+        acc[j] = fmaf(av.w, b3, acc[j]);
+      }
+    }
     __syncthreads();
   }
-  if (row < M && col < N) c[(int64_t)row * N + col] = acc;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (row0 + ty + 8 * j < M && col < N) c[(int64_t)(row0 + ty + 8 * j) * N + col] = acc[j];
 }
 
 __global__ void gather_kernel(float* out, const float* table, int64_t vocab, int64_t dim, const float* ids, int64_t n_ids) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t total = n_ids * dim;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = o / dim, c = o - r * dim;
@@ -230,6 +293,8 @@ __global__ void gather_kernel(float* out, const float* table, int64_t vocab, int
 // im2col of the last axis: out[bc, o, k] = a[bc, o*stride + k*dilation]   (src/Execution.jl:481-504)
 __global__ void unfold1d_kernel(float* out, const float* a, int64_t BC, int64_t Lin, int64_t O, int64_t K, int64_t stride,
                                 int64_t dilation) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t total = BC * O * K;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = i % K, o = (i / K) % O, bc = i / (K * O);
@@ -238,6 +303,8 @@ __global__ void unfold1d_kernel(float* out, const float* a, int64_t BC, int64_t 
 }
 
 __global__ void cumsum_kernel(float* out, const float* in, int64_t rows, int64_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= rows) return;
   float acc = 0.f;
@@ -248,6 +315,8 @@ __global__ void cumsum_kernel(float* out, const float* in, int64_t rows, int64_t
 __global__ void __launch_bounds__(256) norm_kernel(float* y, const float* x, const float* w, const float* bias,
                                                    int64_t n, float eps, int mean_centre) {
   __shared__ float red[8];
+  pdl_launch_dependents();
+  pdl_wait();
   const int tid = threadIdx.x;
   const float* xr = x + blockIdx.x * n;
   float* yr = y + blockIdx.x * n;
@@ -281,6 +350,8 @@ __global__ void __launch_bounds__(256) norm_kernel(float* y, const float* x, con
 }
 
 __global__ void silu_gate_kernel(float* out, const float* gate, const float* up, int64_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
     const float a = gate[o];
     const float e = exp2f((a * -1.0f) * kInvLn2);
@@ -290,6 +361,8 @@ __global__ void silu_gate_kernel(float* out, const float* gate, const float* up,
 }
 
 __global__ void rope_kernel(float* out, const float* x, int64_t BH, int64_t S, int64_t D, int64_t prev_seq, float l2base) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t half = D / 2;
   const int64_t total = BH * S * half;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
@@ -310,6 +383,8 @@ __global__ void rope_kernel(float* out, const float* x, int64_t BH, int64_t S, i
 __global__ void __launch_bounds__(256) argmax_kernel(int32_t* out, const float* x, int64_t n) {
   __shared__ float sv[256];
   __shared__ int si[256];
+  pdl_launch_dependents();
+  pdl_wait();
   const int tid = threadIdx.x;
   const float* row = x + blockIdx.x * n;
   float best = -INFINITY;
@@ -337,6 +412,9 @@ int grid_for(int64_t total) {
   if (g < 1) g = 1;
   return (int)g;
 }
+
+// element counts (an operand is never larger than what a 32-bit index of the output reaches through its strides, which stay 64-bit)
+bool fits32(int64_t total) { return total <= 0x7fffffff; }
 
 int32_t check_dims(int32_t rank, const int64_t* dims, int64_t* total) {
   LMB_REQUIRE(rank >= 0 && rank <= kMaxRank, "rank %d outside 0..%d", rank, kMaxRank);
@@ -407,7 +485,7 @@ extern "C" int32_t lmb200_ew(lmb200_ctx h, int32_t opcode, float* out, int32_t o
     LMB_TRY(check_dims(c_rank, c_dims, &tmp));
     LMB_TRY(bcast_strides(out_rank, out_dims, c_rank, c_dims, ix.sc, "ew c"));
   }
-  ew_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(opcode, out, a, binary ? b : nullptr, ternary ? c : nullptr, ix, total);
+  LMB_CUDA(launch_k(fits32(total) ? ew_kernel<uint32_t> : ew_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, opcode, out, a, binary ? b : nullptr, ternary ? c : nullptr, ix, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -448,7 +526,7 @@ extern "C" int32_t lmb200_fused_ew(lmb200_ctx h, float* out, int32_t out_rank, c
   }
   LMB_REQUIRE(depth == 1, "fused_ew: the program leaves %d values", depth);
   if (total == 0) return LMB200_OK;
-  fused_ew_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(out, pg, total);
+  LMB_CUDA(launch_k(fits32(total) ? fused_ew_kernel<uint32_t> : fused_ew_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, pg, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -464,7 +542,7 @@ extern "C" int32_t lmb200_reduce(lmb200_ctx h, int32_t kind, float* out, const f
   int64_t outer = 1, inner = 1;
   for (int i = 0; i < axis; ++i) outer *= dims[i];
   for (int i = axis + 1; i < rank; ++i) inner *= dims[i];
-  reduce_kernel<<<grid_for(outer * inner), 256, 0, ctx->stream>>>(kind, out, in, outer, dims[axis], inner);
+  LMB_CUDA(launch_k(reduce_kernel, dim3((unsigned)(grid_for(outer * inner))), dim3(256), 0, ctx->stream, kind, out, in, outer, dims[axis], inner));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -489,7 +567,7 @@ extern "C" int32_t lmb200_matmul(lmb200_ctx h, float* out, const float* a, int32
       LMB_REQUIRE(a_dims[i] == b_dims[i], "Batch dimensions must match: %lld vs %lld", (long long)a_dims[i], (long long)b_dims[i]);
   LMB_REQUIRE(batch <= 65535, "matmul: batch %lld too large", (long long)batch);
   dim3 grid((unsigned)ceil_div(N, 32), (unsigned)ceil_div(M, 32), (unsigned)batch);
-  matmul_kernel<<<grid, dim3(32, 32), 0, ctx->stream>>>(out, a, b, (int)M, (int)N, (int)K, M * K, b_rank > 2 ? K * N : 0, M * N);
+  LMB_CUDA(launch_k(matmul_kernel, grid, dim3(kMatmulThreads), 0, ctx->stream, out, a, b, (int)M, (int)N, (int)K, M * K, b_rank > 2 ? K * N : 0, M * N));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -512,7 +590,7 @@ extern "C" int32_t lmb200_permute(lmb200_ctx h, float* out, const float* in, int
     gt.out_d[k] = in_dims[perm[k]];
     gt.st[k] = in_st[perm[k]];
   }
-  strided_copy_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(out, in, gt, total);
+  LMB_CUDA(launch_k(fits32(total) ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -529,7 +607,7 @@ extern "C" int32_t lmb200_reshape_colmajor(lmb200_ctx h, float* out, const float
   rs.in_rank = in_rank; rs.out_rank = out_rank;
   for (int i = 0; i < in_rank; ++i) rs.in_d[i] = in_dims[i];
   for (int i = 0; i < out_rank; ++i) rs.out_d[i] = out_dims[i];
-  reshape_cm_kernel<<<grid_for(to), 256, 0, ctx->stream>>>(out, in, rs, to);
+  LMB_CUDA(launch_k(fits32(to) ? reshape_cm_kernel<uint32_t> : reshape_cm_kernel<int64_t>, dim3((unsigned)(grid_for(to))), dim3(256), 0, ctx->stream, out, in, rs, to));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -551,7 +629,7 @@ extern "C" int32_t lmb200_expand(lmb200_ctx h, float* out, const float* in, int3
     else { gt.out_d[k] = in_dims[j]; gt.st[k] = in_st[j]; ++j; }
   }
   const int64_t total = ti * size;
-  strided_copy_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(out, in, gt, total);
+  LMB_CUDA(launch_k(fits32(total) ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -575,7 +653,7 @@ extern "C" int32_t lmb200_slice(lmb200_ctx h, float* out, const float* in, int32
     mul *= in_dims[k];
     total *= e - s;
   }
-  strided_copy_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(out, in, gt, total);
+  LMB_CUDA(launch_k(fits32(total) ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -595,7 +673,7 @@ extern "C" int32_t lmb200_pad(lmb200_ctx h, float* out, const float* in, int32_t
     pd.out_d[k] = in_dims[k] + left[k] + right[k];
     total *= pd.out_d[k];
   }
-  pad_kernel<<<grid_for(total), 256, 0, ctx->stream>>>(out, in, pd, total);
+  LMB_CUDA(launch_k(fits32(total) ? pad_kernel<uint32_t> : pad_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, pd, total));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -604,7 +682,7 @@ extern "C" int32_t lmb200_gather(lmb200_ctx h, float* out, const float* table, i
                                  const float* ids, int64_t n_ids) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && table && ids && vocab >= 1 && dim >= 1 && n_ids >= 1, "gather: bad argument");
-  gather_kernel<<<grid_for(n_ids * dim), 256, 0, ctx->stream>>>(out, table, vocab, dim, ids, n_ids);
+  LMB_CUDA(launch_k(gather_kernel, dim3((unsigned)(grid_for(n_ids * dim))), dim3(256), 0, ctx->stream, out, table, vocab, dim, ids, n_ids));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -615,7 +693,7 @@ extern "C" int32_t lmb200_unfold1d(lmb200_ctx h, float* out, const float* in, in
   LMB_REQUIRE(out && in && rows >= 1 && kernel >= 1 && stride >= 1 && dilation >= 1, "unfold: bad argument");
   const int64_t O = (length - dilation * (kernel - 1) - 1) / stride + 1;
   LMB_REQUIRE(O >= 1, "unfold: length %lld too short for kernel %lld", (long long)length, (long long)kernel);
-  unfold1d_kernel<<<grid_for(rows * O * kernel), 256, 0, ctx->stream>>>(out, in, rows, length, O, kernel, stride, dilation);
+  LMB_CUDA(launch_k(unfold1d_kernel, dim3((unsigned)(grid_for(rows * O * kernel))), dim3(256), 0, ctx->stream, out, in, rows, length, O, kernel, stride, dilation));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -623,7 +701,7 @@ extern "C" int32_t lmb200_unfold1d(lmb200_ctx h, float* out, const float* in, in
 extern "C" int32_t lmb200_cumsum_last(lmb200_ctx h, float* out, const float* in, int64_t rows, int64_t n) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && in && rows >= 1 && n >= 1, "cumsum: bad argument");
-  cumsum_kernel<<<(unsigned)ceil_div(rows, 128), 128, 0, ctx->stream>>>(out, in, rows, n);
+  LMB_CUDA(launch_k(cumsum_kernel, dim3((unsigned)(ceil_div(rows, 128))), dim3(128), 0, ctx->stream, out, in, rows, n));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -632,7 +710,7 @@ extern "C" int32_t lmb200_rmsnorm_scale(lmb200_ctx h, float* y, const float* x, 
                                         int64_t n, float eps) {
   CTX_OR_FAIL();
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "rmsnorm: bad argument");
-  norm_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(y, x, w, nullptr, n, eps, 0);
+  LMB_CUDA(launch_k(norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, nullptr, n, eps, 0));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -641,7 +719,7 @@ extern "C" int32_t lmb200_layernorm(lmb200_ctx h, float* y, const float* x, cons
                                     int64_t rows, int64_t n, float eps) {
   CTX_OR_FAIL();
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "layernorm: bad argument");
-  norm_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(y, x, w, bias, n, eps, 1);
+  LMB_CUDA(launch_k(norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, bias, n, eps, 1));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -649,7 +727,7 @@ extern "C" int32_t lmb200_layernorm(lmb200_ctx h, float* y, const float* x, cons
 extern "C" int32_t lmb200_silu_gate(lmb200_ctx h, float* out, const float* gate, const float* up, int64_t n) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && gate && up && n >= 1, "silu_gate: bad argument");
-  silu_gate_kernel<<<grid_for(n), 256, 0, ctx->stream>>>(out, gate, up, n);
+  LMB_CUDA(launch_k(silu_gate_kernel, dim3((unsigned)(grid_for(n))), dim3(256), 0, ctx->stream, out, gate, up, n));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -658,7 +736,7 @@ extern "C" int32_t lmb200_rope(lmb200_ctx h, float* out, const float* x, int64_t
                                int64_t prev_seq, float base) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && x && B >= 1 && H >= 1 && S >= 1 && D >= 2 && D % 2 == 0, "rope: bad argument");
-  rope_kernel<<<grid_for(B * H * S * (D / 2)), 256, 0, ctx->stream>>>(out, x, B * H, S, D, prev_seq, log2f(base));
+  LMB_CUDA(launch_k(rope_kernel, dim3((unsigned)(grid_for(B * H * S * (D / 2)))), dim3(256), 0, ctx->stream, out, x, B * H, S, D, prev_seq, log2f(base)));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -666,7 +744,7 @@ extern "C" int32_t lmb200_rope(lmb200_ctx h, float* out, const float* x, int64_t
 extern "C" int32_t lmb200_argmax(lmb200_ctx h, int32_t* out, const float* x, int64_t rows, int64_t n) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && x && rows >= 1 && n >= 1, "argmax: bad argument");
-  argmax_kernel<<<(unsigned)rows, 256, 0, ctx->stream>>>(out, x, n);
+  LMB_CUDA(launch_k(argmax_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, out, x, n));
   LAUNCHED();
   return LMB200_OK;
 }
