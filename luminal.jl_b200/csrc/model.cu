@@ -1471,7 +1471,8 @@ int32_t advance_launch(Session* S, cudaStream_t st) {
 
 namespace {
 
-// The fused decode step of a bf16 Llama / Phi-3: five launches per layer.  The residual add and the
+// The fused decode step of a bf16 Llama / Phi-3: two launches per layer (attention, and the GEMVs from there to the next attention as
+// one chain), or five where every GEMV is its own launch (tensor parallelism).  The residual add and the
 // RMSNorm around every Linear (src/NN.jl:406-414, 149-161) are carried by the projections themselves:
 // o_proj and down_proj finish with EPI_RESID_NORM (under tensor parallelism including the all-reduce of
 // their partial sums), q/k/v, gate/up and the head multiply their accumulators by the norm's

@@ -13,7 +13,7 @@ namespace {
 // A traced graph is a chain of hundreds of these, most of a microsecond's work, so what counts is the time from one to the next:
 // all are launched programmatically (each waits for its predecessor before it touches memory), and index arithmetic is 32-bit
 // (I = uint32_t) wherever the element counts allow: a 64-bit division is a subroutine of about a hundred instructions.
-// The small Llama's 32-token graph (404 kernels): 1522 -> 1343 us a call.
+// The small Llama's 32-token graph (404 kernels): 1522 -> 1343 us a call, 1148 with the matmul below.
 constexpr int kMaxRank = 8;
 constexpr float kInvLn2 = 1.4426950408889634f;
 constexpr float kHalfPi = 1.5707963267948966f;
@@ -230,53 +230,71 @@ __global__ void reduce_kernel(int kind, float* out, const float* in, int64_t out
   }
 }
 
-// C[bt] = A[bt] (MxK) * B[bt] (KxN), 32x32 tiles, plain fp32 FMAs in ascending k.  With one output per thread the two
-// shared-memory reads per FMA bound it (64 wavefronts per k); a thread has four rows of one column now and reads its A values four k at
-// a time (16 wavefronts), and the next tile is on its way from global memory while this one is multiplied.
-constexpr int kMatmulThreads = 256;
+// C[bt] = A[bt] (MxK) * B[bt] (KxN), 32x32 tiles, plain fp32 FMAs.  A traced graph's products are a few tiles with K of a few hundred:
+// a chain of k steps, each a trip to L2, which 32 k at a time took 13 to 18 us for 32 x 256 x 256.  Now a step is 128 k, of
+// which every warp multiplies 16 for the whole tile (a column and 32 rows per thread: 9 shared-memory reads for 32 FMAs), the next step
+// is on its way meanwhile, and the eight warps' sums are added in warp order at the end.
+constexpr int kMatmulThreads = 256, kMatmulK = 128, kMatmulPitch = 36;
 __global__ void __launch_bounds__(kMatmulThreads) matmul_kernel(float* C, const float* A, const float* Bm, int M, int N, int K,
                                                                 int64_t sA, int64_t sB, int64_t sC) {
-  __shared__ __align__(16) float As[32][36], Bs[32][33];
+  __shared__ __align__(16) float buf[kMatmulK * (kMatmulPitch + 32)];
+  float* As = buf;                                       // [k][row], rows padded to 36
+  float* Bs = buf + kMatmulK * kMatmulPitch;             // [k][column]
   pdl_launch_dependents();
   pdl_wait();
   const int bt = blockIdx.z;
   const float* a = A + bt * sA;
   const float* b = Bm + bt * sB;
   float* c = C + bt * sC;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;        // rows ty, ty + 8, ty + 16, ty + 24
+  const int tx = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int row0 = blockIdx.y * 32, col = blockIdx.x * 32 + tx;
-  float an[4], bn[4], acc[4] = {0.f, 0.f, 0.f, 0.f};
+  float an[16], bn[16], acc[32];
+#pragma unroll
+  for (int r = 0; r < 32; ++r) acc[r] = 0.f;
   auto fetch = [&](int k0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int r = ty + 8 * j;
-      an[j] = (row0 + r < M && k0 + tx < K) ? a[(int64_t)(row0 + r) * K + k0 + tx] : 0.f;
-      bn[j] = (k0 + r < K && col < N) ? b[(int64_t)(k0 + r) * N + col] : 0.f;
+    for (int j = 0; j < 16; ++j) {
+      const int r = row0 + w + 8 * (j >> 2), ka = k0 + tx + 32 * (j & 3), kb = k0 + w + 8 * j;
+      an[j] = (r < M && ka < K) ? a[(int64_t)r * K + ka] : 0.f;
+      bn[j] = (kb < K && col < N) ? b[(int64_t)kb * N + col] : 0.f;
     }
   };
   fetch(0);
-  for (int k0 = 0; k0 < K; k0 += 32) {
+  for (int k0 = 0; k0 < K; k0 += kMatmulK) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { As[ty + 8 * j][tx] = an[j]; Bs[ty + 8 * j][tx] = bn[j]; }
+    for (int j = 0; j < 16; ++j) {
+      As[(tx + 32 * (j & 3)) * kMatmulPitch + w + 8 * (j >> 2)] = an[j];
+      Bs[(w + 8 * j) * 32 + tx] = bn[j];
+    }
     __syncthreads();
-    if (k0 + 32 < K) fetch(k0 + 32);
+    if (k0 + kMatmulK < K) fetch(k0 + kMatmulK);
+    if (k0 + 16 * w < K) {
+#pragma unroll 4
+      for (int k = 16 * w; k < 16 * w + 16; ++k) {
+        const float bv = Bs[k * 32 + tx];
 #pragma unroll
-    for (int k = 0; k < 32; k += 4) {
-      const float b0 = Bs[k][tx], b1 = Bs[k + 1][tx], b2 = Bs[k + 2][tx], b3 = Bs[k + 3][tx];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 av = *reinterpret_cast<const float4*>(&As[ty + 8 * j][k]);
-        acc[j] = fmaf(av.x, b0, acc[j]);
-        acc[j] = fmaf(av.y, b1, acc[j]);
-        acc[j] = fmaf(av.z, b2, acc[j]);
-        acc[j] = fmaf(av.w, b3, acc[j]);
+        for (int r = 0; r < 32; r += 4) {
+          const float4 av = *reinterpret_cast<const float4*>(&As[k * kMatmulPitch + r]);
+          acc[r] = fmaf(av.x, bv, acc[r]);
+          acc[r + 1] = fmaf(av.y, bv, acc[r + 1]);
+          acc[r + 2] = fmaf(av.z, bv, acc[r + 2]);
+          acc[r + 3] = fmaf(av.w, bv, acc[r + 3]);
+        }
       }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (row0 + ty + 8 * j < M && col < N) c[(int64_t)(row0 + ty + 8 * j) * N + col] = acc[j];
+  for (int r = 0; r < 32; ++r) buf[(w * 32 + r) * 32 + tx] = acc[r];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = 4 * w + j;
+    float t = 0.f;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) t += buf[(v * 32 + r) * 32 + tx];
+    if (row0 + r < M && col < N) c[(int64_t)(row0 + r) * N + col] = t;
+  }
 }
 
 __global__ void gather_kernel(float* out, const float* table, int64_t vocab, int64_t dim, const float* ids, int64_t n_ids) {
