@@ -41,14 +41,14 @@ constexpr int kEpiStageBytes = 32 * 80;        // per epilogue warp: 32 tokens x
 constexpr float kInvLn2 = 1.4426950408889634f;
 constexpr float kHalfPi = 1.5707963267948966f;
 
-enum GemmEpilogue { GEMM_STORE_F32 = 0, GEMM_SILU_GATE = 1, GEMM_QKV_ROPE = 2, GEMM_AFFINE = 3, GEMM_CROSS_KV = 4, GEMM_SEGMENTS = 5 };
+enum GemmEpilogue { GEMM_STORE_F32 = 0, GEMM_SILU_GATE = 1, GEMM_QKV_ROPE = 2, GEMM_AFFINE = 3, GEMM_CROSS_KV = 4, GEMM_SEGMENTS = 5, GEMM_ADD_F32 = 6 };
 
 struct GemmParams {
   const __nv_bfloat16* W = nullptr;     // canonical 128 x 128 units, unit (row group, k step) at (rg * KS + ks) * 16384
   const __nv_bfloat16* X = nullptr;     // [T, ldx] row-major
   int ldx = 0, T = 0, rows = 0, K = 0;
   int epi = GEMM_STORE_F32;
-  float* out = nullptr;                 // GEMM_STORE_F32: out[token * ldo + row]
+  float* out = nullptr;                 // GEMM_STORE_F32: out[token * ldo + row]; GEMM_ADD_F32: added to it
   int ldo = 0;
   __nv_bfloat16* act = nullptr;         // GEMM_SILU_GATE: act[token * ld_act + i], rows interleaved 8 gate / 8 up
   int ld_act = 0, n_act = 0;
@@ -194,9 +194,16 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32
   const int lane = threadIdx.x & 31, n_tok = min(32, t_end - t0);
   __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(stage);
   const int row0 = row & ~31;                          // the warp's first row: rows row0 .. row0 + 31 (a multiple of 32)
-  if (EPI == GEMM_STORE_F32) {
+  if (EPI == GEMM_STORE_F32 || EPI == GEMM_ADD_F32) {
     if (row < p.rows) {
       float* out = p.out + (int64_t)t0 * p.ldo + row;
+      if (EPI == GEMM_ADD_F32) {                       // every tile is one CTA's: all reads first, then the stores
+        float old[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) old[i] = i < n_tok ? out[(int64_t)i * p.ldo] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] += old[i];
+      }
 #pragma unroll
       for (int i = 0; i < 32; ++i)
         if (i < n_tok) out[(int64_t)i * p.ldo] = v[i];
@@ -808,6 +815,7 @@ int32_t gemm_launch(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
     case GEMM_QKV_ROPE: return gemm_launch_epi<GEMM_QKV_ROPE>(ctx, p, st);
     case GEMM_AFFINE: return gemm_launch_epi<GEMM_AFFINE>(ctx, p, st);
     case GEMM_CROSS_KV: return gemm_launch_epi<GEMM_CROSS_KV>(ctx, p, st);
+    case GEMM_ADD_F32: return gemm_launch_epi<GEMM_ADD_F32>(ctx, p, st);
     default: return gemm_launch_epi<GEMM_SEGMENTS>(ctx, p, st);
   }
 }
@@ -995,6 +1003,7 @@ int32_t prefill_configure() {
   LMB_TRY(gemm_configure<GEMM_QKV_ROPE>());
   LMB_TRY(gemm_configure<GEMM_AFFINE>());
   LMB_TRY(gemm_configure<GEMM_CROSS_KV>());
+  LMB_TRY(gemm_configure<GEMM_ADD_F32>());
   return gemm_configure<GEMM_SEGMENTS>();
 }
 
@@ -1017,8 +1026,11 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows&
   const int B = S->B, hid = c.hidden, L = c.n_layers, D = M->D;
   const int T = ragged.total > 0 ? ragged.total : B * n;
   const int qw = M->Hl * D, kvw = M->KVl * D;
+  // On one rank o_proj and down_proj add to the residual rows themselves: 14 bytes per element with the norm that follows, 18 by way of a
+  // separate sum.  Under tensor parallelism the ranks' partial sums are reduced first.
+  const bool fold = c.tp_size == 1 || M->tp_solo;
   // one scratch block per session, kept for the next prompt of the same or a smaller size
-  const int64_t sizes[9] = {(int64_t)T * hid * 4, (int64_t)T * hid * 4, (int64_t)T * hid * 2, (int64_t)T * qw * 2, (int64_t)T * kvw * 2,
+  const int64_t sizes[9] = {(int64_t)T * hid * 4, fold ? 0 : (int64_t)T * hid * 4, (int64_t)T * hid * 2, (int64_t)T * qw * 2, (int64_t)T * kvw * 2,
                             (int64_t)T * kvw * 2, (int64_t)T * qw * 2, (int64_t)T * M->inter_l * 2, (int64_t)n * (D / 2) * 8};
   int64_t offs[9], total = 0;
   for (int i = 0; i < 9; ++i) { offs[i] = total; total += round_up(sizes[i], 256); }
@@ -1034,7 +1046,7 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows&
   }
   char* base = reinterpret_cast<char*>(S->prefill_buf);
   float* x = reinterpret_cast<float*>(base + offs[0]);
-  float* delta = reinterpret_cast<float*>(base + offs[1]);
+  float* delta = fold ? nullptr : reinterpret_cast<float*>(base + offs[1]);
   __nv_bfloat16* xn = reinterpret_cast<__nv_bfloat16*>(base + offs[2]);
   __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(base + offs[3]);
   __nv_bfloat16* kb = reinterpret_cast<__nv_bfloat16*>(base + offs[4]);
@@ -1048,7 +1060,7 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows&
   ctx->launches++;
   const size_t norm_smem = (size_t)hid * sizeof(float);
   auto reduce = [&](float* buf) -> int32_t {          // row-parallel projection under tensor parallelism
-    if (c.tp_size > 1 && !M->tp_solo) return nccl_allreduce_f32(ctx, buf, (int64_t)T * hid, st);
+    if (!fold) return nccl_allreduce_f32(ctx, buf, (int64_t)T * hid, st);
     return LMB200_OK;
   };
   FlashView fv;
@@ -1076,7 +1088,7 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows&
     {
       GemmParams p;
       p.W = reinterpret_cast<const __nv_bfloat16*>(W.wo); p.X = attn; p.ldx = qw; p.T = T; p.rows = hid; p.K = qw;
-      p.epi = GEMM_STORE_F32; p.out = delta; p.ldo = hid;
+      p.epi = fold ? GEMM_ADD_F32 : GEMM_STORE_F32; p.out = fold ? x : delta; p.ldo = hid;
       LMB_TRY(gemm_launch(ctx, p, st));
       LMB_TRY(reduce(delta));
     }
@@ -1091,7 +1103,7 @@ int32_t prefill_gemm(Session* S, const int* tokens_dev, int n, const RaggedRows&
     {
       GemmParams p;
       p.W = reinterpret_cast<const __nv_bfloat16*>(W.wdown); p.X = act; p.ldx = M->inter_l; p.T = T; p.rows = hid; p.K = M->inter_l;
-      p.epi = GEMM_STORE_F32; p.out = delta; p.ldo = hid;
+      p.epi = fold ? GEMM_ADD_F32 : GEMM_STORE_F32; p.out = fold ? x : delta; p.ldo = hid;
       LMB_TRY(gemm_launch(ctx, p, st));
       LMB_TRY(reduce(delta));
     }
