@@ -81,7 +81,7 @@ struct GemmParams {
 __device__ __forceinline__ float gelu_ref(float a) {
   const float inner = (0.7978845608f * a) * (1.0f + (0.044715f * a) * a);
   const float z = inner * 2.0f;
-  const float sg = __fdividef(1.0f, 1.0f + exp2f((z * -1.0f) * kInvLn2));
+  const float sg = 1.0f / (1.0f + exp2f((z * -1.0f) * kInvLn2));
   const float th = sg * 2.0f + -1.0f;
   return (a * 0.5f) * (1.0f + th);
 }
@@ -165,10 +165,10 @@ __device__ __forceinline__ void segment_epilogue(const GemmParams& p, float (&v)
     for (int i = 0; i < 32; ++i) { const float y = fmaxf(v[i], 0.f); v[i] = y * y; }
   } else if (sg.kind == SEG_SILU) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __fdividef(v[i], 1.0f + expf(-v[i]));
+    for (int i = 0; i < 32; ++i) v[i] = v[i] / (1.0f + expf(-v[i]));
   } else if (sg.kind == SEG_SIGMOID) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __fdividef(1.0f, 1.0f + expf(-v[i]));
+    for (int i = 0; i < 32; ++i) v[i] = sigmoid_f32(v[i]);
   }
   // bf16: the warp's 32 x 32 block is turned through shared memory and stored as runs of 64 bytes
 #pragma unroll
@@ -294,7 +294,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, float (&v)[32
       const float got = __shfl_xor_sync(0xffffffffu, hi ? v[i] : v[i + 16], 8);
       const float a = hi ? got : v[i], u = hi ? v[i + 16] : got;
       const float ex = exp2f((a * -1.0f) * kInvLn2);            // src/HighLevelOps.jl:153-160
-      const float sg = __fdividef(1.0f, 1.0f + ex);
+      const float sg = 1.0f / (1.0f + ex);
       st[(i + 16 * hi) * kEpiPitch + col] = __float2bfloat16_rn((a * sg) * u);
     }
     __syncwarp();

@@ -119,3 +119,33 @@ print("single ok")
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, LMB200_GEMM_PAIR="0"), capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "single ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_prompt_silu_far_below_zero(lib_built, device):
+    """SiLU of -88 is -88 / (1 + e^88): the quotient of a full-precision division is a subnormal number, that of an approximate one is 0 (its
+    divisor lies above 2^126).  A large up-projection makes the difference show in the logits."""
+    L = lib_built
+    cfg = dict(n_layers=1, hidden=128, n_heads=2, n_kv_heads=2, intermediate=64, vocab=96, eps=1e-5, rope_base=10000.0)
+    rng = np.random.default_rng(3)
+    w = {k: np.zeros_like(v) for k, v in O.synth_llama_weights(cfg, seed=3).items()}
+    for k in w:
+        if k.endswith("norm.weight"):
+            w[k][:] = 1.0
+    embed = rng.choice([-1.0, 1.0], (96, 128))                     # rows of rms 1 whose first feature is 1
+    embed[:, 0] = 1.0
+    w["model.embed_tokens.weight"] = embed.astype(np.float32)
+    w["lm_head.weight"] = O.bf16_round(rng.standard_normal((96, 128)).astype(np.float32))
+    w["model.layers.0.mlp.gate_proj.weight"][:, 0] = -88.0
+    w["model.layers.0.mlp.up_proj.weight"][:, 0] = 2.0 ** 100
+    down = (rng.choice([-1.0, 1.0], (128, 64)) * 2.0 ** 18).astype(np.float32)
+    w["model.layers.0.mlp.down_proj.weight"] = down
+    prompt = rng.integers(0, 96, (1, 40)).astype(np.int32)
+    ref = O.CachedLlama(w, cfg, 1, 48).forward(prompt)[:, -1, :]
+    w["model.layers.0.mlp.down_proj.weight"] = down * 0.0
+    without = O.CachedLlama(w, cfg, 1, 48).forward(prompt)[:, -1, :]
+    w["model.layers.0.mlp.down_proj.weight"] = down
+    assert np.linalg.norm(ref - without) > 0.2 * np.linalg.norm(ref)
+    model, sess = make(L, device, cfg, w, 1, 48)
+    got = sess.prefill(prompt)
+    assert np.linalg.norm(got - ref) <= 4e-2 * np.linalg.norm(ref)
+    sess.close(); model.close()
