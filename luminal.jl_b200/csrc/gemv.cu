@@ -2215,8 +2215,10 @@ int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMax + 1) * kChainLin
 int32_t GemvChain::add(const GemvParams& p) {
   if (clusters == 0) return gemv_launch(ctx, LMB200_BF16, p, stream);
   // Every tile costs an exchange inside the cluster, about 2.4 us.  A GEMV of several tiles per cluster whose tiles stream for less than
-  // that (a unit is 0.57 us) is better off alone: 51865 x 512 takes 12 us by itself and 31 us here.
-  if (ceil_div(p.rows, 128) > clusters && p.K <= 3 * 128 * kChainC) {
+  // that (a unit is 0.57 us) is better off alone: 51865 x 512 takes 12 us by itself and 31 us here.  Not where a norm follows: its consumer
+  // reads the slots that the chain kernel leaves (slots()), a launch of its own leaves as many as its plan has CTAs.
+  const bool norm = p.epi == EPI_RESID_NORM || p.epi == EPI_POST_NORM;
+  if (!norm && ceil_div(p.rows, 128) > clusters && p.K <= 3 * 128 * kChainC) {
     LMB_TRY(flush());
     return gemv_launch(ctx, LMB200_BF16, p, stream);
   }

@@ -186,7 +186,7 @@ struct GemvChain {
   int n = 0;
   int32_t add(const GemvParams& p);
   int32_t flush();                           // before anything that reads the last GEMV's output
-  // ssq slots an EPI_RESID_NORM of these rows leaves
+  // ssq slots an EPI_RESID_NORM of these rows leaves: with clusters, add() and flush() run every one in the chain kernel
   int slots(const GemvPlan& pl, int rows) const { return clusters ? (int)ceil_div(rows, 128) * kChainC : gemv_plan_ctas(pl, rows); }
 };
 int gemv_chain_max_clusters(const Ctx* ctx, int B);
