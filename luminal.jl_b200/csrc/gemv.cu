@@ -2204,11 +2204,24 @@ int gemv_plan_ctas(const GemvPlan& pl, int rows) {
   return pl.cluster >= 1 ? (int)ceil_div(rows, 128) * pl.cluster : pl.grid;
 }
 
-int gemv_chain_max_clusters(const Ctx* ctx, int B) {
-  (void)ctx;
-  const char* e = getenv("LMB200_GEMV_CHAIN");                  // 0: one launch per GEMV (A/B runs)
+// What the chain saves per GEMV is a launch, about 6 us of which its ring covers 3; what it costs is that a row group has four CTAs.  By
+// itself a projection runs on clusters of eight while 15 of them hold its row groups, and then streams faster than here, unless it is so
+// short that eight, or four, have no unit of k each.  Hence chained up to 3 and from 16 row groups of the residual width on.  Per layer of a
+// Llama, one launch per GEMV -> chained, batch 1 | 32: width 256, feed-forward 704 28 -> 26 | 32 -> 30 us; 512, 1408 26.1 -> 27.4 | 29.6 -> 29.8;
+// 1024, 2816 30.2 -> 33.2 | 34.8 -> 40.8; 1536, 4224 39.0 -> 41.9 | 50.0 -> 51.7; 2048, 5632 53.2 -> 47.4 | 64.4 -> 58.9; 3072, 8448 69.6 -> 63.2 |
+// 85.5 -> 82.2 (1792 and 1920 go either way with the feed-forward's width).  A Gibutar's chains of two GEMVs: the same line, from 24 row groups on
+// above 16 sequences, where an exchange moves twice the bytes (eight layers, batch 16 | 32: 2048 458 -> 445 | 577 -> 598 us; four, 3072 351 -> 348 |
+// 397 -> 379).  Sublayers normed on their output make chains of six GEMVs, which gain at every width (Kevatar, four layers, batch 16: 512
+// 238 -> 216 us, 1024 277 -> 247, 2048 387 -> 330).
+int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms) {
+  const char* e = getenv("LMB200_GEMV_CHAIN");                  // 0: one launch per GEMV, 1: chained wherever it can be (A/B runs)
   if ((e && atoi(e) == 0) || g_variant != GEMV_TCGEN05) return 0;
-  return Layout<__nv_bfloat16>::batch_pad(B) == 16 ? chain_clusters<16>() : chain_clusters<32>();
+  const int64_t groups = ceil_div(width, 128);
+  if (groups * kChainC > kSsqSlots) return 0;                   // a projection leaves 4 sums of squares per row group
+  const bool wide_batch = Layout<__nv_bfloat16>::batch_pad(B) > 16;
+  if (!e && per_chain < 6 && groups > 3 && groups < (per_chain < 4 && wide_batch ? 24 : 16)) return 0;
+  const int n = wide_batch ? chain_clusters<32>() : chain_clusters<16>();
+  return output_norms && groups > n ? 0 : n;                    // an output norm needs every row group resident at once
 }
 int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMax + 1) * kChainLine * 4; }
 

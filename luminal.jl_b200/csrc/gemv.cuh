@@ -174,9 +174,10 @@ void gemv_prefetch_next(GemvParams& p, const Ctx* ctx, int dtype, const void* ne
 int32_t gemv_launch(Ctx* ctx, int dtype, GemvParams p, cudaStream_t stream);
 
 // A run of bf16 GEMVs, each reading what the one before it wrote, as one launch (gemv_chain_kernel).  `clusters` is
-// gemv_chain_max_clusters for the batch; 0 launches every GEMV by itself.  One rank only.
+// gemv_chain_clusters for the session; 0 launches every GEMV by itself.  One rank only.
 constexpr int kChainMax = 8;                 // GEMVs per launch
 constexpr int kChainC = 4;                   // CTAs per cluster
+constexpr int kSsqSlots = 256;               // of a session's ssq buffer, 32 floats each
 struct GemvChain {
   Ctx* ctx = nullptr;
   cudaStream_t stream = nullptr;
@@ -189,7 +190,9 @@ struct GemvChain {
   // ssq slots an EPI_RESID_NORM of these rows leaves: with clusters, add() and flush() run every one in the chain kernel
   int slots(const GemvPlan& pl, int rows) const { return clusters ? (int)ceil_div(rows, 128) * kChainC : gemv_plan_ctas(pl, rows); }
 };
-int gemv_chain_max_clusters(const Ctx* ctx, int B);
+// Clusters for a session whose residual rows are `width` wide and whose chains have per_chain GEMVs, 0: one launch per GEMV.  output_norms:
+// EPI_POST_NORMs are among them
+int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms);
 int64_t gemv_chain_scratch_bytes();
 
 }  // namespace lmb

@@ -1471,14 +1471,13 @@ int32_t layered_session_create(Model* M, int batch, int max_ctx, lmb200_session*
     }
     S->p_head = take(gemv_plan(ctx, c.dtype, batch, M->m_head.rows, M->m_head.K));
     S->embed_rows_per_cta = 32 * (int)ceil_div(c.hidden, 32 * 256);
-    // A chained projection fills 4 of the 256 slots per row group, and an output norm needs every row group resident at once.
-    if (const int n = gemv_chain_max_clusters(ctx, batch); ceil_div(c.hidden, 128) <= std::min(post_norm(M) ? n : 64, 64)) S->chain_clusters = n;
+    S->chain_clusters = gemv_chain_clusters(batch, c.hidden, post_norm(M) ? 6 : 2, post_norm(M));
     if (S->chain_clusters) alloc((void**)&S->chain_done, gemv_chain_scratch_bytes());
     auto x_bytes = [&](int64_t K) { return Layout<__nv_bfloat16>::x_elems((int)K, S->Bp) * 2; };
     alloc(&S->xn, x_bytes(c.hidden));
     alloc(&S->act, x_bytes(max_over(M, [](const LayerSpec& s) { return s.m_out.K; })));
     alloc((void**)&S->xT, (int64_t)round_up(c.hidden, 128) * S->Bp * 4);
-    alloc((void**)&S->ssq, (int64_t)256 * 32 * 4);
+    alloc((void**)&S->ssq, (int64_t)kSsqSlots * 32 * 4);
     alloc((void**)&S->gemv_partials, max_part * 4);
     alloc((void**)&S->gemv_counters, (int64_t)max_cnt * 4);
     alloc((void**)&Z.proj, batch * max_over(M, [](const LayerSpec& s) { return s.n_store; }) * 4);

@@ -1983,8 +1983,7 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
       else fused = false;
     }
     S->fused = fused;
-    // ssq has 256 slots, of which a chained projection fills 4 per row group
-    if (fused && c.tp_size == 1 && ceil_div(c.hidden, 128) * kChainC <= 256 && !whisper) S->chain_clusters = gemv_chain_max_clusters(ctx, batch);
+    if (fused && c.tp_size == 1 && !whisper) S->chain_clusters = gemv_chain_clusters(batch, c.hidden, 4, false);
     S->embed_rows_per_cta = 32 * (int)ceil_div(c.hidden, 32 * 256);
     // The head is replicated; under tensor parallelism every rank multiplies only its share of the rows and the ranks
     // exchange their best (logit, id) pairs (LMB200_TP_HEAD=replicated keeps every rank on the whole head, A/B runs).
@@ -2047,9 +2046,9 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
   alloc((void**)&S->attn_counters, (int64_t)S->B * M->KVl * 4);
   if (S->fused) {
     alloc((void**)&S->xT, (int64_t)round_up(c.hidden, 128) * S->Bp * 4);
-    alloc((void**)&S->ssq, (int64_t)256 * 32 * 4);
+    alloc((void**)&S->ssq, (int64_t)kSsqSlots * 32 * 4);
     if (S->chain_clusters) alloc((void**)&S->chain_done, gemv_chain_scratch_bytes());
-    if (whisper) alloc((void**)&S->sum_slots, (int64_t)256 * 32 * 4);
+    if (whisper) alloc((void**)&S->sum_slots, (int64_t)kSsqSlots * 32 * 4);
   }
   if (S->head_sliced) alloc((void**)&S->logits_slice, (int64_t)batch * S->head_pitch * 4);
   S->host_pos_v.assign(batch, 0);
