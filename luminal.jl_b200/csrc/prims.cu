@@ -10,10 +10,13 @@
 namespace lmb {
 namespace {
 
-// A traced graph is a chain of hundreds of these, most of a microsecond's work, so what counts is the time from one to the next:
-// all are launched programmatically (each waits for its predecessor before it touches memory), and index arithmetic is 32-bit
-// (I = uint32_t) wherever the element counts allow: a 64-bit division is a subroutine of about a hundred instructions.
-// The small Llama's 32-token graph (404 kernels): 1522 -> 1343 us a call, 1148 with the matmul below.
+// A traced graph is a chain of hundreds of these, most of a microsecond's work, so what counts is the time from one to the next.  Kernels with a
+// short thread per output element are launched programmatically (each waits for its predecessor before it touches memory).  The others, whose
+// CTAs work for a while -- products, reductions, scans, norms -- start in plain order: CTAs that become resident early pile up on the SMs that
+// were free first, and the kernel is as slow as the fullest of them (sums of 65536 rows of 1024: 274 us in plain order, 366 otherwise; scans 700 and
+// 1050).  Index arithmetic is 32-bit (I = uint32_t) wherever the element counts allow: a 64-bit division is a subroutine of about a hundred instructions.
+// The small Llama's 32-token graph (404 kernels), per call: 1431 -> 985 us with the
+// matmul below (1126 with all of them programmatic).
 constexpr int kMaxRank = 8;
 constexpr float kInvLn2 = 1.4426950408889634f;
 constexpr float kHalfPi = 1.5707963267948966f;
@@ -560,7 +563,7 @@ extern "C" int32_t lmb200_reduce(lmb200_ctx h, int32_t kind, float* out, const f
   int64_t outer = 1, inner = 1;
   for (int i = 0; i < axis; ++i) outer *= dims[i];
   for (int i = axis + 1; i < rank; ++i) inner *= dims[i];
-  LMB_CUDA(launch_k(reduce_kernel, dim3((unsigned)(grid_for(outer * inner))), dim3(256), 0, ctx->stream, kind, out, in, outer, dims[axis], inner));
+  LMB_CUDA(launch_k_opt(false, reduce_kernel, dim3((unsigned)(grid_for(outer * inner))), dim3(256), 0, ctx->stream, kind, out, in, outer, dims[axis], inner));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -585,7 +588,7 @@ extern "C" int32_t lmb200_matmul(lmb200_ctx h, float* out, const float* a, int32
       LMB_REQUIRE(a_dims[i] == b_dims[i], "Batch dimensions must match: %lld vs %lld", (long long)a_dims[i], (long long)b_dims[i]);
   LMB_REQUIRE(batch <= 65535, "matmul: batch %lld too large", (long long)batch);
   dim3 grid((unsigned)ceil_div(N, 32), (unsigned)ceil_div(M, 32), (unsigned)batch);
-  LMB_CUDA(launch_k(matmul_kernel, grid, dim3(kMatmulThreads), 0, ctx->stream, out, a, b, (int)M, (int)N, (int)K, M * K, b_rank > 2 ? K * N : 0, M * N));
+  LMB_CUDA(launch_k_opt(false, matmul_kernel, grid, dim3(kMatmulThreads), 0, ctx->stream, out, a, b, (int)M, (int)N, (int)K, M * K, b_rank > 2 ? K * N : 0, M * N));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -719,7 +722,7 @@ extern "C" int32_t lmb200_unfold1d(lmb200_ctx h, float* out, const float* in, in
 extern "C" int32_t lmb200_cumsum_last(lmb200_ctx h, float* out, const float* in, int64_t rows, int64_t n) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && in && rows >= 1 && n >= 1, "cumsum: bad argument");
-  LMB_CUDA(launch_k(cumsum_kernel, dim3((unsigned)(ceil_div(rows, 128))), dim3(128), 0, ctx->stream, out, in, rows, n));
+  LMB_CUDA(launch_k_opt(false, cumsum_kernel, dim3((unsigned)(ceil_div(rows, 128))), dim3(128), 0, ctx->stream, out, in, rows, n));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -728,7 +731,7 @@ extern "C" int32_t lmb200_rmsnorm_scale(lmb200_ctx h, float* y, const float* x, 
                                         int64_t n, float eps) {
   CTX_OR_FAIL();
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "rmsnorm: bad argument");
-  LMB_CUDA(launch_k(norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, nullptr, n, eps, 0));
+  LMB_CUDA(launch_k_opt(false, norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, nullptr, n, eps, 0));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -737,7 +740,7 @@ extern "C" int32_t lmb200_layernorm(lmb200_ctx h, float* y, const float* x, cons
                                     int64_t rows, int64_t n, float eps) {
   CTX_OR_FAIL();
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "layernorm: bad argument");
-  LMB_CUDA(launch_k(norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, bias, n, eps, 1));
+  LMB_CUDA(launch_k_opt(false, norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, bias, n, eps, 1));
   LAUNCHED();
   return LMB200_OK;
 }
@@ -762,7 +765,7 @@ extern "C" int32_t lmb200_rope(lmb200_ctx h, float* out, const float* x, int64_t
 extern "C" int32_t lmb200_argmax(lmb200_ctx h, int32_t* out, const float* x, int64_t rows, int64_t n) {
   CTX_OR_FAIL();
   LMB_REQUIRE(out && x && rows >= 1 && n >= 1, "argmax: bad argument");
-  LMB_CUDA(launch_k(argmax_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, out, x, n));
+  LMB_CUDA(launch_k_opt(false, argmax_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, out, x, n));
   LAUNCHED();
   return LMB200_OK;
 }
