@@ -132,7 +132,29 @@ flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const 
   if (warp >= 5) {
     // ------------------------------ loaders ------------------------------
     const int lw = warp - 5, lt = tid - 5 * 32;
-#pragma unroll 4
+    auto load_kv = [&](int j) {
+      const int s = j % kStages;
+      mbar_wait(&kv_empty[s], ((j / kStages) & 1) ^ 1, dead, err);
+      if (lane == 0) {
+        mbar_expect_tx(&kv_full[s], (uint32_t)(4 * SM::kKV));
+        unsigned char* st = smem + SM::offKV + s * 4 * SM::kKV;
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+#pragma unroll
+          for (int sub = 0; sub < D / W; ++sub) {
+            tma_load_4d(st + part * SM::kKV + sub * kSub, &kmap, sub * W, j * kBN, bh, part, &kv_full[s]);
+            tma_load_4d(st + (2 + part) * SM::kKV + sub * kSub, &vmap, sub * W, j * kBN, bh, part, &kv_full[s]);
+          }
+        }
+      }
+      __syncwarp();
+    };
+    // One CTA per SM: nothing else hides the start, so K and V are on their way while Q is split, and more of Q is in flight
+    // ([2, 16, 1531, 96] causal: 147 -> 143 us).  With two per SM the order makes no difference for the better (80.8, 82.3).
+    constexpr int kEarly = SM::kCtas == 1 ? kStages : 0, kUnroll = SM::kCtas == 1 ? 8 : 4;
+    if (lw == 0)
+      for (int j = 0; j < min(nt, kEarly); ++j) load_kv(j);
+#pragma unroll kUnroll
     for (int i = lt; i < kBM * (D / 8); i += kLoaders) {
       const int row = i / (D / 8), c8 = i - row * (D / 8), qi = q0 + row;
       float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
@@ -149,25 +171,8 @@ flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const 
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(&q_full);
-    if (lw == 0) {
-      for (int j = 0; j < nt; ++j) {
-        const int s = j % kStages;
-        mbar_wait(&kv_empty[s], ((j / kStages) & 1) ^ 1, dead, err);
-        if (lane == 0) {
-          mbar_expect_tx(&kv_full[s], (uint32_t)(4 * SM::kKV));
-          unsigned char* st = smem + SM::offKV + s * 4 * SM::kKV;
-#pragma unroll
-          for (int part = 0; part < 2; ++part) {
-#pragma unroll
-            for (int sub = 0; sub < D / W; ++sub) {
-              tma_load_4d(st + part * SM::kKV + sub * kSub, &kmap, sub * W, j * kBN, bh, part, &kv_full[s]);
-              tma_load_4d(st + (2 + part) * SM::kKV + sub * kSub, &vmap, sub * W, j * kBN, bh, part, &kv_full[s]);
-            }
-          }
-        }
-        __syncwarp();
-      }
-    }
+    if (lw == 0)
+      for (int j = kEarly; j < nt; ++j) load_kv(j);
   } else if (warp == 4) {
     // ------------------------------ MMA issue ------------------------------
     constexpr uint32_t kIdescS = idesc_bf16(kBM, kBN, false, false);
