@@ -94,7 +94,7 @@ __global__ void split_hi_lo_kernel(const float* __restrict__ k, const float* __r
 template <int D>
 __global__ void __launch_bounds__(kThreads, SmemF<D>::kCtas)
 flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const __grid_constant__ CUtensorMap kmap,
-                    const __grid_constant__ CUtensorMap vmap, int64_t BH, int S, float scale, int causal, int* err) {
+                    const __grid_constant__ CUtensorMap vmap, int S, float scale, int causal, int* err) {
   using namespace tc;
   typedef SmemF<D> SM;
   constexpr int W = D % 64 == 0 ? 64 : 32;
@@ -402,7 +402,7 @@ int32_t flash_tc_f32_launch(Ctx* ctx, float* out, const float* q, const float* k
   if (rc == LMB200_OK) {
     dim3 grid((unsigned)ceil_div(S, kBM), (unsigned)BH);
 #define LMB_FLASH(DD) \
-  flash_tc_f32_kernel<DD><<<grid, kThreads, SmemF<DD>::total + 1024, ctx->stream>>>(out, q, kmap, vmap, BH, (int)S, scale, causal, ctx->dev_err)
+  flash_tc_f32_kernel<DD><<<grid, kThreads, SmemF<DD>::total + 1024, ctx->stream>>>(out, q, kmap, vmap, (int)S, scale, causal, ctx->dev_err)
     if (D == 128) LMB_FLASH(128);
     else if (D == 96) LMB_FLASH(96);
     else if (D == 64) LMB_FLASH(64);
