@@ -741,7 +741,9 @@ int32_t gemm_launch_epi(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
   // The tile: waves x clocks of a tile.  A 64-k step costs what its operands take to arrive (64 bytes a clock and SM) or the MMA,
   // whichever is longer -- 512 clocks for a CTA pair's 256 x 256, 768 / 512 / 384 for 128 rows x 256 / 128 / 64 tokens -- and the last
   // tile's epilogue, which nothing overlaps, about 12 clocks a token.  Large products take CTA pairs; few tokens or few rows take the
-  // tile that still fills the SMs (128 rows x 2096 tokens, K 2048: 9 CTAs of 256 tokens took 124 us).
+  // tile that still fills the SMs (128 rows x 2096 tokens, K 2048: 9 CTAs of 256 tokens took 124 us).  Where rows that are no multiple of
+  // 256 leave 256 or 128 tokens, a step of 128 counts for the 528 clocks that it measures: two waves of 256 are faster than three of 128
+  // (two layers of 3200, feed-forward 8640, 1500 tokens: 1022 -> 909 us, 987 with 256 tokens always).
   // LMB200_GEMM_BN=64|128|256 and LMB200_GEMM_PAIR=0 force a choice for A/B runs.
   static const int forced_bn = [] { const char* e = getenv("LMB200_GEMM_BN"); return e ? atoi(e) : 0; }();
   static const bool pair_on = [] { const char* e = getenv("LMB200_GEMM_PAIR"); return !(e && atoi(e) == 0); }();
@@ -752,9 +754,10 @@ int32_t gemm_launch_epi(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
     const int64_t cost = ceil_div(tiles, resident) * steps * clocks + 12 * std::min(bn, 256);
     if (best < 0 || cost < best) { best = cost; BN = bn; }
   };
-  if (pair_on && !conv && p.rows % 256 == 0 && (!forced_bn || forced_bn == 256)) offer(512, 512, n_rg / 2 * seqs * ceil_div(n_own, 256), max_pairs);
+  const bool pairs_fit = pair_on && !conv && p.rows % 256 == 0;
+  if (pairs_fit && (!forced_bn || forced_bn == 256)) offer(512, 512, n_rg / 2 * seqs * ceil_div(n_own, 256), max_pairs);
   if (forced_bn == 0 || forced_bn == 256) offer(256, 768, n_rg * seqs * ceil_div(n_own, 256), ctx->sm_count);
-  if (forced_bn == 0 || forced_bn == 128) offer(128, 512, n_rg * seqs * ceil_div(n_own, 128), ctx->sm_count);
+  if (forced_bn == 0 || forced_bn == 128) offer(128, pairs_fit ? 512 : 528, n_rg * seqs * ceil_div(n_own, 128), ctx->sm_count);
   if (forced_bn == 0 || forced_bn == 64) offer(64, 384, n_rg * seqs * ceil_div(n_own, 64), ctx->sm_count);
   const bool pair = BN == 512;
   CUtensorMap xmap;
