@@ -744,8 +744,9 @@ int32_t gemm_launch_epi(Ctx* ctx, const GemmParams& p, cudaStream_t st) {
   // tile that still fills the SMs (128 rows x 2096 tokens, K 2048: 9 CTAs of 256 tokens took 124 us).  Where rows that are no multiple of
   // 256 leave 256 or 128 tokens, a step of 128 counts for the 528 clocks that it measures: two waves of 256 are faster than three of 128
   // (two layers of 3200, feed-forward 8640, 1500 tokens: 1022 -> 909 us, 987 with 256 tokens always).
-  // LMB200_GEMM_BN=64|128|256 and LMB200_GEMM_PAIR=0 force a choice for A/B runs.
-  static const int forced_bn = [] { const char* e = getenv("LMB200_GEMM_BN"); return e ? atoi(e) : 0; }();
+  // For A/B runs LMB200_GEMM_BN=64|128|256 forces the tokens per tile (256: in pairs or not, other values: no choice) and LMB200_GEMM_PAIR=0
+  // leaves out the pairs.
+  static const int forced_bn = [] { const char* e = getenv("LMB200_GEMM_BN"); const int n = e ? atoi(e) : 0; return n == 64 || n == 128 || n == 256 ? n : 0; }();
   static const bool pair_on = [] { const char* e = getenv("LMB200_GEMM_PAIR"); return !(e && atoi(e) == 0); }();
   const int64_t n_rg = ceil_div(p.rows, 128), steps = ceil_div(p.K, 64);
   int BN = 0;

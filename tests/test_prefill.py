@@ -149,3 +149,24 @@ def test_prompt_silu_far_below_zero(lib_built, device):
     got = sess.prefill(prompt)
     assert np.linalg.norm(got - ref) <= 4e-2 * np.linalg.norm(ref)
     sess.close(); model.close()
+
+
+def test_unknown_tile_width_is_no_choice(lib_built):
+    """LMB200_GEMM_BN takes 64, 128 and 256; any other value leaves the choice to the rule (read once per process, hence the child)."""
+    import subprocess
+    import sys
+    code = ("import luminal_jl_b200 as L, numpy as np\n"
+            "from luminal_jl_b200 import _lib\n"
+            "m = L.Model(L.get_device(), n_layers=1, hidden=256, n_heads=4, n_kv_heads=4, intermediate=256, vocab=64, eps=1e-5, rope_base=1e4, dtype='bf16')\n"
+            "m.init_random(seed=1, sigma=0.02)\n"
+            "s = L.Session(m, 1, 64)\n"
+            "print(repr(float(np.abs(s.prefill(np.arange(40, dtype=np.int32)[None])).sum())))\n")
+    got = {}
+    for bn in (None, "32", "128"):
+        env = {k: v for k, v in os.environ.items() if k != "LMB200_GEMM_BN"}
+        if bn:
+            env["LMB200_GEMM_BN"] = bn
+        r = subprocess.run([sys.executable, "-c", code], env=env, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-500:]
+        got[bn] = float(r.stdout.split()[-1])
+    assert got["32"] == got[None] and abs(got["128"] - got[None]) <= 1e-2 * got[None]
