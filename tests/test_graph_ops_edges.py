@@ -42,3 +42,14 @@ def test_f32_attention_head_dims(lib_built, device, heads, hidden):
     tok, log = L.greedy_generate(sess, prompt, 4, want_logits=True)
     assert np.abs(log - ref_log).max() <= LOGIT_TOL and np.array_equal(tok, ref_tok)
     sess.close(); model.close()
+
+
+@pytest.mark.parametrize("dims,perm", [((96, 100, 4000), (2, 1, 0)), ((96, 1000, 400), (2, 1, 0)), ((16, 1500, 1500), (1, 2, 0)), ((7, 33, 65), (2, 0, 1))])
+def test_permute_routes(lib_built, device, dims, perm):
+    """Either index width, around the rule on the distance between a warp's reads (1.6 MB, 1.6 MB, too few lanes, small)."""
+    a = torch.arange(int(np.prod(dims)), device="cuda", dtype=torch.int32).view(torch.float32).view(dims)        # bit patterns, all different
+    out = torch.empty([dims[p] for p in perm], device="cuda")
+    torch.cuda.synchronize()
+    _lib.call("lmb200_permute", device.handle, ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(a.data_ptr()), len(dims), _lib.dims(dims), (ctypes.c_int32 * len(dims))(*perm))
+    device.sync()
+    assert torch.equal(out.view(torch.int32), a.view(torch.int32).permute(perm))
