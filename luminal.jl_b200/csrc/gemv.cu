@@ -1501,8 +1501,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
 //   Clusters of 4: 33 of them fit a B200 (132 SMs, which stream at the same 7.1 TB/s as 148); of 8 only 15 fit, one short of the 16
 //   row groups of a 2048-wide model, and of 2 a narrow projection would leave half the chip idle.
 //   Measured (8 layers, per step, one launch per GEMV -> chained): Llama-3-8B shape at 1031 keys, batch 1 1044 -> 955 us, batch 32
-//   1252 -> 1143 us; Phi-3-mini batch 16 at 2052 keys 760 -> 693 us; Kevatar width 2048 batch 16 825 -> 734 us.  The Whisper decoder
-//   (512 wide, one unit per tile) got slower, 327 -> 350 us, and keeps its launches.
+//   1252 -> 1143 us; Phi-3-mini batch 16 at 2052 keys 760 -> 693 us; Kevatar width 2048 batch 16 825 -> 734 us.  gemv_chain_clusters has the rule.
+//   LayerNorms (sums of x beside those of squares) are not built in: the Whisper decoder, which needs them, was slower chained at width 512,
+//   327 -> 350 us a step, one unit of k per tile; larger Whispers have not been measured.
 //   warp 0 weights, 1 MMA, 2..5 epilogue, 6 activations.
 // =============================================================================================
 constexpr int kChainThreads = 7 * 32;
@@ -1585,9 +1586,9 @@ __device__ __forceinline__ void chain_resid_tile(const GemvParams& p, const Chai
   constexpr int BG = N / 8;
   const int lane = e & 31, we = e >> 5, bg = e & 3, rl = e >> 2, grow = row0 + rl;
   const bool valid = bg < BG && grow < p.rows;
-  float ssq[8], sxv[8];
+  float ssq[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) ssq[i] = sxv[i] = 0.f;
+  for (int i = 0; i < 8; ++i) ssq[i] = 0.f;
   if (valid) {
     float acc[8];
 #pragma unroll
@@ -1608,7 +1609,6 @@ __device__ __forceinline__ void chain_resid_tile(const GemvParams& p, const Chai
     for (int i = 0; i < 8; ++i) {
       o[8 * i] = __float2bfloat16_rn(xv[i] * h.gain);
       ssq[i] = xv[i] * xv[i];
-      sxv[i] = xv[i];
     }
     if (p.rn.capture) {
 #pragma unroll
@@ -1616,25 +1616,18 @@ __device__ __forceinline__ void chain_resid_tile(const GemvParams& p, const Chai
         if (8 * bg + i < p.B) p.rn.capture[(size_t)(8 * bg + i) * p.rows + grow] = xv[i];
     }
   }
-  auto fold = [&](float (&v)[8], float* out) {                 // over the tile's 32 rows, in a fixed order
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 4);
-      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 8);
-      v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
-    }
-    if (lane < 4) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s_red[we * 32 + 8 * lane + i] = v[i];
-    }
-    asm volatile("bar.sync 1, 128;\n" ::: "memory");
-    if (e < 32) out[(size_t)slot * 32 + e] = ((s_red[e] + s_red[32 + e]) + s_red[64 + e]) + s_red[96 + e];
-  };
-  fold(ssq, p.rn.ssq);
-  if (p.rn.sum) {
-    asm volatile("bar.sync 1, 128;\n" ::: "memory");           // s_red has been read
-    fold(sxv, p.rn.sum);
+  for (int i = 0; i < 8; ++i) {                                // over the tile's 32 rows, in a fixed order
+    ssq[i] += __shfl_xor_sync(0xffffffffu, ssq[i], 4);
+    ssq[i] += __shfl_xor_sync(0xffffffffu, ssq[i], 8);
+    ssq[i] += __shfl_xor_sync(0xffffffffu, ssq[i], 16);
   }
+  if (lane < 4) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_red[we * 32 + 8 * lane + i] = ssq[i];
+  }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  if (e < 32) p.rn.ssq[(size_t)slot * 32 + e] = ((s_red[e] + s_red[32 + e]) + s_red[64 + e]) + s_red[96 + e];
 }
 
 // EPI_POST_NORM for the 32 rows this CTA finalises; protocol, arithmetic and order as in post_norm_tile.  The op's CTAs (n of
@@ -2247,7 +2240,7 @@ int32_t GemvChain::flush() {
   ChainParams P;
   int most = 1;
   for (int i = 0; i < count; ++i) {
-    LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1, "gemv chain: op %d cannot run here", i);
+    LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1 && !op[i].rn.sum && !op[i].inv.sum, "gemv chain: op %d cannot run here", i);
     LMB_REQUIRE(op[i].epi != EPI_POST_NORM || ceil_div(op[i].rows, 128) <= std::min(clusters, kPushMaxCtas / kChainC),
                 "gemv chain: %d rows are more than one wave", op[i].rows);
     P.op[i] = op[i];
