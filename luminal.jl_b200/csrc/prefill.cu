@@ -78,6 +78,8 @@ struct GemmParams {
 };
 
 // GELU with the reference's tanh (src/HighLevelOps.jl:162-168): tanh z = sigmoid(2z) * 2 - 1
+// Divides in full precision, as the other epilogues' SiLU and sigmoid do: an approximate quotient is 2 ulp off, 0 where the divisor lies above 2^126,
+// and would save 13 % of a Whisper-base encoder (eight clips: 2.25 ms for 2.54).
 __device__ __forceinline__ float gelu_ref(float a) {
   const float inner = (0.7978845608f * a) * (1.0f + (0.044715f * a) * a);
   const float z = inner * 2.0f;
