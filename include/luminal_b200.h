@@ -84,7 +84,8 @@ int32_t lmb200_launch_count(lmb200_ctx ctx, int64_t* count);
  * keeps those buffers alive and unchanged in place); calls that copy to or from the host, allocate, free, wait, or
  * belong to a model or session are refused with an error and leave the device untouched.  capture_end returns the
  * instantiated graph, or an error if something recorded cannot be replayed; graph_launch enqueues one replay on the
- * context's stream. */
+ * context's stream.  Runs of small primitive steps are replayed as one kernel, which computes every step's output (the
+ * same bits) in an order that respects what each reads and writes, not necessarily the recorded one. */
 int32_t lmb200_capture_begin(lmb200_ctx ctx);
 int32_t lmb200_capture_end(lmb200_ctx ctx, uint64_t* graph_out);
 int32_t lmb200_graph_launch(lmb200_ctx ctx, uint64_t graph);

@@ -9,6 +9,7 @@
 #include <thread>
 
 #include "common.cuh"
+#include "recorded.cuh"
 #include "gemv.cuh"
 #include "model.cuh"
 #include "pdl.cuh"
@@ -340,6 +341,7 @@ extern "C" int32_t lmb200_shutdown(lmb200_ctx h) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   peer_teardown(c);
+  record_drop(c);
   if (c->nccl_comm && g_nccl.CommDestroy) g_nccl.CommDestroy(c->nccl_comm);
   cudaStreamDestroy(c->own_stream);
   cudaFreeHost(c->dev_err);
@@ -376,6 +378,7 @@ struct HostGraph {
   Ctx* ctx = nullptr;
   cudaGraphExec_t exec = nullptr;
   int64_t nodes = 0;                 // kernels one replay launches
+  std::vector<void*> programs;       // device memory its kernels read (record_finish)
 };
 HostGraph* graph_from(uint64_t h) {
   HostGraph* g = reinterpret_cast<HostGraph*>(h);
@@ -392,6 +395,7 @@ extern "C" int32_t lmb200_capture_begin(lmb200_ctx h) {
   LMB_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   c->capturing = true;
   c->capture_launches0 = c->launches;
+  record_begin(c);
   return LMB200_OK;
 }
 
@@ -407,16 +411,19 @@ extern "C" int32_t lmb200_capture_end(lmb200_ctx h, uint64_t* graph_out) {
   c->launches = c->capture_launches0;                      // recorded, not run
   if (e != cudaSuccess || !g) {
     cudaGetLastError();
+    record_drop(c);
     if (g) cudaGraphDestroy(g);
     return fail(LMB200_ECUDA, "capture_end: the recorded calls cannot be replayed (%s)", cudaGetErrorString(e));
   }
-  if (!graph_out) { cudaGraphDestroy(g); return fail(LMB200_EINVAL, "capture_end: null argument"); }
+  if (!graph_out) { cudaGraphDestroy(g); record_drop(c); return fail(LMB200_EINVAL, "capture_end: null argument"); }
   HostGraph* G = new HostGraph();
   G->ctx = c; G->nodes = nodes;
+  record_finish(c, &g, &G->programs, &G->nodes);
   const cudaError_t ei = cudaGraphInstantiate(&G->exec, g, 0);
   cudaGraphDestroy(g);
   if (ei != cudaSuccess) {
     cudaGetLastError();
+    for (void* p : G->programs) cudaFree(p);
     delete G;
     return fail(LMB200_ECUDA, "capture_end: cudaGraphInstantiate failed (%s)", cudaGetErrorString(ei));
   }
@@ -445,6 +452,7 @@ extern "C" int32_t lmb200_graph_destroy(lmb200_ctx h, uint64_t graph) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
   cudaGraphExecDestroy(G->exec);
+  for (void* p : G->programs) cudaFree(p);
   G->magic = 0;
   delete G;
   if (--c->live_graphs <= 0) {                 // nothing can replay a read of the retired scratch blocks any more

@@ -72,6 +72,7 @@ struct Ctx {
   // instead of run; calls that copy to or from the host, allocate, free or wait are refused meanwhile
   bool capturing = false;
   int64_t capture_launches0 = 0;
+  void* recorder = nullptr;        // the primitive steps of the open capture (recorded.cuh)
   bool scratch_in_graph = false;   // a recorded graph reads `scratch`: when it must grow, the old block is retired, not freed
   std::vector<void*> retired_scratch;   // blocks recorded graphs may still read; freed with the last graph or at shutdown
   int live_graphs = 0;

@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "pdl.cuh"
+#include "recorded.cuh"
 
 namespace lmb {
 namespace {
@@ -15,10 +16,8 @@ namespace {
 // CTAs work for a while -- products, reductions, scans, norms -- start in plain order: CTAs that become resident early pile up on the SMs that
 // were free first, and the kernel is as slow as the fullest of them (sums of 65536 rows of 1024: 274 us in plain order, 366 otherwise; scans 700 and
 // 1050).  Index arithmetic is 32-bit (I = uint32_t) wherever the element counts allow: a 64-bit division is a subroutine of about a hundred instructions.
-// The small Llama's 32-token graph (404 kernels), per call: 1431 -> 985 us with the
-// matmul below (1126 with all of them programmatic).
-constexpr int kMaxRank = 8;
-constexpr float kInvLn2 = 1.4426950408889634f;
+// The small Llama's 32-token graph as 404 kernels, per call: 1431 -> 985 us with the
+// matmul below (1126 with all of them programmatic); recorded graphs run such steps as one kernel (recorded.cu).
 constexpr float kHalfPi = 1.5707963267948966f;
 
 struct Idx {
@@ -26,27 +25,6 @@ struct Idx {
   int64_t out_d[kMaxRank];
   int64_t sa[kMaxRank], sb[kMaxRank], sc[kMaxRank];   // operand strides (0 = broadcast)
 };
-
-__device__ __forceinline__ float apply_op(int op, float a, float b, float c) {
-  switch (op) {
-    case LMB200_OP_ADD: return a + b;
-    case LMB200_OP_MUL: return a * b;
-    case LMB200_OP_MOD: return fmodf(a, b);
-    case LMB200_OP_LESSTHAN: return a < b ? 1.0f : 0.0f;
-    case LMB200_OP_MAX: return fmaxf(a, b);
-    case LMB200_OP_LOG2: return log2f(a);
-    case LMB200_OP_EXP2: return exp2f(a);
-    case LMB200_OP_SIN: return sinf(a);
-    case LMB200_OP_COS: return cosf(a);
-    case LMB200_OP_SQRT: return sqrtf(a);
-    case LMB200_OP_RECIP: return 1.0f / a;
-    case LMB200_OP_RELU: return fmaxf(a, 0.0f);
-    case LMB200_OP_COPY: return a;
-    case LMB200_OP_FUSED_MUL_ADD: return __fadd_rn(__fmul_rn(a, b), c);   // (a .* b) .+ c, two roundings
-    case LMB200_OP_FUSED_ADD_RELU: return fmaxf(a + b, 0.0f);
-  }
-  return 0.f;
-}
 
 template <typename I>
 __global__ void ew_kernel(int op, float* out, const float* a, const float* b, const float* c, Idx ix, int64_t total) {
@@ -68,9 +46,6 @@ __global__ void ew_kernel(int op, float* out, const float* a, const float* b, co
 // interpreted per output element with every operation rounded to float32 on its own (no
 // contraction), so the result equals running the group's nodes one by one.
 // Stands in for FusedElementwiseOp (src/Compiler.jl:323-357, executor src/Execution.jl:552-563).
-constexpr int kFusedMaxInputs = 8, kFusedMaxInstr = 64, kFusedMaxStack = 16;
-enum FusedOp { F_PUSH_IN = 0, F_PUSH_CONST = 1, F_ADD = 2, F_MUL = 3, F_MOD = 4, F_LT = 5, F_MAX = 6, F_LOG2 = 7, F_EXP2 = 8,
-               F_SIN = 9, F_COS = 10, F_SQRT = 11, F_RECIP = 12, F_RELU = 13, F_FMA = 14, F_ADD_RELU = 15 };
 struct FusedProgram {
   int n_in, n_instr, rank;
   int64_t out_d[kMaxRank];
@@ -107,31 +82,11 @@ __global__ void fused_ew_kernel(float* out, const FusedProgram pg, int64_t total
         continue;
       }
       if (op >= F_LOG2 && op <= F_RELU) {
-        const float a = stack[sp - 1];
-        float r = a;
-        switch (op) {
-          case F_LOG2: r = log2f(a); break;
-          case F_EXP2: r = exp2f(a); break;
-          case F_SIN: r = sinf(a); break;
-          case F_COS: r = cosf(a); break;
-          case F_SQRT: r = sqrtf(a); break;
-          case F_RECIP: r = 1.0f / a; break;
-          case F_RELU: r = fmaxf(a, 0.0f); break;
-        }
-        stack[sp - 1] = r;
+        stack[sp - 1] = fused_unary(op, stack[sp - 1]);
         continue;
       }
       const float b = stack[--sp], a = stack[sp - 1];
-      float r = 0.f;
-      switch (op) {
-        case F_ADD: r = __fadd_rn(a, b); break;
-        case F_MUL: r = __fmul_rn(a, b); break;
-        case F_MOD: r = fmodf(a, b); break;
-        case F_LT: r = a < b ? 1.0f : 0.0f; break;
-        case F_MAX: r = fmaxf(a, b); break;
-        case F_ADD_RELU: r = fmaxf(__fadd_rn(a, b), 0.0f); break;
-      }
-      stack[sp - 1] = r;
+      stack[sp - 1] = fused_binary(op, a, b);
     }
     out[o] = stack[0];
   }
@@ -374,10 +329,7 @@ __global__ void silu_gate_kernel(float* out, const float* gate, const float* up,
   pdl_launch_dependents();
   pdl_wait();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += (int64_t)gridDim.x * blockDim.x) {
-    const float a = gate[o];
-    const float e = exp2f((a * -1.0f) * kInvLn2);
-    const float sg = 1.0f / (1.0f + e);
-    out[o] = (a * sg) * up[o];
+    out[o] = silu_gate(gate[o], up[o]);
   }
 }
 
@@ -480,6 +432,28 @@ using namespace lmb;
   ctx->launches++;          \
   LMB_CUDA(cudaGetLastError())
 
+namespace {
+
+// between capture_begin and capture_end: what was just launched, for record_finish()
+RecordedStep step_of(StepKind kind, float* out, int rank, const int64_t* d, std::vector<StepView> in) {
+  RecordedStep s;
+  s.kind = kind; s.out = out; s.rank = rank; s.in = std::move(in);
+  for (int k = 0; k < rank; ++k) s.d[k] = d[k];
+  return s;
+}
+
+// a movement: per output axis the source axis + 1 (0: none), then per source axis where it starts
+RecordedStep movement(float* out, int rank, const int64_t* d, const StepView& in, const int* axis, const int64_t* start) {
+  RecordedStep s = step_of(STEP_COPY, out, rank, d, {in});
+  s.arg.assign(2 * kMaxRank, 0);
+  for (int k = 0; k < rank; ++k) s.arg[k] = axis[k];
+  if (start)
+    for (int k = 0; k < in.rank; ++k) s.arg[kMaxRank + k] = (int)start[k];
+  return s;
+}
+
+}  // namespace
+
 extern "C" int32_t lmb200_ew(lmb200_ctx h, int32_t opcode, float* out, int32_t out_rank, const int64_t* out_dims,
                              const float* a, int32_t a_rank, const int64_t* a_dims, const float* b, int32_t b_rank,
                              const int64_t* b_dims, const float* c, int32_t c_rank, const int64_t* c_dims) {
@@ -508,6 +482,13 @@ extern "C" int32_t lmb200_ew(lmb200_ctx h, int32_t opcode, float* out, int32_t o
   }
   LMB_CUDA(launch_k(fits32(total) ? ew_kernel<uint32_t> : ew_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, opcode, out, a, binary ? b : nullptr, ternary ? c : nullptr, ix, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    RecordedStep r = step_of(STEP_EW, out, out_rank, out_dims, {step_tensor(a, a_rank, a_dims)});
+    if (binary) r.in.push_back(step_tensor(b, b_rank, b_dims));
+    if (ternary) r.in.push_back(step_tensor(c, c_rank, c_dims));
+    r.op = opcode;
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -549,6 +530,14 @@ extern "C" int32_t lmb200_fused_ew(lmb200_ctx h, float* out, int32_t out_rank, c
   if (total == 0) return LMB200_OK;
   LMB_CUDA(launch_k(fits32(total) ? fused_ew_kernel<uint32_t> : fused_ew_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, pg, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    RecordedStep r = step_of(STEP_FUSED, out, out_rank, out_dims, {});
+    const int64_t* id = in_dims;
+    for (int i = 0; i < n_inputs; id += in_ranks[i], ++i) r.in.push_back(step_tensor(inputs[i], in_ranks[i], id));
+    r.arg.assign(ops, ops + n_instr);
+    r.val.assign(args, args + n_instr);
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -565,6 +554,15 @@ extern "C" int32_t lmb200_reduce(lmb200_ctx h, int32_t kind, float* out, const f
   for (int i = axis + 1; i < rank; ++i) inner *= dims[i];
   LMB_CUDA(launch_k_opt(false, reduce_kernel, dim3((unsigned)(grid_for(outer * inner))), dim3(256), 0, ctx->stream, kind, out, in, outer, dims[axis], inner));
   LAUNCHED();
+  if (ctx->recorder) {
+    int64_t od[kMaxRank];
+    int n = 0;
+    for (int i = 0; i < rank; ++i)
+      if (i != axis) od[n++] = dims[i];
+    RecordedStep r = step_of(STEP_REDUCE, out, n, od, {step_tensor(in, rank, dims)});
+    r.op = kind; r.n = dims[axis]; r.inner = inner;
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -590,6 +588,11 @@ extern "C" int32_t lmb200_matmul(lmb200_ctx h, float* out, const float* a, int32
   dim3 grid((unsigned)ceil_div(N, 32), (unsigned)ceil_div(M, 32), (unsigned)batch);
   LMB_CUDA(launch_k_opt(false, matmul_kernel, grid, dim3(kMatmulThreads), 0, ctx->stream, out, a, b, (int)M, (int)N, (int)K, M * K, b_rank > 2 ? K * N : 0, M * N));
   LAUNCHED();
+  if (ctx->recorder) {
+    int64_t od[kMaxRank];
+    for (int i = 0; i < a_rank; ++i) od[i] = i == a_rank - 1 ? N : a_dims[i];
+    record_step(ctx, step_of(STEP_MATMUL, out, a_rank, od, {step_tensor(a, a_rank, a_dims), step_tensor(b, b_rank, b_dims)}));
+  }
   return LMB200_OK;
 }
 
@@ -617,6 +620,11 @@ extern "C" int32_t lmb200_permute(lmb200_ctx h, float* out, const float* in, int
   const bool far = rank > 0 && total > (1 << 25) && gt.out_d[rank - 1] >= 32 && gt.st[rank - 1] * 4 > (1 << 20);
   LMB_CUDA(launch_k(fits32(total) && !far ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    int axis[kMaxRank];
+    for (int k = 0; k < rank; ++k) axis[k] = perm[k] + 1;
+    record_step(ctx, movement(out, rank, gt.out_d, step_tensor(in, rank, in_dims), axis, nullptr));
+  }
   return LMB200_OK;
 }
 
@@ -634,6 +642,9 @@ extern "C" int32_t lmb200_reshape_colmajor(lmb200_ctx h, float* out, const float
   for (int i = 0; i < out_rank; ++i) rs.out_d[i] = out_dims[i];
   LMB_CUDA(launch_k(fits32(to) ? reshape_cm_kernel<uint32_t> : reshape_cm_kernel<int64_t>, dim3((unsigned)(grid_for(to))), dim3(256), 0, ctx->stream, out, in, rs, to));
   LAUNCHED();
+  if (ctx->recorder) {
+    record_step(ctx, step_of(STEP_RESHAPE, out, out_rank, out_dims, {step_tensor(in, in_rank, in_dims)}));
+  }
   return LMB200_OK;
 }
 
@@ -656,6 +667,11 @@ extern "C" int32_t lmb200_expand(lmb200_ctx h, float* out, const float* in, int3
   const int64_t total = ti * size;
   LMB_CUDA(launch_k(fits32(total) ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    int source[kMaxRank];
+    for (int k = 0, j = 0; k < gt.rank; ++k) source[k] = k == axis ? 0 : ++j;
+    record_step(ctx, movement(out, gt.rank, gt.out_d, step_tensor(in, in_rank, in_dims), source, nullptr));
+  }
   return LMB200_OK;
 }
 
@@ -680,6 +696,12 @@ extern "C" int32_t lmb200_slice(lmb200_ctx h, float* out, const float* in, int32
   }
   LMB_CUDA(launch_k(fits32(total) ? strided_copy_kernel<uint32_t> : strided_copy_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, gt, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    int source[kMaxRank];
+    int64_t from[kMaxRank];
+    for (int k = 0; k < rank; ++k) { source[k] = k + 1; from[k] = starts[k] < 0 ? 0 : starts[k]; }
+    if (fits32(ti)) record_step(ctx, movement(out, rank, gt.out_d, step_tensor(in, rank, in_dims), source, from));
+  }
   return LMB200_OK;
 }
 
@@ -700,6 +722,11 @@ extern "C" int32_t lmb200_pad(lmb200_ctx h, float* out, const float* in, int32_t
   }
   LMB_CUDA(launch_k(fits32(total) ? pad_kernel<uint32_t> : pad_kernel<int64_t>, dim3((unsigned)(grid_for(total))), dim3(256), 0, ctx->stream, out, in, pd, total));
   LAUNCHED();
+  if (ctx->recorder) {
+    RecordedStep r = step_of(STEP_PAD, out, rank, pd.out_d, {step_tensor(in, rank, in_dims)});
+    for (int k = 0; k < rank; ++k) r.arg.push_back((int)left[k]);
+    if (fits32(total)) record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -709,6 +736,12 @@ extern "C" int32_t lmb200_gather(lmb200_ctx h, float* out, const float* table, i
   LMB_REQUIRE(out && table && ids && vocab >= 1 && dim >= 1 && n_ids >= 1, "gather: bad argument");
   LMB_CUDA(launch_k(gather_kernel, dim3((unsigned)(grid_for(n_ids * dim))), dim3(256), 0, ctx->stream, out, table, vocab, dim, ids, n_ids));
   LAUNCHED();
+  if (ctx->recorder) {
+    const int64_t od[2] = {n_ids, dim}, td[2] = {vocab, dim};
+    RecordedStep r = step_of(STEP_GATHER, out, 2, od, {step_tensor(table, 2, td), step_tensor(ids, 1, &n_ids)});
+    r.n = vocab; r.inner = dim;
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -728,6 +761,12 @@ extern "C" int32_t lmb200_cumsum_last(lmb200_ctx h, float* out, const float* in,
   LMB_REQUIRE(out && in && rows >= 1 && n >= 1, "cumsum: bad argument");
   LMB_CUDA(launch_k_opt(false, cumsum_kernel, dim3((unsigned)(ceil_div(rows, 128))), dim3(128), 0, ctx->stream, out, in, rows, n));
   LAUNCHED();
+  if (ctx->recorder) {
+    const int64_t od[2] = {rows, n};
+    RecordedStep r = step_of(STEP_CUMSUM, out, 2, od, {step_tensor(in, 2, od)});
+    r.n = n;
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -737,6 +776,13 @@ extern "C" int32_t lmb200_rmsnorm_scale(lmb200_ctx h, float* y, const float* x, 
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "rmsnorm: bad argument");
   LMB_CUDA(launch_k_opt(false, norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, nullptr, n, eps, 0));
   LAUNCHED();
+  if (ctx->recorder) {
+    const int64_t od[2] = {rows, n};
+    RecordedStep r = step_of(STEP_NORM, y, 2, od, {step_tensor(x, 2, od), step_tensor(w, 1, &n), step_tensor(nullptr, 1, &n)});
+    r.op = 0; r.n = n;
+    r.val = {eps};
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -746,6 +792,13 @@ extern "C" int32_t lmb200_layernorm(lmb200_ctx h, float* y, const float* x, cons
   LMB_REQUIRE(y && x && rows >= 1 && n >= 1, "layernorm: bad argument");
   LMB_CUDA(launch_k_opt(false, norm_kernel, dim3((unsigned)(rows)), dim3(256), 0, ctx->stream, y, x, w, bias, n, eps, 1));
   LAUNCHED();
+  if (ctx->recorder) {
+    const int64_t od[2] = {rows, n};
+    RecordedStep r = step_of(STEP_NORM, y, 2, od, {step_tensor(x, 2, od), step_tensor(w, 1, &n), step_tensor(bias, 1, &n)});
+    r.op = 1; r.n = n;
+    r.val = {eps};
+    record_step(ctx, std::move(r));
+  }
   return LMB200_OK;
 }
 
@@ -754,6 +807,9 @@ extern "C" int32_t lmb200_silu_gate(lmb200_ctx h, float* out, const float* gate,
   LMB_REQUIRE(out && gate && up && n >= 1, "silu_gate: bad argument");
   LMB_CUDA(launch_k(silu_gate_kernel, dim3((unsigned)(grid_for(n))), dim3(256), 0, ctx->stream, out, gate, up, n));
   LAUNCHED();
+  if (ctx->recorder) {
+    record_step(ctx, step_of(STEP_SILU, out, 1, &n, {step_tensor(gate, 1, &n), step_tensor(up, 1, &n)}));
+  }
   return LMB200_OK;
 }
 

@@ -1,0 +1,111 @@
+"""Replays of recorded graphs (runs of primitive steps as one kernel) against the same steps called one by one, bit for bit and in every buffer."""
+import numpy as np
+import pytest
+
+import luminal_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def every_buffer(cg):
+    return {nid: a.numpy() for nid, a in cg.results.items()}
+
+
+def same_bits(L, device, g, inputs, varied=(), **kw):
+    recorded, plain = L.compile(g, device, **kw), L.compile(g, device, capture=False, **kw)
+    for turn in range(3):                                          # step by step, then two replays on other values
+        for nid in varied:
+            inputs[nid] = np.roll(inputs[nid], turn)
+        recorded(inputs), plain(inputs)
+        a, b = every_buffer(recorded), every_buffer(plain)
+        keep = kw.get("outputs") or a
+        for nid in keep:
+            assert np.array_equal(a[nid].view(np.int32), b[nid].view(np.int32)), (turn, nid, type(g.nodes[nid - 1].op).__name__, a[nid].shape)
+    before = device.launch_count()
+    recorded(inputs)
+    launches = device.launch_count() - before
+    recorded.close()
+    return launches, recorded.kernel_count()
+
+
+@pytest.mark.parametrize("cfg,batch,tokens", [(dict(hidden=64, n_heads=4, n_kv_heads=2, intermediate=96), 2, 16), (dict(hidden=48, n_heads=3, n_kv_heads=3, intermediate=40), 1, 2),
+                                              (dict(hidden=256, n_heads=8, n_kv_heads=8, intermediate=688), 1, 33), (dict(hidden=512, n_heads=8, n_kv_heads=2, intermediate=1408), 3, 70)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_llama_graphs(lib_built, device, cfg, batch, tokens, shared):
+    L = lib_built
+    g, reg = L.Graph(), {}
+    net = L.nn.Llama(g, reg, vocab_size=300, n_layers=2, **cfg)
+    tok = L.tensor(g, [batch, tokens])
+    out = net(tok, 0)
+    inputs = {t.id: O.synth_normal(3, t.id, t.shape, 0.3) for t in reg.values()}
+    inputs[tok.id] = O.synth_tokens(5, 999, (batch, tokens), 300).astype(np.float32)
+    launches, steps = same_bits(L, device, g, inputs, [tok.id], **(dict(outputs=[out.id]) if shared else {}))
+    if not shared and cfg["hidden"] <= 256:
+        assert launches == 1 and steps > 100                       # small graphs are one kernel; with shared blocks their order may not allow it
+
+
+def random_graph(G, rng, steps):
+    """Movements on movements, broadcasts, reductions, products and element-wise steps on whatever is there."""
+    g = G.Graph()
+    pool = [G.tensor(g, [int(n) for n in rng.integers(1, 7, int(rng.integers(1, 5)))]) for _ in range(3)]
+    pool.append(G.tensor(g, [int(rng.integers(2, 40)), int(rng.integers(2, 40))]))
+    leaves = list(pool)
+    for _ in range(steps):
+        a = pool[-1 - int(rng.integers(min(4, len(pool))))] if rng.random() < 0.7 else pool[int(rng.integers(len(pool)))]
+        r, size = len(a.shape), int(np.prod(a.shape))
+        kind = int(rng.integers(11))
+        if kind == 0:
+            t = G.permute(a, [int(i) + 1 for i in rng.permutation(r)])
+        elif kind == 1:
+            d = [x for x in range(1, size + 1) if size % x == 0]
+            x = int(rng.choice(d))
+            y = int(rng.choice([z for z in range(1, size // x + 1) if (size // x) % z == 0]))
+            t = G.reshape(a, [x, y, size // x // y][:: int(rng.choice([1, -1]))])
+        elif kind == 2 and r < 6 and size < 4000:
+            t = G.expand(a, int(rng.integers(1, r + 2)), int(rng.integers(1, 5)))
+        elif kind == 3:
+            lo = [int(rng.integers(n)) for n in a.shape]
+            t = G.slice_(a, [(s, int(rng.integers(s + 1, n + 1))) for s, n in zip(lo, a.shape)])
+        elif kind == 4 and size < 4000:
+            t = G.pad(a, [(int(rng.integers(3)), int(rng.integers(3))) for _ in a.shape])
+        elif kind == 5 and r > 1:
+            t = (G.sum_ if rng.random() < 0.5 else G.max_reduce)(a, int(rng.integers(1, r + 1)))
+        elif kind == 6 and 2 <= r <= 4:
+            m = G.permute(a, list(range(1, r - 1)) + [r, r - 1])
+            t = G.matmul(a, m) * np.float32(0.05) if rng.random() < 0.5 else G.matmul(m, a) * np.float32(0.05)
+        elif kind == 7:
+            t = G.cumsum_last_dim(a) * np.float32(0.25)
+        elif kind == 8:
+            t = a * np.float32(0.5) + G.permute(G.permute(a, list(range(r, 0, -1))), list(range(r, 0, -1)))
+        elif kind == 9:
+            t = G.sin(a) if rng.random() < 0.5 else G.relu(a) + np.float32(0.125)
+        else:
+            t = G.std_norm(a, r) if size > 1 else G.exp2(a * np.float32(0.01))
+        pool.append(t)
+    return g, leaves
+
+
+@pytest.mark.parametrize("seed", range(24))
+@pytest.mark.parametrize("fuse", [True, False])
+def test_random_graphs(lib_built, device, seed, fuse):
+    rng = np.random.default_rng(seed)
+    g, leaves = random_graph(lib_built.graph, rng, 40)
+    inputs = {t.id: rng.standard_normal(t.shape).astype(np.float32) for t in leaves}
+    same_bits(lib_built, device, g, inputs, [t.id for t in leaves], fuse=fuse)
+
+
+def test_large_steps_stay_kernels(lib_built, device):
+    """Element-wise steps and products beyond the rule's sizes between small ones, and values the products' order must carry: infinities and NaN."""
+    G = lib_built.graph
+    rng = np.random.default_rng(1)
+    g = G.Graph()
+    a, w = G.tensor(g, [700, 800]), G.tensor(g, [900, 800])
+    small = G.sum_(G.exp2(G.permute(a, [2, 1]) * np.float32(0.1)), 2)
+    big = G.matmul(G.relu(a) + np.float32(1.0), G.permute(w, [2, 1]))
+    out = G.sum_(big * np.float32(0.01), 1) + G.sum_(G.permute(w, [2, 1]), 1)
+    tail = G.permute(G.expand(out, 1, 3), [2, 1]) * np.float32(2.0)
+    tail = G.max_reduce(tail + G.reshape(G.sum_(small, 1) * np.float32(0.0) + np.float32(1.0), [1]), 1)
+    x = rng.standard_normal((700, 800)).astype(np.float32)
+    x[3, 5], x[7, 9], x[11, 2] = np.inf, -np.inf, np.nan
+    launches, steps = same_bits(lib_built, device, g, {a.id: x, w.id: rng.standard_normal((900, 800)).astype(np.float32)}, [w.id])
+    assert launches < steps
