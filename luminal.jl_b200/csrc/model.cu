@@ -8,6 +8,7 @@
 
 #include "model.cuh"
 #include "pdl.cuh"
+#include "whisper_step.cuh"
 
 namespace lmb {
 
@@ -1696,6 +1697,26 @@ int32_t whisper_fold(Model* M) {
   return LMB200_OK;
 }
 
+// The layers' table of the two-launch Whisper step, on the device (outside of any capture).
+int32_t whisper_step_table(Session* S) {
+  Model* M = S->m;
+  const int L = M->cfg.n_layers;
+  WhisperStepLayer table[kWhisperStepLayers] = {};
+  for (int l = 0; l < L; ++l) {
+    const LayerWeights& W = M->layers[l];
+    const auto w = [](const void* m) { return reinterpret_cast<const __nv_bfloat16*>(m); };
+    WhisperStepLayer& y = table[l];
+    y.wqkv = w(W.wqkv); y.wo = w(W.wo); y.wqc = w(W.wq_cross); y.woc = w(W.wo_cross); y.wfc1 = w(W.wgu); y.wfc2 = w(W.wdown);
+    y.wg_qkv = W.wg_qkv; y.bf_qkv = W.bf_qkv; y.b_o = W.b_o; y.gain_cross = W.cross_norm;
+    y.wg_qc = W.wg_qc; y.bf_qc = W.bf_qc; y.b_oc = W.b_o_cross; y.gain_ffn = W.ffn_norm;
+    y.wg_fc1 = W.wg_fc1; y.bf_fc1 = W.bf_fc1; y.b_fc2 = W.b_fc2; y.gain_next = l + 1 < L ? M->layers[l + 1].attn_norm : M->final_norm;
+    y.kv = reinterpret_cast<__nv_bfloat16*>(S->kv) + (int64_t)l * S->kv_layer_stride;
+    y.cross = reinterpret_cast<const __nv_bfloat16*>(S->cross_kv) + (int64_t)l * S->cross_layer_stride;
+    y.capture = S->capture_on ? S->capture + (int64_t)l * S->B * M->cfg.hidden : nullptr;
+  }
+  return whisper_step_layers(table, L, S->whisper_step, M->ctx->stream);
+}
+
 // The fused decode step of the bf16 Whisper decoder: eight launches per layer instead of eleven.  As in the Llama
 // step the residual add and the norm around every Linear ride on the projections: out_proj (self and cross) and fc2
 // finish with EPI_RESID_NORM (their own bias added on the way), which leaves x * gain and the per-sequence sums of x
@@ -1708,6 +1729,26 @@ int32_t enqueue_whisper_step_fused(Session* S, cudaStream_t st, bool with_head) 
   const int dt = c.dtype;
   const int B = S->B, hid = c.hidden, L = c.n_layers;
   const float qk_scale = powf((float)hid / (float)c.n_heads, -0.25f);
+  if (S->whisper_step) {                                   // two launches, or the layers' and the position's where there is no head
+    WhisperStepParams p;
+    p.n_layers = L; p.B = B; p.Bp = S->Bp; p.H = M->Hl; p.hidden = hid; p.ffn = c.intermediate; p.vocab = c.vocab; p.q_pitch = S->q_pitch;
+    p.cross_len = c.cross_len; p.eps = c.rms_eps; p.qk_scale = qk_scale;
+    p.kv_b = S->kv_batch_stride; p.kv_h = S->kv_head_stride; p.cross_b = S->cross_batch_stride; p.cross_h = S->cross_head_stride;
+    p.tokens = S->tokens; p.pos = S->pos; p.embed = reinterpret_cast<const __nv_bfloat16*>(M->embed); p.pos_emb = M->pos_emb;
+    p.gain_first = M->layers[0].attn_norm;
+    p.x = S->xT; p.ssq = S->ssq; p.sum = S->sum_slots;
+    p.xn = reinterpret_cast<__nv_bfloat16*>(S->xn); p.q = reinterpret_cast<__nv_bfloat16*>(S->qbuf);
+    p.attn = reinterpret_cast<__nv_bfloat16*>(S->attn_out); p.act = reinterpret_cast<__nv_bfloat16*>(S->act);
+    p.with_head = with_head;
+    p.head = reinterpret_cast<const __nv_bfloat16*>(M->embed_tiled); p.wg_head = M->wg_head; p.bf_head = M->bf_head;
+    p.logits = S->logits; p.logits_pitch = S->logits_pitch;
+    p.hist = S->tok_hist; p.step_ctr = S->step_ctr; p.stop = S->stop; p.limit = S->limit;
+    LMB_TRY(whisper_step_launch(ctx, p, S->whisper_step, st));
+    if (with_head) return LMB200_OK;
+    LMB_CUDA(launch_k(advance_kernel, dim3(1), dim3(32), 0, st, S->pos, (const int*)S->limit, S->B, S->step_ctr, (unsigned long long*)nullptr));
+    ctx->launches++;
+    return LMB200_OK;
+  }
   {
     const int rows_per = S->embed_rows_per_cta;
     const int grid = (int)ceil_div(hid, rows_per);
@@ -1867,6 +1908,7 @@ int32_t ensure_graphs(Session* S) {
   Ctx* ctx = S->m->ctx;
   if (S->graph_full && S->graph_stream == ctx->stream) return LMB200_OK;
   drop_graphs(S);
+  if (S->whisper_step) LMB_TRY(whisper_step_table(S));
   LMB_TRY(capture_one(S, ctx->stream, 1, &S->graph_full, &S->graph_nodes_full));
   LMB_TRY(capture_one(S, ctx->stream, 0, &S->graph_body, &S->graph_nodes_body));
   if (S->head_sliced) LMB_TRY(capture_one(S, ctx->stream, 2, &S->graph_tok, &S->graph_nodes_tok));
@@ -2049,6 +2091,8 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
     alloc((void**)&S->ssq, (int64_t)kSsqSlots * 32 * 4);
     if (S->chain_clusters) alloc((void**)&S->chain_done, gemv_chain_scratch_bytes());
     if (whisper) alloc((void**)&S->sum_slots, (int64_t)kSsqSlots * 32 * 4);
+    if (whisper && c.tp_size == 1 && whisper_step_fits(batch, M->D, M->Hl, M->KVl, c.hidden, c.intermediate, c.n_layers))
+      alloc(&S->whisper_step, whisper_step_scratch_bytes(batch, M->Hl, c.n_layers, ctx->sm_count));
   }
   if (S->head_sliced) alloc((void**)&S->logits_slice, (int64_t)batch * S->head_pitch * 4);
   S->host_pos_v.assign(batch, 0);
@@ -2076,7 +2120,7 @@ extern "C" int32_t lmb200_session_destroy(lmb200_session h) {
   cudaFree(S->attn_out); cudaFree(S->act); cudaFree(S->tokens); cudaFree(S->pos); cudaFree(S->limit); cudaFree(S->step_ctr); cudaFree(S->ragged_logits);
   cudaFree(S->tok_hist); cudaFree(S->prompt); cudaFree(S->gemv_partials); cudaFree(S->gemv_counters); cudaFree(S->chain_done);
   cudaFree(S->part_o); cudaFree(S->part_ml); cudaFree(S->attn_counters); cudaFree(S->prefill_buf); cudaFree(S->capture);
-  cudaFree(S->xT); cudaFree(S->ssq); cudaFree(S->sum_slots); cudaFree(S->logits_slice); cudaFree(S->stop);
+  cudaFree(S->xT); cudaFree(S->ssq); cudaFree(S->sum_slots); cudaFree(S->whisper_step); cudaFree(S->logits_slice); cudaFree(S->stop);
   S->magic = 0;
   delete S;
   return LMB200_OK;
