@@ -8,6 +8,7 @@
 
 #include "model.cuh"
 #include "pdl.cuh"
+#include "llama_step.cuh"
 #include "whisper_step.cuh"
 
 namespace lmb {
@@ -1422,6 +1423,33 @@ int32_t enqueue_step_t(Session* S, cudaStream_t st, bool with_head) {
   return LMB200_OK;
 }
 
+// The small float32 Llama's step as one launch (llama_step.cuh), and its layers' table (outside of any capture).
+int32_t enqueue_llama_step(Session* S, cudaStream_t st, bool with_head) {
+  Model* M = S->m;
+  const lmb200_model_config& c = M->cfg;
+  const auto f = [](void* p) { return reinterpret_cast<float*>(p); };
+  LlamaStepParams p;
+  p.n_layers = c.n_layers; p.B = S->B; p.Hl = M->Hl; p.KVl = M->KVl; p.G = M->G; p.hidden = c.hidden; p.ffn = c.intermediate; p.vocab = c.vocab;
+  p.logits_pitch = S->logits_pitch; p.with_head = with_head; p.eps = c.rms_eps; p.scale = 1.0f / sqrtf((float)M->D);
+  p.kv_b = S->kv_batch_stride; p.kv_h = S->kv_head_stride;
+  p.tokens = S->tokens; p.pos = S->pos; p.hist = S->tok_hist; p.step_ctr = S->step_ctr; p.stop = S->stop; p.limit = S->limit;
+  p.embed = f(M->embed); p.gain_final = M->final_norm; p.head = f(M->lm_head); p.inv_freq = M->inv_freq;
+  p.x = S->x; p.q = f(S->qbuf); p.attn = f(S->attn_out); p.act = f(S->act); p.logits = S->logits;
+  return llama_step_launch(M->ctx, p, M->D, S->llama_step, st);
+}
+
+int32_t llama_step_table(Session* S) {
+  Model* M = S->m;
+  std::vector<LlamaStepLayer> table(M->cfg.n_layers);
+  for (int l = 0; l < M->cfg.n_layers; ++l) {
+    const LayerWeights& W = M->layers[l];
+    const auto f = [](void* p) { return reinterpret_cast<float*>(p); };
+    table[l] = {f(W.wqkv), f(W.wo), f(W.wgu), f(W.wdown), W.attn_norm, W.ffn_norm, f(S->kv) + (int64_t)l * S->kv_layer_stride,
+                S->capture_on ? S->capture + (int64_t)l * S->B * M->cfg.hidden : nullptr};
+  }
+  return llama_step_layers(table.data(), M->cfg.n_layers, S->llama_step, M->ctx->stream);
+}
+
 // Exchange parameters of the projection that carries reduction `index` of the step (2l: o_proj, 2l + 1:
 // down_proj) when it runs EPI_RESID_NORM under tensor parallelism.
 PeerPush peer_push(Session* S, int index) {
@@ -1850,6 +1878,7 @@ int32_t enqueue_step(Session* S, cudaStream_t st, int head) {
   if (S->m->cfg.arch == LMB200_ARCH_LAYERED) return layered_enqueue_step(S, st, with_head);
   if (S->fused && S->m->cfg.arch == LMB200_ARCH_WHISPER_DECODER) return enqueue_whisper_step_fused(S, st, with_head);
   if (S->fused) return enqueue_step_fused(S, st, head);
+  if (S->llama_step) return enqueue_llama_step(S, st, with_head);
   if (S->m->cfg.arch == LMB200_ARCH_WHISPER_DECODER)
     return S->m->cfg.dtype == LMB200_BF16 ? enqueue_whisper_step_t<__nv_bfloat16>(S, st, with_head)
                                           : enqueue_whisper_step_t<float>(S, st, with_head);
@@ -1909,6 +1938,7 @@ int32_t ensure_graphs(Session* S) {
   if (S->graph_full && S->graph_stream == ctx->stream) return LMB200_OK;
   drop_graphs(S);
   if (S->whisper_step) LMB_TRY(whisper_step_table(S));
+  if (S->llama_step) LMB_TRY(llama_step_table(S));
   LMB_TRY(capture_one(S, ctx->stream, 1, &S->graph_full, &S->graph_nodes_full));
   LMB_TRY(capture_one(S, ctx->stream, 0, &S->graph_body, &S->graph_nodes_body));
   if (S->head_sliced) LMB_TRY(capture_one(S, ctx->stream, 2, &S->graph_tok, &S->graph_nodes_tok));
@@ -2094,6 +2124,12 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
     if (whisper && c.tp_size == 1 && whisper_step_fits(batch, M->D, M->Hl, M->KVl, c.hidden, c.intermediate, c.n_layers))
       alloc(&S->whisper_step, whisper_step_scratch_bytes(batch, M->Hl, c.n_layers, ctx->sm_count));
   }
+  {
+    const char* fe = getenv("LMB200_FUSED_STEP");
+    if (!(fe && atoi(fe) == 0) && c.dtype == LMB200_F32 && !whisper && c.tp_size == 1 && ctx->peer_n <= 1 &&
+        llama_step_fits(batch, M->D, c.hidden, c.intermediate, c.vocab, c.n_layers, S->cap))
+      alloc(&S->llama_step, llama_step_scratch_bytes(c.n_layers, ctx->sm_count));
+  }
   if (S->head_sliced) alloc((void**)&S->logits_slice, (int64_t)batch * S->head_pitch * 4);
   S->host_pos_v.assign(batch, 0);
   if (rc == LMB200_OK) rc = set_limits(S, nullptr);
@@ -2120,7 +2156,7 @@ extern "C" int32_t lmb200_session_destroy(lmb200_session h) {
   cudaFree(S->attn_out); cudaFree(S->act); cudaFree(S->tokens); cudaFree(S->pos); cudaFree(S->limit); cudaFree(S->step_ctr); cudaFree(S->ragged_logits);
   cudaFree(S->tok_hist); cudaFree(S->prompt); cudaFree(S->gemv_partials); cudaFree(S->gemv_counters); cudaFree(S->chain_done);
   cudaFree(S->part_o); cudaFree(S->part_ml); cudaFree(S->attn_counters); cudaFree(S->prefill_buf); cudaFree(S->capture);
-  cudaFree(S->xT); cudaFree(S->ssq); cudaFree(S->sum_slots); cudaFree(S->whisper_step); cudaFree(S->logits_slice); cudaFree(S->stop);
+  cudaFree(S->xT); cudaFree(S->ssq); cudaFree(S->sum_slots); cudaFree(S->whisper_step); cudaFree(S->llama_step); cudaFree(S->logits_slice); cudaFree(S->stop);
   S->magic = 0;
   delete S;
   return LMB200_OK;

@@ -169,6 +169,7 @@ struct Session {
   unsigned* attn_counters = nullptr;   // [B*KVl], zero between launches
   float* sum_slots = nullptr;          // fused Whisper step: per-CTA sums of x beside ssq (LayerNorm's mean)
   void* whisper_step = nullptr;        // its scratch: the step runs as two launches (whisper_step.cuh)
+  void* llama_step = nullptr;          // its scratch: the small float32 step runs as one launch (llama_step.cuh)
   void* prefill_buf = nullptr;         // scratch of the GEMM prompt phase, kept between prompts
   int64_t prefill_bytes = 0;
   int keys_per_cta = 0, nsplit = 0;
