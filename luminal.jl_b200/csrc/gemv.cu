@@ -1946,14 +1946,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
             }
           }
         }
+        const bool last = r + ncl >= nrbg && o + 1 < P.n_ops;
+        if (last) asm volatile("fence.proxy.async;\n" ::: "memory");
         asm volatile("bar.sync 1, 128;\n" ::: "memory");         // the receive buffer has been read
-        if (e < kChainC) mbar_arrive_remote(dsmem_addr(smem_u32(&send_ok), (uint32_t)e));
-      }
-      if (o + 1 < P.n_ops) {
         // the barrier puts every thread's stores before thread 0's release, which covers them
-        asm volatile("fence.proxy.async;\n" ::: "memory");
-        asm volatile("bar.sync 1, 128;\n" ::: "memory");
-        if (e == 0) asm volatile("fence.acq_rel.gpu;\nred.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
+        if (last && e == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
+        if (e < kChainC) mbar_arrive_remote(dsmem_addr(smem_u32(&send_ok), (uint32_t)e));
       }
     }
   }
