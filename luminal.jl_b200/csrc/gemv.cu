@@ -1509,11 +1509,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
 constexpr int kChainThreads = 7 * 32;
 constexpr int kChainLine = 32;               // counters are a 128-byte line apart
 
+template <int M>
 struct ChainParams {
-  GemvParams op[kChainMax];
+  GemvParams op[M];
   int n_ops = 0;
-  unsigned* done = nullptr;                  // [kChainMax + 1] lines, zero between launches; the last one counts exits
+  unsigned* done = nullptr;                  // [kChainMaxAttend + 1] lines, zero between launches; the last one counts exits
 };
+// D > 0: the kernel with attention at that head dimension
+template <int D> using ChainParamsOf = ChainParams<(D > 0 ? kChainMaxAttend : kChainMax)>;
 
 template <int N> constexpr int kChainStages = N == 16 ? 6 : 5;
 template <int N> constexpr size_t chain_smem() { return (size_t)kChainStages<N> * (kWStage + N * 256) + 128 * N * 4 + 1024; }
@@ -1544,9 +1547,10 @@ __device__ __forceinline__ void mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
   }
 }
-// the CTAs that take part in op o
-__device__ __forceinline__ unsigned chain_ctas(const ChainParams& P, int o, int ncl) {
-  return (unsigned)(min(ncl, (P.op[o].rows + 127) >> 7) * kChainC);
+// the CTAs that take part in a link
+__device__ __forceinline__ unsigned chain_ctas(const GemvParams& p, int ncl) {
+  if (p.epi == EPI_ATTEND) return (unsigned)min(ncl * kChainC, p.B * p.KVl * p.ksplit);
+  return (unsigned)(min(ncl, (p.rows + 127) >> 7) * kChainC);
 }
 __device__ __forceinline__ void chain_wait_done(const unsigned* done, unsigned want, bool& dead, int* err) {
   if (dead) return;
@@ -1554,6 +1558,21 @@ __device__ __forceinline__ void chain_wait_done(const unsigned* done, unsigned w
   for (;;) {
     unsigned seen;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(done) : "memory");
+    if (seen >= want) return;
+    if (clock64() - t0 > kWaitLimit) {
+      dead = true;
+      if (err) atomicExch(err, 1);
+      return;
+    }
+  }
+}
+
+__device__ __forceinline__ void chain_wait_shared(const unsigned* count, unsigned want, bool& dead, int* err) {
+  if (dead) return;
+  const long long t0 = clock64();
+  for (;;) {
+    unsigned seen;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];\n" : "=r"(seen) : "r"(smem_u32(count)) : "memory");
     if (seen >= want) return;
     if (clock64() - t0 > kWaitLimit) {
       dead = true;
@@ -1740,8 +1759,165 @@ __device__ __forceinline__ void chain_post_tile(const GemvParams& p, const Chain
   if (p.pn.ssq) publish(p.pn.ssq, false);
 }
 
-template <int N, bool X>
-__global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __grid_constant__ ChainParams P, int* err) {
+// Decode attention as a link (EPI_ATTEND; the launched kernel's arithmetic, attention.cu).  A unit is one of `ksplit` parts of one sequence's key head;
+// CTA i takes units i, i + grid, ...  Keys and values come through the weights' ring, 64 keys (four blocks of the tiled cache) a stage: all but a sequence's
+// newest are in the cache since earlier steps, so the producer fetches them while the projections before still run, and only the stage with the newest
+// key waits for q/k/v.  Each epilogue warp takes one block of 16 keys of a stage.
+struct ChainUnit { int bk, b, kvl, T, part, parts, begin, end; };      // keys begin .. end - 1; begin >= end: nothing
+__device__ __forceinline__ ChainUnit chain_unit(const GemvParams& p, int u) {
+  ChainUnit w;
+  const int pairs = p.B * p.KVl;
+  w.part = u / pairs;
+  w.bk = u - w.part * pairs;
+  w.b = w.bk / p.KVl;
+  w.kvl = w.bk - w.b * p.KVl;
+  w.T = p.pos[w.b] + 1;
+  const int even = (((w.T + p.ksplit - 1) / p.ksplit + 63) >> 6) << 6, per = even < p.kc_per_split ? even : p.kc_per_split;
+  w.parts = (w.T + per - 1) / per;
+  w.begin = w.part * per;
+  w.end = min(w.T, w.begin + per);
+  return w;
+}
+// stages of a link's units that fall to this CTA
+__device__ __forceinline__ int chain_attend_stages(const GemvParams& p) {
+  int n = 0;
+  for (int u = blockIdx.x; u < p.B * p.KVl * p.ksplit; u += gridDim.x) {
+    const ChainUnit w = chain_unit(p, u);
+    n += max(0, (w.end - w.begin + 63) >> 6);
+  }
+  return n;
+}
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(d) : "r"(a));
+  return d;
+}
+
+// One unit, by the 128 epilogue threads.  it: the ring's place, which it moves on.  scratch: 128 N floats, of which a warp's heads take G D.
+template <int D, int N, int ST>
+__device__ __forceinline__ void chain_attend(const GemvParams& p, const ChainUnit& u, int& it, const unsigned char* ring, uint64_t* full_bar, uint64_t* empty_bar,
+                                             float* scratch, float* s_ml, int e, bool& dead, int* err) {
+  constexpr int DK = D / 16, kStage = kWStage + N * 256;
+  const int lane = e & 31, warp = e >> 5, g = lane >> 2, t = lane & 3, G = p.Hl / p.KVl;
+  const float c = p.qk_scale * kInvLn2;
+  uint32_t qf[DK][2];
+  {
+    const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q_out) + (int64_t)u.b * p.q_pitch + (u.kvl * G + g) * D;
+#pragma unroll
+    for (int k = 0; k < DK; ++k) {
+      qf[k][0] = g < G ? *reinterpret_cast<const uint32_t*>(q + 16 * k + 2 * t) : 0u;
+      qf[k][1] = g < G ? *reinterpret_cast<const uint32_t*>(q + 16 * k + 2 * t + 8) : 0u;
+    }
+  }
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f, o[DK][4];
+#pragma unroll
+  for (int k = 0; k < DK; ++k) o[k][0] = o[k][1] = o[k][2] = o[k][3] = 0.f;
+  for (int key = u.begin; key < u.end; key += 64, ++it) {
+    const int s = it % ST;
+    mbar_wait(&full_bar[s], (it / ST) & 1, dead, err);
+    const int key0 = key + 16 * warp;
+    if (key0 < u.end) {
+      const uint4* blk = reinterpret_cast<const uint4*>(ring + (size_t)s * kStage) + warp * (4 * D) + lane;
+      float sc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < DK; ++k) mma_bf16_16816(sc, blk[32 * k], qf[k][0], qf[k][1]);
+      if (key0 + g >= u.end) sc[0] = sc[1] = -INFINITY;
+      if (key0 + g + 8 >= u.end) sc[2] = sc[3] = -INFINITY;
+      float b0 = fmaxf(sc[0], sc[2]), b1 = fmaxf(sc[1], sc[3]);
+#pragma unroll
+      for (int off = 4; off < 32; off <<= 1) {
+        b0 = fmaxf(b0, __shfl_xor_sync(0xffffffffu, b0, off));
+        b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, off));
+      }
+      const float n0 = fmaxf(m0, b0), n1 = fmaxf(m1, b1);
+      const float a0 = exp2f((m0 - n0) * c), a1 = exp2f((m1 - n1) * c);
+      const float p00 = exp2f((sc[0] - n0) * c), p01 = exp2f((sc[1] - n1) * c), p10 = exp2f((sc[2] - n0) * c), p11 = exp2f((sc[3] - n1) * c);
+      l0 = l0 * a0 + (p00 + p10);
+      l1 = l1 * a1 + (p01 + p11);
+      m0 = n0;
+      m1 = n1;
+      const uint32_t pb0 = movmatrix_trans(pack_bf16x2(p00, p01)), pb1 = movmatrix_trans(pack_bf16x2(p10, p11));
+#pragma unroll
+      for (int k = 0; k < DK; ++k) {
+        o[k][0] *= a0; o[k][1] *= a1; o[k][2] *= a0; o[k][3] *= a1;
+        mma_bf16_16816(o[k], blk[32 * (DK + k)], pb0, pb1);
+      }
+    }
+    asm volatile("bar.sync 1, 128;\n" ::: "memory");             // the stage has been read
+    if (e == 0) mbar_arrive(&empty_bar[s]);
+  }
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, off);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (2 * t + h < G) {
+      float* so = scratch + (warp * G + 2 * t + h) * D;
+#pragma unroll
+      for (int k = 0; k < DK; ++k) { so[16 * k + g] = o[k][h]; so[16 * k + g + 8] = o[k][2 + h]; }
+      if (g == 0) { s_ml[warp * 8 + 2 * t + h] = h ? m1 : m0; s_ml[32 + warp * 8 + 2 * t + h] = h ? l1 : l0; }
+    }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.act);
+  const int64_t slot0 = (int64_t)u.bk * p.ksplit, slot = slot0 + u.part;
+  for (int i = e; i < G * D; i += 128) {
+    const int h = i / D, d = i - h * D;
+    float M = s_ml[h], acc = 0.f, sum = 0.f;
+#pragma unroll
+    for (int w = 1; w < 4; ++w) M = fmaxf(M, s_ml[w * 8 + h]);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float f = exp2f((s_ml[w * 8 + h] - M) * c);
+      acc += f * scratch[(w * G + h) * D + d];
+      sum += f * s_ml[32 + w * 8 + h];
+    }
+    if (u.parts == 1) {
+      out[xcanon_offset(u.b, (u.kvl * G + h) * D + d, N)] = __float2bfloat16_rn(acc * (1.0f / sum));
+    } else {
+      p.partials[(slot * G + h) * D + d] = acc;
+      if (d == 0) { p.out[(slot * G + h) * 2] = M * c; p.out[(slot * G + h) * 2 + 1] = sum; }        // the maximum in log2 units
+    }
+  }
+  if (u.parts == 1) return;
+  // the CTA that finishes last for this sequence's head merges the parts, as the launched kernel does
+  __threadfence();
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  if (e == 0) {
+    const unsigned before = atomicAdd(&p.counters[u.bk], 1u);
+    s_ml[64] = before == (unsigned)u.parts - 1u ? 1.f : 0.f;
+    if (before == (unsigned)u.parts - 1u) p.counters[u.bk] = 0u;
+  }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  if (s_ml[64] == 0.f) return;
+  __threadfence();
+  float *w_m = scratch, *w_l = scratch + u.parts * G;             // [part][head]
+  for (int i = e; i < u.parts * G; i += 128) {
+    const float2 v = __ldcg(reinterpret_cast<const float2*>(p.out + (slot0 * G + i) * 2));
+    w_m[i] = v.x;
+    w_l[i] = v.y;
+  }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  for (int i = e; i < G * D; i += 128) {
+    const int h = i / D, d = i - h * D;
+    float M = -INFINITY, sum = 0.f, acc = 0.f;
+    for (int s = 0; s < u.parts; ++s) M = fmaxf(M, w_m[s * G + h]);
+    for (int s = 0; s < u.parts; ++s) sum += exp2f(w_m[s * G + h] - M) * w_l[s * G + h];
+    const float* po = p.partials + (slot0 * G + h) * D + d;
+#pragma unroll 8
+    for (int s = 0; s < u.parts; ++s) acc += exp2f(w_m[s * G + h] - M) * __ldcg(po + (int64_t)s * G * D);
+    out[xcanon_offset(u.b, (u.kvl * G + h) * D + d, N)] = __float2bfloat16_rn(acc * (1.0f / sum));
+  }
+}
+
+template <int N, bool X, int D>
+__global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __grid_constant__ ChainParamsOf<D> P, int* err) {
   constexpr int ST = kChainStages<N>;
   constexpr int kXStage = N * 256;
   constexpr int kStage = kWStage + kXStage;
@@ -1754,6 +1930,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
   __shared__ __align__(8) uint64_t acc_empty[2];
   __shared__ __align__(8) uint64_t recv_full;                    // the four parts of this CTA's rows have arrived
   __shared__ __align__(8) uint64_t send_ok;                      // every CTA of the cluster has read its receive buffer
+  __shared__ unsigned attended;                                  // attentions whose stages in this CTA have been read
   __shared__ uint32_t tmem_base_slot;
   __shared__ float s_inv_buf[64];
   __shared__ float s_red[128];
@@ -1771,6 +1948,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
     mbar_init(&acc_empty[0], 4); mbar_init(&acc_empty[1], 4);
     mbar_init(&recv_full, 1);
     mbar_init(&send_ok, kChainC);
+    attended = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) {
@@ -1792,7 +1970,32 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
       uint64_t pol_w;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(pol_w));
       int it = 0;
+      bool after_launch = false;
       for (int o = 0; o < P.n_ops; ++o) {
+        if (D > 0 && P.op[o].epi == EPI_ATTEND) {
+          const GemvParams& p = P.op[o];
+          if (!after_launch) pdl_wait();                         // positions and cache, unlike weights, are the step's
+          after_launch = true;
+          bool fresh = o == 0;
+          for (int u = blockIdx.x; u < p.B * p.KVl * p.ksplit; u += gridDim.x) {
+            const ChainUnit w = chain_unit(p, u);
+            const __nv_bfloat16* kv = reinterpret_cast<const __nv_bfloat16*>(p.kv_layer) + w.b * p.kv_batch_stride + w.kvl * p.kv_head_stride;
+            for (int key = w.begin; key < w.end; key += 64, ++it) {
+              if (!fresh && key + 64 >= w.T) {                   // the newest key and value come from the projection before
+                chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P.op[o - 1], ncl), dead, err);
+                asm volatile("fence.proxy.async;\n" ::: "memory");
+                fresh = true;
+              }
+              const int s = it % ST, k = it / ST;
+              const uint32_t bytes = (uint32_t)(min(4, (w.end - key + 15) >> 4) * 64 * D);
+              mbar_wait(&empty_bar[s], (k & 1) ^ 1, dead, err);
+              mbar_expect_tx(&full_bar[s], bytes);
+              bulk_g2s(smem + s * kStage, kv + (int64_t)(key >> 4) * (32 * D), bytes, &full_bar[s], pol_w);
+              mbar_arrive(&full_bar[s]);                         // (there are no activations)
+            }
+          }
+          continue;
+        }
         const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
         const int ks0 = c * KS / kChainC, ks1 = (c + 1) * KS / kChainC;
         const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(P.op[o].W);
@@ -1815,11 +2018,15 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
       asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(pol_x));
       int it = 0;
       for (int o = 0; o < P.n_ops; ++o) {
+        if (D > 0 && P.op[o].epi == EPI_ATTEND) {
+          it += chain_attend_stages(P.op[o]);
+          continue;
+        }
         const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
         const int ks0 = c * KS / kChainC, ks1 = (c + 1) * KS / kChainC;
         if (cid >= nrbg || ks0 >= ks1) continue;
         if (o > 0) {
-          chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P, o - 1, ncl), dead, err);
+          chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P.op[o - 1], ncl), dead, err);
           asm volatile("fence.proxy.async;\n" ::: "memory");      // the bulk copies read what the epilogues stored
         }
         const __nv_bfloat16* xsrc = reinterpret_cast<const __nv_bfloat16*>(P.op[o].x);
@@ -1837,7 +2044,17 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
   } else if (warp == 1) {
     // ---------------- MMA issue ----------------
     int it = 0, seg = 0;
+    unsigned attentions = 0;
     for (int o = 0; o < P.n_ops; ++o) {
+      if (D > 0 && P.op[o].epi == EPI_ATTEND) {
+        if (attentions == 0) pdl_wait();
+        const int n = chain_attend_stages(P.op[o]);
+        // Not before they have been read: a barrier's parity tells a stage's fills apart only from the one before, and the stages skipped here may
+        // go round the ring several times.
+        if (n > 0) chain_wait_shared(&attended, ++attentions, dead, err);
+        it += n;
+        continue;
+      }
       const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
       const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
       if (n_steps == 0) continue;
@@ -1874,14 +2091,35 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
     const uint32_t to = dsmem_addr(smem_u32(recv) + (uint32_t)((c * 32 + lane) * N * 4), (uint32_t)q);
     const uint32_t to_bar = dsmem_addr(smem_u32(&recv_full), (uint32_t)q);
     int seg = 0, g = 0;                        // accumulators drained, tiles exchanged
+    int it = 0;                                // the ring's stages, which only attention reads here
     for (int o = 0; o < P.n_ops; ++o) {
       const GemvParams& p = P.op[o];
+      if (D > 0 && p.epi == EPI_ATTEND) {
+        const int units = p.B * p.KVl * p.ksplit;
+        if ((int)blockIdx.x >= units) continue;
+        if (o > 0) {
+          if (e == 0) chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P.op[o - 1], ncl), dead, err);
+          asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        }
+        // the receive buffer is free: what the peers send next needs this link's outputs
+        const int it0 = it;
+        for (int u = blockIdx.x; u < units; u += gridDim.x) {
+          const ChainUnit w = chain_unit(p, u);
+          if (w.begin < w.end) chain_attend<(D > 0 ? D : 64), N, ST>(p, w, it, smem, full_bar, empty_bar, const_cast<float*>(reinterpret_cast<const float*>(recv)), s_red, e, dead, err);
+        }
+        asm volatile("fence.proxy.async;\n" ::: "memory");
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        if (e == 0 && it != it0) asm volatile("red.release.cta.shared.add.u32 [%0], 1;\n" ::"r"(smem_u32(&attended)) : "memory");
+        if (e == 0 && o + 1 < P.n_ops) asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
+        continue;
+      }
       const int KS = (p.K + 127) >> 7, nrbg = (p.rows + 127) >> 7;
       const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
       if (cid >= nrbg) continue;
+      if (D > 0) it += n_steps * ((nrbg - cid + ncl - 1) / ncl);
       const float* s_inv = p.inv.ssq ? s_inv_buf : nullptr;
       if (o > 0) {
-        if (e == 0) chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P, o - 1, ncl), dead, err);
+        if (e == 0) chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P.op[o - 1], ncl), dead, err);
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
       }
       compute_inv_scale(p.inv, s_inv_buf, e);
@@ -1967,10 +2205,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
   if (tid == 0) {                              // the last CTA out leaves the counters empty
-    unsigned* gone = P.done + kChainMax * kChainLine;
+    unsigned* gone = P.done + kChainMaxAttend * kChainLine;
     __threadfence();
     if (atomicAdd(gone, 1u) == gridDim.x - 1u) {
-      for (int o = 0; o < kChainMax; ++o) P.done[o * kChainLine] = 0u;
+      for (int o = 0; o < P.n_ops; ++o) P.done[o * kChainLine] = 0u;
       *gone = 0u;
     }
   }
@@ -2085,23 +2323,44 @@ int chain_clusters() {
   cudaLaunchConfig_t cfg = chain_config<N>(attr, 1, 0);
   cfg.numAttrs = 1;
   int n = 0, m = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemv_chain_kernel<N, false>, &cfg) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&m, gemv_chain_kernel<N, true>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, gemv_chain_kernel<N, false, 0>, &cfg) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&m, gemv_chain_kernel<N, true, 0>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return std::min(n, m);
 }
 
-template <int N>
-int32_t launch_chain(Ctx* ctx, const ChainParams& P, int clusters, cudaStream_t stream) {
+template <int N, int D>
+int32_t launch_chain_of(Ctx* ctx, const GemvParams* op, int n, unsigned* done, int clusters, cudaStream_t stream) {
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = chain_config<N>(attr, clusters, stream);
+  static_assert(sizeof(ChainParamsOf<D>) <= 32 * 1024 - 64, "kernel parameters");
+  ChainParamsOf<D> P;
   bool x = false;
-  for (int i = 0; i < P.n_ops; ++i) x = x || layered_epilogue(P.op[i]);
-  LMB_CUDA(cudaLaunchKernelEx(&cfg, x ? gemv_chain_kernel<N, true> : gemv_chain_kernel<N, false>, P, ctx->dev_err));
+  for (int i = 0; i < n; ++i) {
+    P.op[i] = op[i];
+    x = x || layered_epilogue(op[i]);
+  }
+  P.n_ops = n;
+  P.done = done;
+  if constexpr (D > 0) {
+    LMB_REQUIRE(!x, "gemv chain: attention beside a layered decoder's projections");
+    LMB_CUDA(cudaLaunchKernelEx(&cfg, gemv_chain_kernel<N, false, D>, P, ctx->dev_err));
+  } else {
+    LMB_CUDA(cudaLaunchKernelEx(&cfg, x ? gemv_chain_kernel<N, true, 0> : gemv_chain_kernel<N, false, 0>, P, ctx->dev_err));
+  }
   ctx->launches++;
   return LMB200_OK;
+}
+template <int N>
+int32_t launch_chain(Ctx* ctx, const GemvParams* op, int n, unsigned* done, int clusters, int D, cudaStream_t stream) {
+  switch (D) {
+    case 0: return launch_chain_of<N, 0>(ctx, op, n, done, clusters, stream);
+    case 64: return launch_chain_of<N, 64>(ctx, op, n, done, clusters, stream);
+    case 96: return launch_chain_of<N, 96>(ctx, op, n, done, clusters, stream);
+    default: return launch_chain_of<N, 128>(ctx, op, n, done, clusters, stream);
+  }
 }
 
 constexpr int kMtF32 = 1;
@@ -2214,7 +2473,29 @@ int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms) {
   const int n = wide_batch ? chain_clusters<32>() : chain_clusters<16>();
   return output_norms && groups > n ? 0 : n;                    // an output norm needs every row group resident at once
 }
-int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMax + 1) * kChainLine * 4; }
+int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMaxAttend + 1) * kChainLine * 4; }
+
+// The four warps' sums of a unit lie in the receive buffer: 128 N floats for 4 G D
+bool gemv_chain_attends(int B, int G, int D) {
+  const char* e = getenv("LMB200_CHAIN_ATTENTION");             // 0: attention as a launch of its own (A/B runs)
+  if (e && atoi(e) == 0) return false;
+  return (D == 64 || D == 96 || D == 128) && G >= 1 && G <= 8 && G * D <= 32 * Layout<__nv_bfloat16>::batch_pad(B);
+}
+
+// One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge).  Parts beyond the first also cost the
+// merge over CTAs, and their pairs of maximum and sum must fit the receive buffer: at most 64.
+void gemv_chain_attention_plan(int clusters, int B, int KVl, int capacity, int* keys_per_cta, int* nsplit) {
+  const int64_t pairs = (int64_t)B * KVl, ctas = (int64_t)clusters * kChainC, cap = round_up(capacity, 64);
+  int64_t best = cap, best_cost = ceil_div(pairs, ctas) * (cap + 48);
+  for (int64_t k = 64; k < cap; k += 64) {
+    const int64_t ns = ceil_div(cap, k);
+    if (ns > 64) continue;
+    const int64_t cost = ceil_div(pairs * ns, ctas) * (k + 48) + 64;
+    if (cost < best_cost) { best_cost = cost; best = k; }
+  }
+  *keys_per_cta = (int)best;
+  *nsplit = (int)ceil_div(cap, best);
+}
 
 int32_t GemvChain::add(const GemvParams& p) {
   if (clusters == 0) return gemv_launch(ctx, LMB200_BF16, p, stream);
@@ -2226,7 +2507,22 @@ int32_t GemvChain::add(const GemvParams& p) {
     LMB_TRY(flush());
     return gemv_launch(ctx, LMB200_BF16, p, stream);
   }
-  if (n == kChainMax) LMB_TRY(flush());
+  if (n == (attention ? kChainMaxAttend : kChainMax)) LMB_TRY(flush());
+  op[n++] = p;
+  return LMB200_OK;
+}
+int32_t GemvChain::add_attention(const AttnParams& a) {
+  LMB_REQUIRE(clusters && attention && a.counters && a.pos, "gemv chain: no attention here");
+  if (n == kChainMaxAttend) LMB_TRY(flush());
+  GemvParams p;
+  p.epi = EPI_ATTEND;
+  p.B = a.B; p.KVl = a.KVl; p.Hl = a.KVl * a.G; p.D = a.D;
+  p.q_out = const_cast<void*>(a.q); p.q_pitch = a.q_pitch;
+  p.kv_layer = const_cast<void*>(a.kv_layer); p.kv_batch_stride = a.kv_batch_stride; p.kv_head_stride = a.kv_head_stride;
+  p.pos = a.pos; p.qk_scale = a.scale;
+  p.ksplit = a.nsplit; p.kc_per_split = a.keys_per_cta;
+  p.partials = a.part_o; p.out = a.part_ml; p.counters = a.counters;
+  p.act = a.out;
   op[n++] = p;
   return LMB200_OK;
 }
@@ -2234,20 +2530,21 @@ int32_t GemvChain::flush() {
   const int count = n;
   n = 0;
   if (count == 0) return LMB200_OK;
-  if (count == 1 && op[0].epi != EPI_RESID_NORM && op[0].epi != EPI_POST_NORM) return gemv_launch(ctx, LMB200_BF16, op[0], stream);
-  ChainParams P;
-  int most = 1;
+  if (count == 1 && op[0].epi != EPI_RESID_NORM && op[0].epi != EPI_POST_NORM && op[0].epi != EPI_ATTEND) return gemv_launch(ctx, LMB200_BF16, op[0], stream);
+  int most = 1, D = 0;
   for (int i = 0; i < count; ++i) {
     LMB_REQUIRE(op[i].B >= 1 && op[i].B <= 32 && op[i].push.n <= 1 && !op[i].rn.sum && !op[i].inv.sum, "gemv chain: op %d cannot run here", i);
     LMB_REQUIRE(op[i].epi != EPI_POST_NORM || ceil_div(op[i].rows, 128) <= std::min(clusters, kPushMaxCtas / kChainC),
                 "gemv chain: %d rows are more than one wave", op[i].rows);
-    P.op[i] = op[i];
+    if (op[i].epi == EPI_ATTEND) {
+      D = op[i].D;
+      most = clusters;
+    }
     most = std::max(most, (int)ceil_div(op[i].rows, 128));
   }
-  P.n_ops = count;
-  P.done = done;
+  LMB_REQUIRE(D > 0 || count <= kChainMax, "gemv chain: %d links", count);
   const int g = std::min(most, clusters);
-  return Layout<__nv_bfloat16>::batch_pad(op[0].B) == 16 ? launch_chain<16>(ctx, P, g, stream) : launch_chain<32>(ctx, P, g, stream);
+  return Layout<__nv_bfloat16>::batch_pad(op[0].B) == 16 ? launch_chain<16>(ctx, op, count, done, g, D, stream) : launch_chain<32>(ctx, op, count, done, g, D, stream);
 }
 
 // Raise the dynamic shared-memory limit of every instantiation once per device, outside any
@@ -2266,10 +2563,16 @@ int32_t gemv_configure() {
   LMB_CFG((gemv_cl_kernel<16, true>), cluster_smem<16>());
   LMB_CFG((gemv_cl_kernel<32, false>), cluster_smem<32>());
   LMB_CFG((gemv_cl_kernel<32, true>), cluster_smem<32>());
-  LMB_CFG((gemv_chain_kernel<16, false>), chain_smem<16>());
-  LMB_CFG((gemv_chain_kernel<16, true>), chain_smem<16>());
-  LMB_CFG((gemv_chain_kernel<32, false>), chain_smem<32>());
-  LMB_CFG((gemv_chain_kernel<32, true>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<16, false, 0>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<16, true, 0>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<32, false, 0>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<32, true, 0>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<16, false, 64>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<32, false, 64>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<16, false, 96>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<32, false, 96>), chain_smem<32>());
+  LMB_CFG((gemv_chain_kernel<16, false, 128>), chain_smem<16>());
+  LMB_CFG((gemv_chain_kernel<32, false, 128>), chain_smem<32>());
 #undef LMB_CFG
   return LMB200_OK;
 }

@@ -2,6 +2,7 @@
 // batch), i.e. a GEMV / skinny GEMM that is bound by streaming W from HBM once.
 // Replaces NN.Linear -> MatMul for S = 1 (src/NN.jl:22-35, src/Execution.jl:56-90).
 #pragma once
+#include "attention.cuh"
 #include "common.cuh"
 
 namespace lmb {
@@ -15,7 +16,8 @@ enum GemvEpilogue {
   EPI_RESID_NORM = 4,  // row-parallel projection + all-reduce + residual add + RMSNorm preparation (ResidNorm below)
   EPI_STORE_ACT = 6,   // like EPI_STORE_RELU2 with act = acc
   EPI_GELU_TOKEN = 7,  // act[b, row] = gelu(acc) * token_table[tokens[b] * token_pitch + row]
-  EPI_POST_NORM = 8    // residual add of the projection's own RMSNorm (PostNorm below)
+  EPI_POST_NORM = 8,   // residual add of the projection's own RMSNorm (PostNorm below)
+  EPI_ATTEND = 9       // no projection: decode attention as a link of a chain (GemvChain::add_attention)
 };
 
 // Exchange of a row-parallel projection's partial results between the tensor-parallel ranks, done by
@@ -175,7 +177,8 @@ int32_t gemv_launch(Ctx* ctx, int dtype, GemvParams p, cudaStream_t stream);
 
 // A run of bf16 GEMVs, each reading what the one before it wrote, as one launch (gemv_chain_kernel).  `clusters` is
 // gemv_chain_clusters for the session; 0 launches every GEMV by itself.  One rank only.
-constexpr int kChainMax = 8;                 // GEMVs per launch
+constexpr int kChainMax = 8;                 // links per launch
+constexpr int kChainMaxAttend = 40;          // with attention among them (one after every q/k/v projection): eight layers
 constexpr int kChainC = 4;                   // CTAs per cluster
 constexpr int kSsqSlots = 256;               // of a session's ssq buffer, 32 floats each
 struct GemvChain {
@@ -183,9 +186,11 @@ struct GemvChain {
   cudaStream_t stream = nullptr;
   int clusters = 0;
   unsigned* done = nullptr;                  // gemv_chain_scratch_bytes(), zero before the first launch
-  GemvParams op[kChainMax];
+  bool attention = false;                    // gemv_chain_attends() for the session: add_attention() may be called
+  GemvParams op[kChainMaxAttend];
   int n = 0;
   int32_t add(const GemvParams& p);
+  int32_t add_attention(const AttnParams& p);
   int32_t flush();                           // before anything that reads the last GEMV's output
   // ssq slots an EPI_RESID_NORM of these rows leaves: with clusters, add() and flush() run every one in the chain kernel
   int slots(const GemvPlan& pl, int rows) const { return clusters ? (int)ceil_div(rows, 128) * kChainC : gemv_plan_ctas(pl, rows); }
@@ -194,5 +199,8 @@ struct GemvChain {
 // EPI_POST_NORMs are among them
 int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms);
 int64_t gemv_chain_scratch_bytes();
+// Whether a chain's attention runs these heads, and its split of the keys (AttnParams::keys_per_cta, nsplit) for a cache of `capacity` positions
+bool gemv_chain_attends(int B, int G, int D);
+void gemv_chain_attention_plan(int clusters, int B, int KVl, int capacity, int* keys_per_cta, int* nsplit);
 
 }  // namespace lmb

@@ -1274,7 +1274,7 @@ GemvParams gemv_params(Session* S, const void* W, const WMap& m, const GemvPlan&
 
 GemvChain gemv_chain(Session* S, cudaStream_t st) {
   GemvChain ch;
-  ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done;
+  ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done; ch.attention = S->chain_attention;
   return ch;
 }
 
@@ -1528,7 +1528,7 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
       p.kv_layer = kv_layer; p.kv_batch_stride = S->kv_batch_stride; p.kv_head_stride = S->kv_head_stride;
       p.inv_freq = M->inv_freq; p.pos = S->pos; p.pos_uniform = S->ragged ? 0 : 1; p.Hl = M->Hl; p.KVl = M->KVl; p.D = M->D;
       LMB_TRY(chain.add(p));
-      LMB_TRY(chain.flush());
+      if (!chain.attention) LMB_TRY(chain.flush());
     }
     {
       AttnParams a;
@@ -1539,7 +1539,12 @@ int32_t enqueue_step_fused(Session* S, cudaStream_t st, int head) {
       a.scale = 1.0f / sqrtf((float)M->D);
       a.part_o = S->part_o; a.part_ml = S->part_ml; a.out = S->attn_out; a.out_tiled_bp = S->Bp;
       a.counters = S->attn_counters;
-      LMB_TRY(attn_decode_launch(ctx, dt, a, st));
+      if (chain.attention) {
+        a.keys_per_cta = S->chain_keys; a.nsplit = S->chain_nsplit;
+        LMB_TRY(chain.add_attention(a));
+      } else {
+        LMB_TRY(attn_decode_launch(ctx, dt, a, st));
+      }
     }
     {  // o_proj + all-reduce + residual add + what the MLP's norm needs
       GemvParams p = gemv_params(S, W.wo, M->m_o, S->p_o, S->attn_out);
@@ -2078,6 +2083,12 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
   }
   int64_t po, pml;
   attn_plan(ctx, batch, M->KVl, M->G, M->D, S->cap, &S->keys_per_cta, &S->nsplit, &po, &pml);
+  if (S->chain_clusters && c.hidden > 15 * 128 && gemv_chain_attends(batch, M->G, M->D)) {
+    S->chain_attention = true;
+    gemv_chain_attention_plan(S->chain_clusters, batch, M->KVl, S->cap, &S->chain_keys, &S->chain_nsplit);
+    po = std::max(po, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * M->D);
+    pml = std::max(pml, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * 2);
+  }
   if (whisper) {
     plan(S->p_qc, M->m_qc);
     S->cross_cap = (int)round_up(c.cross_len, 64);

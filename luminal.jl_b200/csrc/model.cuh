@@ -164,6 +164,8 @@ struct Session {
   unsigned* gemv_counters = nullptr;
   unsigned* chain_done = nullptr;      // GemvChain::done
   int chain_clusters = 0;              // > 0: the fused step runs its GEMVs in chains
+  bool chain_attention = false;        // ... with the attention among them, and its split of the keys
+  int chain_keys = 0, chain_nsplit = 0;
   float* part_o = nullptr;
   float* part_ml = nullptr;
   unsigned* attn_counters = nullptr;   // [B*KVl], zero between launches
