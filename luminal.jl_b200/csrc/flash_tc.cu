@@ -25,7 +25,8 @@
 // (Earlier forms: keys in tiles of 64 with P through shared memory -- 16 + 8 small MMAs per 64 keys,
 // all operands from shared memory, 160 KB of operand reads per 128 keys and tile -- ran at 709
 // TFLOP/s on [4, 32, 4096, 128]; 128-key tiles with P in tensor memory 729; two softmax threads
-// per row 948; packed float32 pairs and three-input maxima in the softmax 959.)
+// per row 948; packed float32 pairs and three-input maxima in the softmax 959; MMAs issued under an elected branch (tc::elect_one) 983 -> 1049
+// on one box.)
 // Causal: key tiles beyond a query tile's diagonal are never computed; inside the diagonal tile
 // keys j > i are masked -- the reference's `if causal && j > i continue`.
 #include <cuda.h>
@@ -259,9 +260,9 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
     // ------------------------------ MMA issue ------------------------------
     constexpr uint32_t kIdescS = idesc_bf16(kBM, kBN, false, false);
     constexpr uint32_t kIdescPV = idesc_bf16(kBM, DV, false, true);          // V is read MN-major
-    mbar_wait(&q_full, 0, dead, err);
-    auto issue_s = [&](int j, int t) {                // S[t] = Q[t] K(j)^T
-      if (lane == 0) {
+    if (elect_one()) {
+      mbar_wait(&q_full, 0, dead, err);
+      auto issue_s = [&](int j, int t) {                // S[t] = Q[t] K(j)^T
         const uint64_t adesc = smem_desc(smem_u32(smem + SM::offQ + t * SM::kQ), kBM * 16, 128);
         const uint32_t sK = smem_u32(smem + SM::offK + ((j - jb) % kStages) * SM::kK);
 #pragma unroll
@@ -270,52 +271,45 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
           mma_f16(tmem + kColS + t * kBN, adesc + (uint64_t)(ks * ((2 * kBM * 16) >> 4)), bdesc, kIdescS, ks ? 1u : 0u);
         }
         commit(&s_full[t]);
-      }
-      __syncwarp();
-    };
-    auto issue_pv = [&](int j, int t) {               // O[t] += P[t] V(j), P read from tensor memory
-      if (lane == 0) {
+      };
+      auto issue_pv = [&](int j, int t) {               // O[t] += P[t] V(j), P read from tensor memory
         const uint64_t bdesc = smem_desc_swz(smem_u32(smem + SM::offV + ((j - jb) % vStages) * SM::kV), kSub, 16 * W, kSwz);
 #pragma unroll
         for (int ks = 0; ks < kBN / 16; ++ks)
           mma_f16_ts(tmem + kColO + t * DV, tmem + kColS + t * kBN + ks * 8, bdesc + (uint64_t)(ks * ((32 * W) >> 4)), kIdescPV,
                      (j > first[t] || ks > 0) ? 1u : 0u);
         if (j == n_tiles[t] - 1) commit(&o_done[t]);
-      }
-      __syncwarp();
-    };
-    if (n_max > jb) {
-      mbar_wait(&k_full[0], 0, dead, err);
-      fence_after();
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-        if (first[t] == jb && n_tiles[t] > jb) issue_s(jb, t);
-      if (lane == 0) commit(&k_empty[0]);
-      __syncwarp();
-    }
-    for (int j = jb; j < n_max; ++j) {
-      const int i = j - jb, s = i % vStages, s1 = (i + 1) % kStages;
-      mbar_wait(&v_full[s], (i / vStages) & 1, dead, err);
-      if (j + 1 < n_max) mbar_wait(&k_full[s1], ((i + 1) / kStages) & 1, dead, err);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (j >= n_tiles[t]) continue;
-        if (WIN && j < first[t]) {                       // the second query tile's window starts one key tile later
-          fence_after();
-          if (j + 1 == first[t] && j + 1 < n_tiles[t]) issue_s(j + 1, t);
-          continue;
-        }
-        mbar_wait(&p_full[t], (j - first[t]) & 1, dead, err);
+      };
+      if (n_max > jb) {
+        mbar_wait(&k_full[0], 0, dead, err);
         fence_after();
-        issue_pv(j, t);
-        if (j + 1 < n_tiles[t]) issue_s(j + 1, t);       // runs after P V(j) in the tensor pipe: S overwrites P's columns
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (first[t] == jb && n_tiles[t] > jb) issue_s(jb, t);
+        commit(&k_empty[0]);
       }
-      if (lane == 0) {
+      for (int j = jb; j < n_max; ++j) {
+        const int i = j - jb, s = i % vStages, s1 = (i + 1) % kStages;
+        mbar_wait(&v_full[s], (i / vStages) & 1, dead, err);
+        if (j + 1 < n_max) mbar_wait(&k_full[s1], ((i + 1) / kStages) & 1, dead, err);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (j >= n_tiles[t]) continue;
+          if (WIN && j < first[t]) {                       // the second query tile's window starts one key tile later
+            fence_after();
+            if (j + 1 == first[t] && j + 1 < n_tiles[t]) issue_s(j + 1, t);
+            continue;
+          }
+          mbar_wait(&p_full[t], (j - first[t]) & 1, dead, err);
+          fence_after();
+          issue_pv(j, t);
+          if (j + 1 < n_tiles[t]) issue_s(j + 1, t);       // runs after P V(j) in the tensor pipe: S overwrites P's columns
+        }
         commit(&v_empty[s]);
         if (j + 1 < n_max) commit(&k_empty[s1]);
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // ------------------------------ softmax + output ------------------------------
     // Two threads per query row: warps 0-7 take keys 0-63 of a tile, warps 8-15 keys 64-127 (a warp reaches the 32

@@ -177,14 +177,14 @@ flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const 
     // ------------------------------ MMA issue ------------------------------
     constexpr uint32_t kIdescS = idesc_bf16(kBM, kBN, false, false);
     constexpr uint32_t kIdescPV = idesc_bf16(kBM, D, false, true);          // V is read MN-major
-    mbar_wait(&q_full, 0, dead, err);
-    // the three partial products of one float32-class product: (hi, hi), (hi, lo), (lo, hi)
-    const int a_part[3] = {0, 0, 1}, b_part[3] = {0, 1, 0};
-    auto issue_pv = [&](int j) {
-      const int s = j % kStages;
-      mbar_wait(&p_full, j & 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+    if (elect_one()) {
+      mbar_wait(&q_full, 0, dead, err);
+      // the three partial products of one float32-class product: (hi, hi), (hi, lo), (lo, hi)
+      const int a_part[3] = {0, 0, 1}, b_part[3] = {0, 1, 0};
+      auto issue_pv = [&](int j) {
+        const int s = j % kStages;
+        mbar_wait(&p_full, j & 1, dead, err);
+        fence_after();
         unsigned char* st = smem + SM::offKV + s * 4 * SM::kKV;
 #pragma unroll
         for (int t3 = 0; t3 < 3; ++t3) {
@@ -195,15 +195,12 @@ flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const 
         }
         commit(&p_empty);
         commit(&kv_empty[s]);
-      }
-      __syncwarp();
-    };
-    for (int j = 0; j < nt; ++j) {
-      const int sb = j & 1, s = j % kStages;
-      mbar_wait(&kv_full[s], (j / kStages) & 1, dead, err);
-      mbar_wait(&s_empty[sb], ((j >> 1) & 1) ^ 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+      };
+      for (int j = 0; j < nt; ++j) {
+        const int sb = j & 1, s = j % kStages;
+        mbar_wait(&kv_full[s], (j / kStages) & 1, dead, err);
+        mbar_wait(&s_empty[sb], ((j >> 1) & 1) ^ 1, dead, err);
+        fence_after();
         unsigned char* st = smem + SM::offKV + s * 4 * SM::kKV;
 #pragma unroll
         for (int t3 = 0; t3 < 3; ++t3) {
@@ -216,11 +213,11 @@ flash_tc_f32_kernel(float* __restrict__ out, const float* __restrict__ q, const 
           }
         }
         commit(&s_full[sb]);
+        if (j >= 1) issue_pv(j - 1);
       }
-      __syncwarp();
-      if (j >= 1) issue_pv(j - 1);
+      if (nt >= 1) issue_pv(nt - 1);
     }
-    if (nt >= 1) issue_pv(nt - 1);
+    __syncwarp();
   } else {
     // ------------------------------ softmax + output: one query row per thread ------------------------------
     const int r = 32 * warp + lane;

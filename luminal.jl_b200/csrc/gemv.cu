@@ -21,6 +21,7 @@
 
 #include "gemv.cuh"
 #include "pdl.cuh"
+#include "tc.cuh"
 
 namespace lmb {
 
@@ -482,6 +483,7 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+using tc::elect_one;
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -1108,18 +1110,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_tc_kernel(const GemvParams
     pdl_wait();
     if (lane == 0) LMB_TRACE(2);
     // ---------------- MMA issue ----------------
-    int it = 0, seg = 0;
-    for (int u = ur.u0; u < ur.u1; ++u, ++it) {
-      const int ks = u % ur.KS;
-      const bool first = (u == ur.u0) || ks == 0;
-      const bool last = (u == ur.u1 - 1) || ks == ur.KS - 1;
-      const int buf = seg & 1;
-      if (first) mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, dead, err);   // epilogue has drained this buffer
-      const int s = it % kStages, k = it / kStages;
-      mbar_wait(&full_bar[s], k & 1, dead, err);
-      tc_fence_after();
-      if (lane == 0 && it == 0) LMB_TRACE(3);
-      if (lane == 0) {
+    if (elect_one()) {
+      int it = 0, seg = 0;
+      for (int u = ur.u0; u < ur.u1; ++u, ++it) {
+        const int ks = u % ur.KS;
+        const bool first = (u == ur.u0) || ks == 0;
+        const bool last = (u == ur.u1 - 1) || ks == ur.KS - 1;
+        const int buf = seg & 1;
+        if (first) mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, dead, err);   // epilogue has drained this buffer
+        const int s = it % kStages, k = it / kStages;
+        mbar_wait(&full_bar[s], k & 1, dead, err);
+        tc_fence_after();
+        if (it == 0) LMB_TRACE(3);
         const uint32_t st = smem_u32(smem + s * kStage);
         const uint64_t adesc = smem_desc(st, 2048, 128);
         const uint64_t bdesc = smem_desc(st + kWStage, N * 16, 128);
@@ -1129,11 +1131,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_tc_kernel(const GemvParams
                      kIdesc, (first && j == 0) ? 0u : 1u);
         tc_commit(&empty_bar[s]);       // stage free once these MMAs have read it
         if (last) tc_commit(&acc_full[buf]);
+        if (last) ++seg;
       }
-      __syncwarp();
-      if (last) ++seg;
+      LMB_TRACE(4);
     }
-    if (lane == 0) LMB_TRACE(4);
+    __syncwarp();
   } else {
     // ---------------- epilogue: warp quarter q owns TMEM lanes / rows 32q .. 32q+31 ----------------
     // A row group whose k range is shared by n > 1 CTAs is folded by all of them together: each
@@ -1407,12 +1409,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
     // ---------------- MMA issue ----------------
     pdl_wait();
     if (lane == 0) LMB_TRACE(2);
-    for (int i = 0; i < n_steps; ++i) {
-      const int s = i % kStages, k = i / kStages;
-      mbar_wait(&full_bar[s], k & 1, dead, err);
-      tc_fence_after();
-      if (lane == 0 && i == 0) LMB_TRACE(3);
-      if (lane == 0) {
+    if (elect_one()) {
+      for (int i = 0; i < n_steps; ++i) {
+        const int s = i % kStages, k = i / kStages;
+        mbar_wait(&full_bar[s], k & 1, dead, err);
+        tc_fence_after();
+        if (i == 0) LMB_TRACE(3);
         const uint32_t sa = smem_u32(smem + s * kStage);
         const uint64_t adesc = smem_desc(sa, 2048, 128);
         const uint64_t bdesc = smem_desc(sa + kWStage, N * 16, 128);
@@ -1423,9 +1425,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
         tc_commit(&empty_bar[s]);
         if (i == n_steps - 1) tc_commit(&acc_full);
       }
-      __syncwarp();
+      LMB_TRACE(4);
     }
-    if (lane == 0) LMB_TRACE(4);
+    __syncwarp();
   } else {
     // ---------------- epilogue warps: send every row to the CTA that finalises it ----------------
     pdl_wait();
@@ -2043,30 +2045,30 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   } else if (warp == 1) {
     // ---------------- MMA issue ----------------
-    int it = 0, seg = 0;
-    unsigned attentions = 0;
-    for (int o = 0; o < P.n_ops; ++o) {
-      if (D > 0 && P.op[o].epi == EPI_ATTEND) {
-        if (attentions == 0) pdl_wait();
-        const int n = chain_attend_stages(P.op[o]);
-        // Not before they have been read: a barrier's parity tells a stage's fills apart only from the one before, and the stages skipped here may
-        // go round the ring several times.
-        if (n > 0) chain_wait_shared(&attended, ++attentions, dead, err);
-        it += n;
-        continue;
-      }
-      const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
-      const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
-      if (n_steps == 0) continue;
-      for (int r = cid; r < nrbg; r += ncl, ++seg) {
-        const int buf = seg & 1;
-        mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, dead, err);
-        tc_fence_after();
-        for (int i = 0; i < n_steps; ++i, ++it) {
-          const int s = it % ST, k = it / ST;
-          mbar_wait(&full_bar[s], k & 1, dead, err);
+    if (elect_one()) {
+      int it = 0, seg = 0;
+      unsigned attentions = 0;
+      for (int o = 0; o < P.n_ops; ++o) {
+        if (D > 0 && P.op[o].epi == EPI_ATTEND) {
+          if (attentions == 0) pdl_wait();
+          const int n = chain_attend_stages(P.op[o]);
+          // Not before they have been read: a barrier's parity tells a stage's fills apart only from the one before, and the stages skipped here may
+          // go round the ring several times.
+          if (n > 0) chain_wait_shared(&attended, ++attentions, dead, err);
+          it += n;
+          continue;
+        }
+        const int KS = (P.op[o].K + 127) >> 7, nrbg = (P.op[o].rows + 127) >> 7;
+        const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
+        if (n_steps == 0) continue;
+        for (int r = cid; r < nrbg; r += ncl, ++seg) {
+          const int buf = seg & 1;
+          mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, dead, err);
           tc_fence_after();
-          if (lane == 0) {
+          for (int i = 0; i < n_steps; ++i, ++it) {
+            const int s = it % ST, k = it / ST;
+            mbar_wait(&full_bar[s], k & 1, dead, err);
+            tc_fence_after();
             const uint32_t sa = smem_u32(smem + s * kStage);
             const uint64_t adesc = smem_desc(sa, 2048, 128);
             const uint64_t bdesc = smem_desc(sa + kWStage, N * 16, 128);
@@ -2077,10 +2079,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
             tc_commit(&empty_bar[s]);
             if (i == n_steps - 1) tc_commit(&acc_full[buf]);
           }
-          __syncwarp();
         }
       }
     }
+    __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   } else {
     // ---------------- epilogue ----------------

@@ -455,17 +455,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
       }
     }
   } else if (warp == kMmaWarp) {
-    constexpr uint32_t kIdesc = idesc_bf16(128, kGemmBN, false, false);
-    int g = 0, n = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
-      const int buf = n & 1;
-      mbar_wait(&acc_empty[buf], ((n >> 1) & 1) ^ 1, dead, err);        // the epilogue has drained this accumulator
-      fence_after();
-      for (int st = 0; st < NS; ++st, ++g) {
-        const int s = g % kGemmStages;
-        mbar_wait(&full[s], (g / kGemmStages) & 1, dead, err);
+    if (elect_one()) {
+      constexpr uint32_t kIdesc = idesc_bf16(128, kGemmBN, false, false);
+      int g = 0, n = 0;
+      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++n) {
+        const int buf = n & 1;
+        mbar_wait(&acc_empty[buf], ((n >> 1) & 1) ^ 1, dead, err);        // the epilogue has drained this accumulator
         fence_after();
-        if (lane == 0) {
+        for (int st = 0; st < NS; ++st, ++g) {
+          const int s = g % kGemmStages;
+          mbar_wait(&full[s], (g / kGemmStages) & 1, dead, err);
+          fence_after();
           const uint32_t sa = smem_u32(smem + s * kStage);
           const uint64_t adesc = smem_desc(sa, 2048, 128);
           const uint64_t bdesc = smem_desc_sw128(sa + kABytes);
@@ -476,9 +476,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const GemmPara
           commit(&empty[s]);
           if (st == NS - 1) commit(&acc_full[buf]);
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else {
     // epilogue of tile n while the MMAs of tile n + 1 fill the other accumulator
     const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
@@ -632,17 +632,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   } else if (warp == kMmaWarp && rank == 1) {
     // CTA 1 issues no MMAs: CTA 0's thread drives both tensor cores
   } else if (warp == kMmaWarp) {
-    constexpr uint32_t kIdesc = idesc_bf16(256, kBN, false, false);
-    int g = 0, n = 0;
-    for (int tile = pair; tile < n_tiles; tile += n_pairs, ++n) {
-      const int buf = n & 1;
-      mbar_wait(&acc_empty[buf], ((n >> 1) & 1) ^ 1, dead, err);        // both CTAs' epilogues have drained this accumulator
-      fence_after();
-      for (int st = 0; st < NS; ++st, ++g) {
-        const int s = g % kPairStages;
-        mbar_wait(&full[s], (g / kPairStages) & 1, dead, err);
+    if (elect_one()) {
+      constexpr uint32_t kIdesc = idesc_bf16(256, kBN, false, false);
+      int g = 0, n = 0;
+      for (int tile = pair; tile < n_tiles; tile += n_pairs, ++n) {
+        const int buf = n & 1;
+        mbar_wait(&acc_empty[buf], ((n >> 1) & 1) ^ 1, dead, err);        // both CTAs' epilogues have drained this accumulator
         fence_after();
-        if (lane == 0) {
+        for (int st = 0; st < NS; ++st, ++g) {
+          const int s = g % kPairStages;
+          mbar_wait(&full[s], (g / kPairStages) & 1, dead, err);
+          fence_after();
           const uint32_t sa = smem_u32(smem + s * kPairStage);
           const uint64_t adesc = smem_desc(sa, 2048, 128);
           const uint64_t bdesc = smem_desc_sw128(sa + kABytes);
@@ -653,9 +653,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           commit_pair(&empty[s]);
           if (st == NS - 1) commit_pair(&acc_full[buf]);
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else {
     const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t acc_empty_remote[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};

@@ -136,48 +136,39 @@ __global__ void __launch_bounds__(kThreads, 1) retention_tc_kernel(const Retenti
     constexpr uint32_t kKK = idesc_bf16(128, 128, false, false), kKM = idesc_bf16(128, 128, false, true), kMM = idesc_bf16(128, 128, true, true);
     const uint32_t base = smem_u32(smem);
     const int ds = (D + 15) >> 4;                        // 16-feature steps (the tiles are zero behind dim)
-    auto scores = [&](int c) {
-      mbar_wait(&tl.q_full, c & 1, dead, err);
-      mbar_wait(&tl.k_full[c & 1], (c >> 1) & 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+    if (elect_one()) {
+      auto scores = [&](int c) {
+        mbar_wait(&tl.q_full, c & 1, dead, err);
+        mbar_wait(&tl.k_full[c & 1], (c >> 1) & 1, dead, err);
+        fence_after();
         for (int ks = 0; ks < ds; ++ks) mma_f16(tmem + kColP, desc_k(base + offQ, ks), desc_k(base + offK + (c & 1) * kTile, ks), kKK, ks ? 1u : 0u);
         commit(&tl.s_full);
-      }
-      __syncwarp();
-    };
-    if (chunks > 0) scores(0);
-    for (int c = 0; c < chunks; ++c) {
-      if (c) mbar_wait(&tl.o_empty, (c - 1) & 1, dead, err);
-      mbar_wait(&tl.st_ready, c & 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+      };
+      if (chunks > 0) scores(0);
+      for (int c = 0; c < chunks; ++c) {
+        if (c) mbar_wait(&tl.o_empty, (c - 1) & 1, dead, err);
+        mbar_wait(&tl.st_ready, c & 1, dead, err);
+        fence_after();
         for (int ks = 0; ks < ds; ++ks) mma_f16(tmem + kColI, desc_k(base + offQ, ks), desc_mn(base + offSh, ks), kKM, ks ? 1u : 0u);
         for (int ks = 0; ks < ds; ++ks) mma_f16(tmem + kColI, desc_k(base + offQ, ks), desc_mn(base + offSl, ks), kKM, 1u);
         commit(&tl.q_empty);
-      }
-      __syncwarp();
-      mbar_wait(&tl.v_full, c & 1, dead, err);
-      mbar_wait(&tl.p_ready, c & 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+        mbar_wait(&tl.v_full, c & 1, dead, err);
+        mbar_wait(&tl.p_ready, c & 1, dead, err);
+        fence_after();
         for (int ks = 0; ks < 8; ++ks) mma_ts(tmem + kColO, tmem + kColP + ks * 8, desc_mn(base + offV, ks), kKM, ks ? 1u : 0u);
         for (int ks = 0; ks < 8; ++ks) mma_ts(tmem + kColO, tmem + kColP + 64 + ks * 8, desc_mn(base + offV, ks), kKM, 1u);
         commit(&tl.o_full);
-      }
-      __syncwarp();
-      mbar_wait(&tl.kt_ready, c & 1, dead, err);
-      fence_after();
-      if (lane == 0) {
+        mbar_wait(&tl.kt_ready, c & 1, dead, err);
+        fence_after();
         for (int ks = 0; ks < 8; ++ks) mma_f16(tmem + kColS, desc_mn(base + offK + (c & 1) * kTile, ks), desc_mn(base + offV, ks), kMM, 1u);
         for (int ks = 0; ks < 8; ++ks) mma_f16(tmem + kColS, desc_mn(base + offKl, ks), desc_mn(base + offV, ks), kMM, 1u);
         commit(&tl.m4_done);
         commit(&tl.v_empty);
         commit(&tl.k_empty[c & 1]);
+        if (c + 1 < chunks) scores(c + 1);
       }
-      __syncwarp();
-      if (c + 1 < chunks) scores(c + 1);
     }
+    __syncwarp();
   } else if (warp >= 8) {
     // ------------------------------ state and weighted keys ------------------------------
     const int half = (warp - 8) >> 2, row = 32 * (warp & 3) + lane;            // state row (feature) / token
