@@ -520,9 +520,9 @@ __device__ __forceinline__ void tmem_load_row<16>(float (&v)[16], uint32_t taddr
 }
 
 // What a row's epilogue reads besides the accumulators; the chain kernel fetches it while the weights stream.
-struct RowConst { float wg, bias, inv_freq; int pos; };
+struct RowConst { float wg, bias, inv_freq, sn, cs; int pos; };      // sn, cs: the rotation where all sequences are at one position
 __device__ __forceinline__ RowConst row_const(const GemvParams& p, int row) {
-  RowConst rc = {0.f, 0.f, 0.f, 0};
+  RowConst rc = {0.f, 0.f, 0.f, 0.f, p.qk_scale, 0};               // (no rotation: q and k rows are only scaled)
   if (row < p.rows) {
     if (p.ln_wg) rc.wg = p.ln_wg[row];
     if (p.bias) rc.bias = p.bias[row];
@@ -530,7 +530,14 @@ __device__ __forceinline__ RowConst row_const(const GemvParams& p, int row) {
   if (p.epi == EPI_QKV_ROPE) {
     rc.pos = p.pos[0];
     const int rb = row >> 4, tiles_per_head = p.D >> 4;
-    if (p.rope && rb / tiles_per_head < p.Hl + p.KVl) rc.inv_freq = p.inv_freq[8 * (rb % tiles_per_head) + (row & 7)];
+    if (p.rope && rb / tiles_per_head < p.Hl + p.KVl) {
+      rc.inv_freq = p.inv_freq[8 * (rb % tiles_per_head) + (row & 7)];
+      if (p.pos_uniform) {
+        const float ang = (float)rc.pos * rc.inv_freq;
+        rc.sn = sinf(ang);
+        rc.cs = sinf(kHalfPi + ang * -1.0f);        // cos(a) = sin(pi/2 - a)
+      }
+    }
   }
   return rc;
 }
@@ -644,13 +651,8 @@ __device__ __forceinline__ void row_epilogue(const GemvParams& p, float (&v)[NV]
   if (hs < p.Hl + p.KVl) {
     // rows g / g+8 of the block are the RoPE pair (d0, d0 + D/2)      src/NN.jl:253-303
     const int d0 = 8 * jj + g;
-    float sn = 0.f, cs = p.qk_scale;                // no rotation: q and k rows are only scaled
+    float sn = rc.sn, cs = rc.cs;
     const float inv_f = rc.inv_freq;
-    if (p.rope) {
-      const float ang = (float)pos * inv_f;
-      sn = sinf(ang);
-      cs = sinf(kHalfPi + ang * -1.0f);             // cos(a) = sin(pi/2 - a)
-    }
     const int d = hi ? d0 + half : d0;
 #pragma unroll
     for (int b = 0; b < N; ++b) {
@@ -1517,6 +1519,9 @@ struct ChainParams {
   int n_ops = 0;
   unsigned* done = nullptr;                  // [kChainMaxAttend + 1] lines, zero between launches; the last one counts exits
 };
+// what a link's epilogue reads of its parameters: all in front of the tensor-parallel exchange, which no chain has
+constexpr int kChainOpBytes = (int)(offsetof(GemvParams, push) + 15) / 16 * 16;
+static_assert(kChainOpBytes <= 480, "two links' parameters beside the barriers in the 2 KB that the ring leaves");
 // D > 0: the kernel with attention at that head dimension
 template <int D> using ChainParamsOf = ChainParams<(D > 0 ? kChainMaxAttend : kChainMax)>;
 
@@ -1888,33 +1893,62 @@ __device__ __forceinline__ void chain_attend(const GemvParams& p, const ChainUni
     }
   }
   if (u.parts == 1) return;
-  // the CTA that finishes last for this sequence's head merges the parts, as the launched kernel does
-  __threadfence();
+  // The CTA that finishes last for this sequence's head merges the parts.  A chain of trips to L2: the counter's one release and acquire cover all
+  // threads' partial results (barriers on both sides), and the first parts' values are on their way while the weights are formed.
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
   if (e == 0) {
-    const unsigned before = atomicAdd(&p.counters[u.bk], 1u);
+    unsigned before;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(&p.counters[u.bk]) : "memory");
     s_ml[64] = before == (unsigned)u.parts - 1u ? 1.f : 0.f;
     if (before == (unsigned)u.parts - 1u) p.counters[u.bk] = 0u;
   }
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
   if (s_ml[64] == 0.f) return;
-  __threadfence();
+  constexpr int kMine = N / 4;                                    // G D <= 32 N outputs, 128 threads
   float *w_m = scratch, *w_l = scratch + u.parts * G;             // [part][head]
+  const float* po = p.partials + slot0 * G * D + e;
+  float v[4][kMine], acc[kMine];
+  auto fetch = [&](int s0) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) v[s][j] = s0 + s < u.parts && e + 128 * j < G * D ? __ldcg(po + (int64_t)(s0 + s) * G * D + 128 * j) : 0.f;
+  };
+  fetch(0);
   for (int i = e; i < u.parts * G; i += 128) {
-    const float2 v = __ldcg(reinterpret_cast<const float2*>(p.out + (slot0 * G + i) * 2));
-    w_m[i] = v.x;
-    w_l[i] = v.y;
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.out + (slot0 * G + i) * 2));
+    w_m[i] = ml.x;
+    w_l[i] = ml.y;
   }
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
-  for (int i = e; i < G * D; i += 128) {
-    const int h = i / D, d = i - h * D;
-    float M = -INFINITY, sum = 0.f, acc = 0.f;
-    for (int s = 0; s < u.parts; ++s) M = fmaxf(M, w_m[s * G + h]);
-    for (int s = 0; s < u.parts; ++s) sum += exp2f(w_m[s * G + h] - M) * w_l[s * G + h];
-    const float* po = p.partials + (slot0 * G + h) * D + d;
-#pragma unroll 8
-    for (int s = 0; s < u.parts; ++s) acc += exp2f(w_m[s * G + h] - M) * __ldcg(po + (int64_t)s * G * D);
-    out[xcanon_offset(u.b, (u.kvl * G + h) * D + d, N)] = __float2bfloat16_rn(acc * (1.0f / sum));
+  if (e < G) {
+    float M = -INFINITY, sum = 0.f;
+    for (int s = 0; s < u.parts; ++s) M = fmaxf(M, w_m[s * G + e]);
+    for (int s = 0; s < u.parts; ++s) sum += exp2f(w_m[s * G + e] - M) * w_l[s * G + e];
+    s_ml[e] = M;
+    s_ml[8 + e] = 1.0f / sum;
+  }
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  for (int i = e; i < u.parts * G; i += 128) w_m[i] = exp2f(w_m[i] - s_ml[i % G]);
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < kMine; ++j) acc[j] = 0.f;
+  for (int s0 = 0; s0 < u.parts; s0 += 4) {
+    if (s0) fetch(s0);
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+      if (s0 + s < u.parts) {
+#pragma unroll
+        for (int j = 0; j < kMine; ++j) {
+          const int i = e + 128 * j;
+          if (i < G * D) acc[j] += w_m[(s0 + s) * G + i / D] * v[s][j];
+        }
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < kMine; ++j) {
+    const int i = e + 128 * j, h = i / D;
+    if (i < G * D) out[xcanon_offset(u.b, (u.kvl * G + h) * D + i - h * D, N)] = __float2bfloat16_rn(acc[j] * s_ml[8 + h]);
   }
 }
 
@@ -1937,6 +1971,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
   __shared__ float s_inv_buf[64];
   __shared__ float s_red[128];
   __shared__ float s_scale[X ? 32 : 1];
+  __shared__ __align__(16) unsigned char s_op[2][kChainOpBytes];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c = (int)cluster_ctarank(), cid = (int)blockIdx.x / kChainC, ncl = (int)gridDim.x / kChainC;
@@ -1968,7 +2003,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
 
   if (warp == 0) {
     // ---------------- weights ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint64_t pol_w;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(pol_w));
       int it = 0;
@@ -2015,7 +2050,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
   } else if (warp == 6) {
     // ---------------- activations ----------------
     pdl_wait();
-    if (lane == 0) {
+    if (elect_one()) {
       uint64_t pol_x;
       asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(pol_x));
       int it = 0;
@@ -2094,14 +2129,26 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
     const uint32_t to_bar = dsmem_addr(smem_u32(&recv_full), (uint32_t)q);
     int seg = 0, g = 0;                        // accumulators drained, tiles exchanged
     int it = 0;                                // the ring's stages, which only attention reads here
+    // The links' parameters, a link ahead: a constant-bank line that is read for the first time takes about half a microsecond, one after the other, and
+    // q/k/v's epilogue needs eight of them.
+    auto fetch_op = [&](int o) {
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(&P.op[o]);
+      for (int i = e; i < kChainOpBytes / 4; i += 128) reinterpret_cast<uint32_t*>(s_op[o & 1])[i] = from[i];
+    };
+    fetch_op(0);
+    asm volatile("bar.sync 1, 128;\n" ::: "memory");
     for (int o = 0; o < P.n_ops; ++o) {
-      const GemvParams& p = P.op[o];
+      const GemvParams& p = *reinterpret_cast<const GemvParams*>(s_op[o & 1]);
       if (D > 0 && p.epi == EPI_ATTEND) {
         const int units = p.B * p.KVl * p.ksplit;
-        if ((int)blockIdx.x >= units) continue;
-        if (o > 0) {
+        if (o > 0 && (int)blockIdx.x < units) {
           if (e == 0) chain_wait_done(P.done + (o - 1) * kChainLine, chain_ctas(P.op[o - 1], ncl), dead, err);
           asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        }
+        if (o + 1 < P.n_ops) fetch_op(o + 1);                     // (the other half: everybody is done with the link before)
+        if ((int)blockIdx.x >= units) {
+          asm volatile("bar.sync 1, 128;\n" ::: "memory");
+          continue;
         }
         // the receive buffer is free: what the peers send next needs this link's outputs
         const int it0 = it;
@@ -2109,7 +2156,6 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
           const ChainUnit w = chain_unit(p, u);
           if (w.begin < w.end) chain_attend<(D > 0 ? D : 64), N, ST>(p, w, it, smem, full_bar, empty_bar, const_cast<float*>(reinterpret_cast<const float*>(recv)), s_red, e, dead, err);
         }
-        asm volatile("fence.proxy.async;\n" ::: "memory");
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
         if (e == 0 && it != it0) asm volatile("red.release.cta.shared.add.u32 [%0], 1;\n" ::"r"(smem_u32(&attended)) : "memory");
         if (e == 0 && o + 1 < P.n_ops) asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
@@ -2117,7 +2163,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
       }
       const int KS = (p.K + 127) >> 7, nrbg = (p.rows + 127) >> 7;
       const int n_steps = (c + 1) * KS / kChainC - c * KS / kChainC;
-      if (cid >= nrbg) continue;
+      if (cid >= nrbg) {
+        if (o + 1 < P.n_ops) fetch_op(o + 1);
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        continue;
+      }
       if (D > 0) it += n_steps * ((nrbg - cid + ncl - 1) / ncl);
       const float* s_inv = p.inv.ssq ? s_inv_buf : nullptr;
       if (o > 0) {
@@ -2125,6 +2175,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
       }
       compute_inv_scale(p.inv, s_inv_buf, e);
+      if (o + 1 < P.n_ops) fetch_op(o + 1);
       for (int r = cid; r < nrbg; r += ncl, ++g) {
         const int row0 = r * 128 + c * 32;
         // what the epilogue reads besides the accumulators, fetched while the weights stream
@@ -2187,9 +2238,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) gemv_chain_kernel(const __gr
           }
         }
         const bool last = r + ncl >= nrbg && o + 1 < P.n_ops;
-        if (last) asm volatile("fence.proxy.async;\n" ::: "memory");
         asm volatile("bar.sync 1, 128;\n" ::: "memory");         // the receive buffer has been read
-        // the barrier puts every thread's stores before thread 0's release, which covers them
+        // The barrier puts every thread's stores before thread 0's release, which covers them.  (The bulk copies that read them are behind a proxy fence
+        // on the reader's side, after its acquire; another one here, by all threads, cost a microsecond per link.)
         if (last && e == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(P.done + o * kChainLine) : "memory");
         if (e < kChainC) mbar_arrive_remote(dsmem_addr(smem_u32(&send_ok), (uint32_t)e));
       }
@@ -2484,15 +2535,16 @@ bool gemv_chain_attends(int B, int G, int D) {
   return (D == 64 || D == 96 || D == 128) && G >= 1 && G <= 8 && G * D <= 32 * Layout<__nv_bfloat16>::batch_pad(B);
 }
 
-// One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge).  Parts beyond the first also cost the
-// merge over CTAs, and their pairs of maximum and sum must fit the receive buffer: at most 64.
+// One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge).  The merge of several parts -- partial
+// results out, a counter, and back -- costs 4 us, in which a CTA streams some 640 keys (Llama-3-8B shape, one sequence of 1031 keys, nine parts: the
+// last one 11.8 us after q/k/v, the others 4.6).  Their pairs of maximum and sum must fit the receive buffer: at most 64 parts.
 void gemv_chain_attention_plan(int clusters, int B, int KVl, int capacity, int* keys_per_cta, int* nsplit) {
   const int64_t pairs = (int64_t)B * KVl, ctas = (int64_t)clusters * kChainC, cap = round_up(capacity, 64);
   int64_t best = cap, best_cost = ceil_div(pairs, ctas) * (cap + 48);
   for (int64_t k = 64; k < cap; k += 64) {
     const int64_t ns = ceil_div(cap, k);
     if (ns > 64) continue;
-    const int64_t cost = ceil_div(pairs * ns, ctas) * (k + 48) + 64;
+    const int64_t cost = ceil_div(pairs * ns, ctas) * (k + 48) + 640;
     if (cost < best_cost) { best_cost = cost; best = k; }
   }
   *keys_per_cta = (int)best;
