@@ -4,10 +4,9 @@
 //
 // One CTA = two tiles of 128 query rows of one (batch, head) sharing the key/value stream, keys in
 // tiles of 128:
-//   2 loader warps : Q by cp.async 16-byte chunks into the canonical core-matrix layout (8 rows x 16
-//                    bytes); then one warp streams K and the other V by TMA (cp.async.bulk.tensor over
-//                    a 4-D map d / key / kv head / batch, 2 stages each): a key tile lands as D / W
-//                    sub-tiles of [128 keys][W head dims] in the 128-byte (W = 64) or 64-byte (W = 32,
+//   2 loader warps : one brings Q and streams K, the other V, by TMA (cp.async.bulk.tensor over 4-D
+//                    maps d / row / head / batch, 2 stages each for K and V): a tile lands as D / W
+//                    sub-tiles of [128 rows][W head dims] in the 128-byte (W = 64) or 64-byte (W = 32,
 //                    head_dim 96) swizzle, which the tensor core reads K-major for Q K^T and MN-major
 //                    for P V;
 //   1 MMA warp     : one thread issues tcgen05.mma for both query tiles -- S = Q K^T (M 128, N 128,
@@ -26,7 +25,14 @@
 // all operands from shared memory, 160 KB of operand reads per 128 keys and tile -- ran at 709
 // TFLOP/s on [4, 32, 4096, 128]; 128-key tiles with P in tensor memory 729; two softmax threads
 // per row 948; packed float32 pairs and three-input maxima in the softmax 959; MMAs issued under an elected branch (tc::elect_one) 983 -> 1049
-// on one box.)
+// on one box; what follows 1047 -> 1126.)
+// A CTA holds the SM alone, so what it does outside its key loop is not hidden by another: 17000 clocks of
+// 136000 with 4096 keys, of 25000 with 256.  Q by TMA before the block's first barrier instead of by copies of
+// 16 bytes (any number of threads: the load path took 14 bytes a clock) has the first scores there after 3600
+// clocks instead of 10400; O through shared memory as whole runs of a row takes 1700 instead of 4500; and a
+// masked tile compares each key once, without branches, which took 10 us off every causal CTA.
+// [4, 32, 4096, 128]: 1048 -> 977 us, causal 752 -> 588; [4, 32, 4096, 64] 1008 -> 935; head_dim 96 causal
+// 723 -> 602; 148 heads of 256 queries 15.4 -> 10.1.
 // Causal: key tiles beyond a query tile's diagonal are never computed; inside the diagonal tile
 // keys j > i are masked -- the reference's `if causal && j > i continue`.
 #include <cuda.h>
@@ -54,11 +60,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
   return y;
-}
-
-// chunk (row, d8) of a [rows x D] row-major tile -> canonical offset [d8][row/8][row%8][16 B]
-__device__ __forceinline__ uint32_t canon(int row, int c8, int rows) {
-  return (uint32_t)(c8 * (rows * 16) + (row >> 3) * 128 + (row & 7) * 16);
 }
 
 // Shared-memory descriptor of a tile in the 128-byte (layout type 2) or 64-byte (type 4) swizzle a
@@ -153,7 +154,7 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uin
 // code of them
 template <int DN, int DR, int DV, int WIN>
 __global__ void __launch_bounds__(kThreads, 1)
-flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q, const __grid_constant__ CUtensorMap kmap,
+flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap qrmap, const __grid_constant__ CUtensorMap kmap,
                    const __grid_constant__ CUtensorMap vmap, const __grid_constant__ CUtensorMap rmap, const FlashView fv, const FlashExtra ex, int S_all,
                    float scale, int causal, int* err) {
   constexpr int D = DN + DR;
@@ -165,7 +166,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   typedef Smem<DN, DR, DV> SM;
   constexpr int kStages = SM::kStages, vStages = SM::vStages;
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t q_full, k_full[kStages], k_empty[kStages], v_full[vStages], v_empty[vStages];
+  __shared__ __align__(8) uint64_t q_full[2], k_full[kStages], k_empty[kStages], v_full[vStages], v_empty[vStages];
   __shared__ __align__(8) uint64_t s_full[2], p_full[2], o_done[2], v_tail;
   __shared__ float xch[2][2][kBM];                    // [tile][column half][row]: the halves' row maxima, later their sums
   __shared__ uint32_t tmem_slot;
@@ -179,10 +180,8 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   const int row0 = ex.cu ? ex.cu[bi] : 0, S = ex.cu ? ex.cu[bi + 1] - row0 : S_all;
   if (q0 >= S) return;                                // a packed sequence shorter than the longest
   const int kv_b = ex.cu ? 0 : bi;
-  const __nv_bfloat16* qb = q + (ex.cu ? row0 * fv.q_s : bi * fv.q_b) + hi * fv.q_h;
   const int kvh = hi / fv.G;
   __nv_bfloat16* ob_base = out + (ex.cu ? row0 * ex.o_s : bi * ex.o_b) + hi * ex.o_h;
-  const int64_t q_s = fv.q_s;
   const int Sk = ex.cu ? S : ex.Sk, q_off = ex.q_off;
   int n_tiles[2], first[2];                           // key tiles first[t] .. n_tiles[t] - 1
 #pragma unroll
@@ -195,13 +194,30 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   const int n_max = max(n_tiles[0], n_tiles[1]);
   const int jb = WIN ? first[0] : 0;                  // the first query tile is never empty and starts no later than the second
 
-  if (tid == 0) {
-    mbar_init(&q_full, kLoaders / 32);
+  auto load_k = [&](int j) {                          // one thread: key tile j into its stage
+    const int s = (j - jb) % kStages;
+    unsigned char* at = smem + SM::offK + s * SM::kK;
+    mbar_expect_tx(&k_full[s], (uint32_t)SM::kK);
+    for (int sub = 0; sub < DN / W; ++sub) tma_load_4d(at + sub * kSub, &kmap, sub * W, row0 + j * kBN, kvh, kv_b, &k_full[s]);
+    for (int sub = 0; sub < DR / W; ++sub) tma_load_4d(at + (DN / W + sub) * kSub, &rmap, sub * W, row0 + j * kBN, 0, kv_b, &k_full[s]);
+  };
+  if (warp == kMmaWarp + 1 && lane == 0) {
+    for (int t = 0; t < 2; ++t) mbar_init(&q_full[t], 1);
     for (int s = 0; s < kStages; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
     for (int s = 0; s < vStages; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 8); mbar_init(&o_done[t], 1); }
     mbar_init(&v_tail, 1);
     mbar_init_fence();
+    // the queries and the first keys are on their way before the block's first barrier
+    for (int t = 0; t < 2; ++t) {
+      if (q0 + t * kBM < S) {
+        unsigned char* at = smem + SM::offQ + t * SM::kQ;
+        mbar_expect_tx(&q_full[t], (uint32_t)SM::kQ);
+        for (int sub = 0; sub < DN / W; ++sub) tma_load_4d(at + sub * kSub, &qmap, sub * W, row0 + q0 + t * kBM, hi, kv_b, &q_full[t]);
+        for (int sub = 0; sub < DR / W; ++sub) tma_load_4d(at + (DN / W + sub) * kSub, &qrmap, sub * W, row0 + q0 + t * kBM, hi, kv_b, &q_full[t]);
+      }
+      if (t == 0 && n_max > jb) load_k(jb);
+    }
   }
   if (warp == kMmaWarp) tmem_alloc(&tmem_slot, kTmemCols);
   fence_before();
@@ -211,49 +227,35 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
   bool dead = false;
 
   if (warp > kMmaWarp) {
-    // ------------------------------ loaders: Q by both warps, then K by one and V by the other ------------------------------
-    const int lw = warp - kMmaWarp - 1, lt = tid - (kMmaWarp + 1) * 32;
-    const uint32_t sQ = smem_u32(smem + SM::offQ);
-    for (int i = lt; i < 2 * kBM * (D / 8); i += kLoaders) {
-      const int row = i / (D / 8), c8 = i - row * (D / 8);
-      const int qi = q0 + row;
-      const int d = c8 * 8;                                  // the padding behind either part of a query is zero
-      const bool valid = qi < S && ((DR == 0 && !WIN) || (d < DN ? d < ex.dn : d - DN < ex.dr));
-      const int src = DR == 0 || d < DN ? d : ex.dn + d - DN;
-      cp_async16(sQ + (row >> 7) * SM::kQ + canon(row & 127, c8, kBM), qb + (int64_t)min(qi, S - 1) * q_s + (valid ? src : 0), valid ? 16u : 0u);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    fence_async_smem();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&q_full);
-    uint64_t* full = lw == 0 ? k_full : v_full;
-    uint64_t* empty = lw == 0 ? k_empty : v_empty;
-    const CUtensorMap* map = lw == 0 ? &kmap : &vmap;
-    const int off = lw == 0 ? SM::offK : SM::offV;
-    const int stages = lw == 0 ? kStages : vStages, stage_bytes = lw == 0 ? SM::kK : SM::kV, subs = (lw == 0 ? DN : DV) / W;
-    for (int j = jb; j < n_max; ++j) {
-      const int s = (j - jb) % stages;
-      mbar_wait(&empty[s], (((j - jb) / stages) & 1) ^ 1, dead, err);
-      const bool tail = ex.cu && lw == 1 && (j + 1) * kBN > Sk;
-      unsigned char* at = smem + off + s * stage_bytes;
-      if (lane == 0) {
-        uint64_t* bar = tail ? &v_tail : &full[s];
-        mbar_expect_tx(bar, (uint32_t)stage_bytes);
-        for (int sub = 0; sub < subs; ++sub) tma_load_4d(at + sub * kSub, map, sub * W, row0 + j * kBN, kvh, kv_b, bar);
-        if (DR > 0 && lw == 0)
-          for (int sub = 0; sub < DR / W; ++sub) tma_load_4d(at + (DN / W + sub) * kSub, &rmap, sub * W, row0 + j * kBN, 0, kv_b, &full[s]);
-      }
-      __syncwarp();
-      if (tail) {
-        // rows behind a packed sequence's end are the next one's: their weight is 0, but 0 times an infinity or NaN over there
-        // would reach this sequence.  Whole rows are cleared, so the swizzle does not matter
-        mbar_wait(&v_tail, 0, dead, err);
-        for (int sub = 0; sub < subs; ++sub)
-          for (int i = (Sk - j * kBN) * (W / 8) + lane; i < kBN * (W / 8); i += 32) reinterpret_cast<uint4*>(at + sub * kSub)[i] = make_uint4(0, 0, 0, 0);
-        fence_async_smem();
+    // ------------------------------ loaders: one warp streams K (its first tile is under way), the other V ------------------------------
+    if (warp == kMmaWarp + 1) {
+      for (int j = jb + 1; j < n_max; ++j) {
+        mbar_wait(&k_empty[(j - jb) % kStages], (((j - jb) / kStages) & 1) ^ 1, dead, err);
+        if (lane == 0) load_k(j);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full[s]);
+      }
+    } else {
+      for (int j = jb; j < n_max; ++j) {
+        const int s = (j - jb) % vStages;
+        mbar_wait(&v_empty[s], (((j - jb) / vStages) & 1) ^ 1, dead, err);
+        const bool tail = ex.cu && (j + 1) * kBN > Sk;
+        unsigned char* at = smem + SM::offV + s * SM::kV;
+        if (lane == 0) {
+          uint64_t* bar = tail ? &v_tail : &v_full[s];
+          mbar_expect_tx(bar, (uint32_t)SM::kV);
+          for (int sub = 0; sub < DV / W; ++sub) tma_load_4d(at + sub * kSub, &vmap, sub * W, row0 + j * kBN, kvh, kv_b, bar);
+        }
+        __syncwarp();
+        if (tail) {
+          // rows behind a packed sequence's end are the next one's: their weight is 0, but 0 times an infinity or NaN over there
+          // would reach this sequence.  Whole rows are cleared, so the swizzle does not matter
+          mbar_wait(&v_tail, 0, dead, err);
+          for (int sub = 0; sub < DV / W; ++sub)
+            for (int i = (Sk - j * kBN) * (W / 8) + lane; i < kBN * (W / 8); i += 32) reinterpret_cast<uint4*>(at + sub * kSub)[i] = make_uint4(0, 0, 0, 0);
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&v_full[s]);
+        }
       }
     }
   } else if (warp == kMmaWarp) {
@@ -261,14 +263,14 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
     constexpr uint32_t kIdescS = idesc_bf16(kBM, kBN, false, false);
     constexpr uint32_t kIdescPV = idesc_bf16(kBM, DV, false, true);          // V is read MN-major
     if (elect_one()) {
-      mbar_wait(&q_full, 0, dead, err);
       auto issue_s = [&](int j, int t) {                // S[t] = Q[t] K(j)^T
-        const uint64_t adesc = smem_desc(smem_u32(smem + SM::offQ + t * SM::kQ), kBM * 16, 128);
+        const uint32_t sQ = smem_u32(smem + SM::offQ + t * SM::kQ);
         const uint32_t sK = smem_u32(smem + SM::offK + ((j - jb) % kStages) * SM::kK);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
-          const uint64_t bdesc = smem_desc_swz(sK + ((16 * ks) / W) * kSub + ((16 * ks) % W) * 2, 16, 16 * W, kSwz);
-          mma_f16(tmem + kColS + t * kBN, adesc + (uint64_t)(ks * ((2 * kBM * 16) >> 4)), bdesc, kIdescS, ks ? 1u : 0u);
+          constexpr auto at = [](int k) { return (uint32_t)(((16 * k) / W) * kSub + ((16 * k) % W) * 2); };
+          const uint64_t adesc = smem_desc_swz(sQ + at(ks), 16, 16 * W, kSwz), bdesc = smem_desc_swz(sK + at(ks), 16, 16 * W, kSwz);
+          mma_f16(tmem + kColS + t * kBN, adesc, bdesc, kIdescS, ks ? 1u : 0u);
         }
         commit(&s_full[t]);
       };
@@ -285,7 +287,11 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
         fence_after();
 #pragma unroll
         for (int t = 0; t < 2; ++t)
-          if (first[t] == jb && n_tiles[t] > jb) issue_s(jb, t);
+          if (first[t] == jb && n_tiles[t] > jb) {
+            mbar_wait(&q_full[t], 0, dead, err);
+            fence_after();
+            issue_s(jb, t);
+          }
         commit(&k_empty[0]);
       }
       for (int j = jb; j < n_max; ++j) {
@@ -297,7 +303,10 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
           if (j >= n_tiles[t]) continue;
           if (WIN && j < first[t]) {                       // the second query tile's window starts one key tile later
             fence_after();
-            if (j + 1 == first[t] && j + 1 < n_tiles[t]) issue_s(j + 1, t);
+            if (j + 1 == first[t] && j + 1 < n_tiles[t]) {
+              mbar_wait(&q_full[t], 0, dead, err);
+              issue_s(j + 1, t);
+            }
             continue;
           }
           mbar_wait(&p_full[t], (j - first[t]) & 1, dead, err);
@@ -343,7 +352,6 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
       p = fma2(p, u, pc[0]);
       return fma2(z, p, plus);
     };
-    auto hidden = [&](int key) { return key >= Sk || (causal && key > q_off + qi) || (WIN && ex.window > 0 && key <= q_off + qi - ex.window); };
     // keys key_lo .. key_lo + key_span are visible to this row
     const int key_hi = min(Sk - 1, causal ? q_off + qi : Sk - 1), key_lo = WIN && ex.window > 0 ? q_off + qi - ex.window + 1 : 0;
     const unsigned key_span = (unsigned)max(key_hi - key_lo, 0);      // (rows behind the last query are never stored)
@@ -352,7 +360,10 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
     for (int j = j0; j < nt; ++j) {
       mbar_wait(&s_full[t], (j - j0) & 1, dead, err);          // S(j) is complete, and with it (pipe order) P V(j - 1): O is at rest
       fence_after();
-      const int key0 = j * kBN + h * 64;
+      const int key0 = j * kBN + h * 64, last_seen = key_hi - key0;
+      // is key key0 + i visible?  One comparison and a select: as a chain of conditions every masked key was a branch of its own, and a
+      // tile on the diagonal took 5 us longer than one inside
+      auto seen = [&](int i) { return WIN ? (unsigned)(key0 + i - key_lo) <= key_span : i <= last_seen; };
       const bool inside = (j + 1) * kBN <= Sk && (!causal || (j + 1) * kBN - 1 <= q_off + q0 + t * kBM) &&
                           (!WIN || ex.window == 0 || j * kBN > q_off + q0 + t * kBM + kBM - 1 - ex.window);   // no key of the tile is masked
       // pass 1: the maximum of this thread's 64 scores
@@ -367,8 +378,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const int key = key0 + qd * 32 + i;
-            if (WIN ? (unsigned)(key - key_lo) <= key_span : !hidden(key)) mx4[i & 3] = fmaxf(mx4[i & 3], sv[i]);
+            mx4[i & 3] = fmaxf(mx4[i & 3], seen(qd * 32 + i) ? sv[i] : -CUDART_INF_F);
           }
         }
       }
@@ -414,7 +424,6 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
           float a0 = sv[i], a1 = sv[i + 1];
-          const int key = key0 + qd * 16 + i;
           float x0, x1;
           if (WIN && capl > 0.f) {
             if (WIN == 2 && (i & 2)) {                     // every other pair on the FMA pipe, the others on the exp2 unit
@@ -425,13 +434,13 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
               unpack2(fma2(pack2(rcp_approx(x0), rcp_approx(x1)), m2capl2, pack2(capl + neg_m, capl + neg_m)), x0, x1);
             }
             if (!inside) {
-              if ((unsigned)(key - key_lo) > key_span) x0 = -CUDART_INF_F;
-              if ((unsigned)(key + 1 - key_lo) > key_span) x1 = -CUDART_INF_F;
+              x0 = seen(qd * 16 + i) ? x0 : -CUDART_INF_F;
+              x1 = seen(qd * 16 + i + 1) ? x1 : -CUDART_INF_F;
             }
           } else {
             if (!inside) {
-              if (hidden(key)) a0 = -CUDART_INF_F;
-              if (hidden(key + 1)) a1 = -CUDART_INF_F;
+              a0 = seen(qd * 16 + i) ? a0 : -CUDART_INF_F;
+              a1 = seen(qd * 16 + i + 1) ? a1 : -CUDART_INF_F;
             }
             unpack2(fma2(pack2(a0, a1), c2, negm2), x0, x1);
           }
@@ -467,23 +476,37 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict
       fence_after();
       float inv = 1.0f / l;
       if (DR > 0 && ex.gate && qi < S) inv *= 1.0f / (1.0f + expf(-ex.gate[((int64_t)bi * S + qi) * ex.gate_pitch + hi]));
-      __nv_bfloat16* ob = ob_base + (int64_t)qi * ex.o_s + h * (DV / 2);
+      // The warp's 32 rows x DV / 2 columns are turned through its share of the tile's query buffer (every product that read it is
+      // done), so that a store instruction writes whole runs of a row: from the threads that hold a row each, it wrote 32 pieces of 16 bytes
+      constexpr int kCols = DV <= D ? DV / 2 : DV / 2 * D / DV, kPieces = kCols / 8;      // columns per pass, 16-byte pieces of them
+      static_assert(kCols % 16 == 0 && (DV / 2) % kCols == 0 && 8 * 32 * kCols * 2 <= SM::kQ, "a warp's share of the query buffer");
+      uint4* st = reinterpret_cast<uint4*>(smem + SM::offQ + t * SM::kQ) + (h * 4 + wq) * (32 * kPieces);
+      auto slot = [](int row, int piece) { return row * kPieces + (kPieces == 8 ? piece ^ (row & 7) : kPieces == 4 ? piece ^ ((row >> 1) & 3) : piece); };
+      const int out_row0 = q0 + t * kBM + 32 * wq;
 #pragma unroll
-      for (int ch = 0; ch < DV / 32; ++ch) {
-        float o[16];
-        tmem_ld16(o, tmem + lane_base + colO + ch * 16);
-        if (qi < S) {
+      for (int c0 = 0; c0 < DV / 2; c0 += kCols) {
+#pragma unroll
+        for (int ch = 0; ch < kCols / 16; ++ch) {
+          float o[16];
+          tmem_ld16(o, tmem + lane_base + colO + c0 + ch * 16);
 #pragma unroll
           for (int i = 0; i < 16; i += 8) {
-            if ((DR > 0 || WIN) && h * (DV / 2) + ch * 16 + i >= ex.dv) continue;      // padding behind the value's width
             uint4 w;
             __nv_bfloat162 a0 = __floats2bfloat162_rn(o[i] * inv, o[i + 1] * inv), a1 = __floats2bfloat162_rn(o[i + 2] * inv, o[i + 3] * inv);
             __nv_bfloat162 a2 = __floats2bfloat162_rn(o[i + 4] * inv, o[i + 5] * inv), a3 = __floats2bfloat162_rn(o[i + 6] * inv, o[i + 7] * inv);
             w.x = *reinterpret_cast<uint32_t*>(&a0); w.y = *reinterpret_cast<uint32_t*>(&a1);
             w.z = *reinterpret_cast<uint32_t*>(&a2); w.w = *reinterpret_cast<uint32_t*>(&a3);
-            *reinterpret_cast<uint4*>(ob + ch * 16 + i) = w;
+            st[slot(lane, ch * 2 + i / 8)] = w;
           }
         }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+          const int row = (i * 32 + lane) / kPieces, piece = (i * 32 + lane) % kPieces, col = h * (DV / 2) + c0 + piece * 8;
+          if (out_row0 + row < S && ((DR == 0 && !WIN) || col < ex.dv))             // (behind ex.dv: padding of the value's width)
+            *reinterpret_cast<uint4*>(ob_base + (int64_t)(out_row0 + row) * ex.o_s + col) = st[slot(row, piece)];
+        }
+        __syncwarp();
       }
       fence_before();
     }
@@ -566,10 +589,11 @@ int32_t flash_tc_launch_view(Ctx* ctx, void* out, const void* q, const void* k, 
                              int64_t S, int64_t D, float scale, int causal, cudaStream_t stream, const int* cu, int64_t total) {
   LMB_REQUIRE(!cu || causal, "flash attention: packed sequences are causal");
   dim3 grid((unsigned)ceil_div(S, 2 * kBM), (unsigned)(B * fv.H));
-  CUtensorMap kmap, vmap;
+  CUtensorMap qmap, kmap, vmap;
   const int W = D % 64 == 0 ? 64 : 32;
   const int64_t n_kv = fv.H / fv.G;
   const int64_t map_B = cu ? 1 : B, map_S = cu ? total : S;
+  LMB_TRY(kv_tensor_map(&qmap, q, fv.H, map_B, map_S, D, fv.q_s, fv.q_h, fv.q_b, W));
   LMB_TRY(kv_tensor_map(&kmap, k, n_kv, map_B, map_S, D, fv.k_s, fv.k_h, fv.k_b, W));
   LMB_TRY(kv_tensor_map(&vmap, v, n_kv, map_B, map_S, D, fv.k_s, fv.k_h, fv.k_b, W));
   FlashExtra ex;
@@ -578,7 +602,7 @@ int32_t flash_tc_launch_view(Ctx* ctx, void* out, const void* q, const void* k, 
   ex.o_b = fv.q_b; ex.o_h = fv.q_h; ex.o_s = fv.q_s;
 #define LMB_FLASH(DD)                                                                                                   \
   flash_tc_kernel<DD, 0, DD, 0><<<grid, kThreads, Smem<DD, 0, DD>::total + 1024, stream>>>(                          \
-      (__nv_bfloat16*)out, (const __nv_bfloat16*)q, kmap, vmap, kmap, fv, ex, (int)S, scale, causal, ctx->dev_err)
+      (__nv_bfloat16*)out, qmap, qmap, kmap, vmap, kmap, fv, ex, (int)S, scale, causal, ctx->dev_err)
   if (D == 128) LMB_FLASH(128);
   else if (D == 96) LMB_FLASH(96);
   else if (D == 64) LMB_FLASH(64);
@@ -602,7 +626,9 @@ int32_t flash_tc_launch_split(Ctx* ctx, void* out, const void* q, const void* k,
   LMB_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && f.q_s % 8 == 0 && f.q_h % 8 == 0 &&
                   f.q_b % 8 == 0 && f.o_s % 8 == 0 && f.o_h % 8 == 0 && f.o_b % 8 == 0,
               "flash attention: query and output rows must start on 16 bytes");
-  CUtensorMap kmap, vmap, rmap;
+  CUtensorMap qmap, qrmap, kmap, vmap, rmap;
+  LMB_TRY(kv_tensor_map(&qmap, q, f.H, B, Sq, f.dn, f.q_s, f.q_h, f.q_b, 64));
+  LMB_TRY(kv_tensor_map(&qrmap, (const __nv_bfloat16*)q + f.dn, f.H, B, Sq, f.dr, f.q_s, f.q_h, f.q_b, 64));
   LMB_TRY(kv_tensor_map(&kmap, k, f.H, B, Sk, f.dn, f.k_s, f.k_h, f.k_b, 64));
   LMB_TRY(kv_tensor_map(&vmap, v, f.H, B, Sk, f.dv, f.v_s, f.v_h, f.v_b, 64));
   LMB_TRY(kv_tensor_map(&rmap, kr, 1, B, Sk, f.dr, f.kr_s, 0, f.kr_b, 64));
@@ -616,7 +642,7 @@ int32_t flash_tc_launch_split(Ctx* ctx, void* out, const void* q, const void* k,
   const dim3 grid((unsigned)ceil_div(Sq, 2 * kBM), (unsigned)(B * f.H));
 #define LMB_FLASH(DN, DV)                                                                                              \
   flash_tc_kernel<DN, 64, DV, 0><<<grid, kThreads, Smem<DN, 64, DV>::total + 1024, stream>>>(                       \
-      (__nv_bfloat16*)out, (const __nv_bfloat16*)q, kmap, vmap, rmap, fv, ex, (int)Sq, scale, 1, ctx->dev_err)
+      (__nv_bfloat16*)out, qmap, qrmap, kmap, vmap, rmap, fv, ex, (int)Sq, scale, 1, ctx->dev_err)
   if (f.dn <= 64 && f.dv <= 64) LMB_FLASH(64, 64);
   else if (f.dn <= 64) LMB_FLASH(64, 128);
   else if (f.dv <= 64) LMB_FLASH(128, 64);
@@ -656,7 +682,8 @@ int32_t flash_tc_launch_window(Ctx* ctx, void* out, const void* q, const void* k
   LMB_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && f.q_s % 8 == 0 && f.q_h % 8 == 0 &&
                   f.q_b % 8 == 0 && f.o_s % 8 == 0 && f.o_h % 8 == 0 && f.o_b % 8 == 0,
               "flash attention: query and output rows must start on 16 bytes");
-  CUtensorMap kmap, vmap;
+  CUtensorMap qmap, kmap, vmap;
+  LMB_TRY(kv_tensor_map(&qmap, q, f.H, B, Sq, f.dn, f.q_s, f.q_h, f.q_b, 64));
   LMB_TRY(kv_tensor_map(&kmap, k, f.H / f.G, B, Sk, f.dn, f.k_s, f.k_h, f.k_b, 64));
   LMB_TRY(kv_tensor_map(&vmap, v, f.H / f.G, B, Sk, f.dv, f.v_s, f.v_h, f.v_b, 64));
   FlashView fv;
@@ -672,7 +699,7 @@ int32_t flash_tc_launch_window(Ctx* ctx, void* out, const void* q, const void* k
   const dim3 grid((unsigned)ceil_div(Sq, 2 * kBM), (unsigned)(B * f.H));
 #define LMB_FLASH(DN, DV, W)                                                                                           \
   flash_tc_kernel<DN, 0, DV, W><<<grid, kThreads, Smem<DN, 0, DV>::total + 1024, stream>>>(                            \
-      (__nv_bfloat16*)out, (const __nv_bfloat16*)q, kmap, vmap, kmap, fv, ex, (int)Sq, scale, 1, ctx->dev_err)
+      (__nv_bfloat16*)out, qmap, qmap, kmap, vmap, kmap, fv, ex, (int)Sq, scale, 1, ctx->dev_err)
 #define LMB_PICK(DN, DV) do { if (poly) LMB_FLASH(DN, DV, 2); else LMB_FLASH(DN, DV, 1); } while (0)
   if (f.dn <= 64 && f.dv <= 64) LMB_PICK(64, 64);
   else if (f.dn <= 64) LMB_PICK(64, 128);
