@@ -14,9 +14,10 @@
 //                    K 128) with P read FROM TENSOR MEMORY (the A operand), accumulating O in tensor
 //                    memory over all key tiles; tcgen05.commit signals mbarriers;
 //   16 softmax warps, two threads per query row (warps w and w + 8 reach the same 32 lanes; each takes
-//                    64 of the tile's 128 keys): tcgen05.ld the scores twice (row maximum, then
-//                    exp2 with the scale folded in), exchange the halves' maxima through shared
-//                    memory, and tcgen05.st P as bf16 pairs over the columns of S.  The running maximum
+//                    64 of the tile's 128 keys): tcgen05.ld the scores (row maximum, then exp2 with
+//                    the scale folded in; read again for the second pass where registers do not
+//                    hold them), exchange the halves' maxima through shared memory, and tcgen05.st
+//                    P as bf16 pairs over the columns of S, in parts that the P V products follow.  The running maximum
 //                    is only raised -- and O rescaled in place -- when it grows by more than 2^8 (p
 //                    stays <= 256, exact in the final O / l).
 // S and P of a tile share their columns, so a tile runs S -> softmax -> P V strictly in turn and the
@@ -25,7 +26,7 @@
 // all operands from shared memory, 160 KB of operand reads per 128 keys and tile -- ran at 709
 // TFLOP/s on [4, 32, 4096, 128]; 128-key tiles with P in tensor memory 729; two softmax threads
 // per row 948; packed float32 pairs and three-input maxima in the softmax 959; MMAs issued under an elected branch (tc::elect_one) 983 -> 1049
-// on one box; what follows 1047 -> 1126.)
+// on one box; what follows 1047 -> 1126; scores held in registers and P in parts 1126 -> 1203.)
 // A CTA holds the SM alone, so what it does outside its key loop is not hidden by another: 17000 clocks of
 // 136000 with 4096 keys, of 25000 with 256.  Q by TMA before the block's first barrier instead of by copies of
 // 16 bytes (any number of threads: the load path took 14 bytes a clock) has the first scores there after 3600
@@ -167,7 +168,14 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
   constexpr int kStages = SM::kStages, vStages = SM::vStages;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t q_full[2], k_full[kStages], k_empty[kStages], v_full[vStages], v_empty[vStages];
-  __shared__ __align__(8) uint64_t s_full[2], p_full[2], o_done[2], v_tail;
+  // A softmax thread keeps the last kHeld of its 64 scores in registers between its two passes over them, so that P may overwrite the
+  // scores after the one barrier at which the halves exchange their maxima, and P goes to the tensor core in kParts parts: P V begins
+  // while the later keys are still being exponentiated.  Registers (96 a thread: 19 warps) and the products' share decide how much of
+  // it pays, [4, 32, 4096, D], all read twice -> as chosen: D 128 (32 held, 2 parts) 977 -> 914 us, all 64 held 1187 (spills);
+  // D 96 causal (64, 2) 602 -> 514, 32 held 577; D 64 (64, 1) 935 -> 881, 2 parts 889, 32 held 942.
+  constexpr int kHeld = WIN ? 0 : DN + DR >= 128 ? 32 : 64;
+  constexpr int kParts = WIN || DN + DR == 64 ? 1 : 2;
+  __shared__ __align__(8) uint64_t s_full[2], p_full[2][kParts], o_done[2], v_tail;
   __shared__ float xch[2][2][kBM];                    // [tile][column half][row]: the halves' row maxima, later their sums
   __shared__ uint32_t tmem_slot;
   constexpr uint32_t kTmemCols = 512;
@@ -205,7 +213,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
     for (int t = 0; t < 2; ++t) mbar_init(&q_full[t], 1);
     for (int s = 0; s < kStages; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
     for (int s = 0; s < vStages; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 8); mbar_init(&o_done[t], 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&o_done[t], 1); for (int i = 0; i < kParts; ++i) mbar_init(&p_full[t][i], 8); }
     mbar_init(&v_tail, 1);
     mbar_init_fence();
     // the queries and the first keys are on their way before the block's first barrier
@@ -277,9 +285,17 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
       auto issue_pv = [&](int j, int t) {               // O[t] += P[t] V(j), P read from tensor memory
         const uint64_t bdesc = smem_desc_swz(smem_u32(smem + SM::offV + ((j - jb) % vStages) * SM::kV), kSub, 16 * W, kSwz);
 #pragma unroll
-        for (int ks = 0; ks < kBN / 16; ++ks)
-          mma_f16_ts(tmem + kColO + t * DV, tmem + kColS + t * kBN + ks * 8, bdesc + (uint64_t)(ks * ((32 * W) >> 4)), kIdescPV,
-                     (j > first[t] || ks > 0) ? 1u : 0u);
+        for (int part = 0; part < kParts; ++part) {
+          mbar_wait(&p_full[t][part], (j - first[t]) & 1, dead, err);
+          fence_after();
+          constexpr int kHalf = kBN / 32, kRun = kHalf / kParts;      // 16-key steps of a half's 64 keys, and of one part of them
+#pragma unroll
+          for (int i = 0; i < 2 * kRun; ++i) {
+            const int ks = (i / kRun) * kHalf + part * kRun + i % kRun;
+            mma_f16_ts(tmem + kColO + t * DV, tmem + kColS + t * kBN + ks * 8, bdesc + (uint64_t)(ks * ((32 * W) >> 4)), kIdescPV,
+                       (j > first[t] || ks > 0) ? 1u : 0u);
+          }
+        }
         if (j == n_tiles[t] - 1) commit(&o_done[t]);
       };
       if (n_max > jb) {
@@ -309,8 +325,6 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
             }
             continue;
           }
-          mbar_wait(&p_full[t], (j - first[t]) & 1, dead, err);
-          fence_after();
           issue_pv(j, t);
           if (j + 1 < n_tiles[t]) issue_s(j + 1, t);       // runs after P V(j) in the tensor pipe: S overwrites P's columns
         }
@@ -324,7 +338,8 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
     // Two threads per query row: warps 0-7 take keys 0-63 of a tile, warps 8-15 keys 64-127 (a warp reaches the 32
     // tensor-memory lanes of its index modulo 4, so warp w and w + 8 see the same rows).  The two halves exchange
     // their row maxima through shared memory and a 64-thread barrier, keep their own partial sums, and each writes
-    // its half of P -- after a second barrier, because P's columns lie over the other half's scores.
+    // its half of P.  P's columns lie over the first half's scores: those that this barrier does not protect, the last
+    // 32 of its 64 (the second half's P), are in registers by then; with windows a second barrier stands before the writes.
     const int h = warp >> 3, t = (warp >> 2) & 1, wq = warp & 3;
     const int r = 32 * wq + lane;
     const int qi = q0 + t * kBM + r;
@@ -367,12 +382,31 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
       const bool inside = (j + 1) * kBN <= Sk && (!causal || (j + 1) * kBN - 1 <= q_off + q0 + t * kBM) &&
                           (!WIN || ex.window == 0 || j * kBN > q_off + q0 + t * kBM + kBM - 1 - ex.window);   // no key of the tile is masked
       // pass 1: the maximum of this thread's 64 scores
+      float held[kHeld ? kHeld : 1];
+      if constexpr (kHeld == 64) {                         // masked once, here
+        tmem_ld64(held, tmem + lane_base + colS);
+        if (!inside) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) held[i] = seen(i) ? held[i] : -CUDART_INF_F;
+        }
+      }
       float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
       for (int qd = 0; qd < 2; ++qd) {
         float sv[32];
-        tmem_ld32(sv, tmem + lane_base + colS + qd * 32);
-        if (inside) {
+        if constexpr (kHeld == 64) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sv[i] = held[qd * 32 + i];
+        } else {
+          tmem_ld32(sv, tmem + lane_base + colS + qd * 32);
+        }
+        if constexpr (kHeld == 32) {
+          if (qd == 1) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) held[i] = sv[i];
+          }
+        }
+        if (kHeld == 64 || inside) {
 #pragma unroll
           for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], sv[i], sv[i + 1]);
         } else {
@@ -413,14 +447,19 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
       if (raise) { l *= exp2f(m - mx); m = mx; }
       if (starts) m = mx;
       const float neg_m = m == -CUDART_INF_F ? 0.f : -m;
-      // pass 2: p = exp2(s c - m) as bf16 pairs, kept in registers until the other half has read its scores too
+      // pass 2: p = exp2(s c - m) as bf16 pairs, P's columns lie over the first half's scores
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};           // four chains of (even, odd) partial sums
       const uint64_t c2 = pack2(c, c), negm2 = pack2(neg_m, neg_m);
       uint32_t packed[32];
 #pragma unroll
       for (int qd = 0; qd < 4; ++qd) {
         float sv[16];
-        tmem_ld16(sv, tmem + lane_base + colS + qd * 16);
+        if (qd * 16 >= 64 - kHeld) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) sv[i] = held[kHeld ? qd * 16 + i - (64 - kHeld) : 0];
+        } else {
+          tmem_ld16(sv, tmem + lane_base + colS + qd * 16);
+        }
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
           float a0 = sv[i], a1 = sv[i + 1];
@@ -438,7 +477,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
               x1 = seen(qd * 16 + i + 1) ? x1 : -CUDART_INF_F;
             }
           } else {
-            if (!inside) {
+            if (kHeld < 64 && !inside) {
               a0 = seen(qd * 16 + i) ? a0 : -CUDART_INF_F;
               a1 = seen(qd * 16 + i + 1) ? a1 : -CUDART_INF_F;
             }
@@ -449,30 +488,33 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
           const __nv_bfloat162 pb2 = __floats2bfloat162_rn(p0, p1);
           packed[qd * 8 + i / 2] = *reinterpret_cast<const uint32_t*>(&pb2);
         }
+        constexpr int kQd = 4 / kParts;
+        if (qd % kQd == kQd - 1) {                           // a part of P is complete
+          if (!kHeld) asm volatile("bar.sync %0, 64;\n" ::"r"(pair_bar) : "memory");      // the other half has read its scores too
+#pragma unroll
+          for (int w0 = (qd - kQd + 1) * 8; w0 < (qd + 1) * 8; w0 += 16) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[i] = packed[w0 + i];
+            tmem_st16_nowait(tmem + lane_base + colP + w0, pk);
+          }
+          tmem_st_wait();
+          fence_before();                  // orders the stores (P, a rescaled O) before the MMAs that the arrive releases
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[t][qd / kQd]);
+        }
       }
       {
         float e, o;
         unpack2(add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3])), e, o);
         l += e + o;
       }
-      asm volatile("bar.sync %0, 64;\n" ::"r"(pair_bar) : "memory");
-      {
-        uint32_t lo[16], hi2[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { lo[i] = packed[i]; hi2[i] = packed[16 + i]; }
-        tmem_st16_nowait(tmem + lane_base + colP, lo);
-        tmem_st16_nowait(tmem + lane_base + colP + 16, hi2);
-      }
-      tmem_st_wait();
-      fence_before();                    // orders the stores (P, a rescaled O) before the MMA that the arrive releases
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
     }
     if (nt > j0) {
+      mbar_wait(&o_done[t], 0, dead, err);            // the last P V has landed, so both halves have read their last maxima
       xch[t][h][r] = l;
       asm volatile("bar.sync %0, 64;\n" ::"r"(pair_bar) : "memory");
       l += xch[t][h ^ 1][r];
-      mbar_wait(&o_done[t], 0, dead, err);            // the last P V has landed
       fence_after();
       float inv = 1.0f / l;
       if (DR > 0 && ex.gate && qi < S) inv *= 1.0f / (1.0f + expf(-ex.gate[((int64_t)bi * S + qi) * ex.gate_pitch + hi]));
@@ -562,15 +604,15 @@ EncodeTiledFn flash_encode_fn() {
   }
   return fn;
 }
-// 4-D map over K or V: dims {d, key, kv head, batch}; a box is [kBN keys][W head dims], swizzled over its W * 2 bytes.  Keys past S and
+// 4-D map over Q, K or V: dims {d, row, head, batch}; a box is [kBN rows][W head dims], swizzled over its W * 2 bytes.  Keys past S and
 // features past D arrive as zeros (the softmax masks the former).
 int32_t kv_tensor_map(CUtensorMap* map, const void* base, int64_t n_kv, int64_t B, int64_t S, int64_t D, int64_t k_s, int64_t k_h, int64_t k_b, int W) {
   EncodeTiledFn enc = flash_encode_fn();
   if (!enc) return fail(LMB200_ECUDA, "flash attention: cuTensorMapEncodeTiled is not available");
   const int64_t head_stride = n_kv > 1 ? k_h : S * k_s;           // a dimension of extent 1 still needs a valid stride
-  const int64_t batch_stride = B > 1 ? k_b : S * k_s * n_kv;
+  const int64_t batch_stride = B > 1 ? k_b : S * k_s;            // (times n_kv it could pass the 2^40 bytes a map's stride may have)
   LMB_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0 && k_s % 8 == 0 && head_stride % 8 == 0 && batch_stride % 8 == 0,
-              "flash attention: K / V base and strides must be multiples of 16 bytes");
+              "flash attention: Q / K / V base and strides must be multiples of 16 bytes");
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)S, (cuuint64_t)n_kv, (cuuint64_t)B};
   const cuuint64_t strides[3] = {(cuuint64_t)k_s * 2, (cuuint64_t)head_stride * 2, (cuuint64_t)batch_stride * 2};
   const cuuint32_t box[4] = {(cuuint32_t)W, (cuuint32_t)kBN, 1, 1};
