@@ -1500,8 +1500,9 @@ int32_t advance_launch(Session* S, cudaStream_t st) {
 
 namespace {
 
-// The fused decode step of a bf16 Llama / Phi-3: two launches per layer (attention, and the GEMVs from there to the next attention as
-// one chain), or five where every GEMV is its own launch (tensor parallelism).  The residual add and the
+// The fused decode step of a bf16 Llama / Phi-3: a launch per eight layers (every GEMV and attention a link of one chain), two launches per
+// layer (attention, and the GEMVs from there to the next attention as one chain) where attention cannot be a link, or five where every
+// GEMV is its own launch (tensor parallelism).  The residual add and the
 // RMSNorm around every Linear (src/NN.jl:406-414, 149-161) are carried by the projections themselves:
 // o_proj and down_proj finish with EPI_RESID_NORM (under tensor parallelism including the all-reduce of
 // their partial sums), q/k/v, gate/up and the head multiply their accumulators by the norm's
@@ -1750,7 +1751,8 @@ int32_t whisper_step_table(Session* S) {
   return whisper_step_layers(table, L, S->whisper_step, M->ctx->stream);
 }
 
-// The fused decode step of the bf16 Whisper decoder: eight launches per layer instead of eleven.  As in the Llama
+// The fused decode step of the bf16 Whisper decoder: two launches where S->whisper_step says so (whisper_step.cu), else eight per
+// layer instead of the eleven with norm kernels.  In that form, as in the Llama
 // step the residual add and the norm around every Linear ride on the projections: out_proj (self and cross) and fc2
 // finish with EPI_RESID_NORM (their own bias added on the way), which leaves x * gain and the per-sequence sums of x
 // and x^2; q/k/v, the cross q projection, fc1 and the tied head apply the LayerNorm to their accumulators
