@@ -576,6 +576,7 @@ struct Planned {
   RecordedStep* s;
   bool own = false;                    // runs as the kernel it was recorded as
   bool is_view = false;                // its output is `view` (of a source that others may read instead)
+  bool redirected = false;             // reads a movement's source in the place of its output, which the recorded kernel names: it can only run in a vm_kernel
   StepView view;
   Range write;
   std::vector<Range> reads;
@@ -668,6 +669,7 @@ bool plan_steps(std::vector<Planned>& plan) {
           if (&v == &p.in[0] && a != 1) continue;
         }
         v = t;
+        p.redirected = true;
       }
     }
     // a movement step is a view of what it reads
@@ -983,7 +985,9 @@ int append_run(Ctx* ctx, cudaGraph_t graph, cudaGraphNode_t* prev, RecordedStep*
   std::vector<void*> mem;
   bool ok = true;
   for (int s = 0; s < stages && ok; s += 2)
-    if (of[s].size() >= 3) {                               // fewer: their own kernels
+    // Fewer than three: their own kernels, unless one reads past a movement.  It then waits for the movement's source only and may stand in front of the
+    // movement, whose output its recorded kernel would read.
+    if (of[s].size() >= 3 || std::any_of(of[s].begin(), of[s].end(), [&](int i) { return plan[i].redirected; })) {
       void* m = nullptr;
       ok = build_program(plan, of[s], ctx->sm_count, &pg[s]) && upload(ctx, pg[s], &vp[s], &m);
       if (m) mem.push_back(m);

@@ -13,7 +13,7 @@ def every_buffer(cg):
 
 def same_bits(L, device, g, inputs, varied=(), **kw):
     recorded, plain = L.compile(g, device, **kw), L.compile(g, device, capture=False, **kw)
-    for turn in range(3):                                          # step by step, then two replays on other values
+    for turn in range(3):                                          # the first call records and replays, the others replay on other values
         for nid in varied:
             inputs[nid] = np.roll(inputs[nid], turn)
         recorded(inputs), plain(inputs)
@@ -109,3 +109,66 @@ def test_large_steps_stay_kernels(lib_built, device):
     x[3, 5], x[7, 9], x[11, 2] = np.inf, -np.inf, np.nan
     launches, steps = same_bits(lib_built, device, g, {a.id: x, w.id: rng.standard_normal((900, 800)).astype(np.float32)}, [w.id])
     assert launches < steps
+
+
+def large_movement(G, tail):
+    """A product that reads past a large movement (a kernel of its own) to the movement's source, alone in front of everything; then large and small steps."""
+    g = G.Graph()
+    w, a = G.tensor(g, [1024, 1024]), G.tensor(g, [32, 1024])
+    m = G.permute(w, [2, 1])
+    x = G.matmul(a, m)
+    big = m * np.float32(0.5) + np.float32(1.0)
+    y = G.sum_(big, 1)
+    for i in range(tail):
+        y = y * np.float32(0.5) + G.sum_(x, 1) * np.float32(0.01 * (i + 1))
+    return g, (w, a), (x, y)
+
+
+@pytest.mark.parametrize("tail", [4, 9])
+@pytest.mark.parametrize("fuse,shared", [(True, False), (False, False), (True, True), (False, True)])
+def test_short_stage_reads_past_a_large_movement(lib_built, device, tail, fuse, shared):
+    g, (w, a), outputs = large_movement(lib_built.graph, tail)
+    rng = np.random.default_rng(tail)
+    inputs = {t.id: rng.standard_normal(t.shape).astype(np.float32) for t in (w, a)}
+    same_bits(lib_built, device, g, inputs, [w.id, a.id], fuse=fuse, **(dict(outputs=[t.id for t in outputs]) if shared else {}))
+
+
+def stages_graph(G, rng, steps):
+    """Steps around the sizes (2^19 elements, 592 product tiles) from which one keeps its own kernel: runs fall apart into stages of one step and more, and
+    small steps read large movements."""
+    g = G.Graph()
+    n = 720                                                        # n x n is just below 2^19, n x 800 above
+    leaves = [G.tensor(g, [n, n]), G.tensor(g, [n, 800]), G.tensor(g, [24, n]), G.tensor(g, [800, 16])]
+    pool = list(leaves)
+    pick = lambda ok: [t for t in pool if ok(t)]  # noqa: E731
+    for _ in range(steps):
+        a = pool[int(rng.integers(len(pool)))]
+        r, size, kind = len(a.shape), int(np.prod(a.shape)), int(rng.integers(7))
+        if kind <= 1:
+            t = G.permute(a, list(range(r, 0, -1)))
+        elif kind == 2:
+            lo = [int(rng.integers(0, 1 + d // 32)) for d in a.shape]
+            t = G.slice_(a, [(s, d) for s, d in zip(lo, a.shape)])
+        elif kind == 3 and r == 2:
+            mates = pick(lambda t: len(t.shape) == 2 and t.shape[0] == a.shape[1] and t.shape[1] * a.shape[0] < 1 << 20)
+            if not mates:
+                continue
+            t = G.matmul(a, mates[int(rng.integers(len(mates)))]) * np.float32(0.01)
+        elif kind == 4 and r > 1:
+            t = G.sum_(a, int(rng.integers(1, r + 1))) * np.float32(0.03)
+        elif kind == 5 and size < 2000 and r < 3:
+            t = G.expand(a, int(rng.integers(1, r + 2)), int(rng.choice([3, 700])))
+        else:
+            mates = pick(lambda t: t.shape == a.shape)
+            t = a * np.float32(0.5) + mates[int(rng.integers(len(mates)))]
+        pool.append(t)
+    return g, leaves, pool[-4:]
+
+
+@pytest.mark.parametrize("seed", range(32))
+@pytest.mark.parametrize("shared", [False, True])
+def test_random_graphs_in_stages(lib_built, device, seed, shared):
+    rng = np.random.default_rng(100 + seed)
+    g, leaves, last = stages_graph(lib_built.graph, rng, 9 + 3 * (seed % 8))
+    inputs = {t.id: rng.standard_normal(t.shape).astype(np.float32) for t in leaves}
+    same_bits(lib_built, device, g, inputs, [t.id for t in leaves], fuse=False, **(dict(outputs=sorted({t.id for t in last})) if shared else {}))
