@@ -282,6 +282,16 @@ __device__ __forceinline__ bool attention_unit(const LlamaStepParams& p, const L
     const float p0 = exp2f((s0 - mn) * kLog2e), p1 = exp2f((s1 - mn) * kLog2e);
     l = l * a + (p0 + p1);
     m = mn;
+    if (16 * kb + 16 > T) {            // what lies behind the context may be no number (an earlier request's), which a weight of 0 would not stop
+#pragma unroll
+      for (int k = 0; k < DU; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int key = 16 * kb + 2 * t + 8 * h;
+          if (key >= T) vf[k][h].x = vf[k][h].z = 0.f;
+          if (key + 1 >= T) vf[k][h].y = vf[k][h].w = 0.f;
+        }
+    }
     const float pa = __shfl_sync(0xffffffffu, p0, 8 * t), pb = __shfl_sync(0xffffffffu, p0, 8 * t + 4);
     const float pc = __shfl_sync(0xffffffffu, p1, 8 * t), pd = __shfl_sync(0xffffffffu, p1, 8 * t + 4);
 #pragma unroll

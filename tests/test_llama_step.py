@@ -60,3 +60,24 @@ def test_layer_outputs_and_unequal_positions(lib_built, device):
         for l in range(cfg["n_layers"]):
             assert np.abs(sess.layer_output(l) - np.asarray(hidden[l]).reshape(1, -1)).max() <= 1e-4 * np.abs(hidden[l]).max()
     sess.close(); model.close()
+
+
+@pytest.mark.parametrize("heads,kv", [(8, 8), (4, 2), (2, 1)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_values_behind_the_context_do_not_count(lib_built, device, heads, kv, bad):
+    """A request that left infinities or NaN in the cache: after a reset, or a step back, what lies behind the context reaches nothing."""
+    L = lib_built
+    cfg = config(256, heads, kv, 200, 97)
+    w = O.synth_llama_weights(cfg, seed=4)
+    model = make_model(L, device, cfg, w, "f32")
+    prompt = O.synth_tokens(4, 1000, (2, 40), cfg["vocab"])
+    sess, clean = L.Session(model, 2, 48), L.Session(model, 2, 48)
+    want = [clean.decode_step(np.ascontiguousarray(prompt[:, i]), want_logits=True)[1] for i in range(40)]
+    for name in ("model.layers.0.self_attn.k_proj.weight", "model.layers.1.self_attn.v_proj.weight"):
+        model.set_weight(name, np.full_like(w[name], bad))
+    assert not np.isfinite(sess.prefill(prompt)).any()
+    model.set_weights(w)
+    sess.reset()
+    for i in range(40):
+        assert np.array_equal(sess.decode_step(np.ascontiguousarray(prompt[:, i]), want_logits=True)[1], want[i]), i
+    sess.close(); clean.close(); model.close()
