@@ -455,6 +455,8 @@ __global__ void __launch_bounds__(kVmThreads, 1) vm_kernel(const VmParams P) {
           ready = v >= (need >> 16);
         }
         if (__all_sync(0xffffffffu, ready)) break;
+        // Not at full rate for long: beside 146 CTAs that ask on, the loads of the two that sum 512 rows of 1000 take three times as long (228 us, 87 so)
+        if (spins > 8u) __nanosleep(spins > 64u ? 200 : 40);
         if ((++spins & 255u) == 0u) {
           const bool over = clock64() - t0 > kVmWaitCycles || *reinterpret_cast<volatile int*>(P.err) != 0;
           if (__any_sync(0xffffffffu, over)) {
