@@ -13,6 +13,7 @@
 #include "recorded.cuh"
 
 #include <algorithm>
+#include <stdlib.h>
 #include <string.h>
 
 namespace lmb {
@@ -569,10 +570,99 @@ int64_t elements(const RecordedStep& s) {
   return t;
 }
 
-// Steps whose own kernel fills the GPU for longer than a launch costs stay kernels: half a million elements (4 MB in and out, 2 us), or four rounds
-// of 32 x 32 product tiles; theirs have more threads per SM, which hides more of the loads' latency.
+int64_t matmul_tiles(const RecordedStep& s, int cols) {
+  int64_t b = 1;
+  for (int k = 0; k + 2 < s.rank; ++k) b *= s.d[k];
+  return b * ceil_div(s.d[s.rank - 2], 32) * ceil_div(s.d[s.rank - 1], cols);
+}
+
+// What a step takes, in microseconds: as the kernel it was recorded as, from one such kernel to the next, and a tile of it in vm_kernel beside the
+// kHandOver of an entry (release, notice, the step's description).  From chains of 8 and of 24 steps of one kind replayed both ways, 170 kinds and
+// sizes: within a quarter of most; among them (own | here) element-wise steps of 4096, 131072 and 520000 elements 1.5 | 1.4, 2.4 | 2.7 and 4.0 | 8.2 us; fusion
+// groups of 41 instructions 6.0 | 6.1 at 4096, 25 | 82 at 520000; products of 1 x 1024 x 1024 18 | 7.3, 128 x 1024 x 1024 18.7 | 18.7, 4096 x 128 x 128
+// 10 | 17; norms of 148 and of 2000 rows of 256 1.8 | 2.2 and 4.5 | 29; sums of 512 rows of 256 35 | 8.7, of 32000 rows of 64 10 | 24.
+constexpr double kHandOver = 0.8, kVmLaunch = 6.0;
+double own_us(const RecordedStep& s) {
+  const double total = (double)elements(s), n = (double)s.n;
+  switch (s.kind) {
+    case STEP_RESHAPE: return 1.9 + total / 1.4e5;
+    case STEP_FUSED: {
+      const double k = (double)s.arg.size();
+      return 1.6 + 0.11 * k + (total > 32768 ? 2.5 + 0.1 * k + total / 520e3 * (5.0 + 0.17 * k) : 0.0);
+    }
+    case STEP_REDUCE:                                      // (rows that start in the same bank of L1 are slower)
+      return s.inner == 1 ? 1.6 + n * (0.0136 + (s.n % 32 ? 0.06 : 0.12) * std::min(total, 256.0) / 256.0) : 1.4 + 0.0155 * n;
+    case STEP_MATMUL: {
+      const double tiles = (double)matmul_tiles(s, 32);
+      return 2.0 + 0.0165 * (double)s.in[0].d[s.in[0].rank - 1] * std::max(1.0, tiles / 148.0) + 0.006 * tiles;
+    }
+    case STEP_CUMSUM: return 1.2 + n * (0.043 + 0.055 * std::min(total / n, 16.0) / 16.0 + 0.06 * std::min(total / n, 256.0) / 256.0);
+    case STEP_NORM: return 1.4 + 0.0008 * n + 0.0011 * total / n + (s.op ? 0.4 : 0.0);
+    default: return 1.3 + total / 2e5;
+  }
+}
+
+struct Tiling { int per; int64_t tiles; };                // elements a thread takes (REDUCE: rows a tile), and the step's tiles
+// cols: columns of a product's tile; spread: other steps wait for this one, which then spreads over the CTAs (a movement nobody waits for takes eight
+// elements a thread)
+Tiling tiling(const RecordedStep& s, int sms, int cols, bool spread) {
+  const int64_t total = elements(s);
+  int per = 1;
+  switch (s.kind) {
+    case STEP_REDUCE:
+      per = s.inner == 1 && s.n <= 256 ? 32 : 1;
+      return {per, ceil_div(total, per == 32 ? 32 : kVmThreads)};
+    case STEP_MATMUL: return {1, matmul_tiles(s, cols)};
+    case STEP_CUMSUM: return {1, ceil_div(total / s.n, kVmThreads)};
+    case STEP_NORM: return {1, total / s.n};
+    default:
+      while (per < 8 && (!spread || ceil_div(total, kVmThreads * per) > sms)) per *= 2;
+      return {per, ceil_div(total, kVmThreads * per)};
+  }
+}
+double tile_us(const RecordedStep& s, const Tiling& t, int cols) {
+  const double n = (double)s.n, per = t.per;
+  switch (s.kind) {
+    case STEP_COPY: return 0.4 + 0.15 * per;
+    case STEP_RESHAPE: return 1.1 + 0.15 * per;
+    case STEP_FUSED: return 0.5 + per * (0.2 + 0.12 * (double)s.arg.size());
+    case STEP_REDUCE: return t.per == 32 ? 1.5 + 0.027 * n : 0.9 + 0.023 * n;
+    case STEP_MATMUL: {
+      const double K = (double)s.in[0].d[s.in[0].rank - 1];
+      return cols == 8 ? 1.0 + 0.0055 * K : cols == 16 ? 1.0 + 0.009 * K : 1.8 + 0.0162 * K;
+    }
+    case STEP_CUMSUM: {
+      const double rows = std::min((double)elements(s) / n, 256.0);
+      return 1.5 + n * (0.0166 + 0.02 * std::min(rows, 16.0) / 16.0 + (rows > 64.0 ? 0.22 : 0.03) * rows / (rows > 64.0 ? 256.0 : 64.0));
+    }
+    case STEP_NORM: return 1.1 + 0.0009 * n + (s.op ? 0.35 : 0.0);
+    default: return 0.35 + 0.4 * per;
+  }
+}
+// columns of a product's tile: the fewest with which it takes one round of the CTAs
+int product_cols(const RecordedStep& s, int sms) {
+  int cols = 8;
+  while (cols < 32 && matmul_tiles(s, cols) > sms) cols *= 2;
+  return cols;
+}
+
+// A step that takes kOwnGain longer here than by its own kernel keeps that kernel.  That ends the vm_kernel in front of it and everything in that has to be
+// done by then, and starts another behind: 30 us for each of three such steps of a 128-token graph of hidden 1024 (907 us a replay, 857 with them inside).
+// Rows beyond 256 elements are summed by a thread each: as fast as the own kernel while nothing else runs, but its loads want the L1 that vm_kernel's shared
+// memory takes (sums of 16 rows of 4096 with a broadcast add between them 107 us, 227 here).  Movements, which nobody waits for, are only bounded in size: half
+// a million elements.
+constexpr double kOwnGain = 16.0;
 constexpr int64_t kOwnElements = 1 << 19;
-constexpr int64_t kOwnTiles = 4 * 148;
+bool own_kernel(const RecordedStep& s, int sms) {
+  if (elements(s) > kOwnElements || s.n > 0x7fffffff) return true;
+  for (const StepView& v : s.in)
+    if (v.base && v.elems > 0x7fffffff) return true;
+  if (s.kind == STEP_COPY) return false;
+  const int cols = s.kind == STEP_MATMUL ? product_cols(s, sms) : 0;
+  const Tiling t = tiling(s, sms, cols, true);
+  if (t.tiles > 65535 || (s.kind == STEP_REDUCE && s.n > 256)) return true;
+  return (double)ceil_div(t.tiles, sms) * (kHandOver + tile_us(s, t, cols)) > own_us(s) + kOwnGain;
+}
 
 struct Planned {
   RecordedStep* s;
@@ -586,12 +676,6 @@ struct Planned {
   int stage = 0, level = 0;            // even stages: one vm_kernel each; odd ones: kernels in order
   std::vector<int> after;              // steps of the same stage it waits for
 };
-
-int64_t matmul_tiles(const RecordedStep& s, int cols) {
-  int64_t b = 1;
-  for (int k = 0; k + 2 < s.rank; ++k) b *= s.d[k];
-  return b * ceil_div(s.d[s.rank - 2], 32) * ceil_div(s.d[s.rank - 1], cols);
-}
 
 // A product's operand as (batch, batch, row, column) strides: leading axes of the view are the batches.
 bool operand_strides(const StepView& v, int64_t st[4], int64_t b[2]) {
@@ -633,25 +717,20 @@ struct Memory {
 };
 
 // Views, stages and dependencies of a run of steps.  false: a step cannot be described.
-bool plan_steps(std::vector<Planned>& plan) {
+bool plan_steps(std::vector<Planned>& plan, int sms) {
   for (Planned& p : plan) {
     const RecordedStep& s = *p.s;
     const int64_t total = elements(s);
     p.write = {reinterpret_cast<uintptr_t>(s.out), reinterpret_cast<uintptr_t>(s.out + total)};
-    p.own = total > kOwnElements;
-    if (s.kind == STEP_REDUCE && (s.in[0].elems > 4 * kOwnElements || s.n > 0x7fffffff)) p.own = true;
-    if (s.kind == STEP_MATMUL && matmul_tiles(s, 32) > kOwnTiles) p.own = true;
-    if (s.kind == STEP_NORM && total / s.n > 65535) p.own = true;
-    for (const StepView& v : s.in)
-      if (v.base && v.elems > 0x7fffffff) p.own = true;
+    p.own = own_kernel(s, sms);
   }
   Memory mem;
   mem.build(plan);
   std::vector<int> dep;
   for (size_t i = 0; i < plan.size(); ++i) {
     Planned& p = plan[i];
-    RecordedStep& s = *p.s;
-    p.in = std::move(s.in);
+    const RecordedStep& s = *p.s;
+    p.in = s.in;
     if (!p.own && s.kind != STEP_REDUCE && s.kind != STEP_GATHER && s.kind != STEP_CUMSUM && s.kind != STEP_NORM) {
       for (StepView& v : p.in) {
         Range r;
@@ -752,18 +831,15 @@ void broadcast(const StepView& v, int rank, const int64_t* d, int64_t* st) {
   for (int k = 0; k < rank; ++k) st[k] = k >= shift && v.d[k - shift] == d[k] && v.d[k - shift] != 1 ? v.st[k - shift] : 0;
 }
 
-// Fills the kernel's form of a step; returns its tiles, 0 if it has none.  cols: columns of a product's tile; waited_for: other steps wait for this one,
-// which then spreads over the CTAs (a movement nobody waits for takes eight elements a thread)
-int64_t encode(const Planned& p, int sms, int cols, bool waited_for, VmOp* q) {
+// Fills the kernel's form of a step; returns its tiles, 0 if it has none.  cols: columns of a product's tile
+int64_t encode(const Planned& p, const Tiling& t, int cols, VmOp* q) {
   const RecordedStep& s = *p.s;
   memset(q, 0, sizeof(*q));
   const int64_t total = elements(s);
   q->kind = s.kind; q->op = s.op; q->out = s.out;
   q->n_in = (int)p.in.size();
   q->total = (int)total;
-  q->per = 1;
-  while (q->per < 8 && (!waited_for || ceil_div(total, kVmThreads * q->per) > sms)) q->per *= 2;
-  int64_t tiles = ceil_div(total, kVmThreads * q->per);
+  q->per = t.per;
   for (size_t i = 0; i < p.in.size(); ++i) q->in[i] = p.in[i].base ? p.in[i].base + p.in[i].offset : nullptr;
   switch (s.kind) {
     case STEP_EW:
@@ -809,8 +885,6 @@ int64_t encode(const Planned& p, int sms, int cols, bool waited_for, VmOp* q) {
     }
     case STEP_REDUCE:
       q->p[0] = (int)s.n; q->p[1] = (int)s.inner;
-      q->per = s.inner == 1 && s.n <= 256 ? 32 : 1;
-      tiles = ceil_div(total, q->per == 32 ? 32 : kVmThreads);
       break;
     case STEP_MATMUL: {
       int64_t sa[4], sb[4], ba[2], bb[2];
@@ -827,7 +901,6 @@ int64_t encode(const Planned& p, int sms, int cols, bool waited_for, VmOp* q) {
         return q->p[2] % 4 == 0 && reinterpret_cast<uintptr_t>(base) % 16 == 0 && (st[0] | st[1] | st[row]) % 4 == 0 && st[5 - row] == 1;
       };
       q->p[6] = (vec(q->in[0], sa, 2) ? 1 : 0) | (vec(q->in[1], sb, 3) ? 2 : 0);
-      tiles = matmul_tiles(s, cols);
       break;
     }
     case STEP_GATHER:
@@ -836,14 +909,12 @@ int64_t encode(const Planned& p, int sms, int cols, bool waited_for, VmOp* q) {
     case STEP_CUMSUM:
       q->total = (int)(total / s.n);
       q->p[0] = (int)s.n;
-      tiles = ceil_div(total / s.n, kVmThreads);
       break;
     case STEP_NORM:
       q->p[0] = (int)s.n; q->f = s.val[0];
-      tiles = total / s.n;
       break;
   }
-  return tiles;
+  return t.tiles;
 }
 
 // One vm_kernel: the steps of a stage, their tiles dealt to the CTAs.  An entry only waits for entries of lower levels, and every CTA's list ascends in
@@ -853,17 +924,23 @@ struct Program {
   std::vector<VmOp> ops;
   std::vector<uint32_t> entries;
   std::vector<int> first;
+  std::vector<int64_t> tiles;
+  std::vector<int> limit;                                                // the last level each step may take: before the first that waits for it
+  int levels = 0;
+  double us = 0.0;                                                       // what a replay of it takes: own_us's measurements
 };
 
-bool build_program(std::vector<Planned>& plan, const std::vector<int>& steps, int sms, Program* out) {
+// Everything but the entries; false: a step cannot be described.
+bool describe_program(const std::vector<Planned>& plan, const std::vector<int>& steps, int sms, Program* out) {
   const int n = (int)steps.size();
   if (n > 65535) return false;
   std::vector<int> index(plan.size(), -1);
   for (int i = 0; i < n; ++i) index[steps[i]] = i;
   int levels = 0;
   for (int i : steps) levels = std::max(levels, plan[i].level + 1);
-  // the last level each step may take: before the first that waits for it
-  std::vector<int> limit(n, levels - 1);
+  out->levels = levels;
+  std::vector<int>& limit = out->limit;
+  limit.assign(n, levels - 1);
   std::vector<bool> waited_for(n, false);
   for (int i = n - 1; i >= 0; --i)
     for (int j : plan[steps[i]].after) {
@@ -875,20 +952,45 @@ bool build_program(std::vector<Planned>& plan, const std::vector<int>& steps, in
   for (int i : steps)
     if (plan[i].s->kind == STEP_MATMUL)
       for (int c = 0; c < 3; ++c) product[3 * plan[i].level + c] += matmul_tiles(*plan[i].s, 8 << c);
-  std::vector<int64_t> tiles(n);
+  std::vector<int64_t>& tiles = out->tiles;
+  tiles.resize(n);
+  // a level takes its longest entry as often as its chain's tiles go round the CTAs; the other tiles lie beside them on all CTAs
+  std::vector<int64_t> chain_tiles(levels, 0);
+  std::vector<double> longest(levels, 0.0);
+  double chain_us = 0.0, rest_us = 0.0;
   out->ops.resize(n);
   for (int i = 0; i < n; ++i) {
     const Planned& p = plan[steps[i]];
     int c = 0;
     while (c < 2 && product[3 * p.level + c] > sms) ++c;
-    tiles[i] = encode(p, sms, 8 << c, waited_for[i], &out->ops[i]);
+    const Tiling t = tiling(*p.s, sms, 8 << c, waited_for[i]);
+    tiles[i] = encode(p, t, 8 << c, &out->ops[i]);
     if (tiles[i] < 1 || tiles[i] > 65535 || (int)p.after.size() > kMaxDeps) return false;
+    const double us = kHandOver + tile_us(*p.s, t, 8 << c);
+    if (limit[i] == p.level) {
+      chain_tiles[p.level] += t.tiles;
+      longest[p.level] = std::max(longest[p.level], us);
+    } else {
+      rest_us += us * (double)t.tiles / sms;
+    }
   }
+  for (int l = 0; l < levels; ++l) chain_us += longest[l] * (double)ceil_div(chain_tiles[l], sms);
+  out->us = kVmLaunch + chain_us + rest_us;
   for (int i = 0; i < n; ++i) {
     const Planned& p = plan[steps[i]];
     out->ops[i].n_dep = (int)p.after.size();
     for (size_t k = 0; k < p.after.size(); ++k) out->ops[i].dep[k] = (uint32_t)index[p.after[k]] | (uint32_t)(tiles[index[p.after[k]]] << 16);
   }
+  return true;
+}
+
+// Deals the tiles to the CTAs.
+void place_program(const std::vector<Planned>& plan, const std::vector<int>& steps, int sms, Program* out) {
+  const int n = (int)steps.size(), levels = out->levels;
+  const std::vector<int64_t>& tiles = out->tiles;
+  const std::vector<int>& limit = out->limit;
+  std::vector<int> index(plan.size(), -1);
+  for (int i = 0; i < n; ++i) index[steps[i]] = i;
   struct Place { int cta, level; uint32_t entry; };
   std::vector<Place> places;
   std::vector<int> used(levels + 1, 0);                                  // CTAs the chain's steps take in a level
@@ -927,41 +1029,51 @@ bool build_program(std::vector<Planned>& plan, const std::vector<int>& steps, in
   for (int c = 0; c <= sms; ++c) out->first.push_back(from[(size_t)c * levels]);
   out->entries.resize(places.size());
   for (const Place& p : places) out->entries[from[(size_t)p.cta * levels + p.level]++] = p.entry;
-  return true;
 }
 
 struct Recorder {
   std::vector<RecordedStep> steps;
 };
 
-// device memory of a program: steps | entries | first | counters
-bool upload(Ctx* ctx, const Program& pg, VmParams* vp, void** mem) {
-  const size_t a = pg.ops.size() * sizeof(VmOp), b = round_up(pg.entries.size() * 4, 16), c = round_up(pg.first.size() * 4, 16), d = (pg.ops.size() + 1) * 4;
-  std::vector<char> host(a + b + c + d, 0);
-  memcpy(host.data(), pg.ops.data(), a);
-  memcpy(host.data() + a, pg.entries.data(), pg.entries.size() * 4);
-  memcpy(host.data() + a + b, pg.first.data(), pg.first.size() * 4);
-  void* p = nullptr;
-  if (cudaMalloc(&p, host.size()) != cudaSuccess) return false;
-  if (cudaMemcpyAsync(p, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->own_stream) != cudaSuccess || cudaStreamSynchronize(ctx->own_stream) != cudaSuccess) {
-    cudaFree(p);
-    return false;
+// Programs in device memory, one allocation for all of a graph's: steps | entries | first | counters of each in turn.
+struct Image {
+  std::vector<char> host;
+  std::vector<VmParams> at;                                // pointers as offsets until place()
+  void add(Ctx* ctx, const Program& pg) {
+    const size_t a = pg.ops.size() * sizeof(VmOp), b = round_up(pg.entries.size() * 4, 16), c = round_up(pg.first.size() * 4, 16), d = round_up((pg.ops.size() + 1) * 4, 16);
+    const size_t o = host.size();
+    host.resize(o + a + b + c + d, 0);
+    memcpy(host.data() + o, pg.ops.data(), a);
+    memcpy(host.data() + o + a, pg.entries.data(), pg.entries.size() * 4);
+    memcpy(host.data() + o + a + b, pg.first.data(), pg.first.size() * 4);
+    VmParams vp;
+    vp.ops = reinterpret_cast<const VmOp*>(o);
+    vp.entries = reinterpret_cast<const uint32_t*>(o + a);
+    vp.first = reinterpret_cast<const int*>(o + a + b);
+    vp.done = reinterpret_cast<unsigned*>(o + a + b + c);
+    vp.n_ops = (int)pg.ops.size();
+    vp.err = ctx->dev_err;
+    at.push_back(vp);
   }
-  char* at = static_cast<char*>(p);
-  vp->ops = reinterpret_cast<const VmOp*>(at);
-  vp->entries = reinterpret_cast<const uint32_t*>(at + a);
-  vp->first = reinterpret_cast<const int*>(at + a + b);
-  vp->done = reinterpret_cast<unsigned*>(at + a + b + c);
-  vp->n_ops = (int)pg.ops.size();
-  vp->err = ctx->dev_err;
-  *mem = p;
-  return true;
-}
+  // false: no device memory; *mem is the caller's to free
+  bool place(Ctx* ctx, void** mem) {
+    if (cudaMalloc(mem, host.size()) != cudaSuccess) { *mem = nullptr; return false; }
+    if (cudaMemcpyAsync(*mem, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->own_stream) != cudaSuccess || cudaStreamSynchronize(ctx->own_stream) != cudaSuccess) return false;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(*mem);
+    for (VmParams& v : at) {
+      v.ops = reinterpret_cast<const VmOp*>(base + reinterpret_cast<uintptr_t>(v.ops));
+      v.entries = reinterpret_cast<const uint32_t*>(base + reinterpret_cast<uintptr_t>(v.entries));
+      v.first = reinterpret_cast<const int*>(base + reinterpret_cast<uintptr_t>(v.first));
+      v.done = reinterpret_cast<unsigned*>(base + reinterpret_cast<uintptr_t>(v.done));
+    }
+    return true;
+  }
+};
 
-// A run shorter than this stays as it was recorded: the cooperative launch and the first trip through its program cost about three recorded kernels.
+// A run shorter than this is not looked at: the kernel's launch alone takes as long as four of the shortest steps.
 constexpr size_t kShortestRun = 6;
 
-// a recorded kernel as it is, behind *prev
+// a recorded kernel as it is, behind *prev (the attributes' copy takes the destination first, whatever the header calls its arguments: read back on both nodes)
 bool append_kernel(cudaGraph_t graph, cudaGraphNode_t* prev, cudaGraphNode_t recorded, int64_t* kernels) {
   cudaKernelNodeParams kp{};
   cudaGraphNode_t node = nullptr;
@@ -973,55 +1085,74 @@ bool append_kernel(cudaGraph_t graph, cudaGraphNode_t* prev, cudaGraphNode_t rec
   return true;
 }
 
-// Appends one run of steps to `graph` behind *prev.  0: it gains nothing from being replaced, 1: done, -1: the graph is no longer usable.
-int append_run(Ctx* ctx, cudaGraph_t graph, cudaGraphNode_t* prev, RecordedStep* steps, size_t n, std::vector<void*>* programs, int64_t* kernels) {
-  std::vector<Planned> plan(n);
+// A new graph is planned, uploaded and rebuilt once: 0.1 to 0.3 ms of its first call, and the estimates are a tenth off.
+constexpr double kWorthIt = 0.92;
+
+// A run of steps as stages: a program of vm_kernel each, or (programs without steps) the recorded kernels.
+struct Run {
+  std::vector<Planned> plan;
+  std::vector<std::vector<int>> of;    // a stage's steps
+  std::vector<Program> pg;
+};
+
+// false: the run gains nothing from being replaced.
+bool plan_run(Ctx* ctx, RecordedStep* steps, size_t n, Run* run) {
+  const char* e = getenv("LMB200_GRAPH_KERNEL");           // 0: recorded kernels only, 1: vm_kernel wherever it can be (A/B runs)
+  if (e && atoi(e) == 0) return false;
+  std::vector<Planned>& plan = run->plan;
+  plan.resize(n);
   for (size_t i = 0; i < n; ++i) plan[i].s = &steps[i];
-  if (!plan_steps(plan)) return 0;
+  if (!plan_steps(plan, ctx->sm_count)) return false;
   int stages = 0;
   for (const Planned& p : plan) stages = std::max(stages, p.stage + 1);
-  std::vector<std::vector<int>> of(stages);
-  for (size_t i = 0; i < n; ++i) of[plan[i].stage].push_back((int)i);
-  std::vector<Program> pg(stages);
-  std::vector<VmParams> vp(stages);
-  std::vector<void*> mem;
-  bool ok = true;
-  for (int s = 0; s < stages && ok; s += 2)
-    // Fewer than three: their own kernels, unless one reads past a movement.  It then waits for the movement's source only and may stand in front of the
-    // movement, whose output its recorded kernel would read.
-    if (of[s].size() >= 3 || std::any_of(of[s].begin(), of[s].end(), [&](int i) { return plan[i].redirected; })) {
-      void* m = nullptr;
-      ok = build_program(plan, of[s], ctx->sm_count, &pg[s]) && upload(ctx, pg[s], &vp[s], &m);
-      if (m) mem.push_back(m);
-    }
-  if (!ok || mem.empty()) {
-    for (void* m : mem) cudaFree(m);
-    cudaGetLastError();
-    return 0;
-  }
-  programs->insert(programs->end(), mem.begin(), mem.end());
+  run->of.resize(stages);
+  for (size_t i = 0; i < n; ++i) run->of[plan[i].stage].push_back((int)i);
+  run->pg.resize(stages);
+  double recorded = 0.0, planned = 0.0;
+  bool any = false;
   for (int s = 0; s < stages; ++s) {
-    if (!pg[s].ops.empty()) {
-      cudaKernelNodeParams kp{};
-      void* args[1] = {&vp[s]};
-      kp.func = (void*)vm_kernel;
-      kp.gridDim = dim3((unsigned)ctx->sm_count);
-      kp.blockDim = dim3(kVmThreads);
-      kp.sharedMemBytes = kBufFloats * 4;
-      kp.kernelParams = args;
-      cudaGraphNode_t node = nullptr;
-      if (cudaGraphAddKernelNode(&node, graph, *prev ? prev : nullptr, *prev ? 1 : 0, &kp) != cudaSuccess) return -1;
-      cudaKernelNodeAttrValue coop{};
-      coop.cooperative = 1;
-      if (cudaGraphKernelNodeSetAttribute(node, cudaKernelNodeAttributeCooperative, &coop) != cudaSuccess) return -1;
-      *prev = node;
-      ++*kernels;
+    double own = 0.0;
+    bool redirected = false;
+    for (int i : run->of[s]) { own += own_us(steps[i]); redirected = redirected || plan[i].redirected; }
+    recorded += own;
+    Program& pg = run->pg[s];
+    if (s % 2 == 0 && !run->of[s].empty() && !describe_program(plan, run->of[s], ctx->sm_count, &pg)) return false;
+    // A stage that is faster as its own kernels runs as those, unless a step reads past a movement: it then waits for the movement's source only and may stand
+    // in front of the movement, whose output its recorded kernel would read.
+    if (!pg.ops.empty() && pg.us >= own && !redirected && !e) pg = Program();
+    planned += pg.ops.empty() ? own : pg.us;
+    any = any || !pg.ops.empty();
+  }
+  if (!any || (!e && planned >= kWorthIt * recorded)) return false;
+  for (int s = 0; s < stages; ++s)
+    if (!run->pg[s].ops.empty()) place_program(plan, run->of[s], ctx->sm_count, &run->pg[s]);
+  return true;
+}
+
+// Appends it to `graph` behind *prev, *vp its first program; false: the graph is no longer usable.
+bool append_run(Ctx* ctx, cudaGraph_t graph, cudaGraphNode_t* prev, const Run& run, VmParams** vp, int64_t* kernels) {
+  for (size_t s = 0; s < run.of.size(); ++s) {
+    if (run.pg[s].ops.empty()) {
+      for (int i : run.of[s])
+        if (!append_kernel(graph, prev, run.plan[i].s->node, kernels)) return false;
       continue;
     }
-    for (int i : of[s])
-      if (!append_kernel(graph, prev, steps[i].node, kernels)) return -1;
+    cudaKernelNodeParams kp{};
+    void* args[1] = {(*vp)++};
+    kp.func = (void*)vm_kernel;
+    kp.gridDim = dim3((unsigned)ctx->sm_count);
+    kp.blockDim = dim3(kVmThreads);
+    kp.sharedMemBytes = kBufFloats * 4;
+    kp.kernelParams = args;
+    cudaGraphNode_t node = nullptr;
+    if (cudaGraphAddKernelNode(&node, graph, *prev ? prev : nullptr, *prev ? 1 : 0, &kp) != cudaSuccess) return false;
+    cudaKernelNodeAttrValue coop{};
+    coop.cooperative = 1;
+    if (cudaGraphKernelNodeSetAttribute(node, cudaKernelNodeAttributeCooperative, &coop) != cudaSuccess) return false;
+    *prev = node;
+    ++*kernels;
   }
-  return 1;
+  return true;
 }
 
 // The chain's kernels in order; false if the graph is anything but a chain of kernels.
@@ -1081,36 +1212,49 @@ void record_finish(Ctx* ctx, cudaGraph_t* graph, std::vector<void*>* programs, i
   record_drop(ctx);
   if (steps.size() < kShortestRun) return;
   std::vector<cudaGraphNode_t> chain;
-  cudaGraph_t made = nullptr;
-  cudaGraphNode_t prev = nullptr;
-  std::vector<void*> mem;
-  int64_t count = 0;
-  bool replaced = false;
-  bool ok = chain_of(*graph, steps, &chain) && cudaFuncSetAttribute(vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBufFloats * 4) == cudaSuccess &&
-            cudaGraphCreate(&made, 0) == cudaSuccess;
-  for (size_t c = 0, i = 0; ok && c < chain.size();) {
+  if (!chain_of(*graph, steps, &chain)) {
+    cudaGetLastError();
+    return;
+  }
+  struct Piece { size_t at, n; bool replaced; };           // kernels of the chain
+  std::vector<Piece> pieces;
+  std::vector<Run> runs;
+  for (size_t c = 0, i = 0; c < chain.size();) {
     size_t n = 0;                                          // recorded steps from this node of the chain on
     while (i + n < steps.size() && c + n < chain.size() && steps[i + n].node == chain[c + n]) ++n;
-    int done = 0;
-    if (n >= kShortestRun) {
-      done = append_run(ctx, made, &prev, &steps[i], n, &mem, &count);
-      replaced |= done > 0;
-      ok = done >= 0;
-    }
+    Run run;
+    const bool replaced = n >= kShortestRun && plan_run(ctx, &steps[i], n, &run);
+    if (replaced) runs.push_back(std::move(run));
+    i += n;
     if (n == 0) n = 1;
-    else i += n;
-    if (done == 0)
-      for (size_t k = c; ok && k < c + n; ++k) ok = append_kernel(made, &prev, chain[k], &count);
+    pieces.push_back({c, n, replaced});
     c += n;
   }
+  if (runs.empty()) return;
+  cudaGraph_t made = nullptr;
+  cudaGraphNode_t prev = nullptr;
+  void* mem = nullptr;
+  int64_t count = 0;
+  Image image;
+  for (const Run& r : runs)
+    for (const Program& pg : r.pg)
+      if (!pg.ops.empty()) image.add(ctx, pg);
+  bool ok = image.place(ctx, &mem) && cudaFuncSetAttribute(vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBufFloats * 4) == cudaSuccess &&
+            cudaGraphCreate(&made, 0) == cudaSuccess;
+  size_t next = 0;
+  VmParams* vp = image.at.data();
+  for (const Piece& p : pieces) {
+    if (ok && p.replaced) ok = append_run(ctx, made, &prev, runs[next++], &vp, &count);
+    for (size_t k = p.at; ok && !p.replaced && k < p.at + p.n; ++k) ok = append_kernel(made, &prev, chain[k], &count);
+  }
   cudaGetLastError();
-  if (ok && replaced) {
+  if (ok) {
     cudaGraphDestroy(*graph);
     *graph = made;
     *kernels = count;
-    *programs = std::move(mem);
+    programs->push_back(mem);
   } else {                                                 // as recorded, then
-    for (void* m : mem) cudaFree(m);
+    cudaFree(mem);
     if (made) cudaGraphDestroy(made);
   }
 }

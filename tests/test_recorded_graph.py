@@ -7,6 +7,12 @@ import luminal_oracle as O
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def wherever_it_can_be(monkeypatch):
+    """The kernel also where the library expects nothing of it: these tests are about what it computes."""
+    monkeypatch.setenv("LMB200_GRAPH_KERNEL", "1")
+
+
 def every_buffer(cg):
     return {nid: a.numpy() for nid, a in cg.results.items()}
 
@@ -172,3 +178,38 @@ def test_random_graphs_in_stages(lib_built, device, seed, shared):
     g, leaves, last = stages_graph(lib_built.graph, rng, 9 + 3 * (seed % 8))
     inputs = {t.id: rng.standard_normal(t.shape).astype(np.float32) for t in leaves}
     same_bits(lib_built, device, g, inputs, [t.id for t in leaves], fuse=False, **(dict(outputs=sorted({t.id for t in last})) if shared else {}))
+
+
+def alternating(G, n, k):
+    g = G.Graph()
+    a = G.tensor(g, [n // 64, 64])
+    t = a
+    for i in range(k):
+        t = t * t if i % 2 else t + a
+    return g, {a.id: np.linspace(-1.0, 1.0, n, dtype=np.float32).reshape(a.shape)}
+
+
+def test_only_where_it_is_expected_to_be_faster(lib_built, device, monkeypatch):
+    """Chains without a movement or a small product stay their recorded kernels; a step of many rounds keeps its kernel among steps that do not."""
+    monkeypatch.delenv("LMB200_GRAPH_KERNEL")
+    L = lib_built
+    for n in (4096, 400_000):
+        g, inputs = alternating(L.graph, n, 12)
+        launches, steps = same_bits(L, device, g, inputs, fuse=False)
+        assert launches == steps == 12
+    g, reg = L.Graph(), {}
+    net = L.nn.Llama(g, reg, vocab_size=300, n_layers=2, hidden=256, n_heads=8, n_kv_heads=8, intermediate=688)
+    tok = L.tensor(g, [1, 33])
+    net(tok, 0)
+    inputs = {t.id: O.synth_normal(3, t.id, t.shape, 0.3) for t in reg.values()}
+    inputs[tok.id] = O.synth_tokens(5, 999, (1, 33), 300).astype(np.float32)
+    assert same_bits(L, device, g, inputs, [tok.id])[0] == 1
+    g = L.Graph()
+    a, w = L.tensor(g, [1, 1024]), L.tensor(g, [1024, 1024])
+    t = a
+    for _ in range(4):
+        t = L.graph.matmul(t, L.graph.permute(w, [2, 1])) * np.float32(0.03)
+    big = L.graph.sum_(L.graph.expand(L.graph.reshape(t, [1024]), 1, 3_000), 2)      # rows of 1024 values: a step that keeps its kernel
+    out = L.graph.permute(L.graph.expand(big, 1, 2), [2, 1]) * np.float32(0.5)
+    launches, steps = same_bits(L, device, g, {a.id: np.ones((1, 1024), np.float32), w.id: O.synth_normal(3, 7, (1024, 1024), 0.3)}, fuse=False)
+    assert 1 < launches < steps
