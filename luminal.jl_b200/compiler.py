@@ -249,6 +249,7 @@ class CompiledGraph:
                           np.asarray([what[1]], np.float32).ctypes.data_as(C.c_void_p), 0, _lib.dims(()), 0)
             elif what[0] != "input":
                 self.steps.append((what, buf))
+        self.records_first = self._records_first()
         # data pre-loaded into the graph (load_weights!, src/Weights.jl:60-91; the sinusoid table of the Whisper
         # encoder) fills its input buffers once, here; the inputs of a call may still overwrite them
         from .device import DeviceArray
@@ -258,6 +259,27 @@ class CompiledGraph:
                 buf = self.results[node_id]
                 _lib.call("lmb200_upload", self.dev.handle, C.c_void_p(buf.ptr), _lib.F32, a.ctypes.data_as(C.c_void_p),
                           len(buf.shape), _lib.dims(buf.shape), 0)
+
+    def _records_first(self):
+        """Whether the first call records the steps and replays them at once instead of running them one by one before it records them.  Not where a step
+        sizes a scratch buffer on its first use, nor where the device would be busy for longer than it takes to issue the steps (8 us each), which
+        it then is while they are recorded.  First call of a new graph, run first -> recorded first: the small Llama's 404 steps (2.2 us of kernels each)
+        5.7 -> 3.7 ms; 212 steps of 5.7 us 3.5 -> 3.4 ms, of 7.5 us 3.5 -> 3.9, of 11.5 us 3.6 -> 5.1."""
+        us, shapes = 0.0, self.graph.shapes                    # beyond a kernel's shortest time
+        for what, out in self.steps:
+            op = what[1] if what[0] == "op" else None
+            t = type(op)
+            if t is G.FlashAttentionOp:
+                return False
+            if t is G.MatMul:
+                us += 0.0165 * shapes[what[2][0] - 1][-1] * max(1.0, out.size / (1024 * 148))
+            elif t is G.SumReduce or t is G.MaxReduce:
+                us += (0.1 if out.size >= 256 else 0.03) * shapes[what[2][0] - 1][op.dim - 1]
+            elif t is G.Function and op.name == "CumSum":
+                us += 0.1 * out.shape[-1]
+            else:
+                us += out.size / 2e5
+        return us <= 6.0 * len(self.steps)
 
     # -- execution -------------------------------------------------------------------------------
     def __call__(self, inputs, device=None):
@@ -270,9 +292,7 @@ class CompiledGraph:
                       len(buf.shape), _lib.dims(buf.shape), 0)
         if self.capture:
             from .device import execute_with_capture
-            if not self.cache and not any(isinstance(what[1], G.FlashAttentionOp) for what, _ in self.steps if what[0] == "op"):
-                # No step sizes a scratch buffer on its first use, so the first call need not run them one by one before it records
-                # them: recorded and replayed at once (the small Llama's graph of 404 steps: 6.3 -> 4.3 ms for a new graph's first call).
+            if not self.cache and self.records_first:
                 try:
                     self.cache["cuda_exec"] = self.dev.capture(self.run_steps)
                 except _lib.LuminalB200Error:

@@ -3,6 +3,7 @@ to_device / from_device (src/Device.jl:9-16, 82-105) for `libluminal_b200.so`.""
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 
@@ -18,7 +19,7 @@ class DeviceArray:
 
     @property
     def size(self):
-        return int(np.prod(self.shape)) if self.shape else 1
+        return int(math.prod(self.shape))
 
     def numpy(self, layout=ROWMAJOR):
         """from_device: float32 NumPy array of the logical shape."""

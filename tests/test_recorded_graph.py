@@ -213,3 +213,20 @@ def test_only_where_it_is_expected_to_be_faster(lib_built, device, monkeypatch):
     out = L.graph.permute(L.graph.expand(big, 1, 2), [2, 1]) * np.float32(0.5)
     launches, steps = same_bits(L, device, g, {a.id: np.ones((1, 1024), np.float32), w.id: O.synth_normal(3, 7, (1024, 1024), 0.3)}, fuse=False)
     assert 1 < launches < steps
+
+
+@pytest.mark.parametrize("rows,records_first", [(8, True), (40_000, False)])
+def test_first_call_records_first_where_the_kernels_are_short(lib_built, device, rows, records_first):
+    """Products of a few rows record before they run, products that keep the device busy run while they are recorded; the first call is the later ones' result."""
+    G = lib_built.graph
+    g = G.Graph()
+    a, w = G.tensor(g, [rows, 256]), G.tensor(g, [256, 256])
+    t = a
+    for _ in range(4):
+        t = G.matmul(t, w)
+    inputs = {a.id: O.synth_normal(3, 1, a.shape, 1.0), w.id: O.synth_normal(3, 2, w.shape, 0.06)}
+    cg = lib_built.compile(g, device)
+    assert cg.records_first is records_first
+    first = cg(inputs)[t.id].numpy()
+    assert "cuda_exec" in cg.cache and np.array_equal(cg(inputs)[t.id].numpy(), first)
+    cg.close()
