@@ -425,10 +425,13 @@ Kernel kernel_of(int B, int D) {
 }  // namespace
 
 // Sizes up to which the one launch was measured to be the faster way (and what its shared memory and registers hold); a context longer than 1024 keys would be
-// one CTA's work per head, which the launched attention splits.
+// one CTA's work per head, which the launched attention splits.  The head is the part that loses: a CTA takes its 16-row units one after the other, 1.1 us each
+// with one sequence and 2.2 with four, where the launched product streams the matrix; a layer gains 4 to 17 us at short contexts.  Launched -> one launch, 8 keys:
+// hidden 64, one layer, vocabulary 32768, one and four sequences 34 -> 42, 35 -> 62 us; 256, one layer, 16384 43 -> 33, 43 -> 46; 256, four layers, 65536
+// 145 -> 111, 152 -> 158; 1024 with 32 heads, 16 layers, 65536 895 -> 701, 960 -> 1054; 1024, 16 layers, 32000, four 1337 -> 958.
 bool llama_step_fits(int B, int D, int hidden, int ffn, int vocab, int n_layers, int capacity) {
   return B <= kLlamaStepBatch && (D == 32 || D == 64 || D == 128) && hidden % 4 == 0 && ffn % 4 == 0 && hidden <= kMaxHidden && ffn <= kMaxFfn && capacity <= 1024 &&
-         vocab <= 65536 && n_layers <= 64;
+         vocab <= (B <= 2 ? 65536 : 32768) && (int64_t)vocab * (1 + B) <= 32768ll * n_layers && n_layers <= 64;
 }
 
 int64_t llama_step_scratch_bytes(int n_layers, int sms) { return layer_bytes(n_layers) + counter_bytes(n_layers) + (int64_t)sms * kLlamaStepBatch * 8; }

@@ -81,3 +81,20 @@ def test_values_behind_the_context_do_not_count(lib_built, device, heads, kv, ba
     for i in range(40):
         assert np.array_equal(sess.decode_step(np.ascontiguousarray(prompt[:, i]), want_logits=True)[1], want[i]), i
     sess.close(); clean.close(); model.close()
+
+
+@pytest.mark.parametrize("vocab,layers,batch,one_launch", [(16384, 1, 1, True), (16385, 1, 1, False), (16384, 1, 2, False), (6553, 1, 4, True), (6554, 1, 4, False),
+                                                           (32768, 8, 3, True), (32769, 8, 3, False)])
+def test_vocabulary_at_the_rule(lib_built, device, vocab, layers, batch, one_launch):
+    L = lib_built
+    cfg = config(64, 2, 2, 40, vocab, layers)
+    w = O.synth_llama_weights(cfg, seed=2)
+    prompt = O.synth_tokens(2, 1000, (batch, 4), vocab)
+    ref = O.CachedLlama(w, cfg, batch, 16).greedy(prompt, 2)[1]
+    model = make_model(L, device, cfg, w, "f32")
+    sess = L.Session(model, batch, 16)
+    before = device.launch_count()
+    logits = sess.prefill(prompt)
+    assert (device.launch_count() - before == 4) is one_launch
+    assert np.abs(logits - ref[:, 0]).max() <= LOGIT_TOL
+    sess.close(); model.close()
