@@ -15,6 +15,7 @@
 #include "pdl.cuh"
 
 #include <math_constants.h>
+#include <stdlib.h>
 
 #include <algorithm>
 
@@ -604,9 +605,15 @@ int64_t counter_bytes(int n_layers) { return round_up((int64_t)(3 + 8 * n_layers
 }  // namespace
 
 // D = 64, one key head per query head, and a batch of two MMA column tiles at most: beyond that the weights' tiles of 16 rows are multiplied with four or
-// more column tiles and the launched step's tcgen05 GEMVs are used.
+// more column tiles and the launched step's tcgen05 GEMVs are used.  With two column tiles only up to a width of 768: at 1024 a sequence's heads are 1.3 to
+// 1.7 rounds of the CTAs and the products outweigh the launches.  Launched -> two launches, a step at 1500 cross-attention keys: width 512, six layers, batch 1, 8, 16
+// 284 -> 164, 316 -> 187, 343 -> 230 us; 768, twelve 577 -> 393, 662 -> 458, 721 -> 667; 1024, 24 1155 -> 915, 1376 -> 1080; batch 12, 16 1461 -> 1501, 1574 -> 1558
+// (380 positions 1556 -> 1631, 1675 -> 1688).  LMB200_WHISPER_STEP=0: launched, 1: wherever it can be (A/B runs).
 bool whisper_step_fits(int B, int D, int heads, int kv_heads, int hidden, int ffn, int n_layers) {
-  return B <= kWhisperStepBatch && D == kD && heads == kv_heads && hidden == heads * kD && ffn % 64 == 0 && hidden <= kMaxHidden && n_layers <= kWhisperStepLayers;
+  const char* e = getenv("LMB200_WHISPER_STEP");
+  if (e && atoi(e) == 0) return false;
+  return B <= kWhisperStepBatch && D == kD && heads == kv_heads && hidden == heads * kD && ffn % 64 == 0 && hidden <= kMaxHidden && n_layers <= kWhisperStepLayers &&
+         (e || B <= 8 || hidden <= 768);
 }
 
 int64_t whisper_step_scratch_bytes(int B, int heads, int n_layers, int sms) { return layer_bytes(n_layers) + counter_bytes(n_layers) + (int64_t)B * heads * kWhisperStepSplits * (kD + 2) * 4 + (int64_t)sms * kWhisperStepBatch * 8; }

@@ -9,6 +9,12 @@ import whisper_oracle as W
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def wherever_it_can_be(monkeypatch):
+    """Also at the sizes the library launches instead: these tests are about what the kernels compute."""
+    monkeypatch.setenv("LMB200_WHISPER_STEP", "1")
+
+
 def config(heads, ffn, layers=2, vocab=203, positions=40):
     return dict(d_model=64 * heads, heads=heads, enc_layers=1, dec_layers=layers, ffn=ffn, vocab=vocab, n_mels=8, max_positions=positions)
 
@@ -76,4 +82,19 @@ def test_larger_batches_keep_the_launched_step(lib_built, device):
     before = device.launch_count()
     sess.decode_step(O.synth_tokens(4, 6, (17,), cfg["vocab"]))
     assert device.launch_count() - before > 8
+    sess.close(); model.close()
+
+
+@pytest.mark.parametrize("heads,batch,two_launches", [(12, 16, True), (13, 9, False), (16, 8, True), (16, 16, False)])
+def test_wide_decoders_at_the_rule(lib_built, device, monkeypatch, heads, batch, two_launches):
+    monkeypatch.delenv("LMB200_WHISPER_STEP")
+    cfg = config(heads, 128)
+    w, kv, model, sess = decoder(lib_built, device, cfg, batch, 20, heads)
+    tok = O.synth_tokens(4, 6, (batch,), cfg["vocab"])
+    ref = W.CachedDecoder(w, cfg, batch, kv).step(tok)
+    chosen, logits = sess.decode_step(tok, want_logits=True)
+    assert np.linalg.norm(logits - ref) <= 4e-2 * np.linalg.norm(ref)
+    before = device.launch_count()
+    sess.decode_step(tok)
+    assert (device.launch_count() - before == 2) is two_launches
     sess.close(); model.close()
