@@ -2519,39 +2519,52 @@ int gemv_plan_ctas(const GemvPlan& pl, int rows) {
 // above 16 sequences, where an exchange moves twice the bytes (eight layers, batch 16 | 32: 2048 458 -> 445 | 577 -> 598 us; four, 3072 351 -> 348 |
 // 397 -> 379).  Sublayers normed on their output make chains of six GEMVs, which gain at every width (Kevatar, four layers, batch 16: 512
 // 238 -> 216 us, 1024 277 -> 247, 2048 387 -> 330).
+constexpr int kChainGroups = 16;
 int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms) {
   const char* e = getenv("LMB200_GEMV_CHAIN");                  // 0: one launch per GEMV, 1: chained wherever it can be (A/B runs)
   if ((e && atoi(e) == 0) || g_variant != GEMV_TCGEN05) return 0;
   const int64_t groups = ceil_div(width, 128);
   if (groups * kChainC > kSsqSlots) return 0;                   // a projection leaves 4 sums of squares per row group
   const bool wide_batch = Layout<__nv_bfloat16>::batch_pad(B) > 16;
-  if (!e && per_chain < 6 && groups > 3 && groups < (per_chain < 4 && wide_batch ? 24 : 16)) return 0;
+  if (!e && per_chain < 6 && groups > 3 && groups < (per_chain < 4 && wide_batch ? 24 : kChainGroups)) return 0;
   const int n = wide_batch ? chain_clusters<32>() : chain_clusters<16>();
   return output_norms && groups > n ? 0 : n;                    // an output norm needs every row group resident at once
 }
 int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMaxAttend + 1) * kChainLine * 4; }
 
-// The four warps' sums of a unit lie in the receive buffer: 128 N floats for 4 G D
-bool gemv_chain_attends(int B, int G, int D) {
-  const char* e = getenv("LMB200_CHAIN_ATTENTION");             // 0: attention as a launch of its own (A/B runs)
-  if (e && atoi(e) == 0) return false;
-  return (D == 64 || D == 96 || D == 128) && G >= 1 && G <= 8 && G * D <= 32 * Layout<__nv_bfloat16>::batch_pad(B);
-}
-
-// One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge).  The merge of several parts -- partial
-// results out, a counter, and back -- costs 4 us, in which a CTA streams some 640 keys (Llama-3-8B shape, one sequence of 1031 keys, nine parts: the
-// last one 11.8 us after q/k/v, the others 4.6).  Their pairs of maximum and sum must fit the receive buffer: at most 64 parts.
-void gemv_chain_attention_plan(int clusters, int B, int KVl, int capacity, int* keys_per_cta, int* nsplit) {
+// One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge), and one of several parts 100 more (partial
+// results out, a counter).  The merge at the end takes 4 us, in which a CTA streams some 640 keys (Llama-3-8B shape, one sequence of 1031 keys, nine parts: the
+// last one 11.8 us after q/k/v, the others 4.6).  Without the 100 a head was cut into too many parts (28 sequences of 8190 keys: 17 rounds of units; the step
+// 1087 us, 954 with two).  The parts' pairs of maximum and sum must fit the receive buffer: at most 64.  The four warps' sums of a unit lie there too: 128 N floats for
+// 4 G D.
+//   Whether it is worth it: the link saves a launch and its latency, but takes whole units, where the launched kernel's many CTAs even out.  What the busiest CTA
+// takes longer than an even spread of the keys tells gains from losses (670 sessions: width 2048 to 8192, head dimension 96 and 128, batch 1 to 32, 64 to 32768 keys;
+// up to the line the link gains 0 to 25 us a layer and loses 3 % at worst, above it loses up to 50 us).  Per layer, launched -> link, Llama-3-8B shape: 1031 keys,
+// batch 1 (841 keys over) -4.9, batch 17 (1151: 136 heads for 132 CTAs) +2.3; 2050 keys, batch 17 (1872) +10; 8190 keys, batch 32 (596) -16.9, batch 30 (1598) -14.8, batch
+// 28 (2450) +4.4, batch 17 (2914) +12.  With a key head per head the launched kernel has a quarter of the parts to merge and is harder to beat: 8190 keys, batch 8 (298) -5.4, 16
+// (1193) +13.5, 20 (1491) -9, 26 (3703) +32.  Head dimension 64 is bound by the work per stage, not by its bytes: 1031 keys, batch 1, 16, 17 -2.1, -2.7, +4.1; 4096
+// keys, batch 1, 16 +1.2, +3.0; 8190 keys, batch 32 +20.
+//   Narrow models are chained up to three row groups, where an attention between is launched: at width 256 and 384 a link gained 5 % at 64 keys and lost up to
+// 12 % at 1031.
+bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, int D, int capacity, int* keys_per_cta, int* nsplit) {
+  const char* e = getenv("LMB200_CHAIN_ATTENTION");             // 0: attention as a launch of its own, 1: a link wherever it can be (A/B runs)
+  if ((e && atoi(e) == 0) || clusters == 0 || ceil_div(width, 128) < kChainGroups) return false;
+  if (!(D == 64 || D == 96 || D == 128) || G < 1 || G > 8 || G * D > 32 * Layout<__nv_bfloat16>::batch_pad(B)) return false;
   const int64_t pairs = (int64_t)B * KVl, ctas = (int64_t)clusters * kChainC, cap = round_up(capacity, 64);
   int64_t best = cap, best_cost = ceil_div(pairs, ctas) * (cap + 48);
   for (int64_t k = 64; k < cap; k += 64) {
     const int64_t ns = ceil_div(cap, k);
     if (ns > 64) continue;
-    const int64_t cost = ceil_div(pairs * ns, ctas) * (k + 48) + 640;
+    const int64_t cost = ceil_div(pairs * ns, ctas) * (k + 148) + 640;
     if (cost < best_cost) { best_cost = cost; best = k; }
   }
   *keys_per_cta = (int)best;
   *nsplit = (int)ceil_div(cap, best);
+  const int64_t even = pairs * cap / ctas, over = best_cost - even, slack = std::min<int64_t>(even, 16000) * 2 / 25;
+  if (e) return true;
+  if (D == 64) return best_cost <= 1050 || (over <= 200 && best_cost <= 2300);
+  if (G < 4 && Layout<__nv_bfloat16>::batch_pad(B) == 16) return over <= 950;
+  return over <= (G < 4 ? 900 : 1050) + slack;
 }
 
 int32_t GemvChain::add(const GemvParams& p) {

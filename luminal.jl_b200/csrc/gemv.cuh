@@ -186,7 +186,7 @@ struct GemvChain {
   cudaStream_t stream = nullptr;
   int clusters = 0;
   unsigned* done = nullptr;                  // gemv_chain_scratch_bytes(), zero before the first launch
-  bool attention = false;                    // gemv_chain_attends() for the session: add_attention() may be called
+  bool attention = false;                    // gemv_chain_attention_plan() for the session: add_attention() may be called
   GemvParams op[kChainMaxAttend];
   int n = 0;
   int32_t add(const GemvParams& p);
@@ -199,8 +199,7 @@ struct GemvChain {
 // EPI_POST_NORMs are among them
 int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms);
 int64_t gemv_chain_scratch_bytes();
-// Whether a chain's attention runs these heads, and its split of the keys (AttnParams::keys_per_cta, nsplit) for a cache of `capacity` positions
-bool gemv_chain_attends(int B, int G, int D);
-void gemv_chain_attention_plan(int clusters, int B, int KVl, int capacity, int* keys_per_cta, int* nsplit);
+// Whether a step's attentions are links of its chains, and then their split of the keys (AttnParams::keys_per_cta, nsplit) for a cache of `capacity` positions
+bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, int D, int capacity, int* keys_per_cta, int* nsplit);
 
 }  // namespace lmb

@@ -1501,7 +1501,7 @@ int32_t advance_launch(Session* S, cudaStream_t st) {
 namespace {
 
 // The fused decode step of a bf16 Llama / Phi-3: a launch per eight layers (every GEMV and attention a link of one chain), two launches per
-// layer (attention, and the GEMVs from there to the next attention as one chain) where attention cannot be a link, or five where every
+// layer (attention, and the GEMVs from there to the next attention as one chain) where attention is faster as a launch, or five where every
 // GEMV is its own launch (tensor parallelism).  The residual add and the
 // RMSNorm around every Linear (src/NN.jl:406-414, 149-161) are carried by the projections themselves:
 // o_proj and down_proj finish with EPI_RESID_NORM (under tensor parallelism including the all-reduce of
@@ -2085,9 +2085,8 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
   }
   int64_t po, pml;
   attn_plan(ctx, batch, M->KVl, M->G, M->D, S->cap, &S->keys_per_cta, &S->nsplit, &po, &pml);
-  if (S->chain_clusters && c.hidden > 15 * 128 && gemv_chain_attends(batch, M->G, M->D)) {
+  if (gemv_chain_attention_plan(S->chain_clusters, c.hidden, batch, M->KVl, M->G, M->D, S->cap, &S->chain_keys, &S->chain_nsplit)) {
     S->chain_attention = true;
-    gemv_chain_attention_plan(S->chain_clusters, batch, M->KVl, S->cap, &S->chain_keys, &S->chain_nsplit);
     po = std::max(po, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * M->D);
     pml = std::max(pml, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * 2);
   }

@@ -12,10 +12,8 @@ pytestmark = pytest.mark.gpu
 def both(L, model, monkeypatch, batch, capacity, contexts, steps, seed):
     """(logits, tokens) of `steps` forced steps behind random caches, with the attention in the chain and launched."""
     out = []
-    for env in (None, "0"):
-        monkeypatch.delenv("LMB200_CHAIN_ATTENTION", raising=False)
-        if env:
-            monkeypatch.setenv("LMB200_CHAIN_ATTENTION", env)
+    for env in ("1", "0"):                                         # 1: also where the library launches it because that is faster
+        monkeypatch.setenv("LMB200_CHAIN_ATTENTION", env)
         sess = L.Session(model, batch, capacity)
         rng = np.random.default_rng(seed)
         sess.fill_kv_random(max(contexts), seed)
@@ -40,6 +38,34 @@ def test_against_launched_attention(lib_built, device, monkeypatch, hidden, head
     # the same products and sums but for the order of the keys' parts: differences of a bf16 rounding of the attention's outputs
     assert rel_err(chain, launched) <= BF16_REL_TOL / 2
     model.close()
+
+
+@pytest.mark.parametrize("hidden,heads,kv", [(2048, 16, 4), (3072, 32, 8), (2048, 32, 8), (2048, 16, 16)])
+@pytest.mark.parametrize("batch,contexts", [(1, [8100]), (1, [20000]), (3, [8100, 63, 4095]), (17, [8000]), (32, [8000])])
+def test_long_contexts_against_launched_attention(lib_built, device, monkeypatch, hidden, heads, kv, batch, contexts):
+    """Hundreds of stages in a link, which go round the ring many times, up to 64 parts a head, units of a second and later round; the steps cross a 64-key stage."""
+    L = lib_built
+    model = L.Model(device, dtype="bf16", n_layers=2, hidden=hidden, n_heads=heads, n_kv_heads=kv, intermediate=512, vocab=500, eps=1e-5, rope_base=10000.0)
+    model.init_random(seed=6, sigma=0.02)
+    contexts = contexts if len(contexts) == batch else contexts * batch
+    chain, launched = both(L, model, monkeypatch, batch, max(contexts) + 70, contexts, 68, batch)
+    # as above; the sums run over more keys, whose weights are the same bf16 values on both sides up to the maximum they are taken against
+    assert np.isfinite(chain).all() and rel_err(chain, launched) <= BF16_REL_TOL / 2
+    model.close()
+
+
+@pytest.mark.parametrize("batch,capacity,link", [(16, 1024, True), (17, 128, True), (17, 4096, False), (20, 8192, False), (32, 8192, True), (1, 8192, True)])
+def test_launched_where_whole_heads_spread_badly(lib_built, device, batch, capacity, link):
+    L = lib_built
+    model = L.Model(device, dtype="bf16", n_layers=4, hidden=2048, n_heads=32 if batch == 20 else 16, n_kv_heads=8, intermediate=512, vocab=300, eps=1e-5, rope_base=10000.0)
+    model.init_random(seed=6, sigma=0.02)
+    sess = L.Session(model, batch, capacity)
+    tok = np.zeros(batch, np.int32)
+    sess.decode_step(tok)
+    before = device.launch_count()
+    sess.decode_step(tok)
+    assert (device.launch_count() - before == 4) is link           # embedding, one chain, token, position; launched: an attention and a chain per layer
+    sess.close(); model.close()
 
 
 def test_deep_model_against_oracle(lib_built, device):
