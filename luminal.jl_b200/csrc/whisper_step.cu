@@ -196,41 +196,34 @@ __device__ __forceinline__ bool gemv_unit(const WhisperStepParams& p, const Whis
   if (joined) {                                            // the cross attention's parts, put together
     const int items = p.B * p.H * 8;
 #pragma unroll 1
-    for (int i0 = tid; i0 < items; i0 += kThreads) {
-      float2 ml[1][kWhisperStepSplits];
-      float4 o[1][kWhisperStepSplits][2];
+    for (int i = tid; i < items; i += kThreads) {
+      const int pair = i >> 3, s0 = pair * p.splits, bb = pair / p.H, hh = pair - bb * p.H;
+      float2 ml[kWhisperStepSplits];
+      float4 o[kWhisperStepSplits][2];
 #pragma unroll
-      for (int j = 0; j < 1; ++j) {
-        const int i = min(i0 + j * kThreads, items - 1), s0 = (i >> 3) * p.splits;
+      for (int s = 0; s < kWhisperStepSplits; ++s)
+        if (s < p.splits) {
+          const float4* part = reinterpret_cast<const float4*>(p.part_o + (size_t)(s0 + s) * kD + 8 * (i & 7));
+          ml[s] = *reinterpret_cast<const float2*>(p.part_ml + 2 * (s0 + s));
+          o[s][0] = part[0];
+          o[s][1] = part[1];
+        }
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, m = -CUDART_INF_F, den = 0.f;
 #pragma unroll
-        for (int s = 0; s < kWhisperStepSplits; ++s)
-          if (s < p.splits) {
-            const float4* part = reinterpret_cast<const float4*>(p.part_o + (size_t)(s0 + s) * kD + 8 * (i & 7));
-            ml[j][s] = *reinterpret_cast<const float2*>(p.part_ml + 2 * (s0 + s));
-            o[j][s][0] = part[0];
-            o[j][s][1] = part[1];
-          }
-      }
+      for (int s = 0; s < kWhisperStepSplits; ++s)
+        if (s < p.splits) m = fmaxf(m, ml[s].x);
 #pragma unroll
-      for (int j = 0; j < 1; ++j) {
-        const int i = min(i0 + j * kThreads, items - 1), pair = i >> 3, bb = pair / p.H, hh = pair - bb * p.H;
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, m = -CUDART_INF_F, den = 0.f;
-#pragma unroll
-        for (int s = 0; s < kWhisperStepSplits; ++s)
-          if (s < p.splits) m = fmaxf(m, ml[j][s].x);
-#pragma unroll
-        for (int s = 0; s < kWhisperStepSplits; ++s)
-          if (s < p.splits) {
-            const float f = exp2f(ml[j][s].x - m);
-            const float4 o0 = o[j][s][0], o1 = o[j][s][1];
-            den += f * ml[j][s].y;
-            v[0] += f * o0.x; v[1] += f * o0.y; v[2] += f * o0.z; v[3] += f * o0.w;
-            v[4] += f * o1.x; v[5] += f * o1.y; v[6] += f * o1.z; v[7] += f * o1.w;
-          }
-        const float inv = 1.0f / den;
-        *reinterpret_cast<uint4*>(sm.x + (hh * 8 + (i & 7)) * (8 * N) + bb * 8) =
-            make_uint4(pack(v[0] * inv, v[1] * inv), pack(v[2] * inv, v[3] * inv), pack(v[4] * inv, v[5] * inv), pack(v[6] * inv, v[7] * inv));
-      }
+      for (int s = 0; s < kWhisperStepSplits; ++s)
+        if (s < p.splits) {
+          const float f = exp2f(ml[s].x - m);
+          const float4 o0 = o[s][0], o1 = o[s][1];
+          den += f * ml[s].y;
+          v[0] += f * o0.x; v[1] += f * o0.y; v[2] += f * o0.z; v[3] += f * o0.w;
+          v[4] += f * o1.x; v[5] += f * o1.y; v[6] += f * o1.z; v[7] += f * o1.w;
+        }
+      const float inv = 1.0f / den;
+      *reinterpret_cast<uint4*>(sm.x + (hh * 8 + (i & 7)) * (8 * N) + bb * 8) =
+          make_uint4(pack(v[0] * inv, v[1] * inv), pack(v[2] * inv, v[3] * inv), pack(v[4] * inv, v[5] * inv), pack(v[6] * inv, v[7] * inv));
     }
     __syncthreads();
   }
