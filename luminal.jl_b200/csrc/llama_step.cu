@@ -9,7 +9,7 @@
 // rows (the layout of the launched kernel's tiles), a warp every eighth chunk of 32 k; lanes, then warps, are added in order.
 #include "llama_step.cuh"
 
-#include <math_constants.h>
+#include "step.cuh"
 
 #include <algorithm>
 
@@ -19,7 +19,6 @@ namespace {
 constexpr int kThreads = 256, kWarps = 8, kAhead = 3;
 constexpr int kMaxHidden = 4 * kThreads, kMaxFfn = 4096;
 constexpr float kLog2e = 1.4426950408889634f, kHalfPi = 1.5707963267948966f;
-constexpr long long kWaitCycles = 4000000000ll;          // about 2 s
 
 enum Piece { QKV, ATTEND, OUT, GATE_UP, DOWN, HEAD };
 
@@ -32,28 +31,6 @@ struct Shared {
   LlamaStepLayer layer[2];                     // the present layer's matrices and the next one's
   int flag;
 };
-
-__device__ __forceinline__ bool wait_units(const LlamaStepParams& p, const unsigned* counter, unsigned need, Shared& sm) {
-  if (threadIdx.x == 0) {
-    const long long t0 = clock64();
-    unsigned spins = 0, v;
-    for (;;) {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-      if (v >= need) break;
-      if ((++spins & 255u) == 0u && (clock64() - t0 > kWaitCycles || *reinterpret_cast<volatile int*>(p.err) != 0)) {
-        *reinterpret_cast<volatile int*>(p.err) = 1;
-        sm.flag = 1;
-        break;
-      }
-    }
-  }
-  __syncthreads();
-  return sm.flag == 0;
-}
-__device__ __forceinline__ void count_unit(unsigned* counter) {
-  __syncthreads();
-  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-}
 
 // the residual row before the layers have written it: the token's embedding (out of range: zeros, as _gather_kernel! does, src/Execution.jl:580-595)
 __device__ __forceinline__ const float* embedding(const LlamaStepParams& p, int b) {
@@ -85,7 +62,7 @@ __device__ __forceinline__ bool gemv_unit(const LlamaStepParams& p, const LlamaS
   fetch(warp);
   float4 gn = make_float4(0.f, 0.f, 0.f, 0.f);
   if (norm && 4 * tid < K) gn = __ldg(reinterpret_cast<const float4*>(gain) + tid);
-  if (need && !wait_units(p, before, need, sm)) return false;
+  if (need && !wait_units(before, need, p.err, &sm.flag)) return false;
   // the input, a multiple of 32 wide
   const int width = 32 * KC, n4 = K >> 2;
   if (norm) {                                              // (hidden <= 4 kThreads: a thread's four features of every row stay in registers)
@@ -240,7 +217,7 @@ __device__ __forceinline__ bool attention_unit(const LlamaStepParams& p, const L
   constexpr int D = 16 * DU;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int b = unit / p.Hl, hl = unit - b * p.Hl, T = p.pos[b] + 1, blocks = (T + 15) >> 4;
-  if (!wait_units(p, before, need, sm)) return false;
+  if (!wait_units(before, need, p.err, &sm.flag)) return false;
   const float* base = L.kv + b * p.kv_b + (hl / p.G) * p.kv_h + lane * 8;
   float4 qv[DU];
   const float* q = p.q + ((size_t)b * p.Hl + hl) * D;
@@ -373,38 +350,11 @@ __global__ void __launch_bounds__(kThreads, 1) llama_step_kernel(const __grid_co
     if (tid < p.B) p.best[cta * kLlamaStepBatch + tid] = make_float2(sm.best[tid][0], __int_as_float(sm.best_id[tid][0]));
   }
   // the last CTA out chooses the tokens, moves the positions and empties the counters for the next step
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    sm.flag = atomicAdd(p.done, 1u) == (unsigned)G - 1u ? 2 : 0;
-    __threadfence();
-  }
-  __syncthreads();
-  if (sm.flag != 2) return;
+  if (!last_block(p.done, &sm.flag)) return;
   for (int b = warp; b < p.B; b += kWarps) {
     if (p.with_head) {
-      float v = -CUDART_INF_F;
-      int i = 0x7fffffff;
-      for (int k = lane; k < G; k += 32) {
-        const float2 o = __ldcg(p.best + k * kLlamaStepBatch + b);
-        const int oi = __float_as_int(o.y);
-        if (o.x > v || (o.x == v && oi < i)) { v = o.x; i = oi; }
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float o = __shfl_xor_sync(0xffffffffu, v, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-        if (o > v || (o == v && oi < i)) { v = o; i = oi; }
-      }
-      if (lane == 0) {
-        const int eot = p.stop[0];                         // stop: end-of-text id or -1, sequences that produced it, whether sequence b did
-        if (eot >= 0) {
-          if (p.stop[2 + b]) i = eot;
-          else if (i == eot) { p.stop[2 + b] = 1; atomicAdd(&p.stop[1], 1); }
-        }
-        p.tokens[b] = i;
-        p.hist[(int64_t)(*p.step_ctr) * p.B + b] = i;
-      }
+      const int id = best_of_blocks(p.best + b, kLlamaStepBatch, lane);
+      if (lane == 0) keep_token(id, b, p.B, p.tokens, p.hist, p.step_ctr, p.stop);
     }
     if (lane == 0 && p.pos[b] < p.limit[b]) p.pos[b] += 1;
   }

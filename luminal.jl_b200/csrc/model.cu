@@ -9,6 +9,7 @@
 #include "model.cuh"
 #include "pdl.cuh"
 #include "llama_step.cuh"
+#include "step.cuh"
 #include "whisper_step.cuh"
 
 namespace lmb {
@@ -478,15 +479,7 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_step_kernel(const float
       const int i = __shfl_xor_sync(0xffffffffu, bi, off);
       take(v, i);
     }
-    if (tid == 0) {
-      const int eot = stop ? stop[0] : -1;
-      if (eot >= 0) {
-        if (stop[2 + b]) bi = eot;
-        else if (bi == eot) { stop[2 + b] = 1; atomicAdd(&stop[1], 1); }
-      }
-      tokens[b] = bi;
-      if (hist) hist[(int64_t)(*step_ctr) * B + b] = bi;
-    }
+    if (tid == 0) keep_token(bi, b, B, tokens, hist, step_ctr, stop);
   }
 }
 
@@ -562,13 +555,7 @@ __global__ void __launch_bounds__(256) argmax_tp_select_kernel(const PeerReduce 
     const int i = __float_as_int(f);
     if (v > best || (v == best && i < bi)) { best = v; bi = i; }
   }
-  const int eot = stop ? stop[0] : -1;
-  if (eot >= 0) {
-    if (stop[2 + b]) bi = eot;
-    else if (bi == eot) { stop[2 + b] = 1; atomicAdd(&stop[1], 1); }
-  }
-  tokens[b] = bi;
-  if (hist) hist[(int64_t)(*step_ctr) * B + b] = bi;
+  keep_token(bi, b, B, tokens, hist, step_ctr, stop);
 }
 
 // First kernel of the fused step: x <- embedding rows (out-of-range ids -> zeros, as _gather_kernel! does,

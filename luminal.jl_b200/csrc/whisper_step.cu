@@ -13,8 +13,8 @@
 #include "whisper_step.cuh"
 
 #include "pdl.cuh"
+#include "step.cuh"
 
-#include <math_constants.h>
 #include <stdlib.h>
 
 #include <algorithm>
@@ -24,7 +24,6 @@ namespace {
 
 constexpr int kThreads = 256, kWarps = 8, kD = 64, kMaxHidden = 1024;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr long long kWaitCycles = 4000000000ll;          // about 2 s
 
 typedef __nv_bfloat16 bf16;
 
@@ -73,29 +72,6 @@ struct Shared {
   WhisperStepLayer layer[2];           // the present layer's matrices and the next one's
   int dead;
 };
-
-// Waits until `need` units of the piece before have been counted; false if that took too long (the flag says so to the host).
-__device__ __forceinline__ bool wait_units(const WhisperStepParams& p, const unsigned* counter, unsigned need, Shared& sm) {
-  if (threadIdx.x == 0) {
-    const long long t0 = clock64();
-    unsigned spins = 0, v;
-    for (;;) {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-      if (v >= need) break;
-      if ((++spins & 255u) == 0u && (clock64() - t0 > kWaitCycles || *reinterpret_cast<volatile int*>(p.err) != 0)) {
-        *reinterpret_cast<volatile int*>(p.err) = 1;
-        sm.dead = 1;
-        break;
-      }
-    }
-  }
-  __syncthreads();
-  return sm.dead == 0;
-}
-__device__ __forceinline__ void count_unit(unsigned* counter) {
-  __syncthreads();
-  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-}
 
 // The input norm's sums of x^2 and x, per warp: four slots a warp at a time, columns along the lanes.
 template <int NT>
@@ -189,7 +165,7 @@ __device__ __forceinline__ bool gemv_unit(const WhisperStepParams& p, const Whis
   const int row = 16 * rt + tid / N, b = tid % N, rr = tid / N;
   const bool live = tid < 16 * N;
   const float bias_row = live ? bias[row] : 0.f, other_row = live ? (norm ? wg : gain)[row] : 0.f;
-  if (!wait_units(p, before, need, sm)) return false;
+  if (!wait_units(before, need, p.err, &sm.dead)) return false;
   float xv = 0.f;
   if (!norm && live) xv = p.x[(size_t)row * p.Bp + b];
   if (norm) input_sums<NT>(p, sm, warp, lane);
@@ -316,7 +292,7 @@ __device__ __forceinline__ bool attention_unit(const WhisperStepParams& p, const
     if (kb0 < end) load(0, kb0);
     if (kb0 + kWarps < end) load(1, kb0 + kWarps);
   }
-  if (!wait_units(p, before, need, sm)) return false;
+  if (!wait_units(before, need, p.err, &sm.dead)) return false;
   if (!CROSS) {
     if (kb0 < end) load(0, kb0);
     if (kb0 + kWarps < end) load(1, kb0 + kWarps);
@@ -439,14 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1) whisper_step_kernel(const __grid_
   }
   // the last CTA out empties the counters for the next step
   const int n_done = 1 + 8 * p.n_layers;
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    sm.dead = atomicAdd(p.done + n_done, 1u) == (unsigned)G - 1u ? 2 : 0;
-    __threadfence();
-  }
-  __syncthreads();
-  if (sm.dead == 2)
+  if (last_block(p.done + n_done, &sm.dead))
     for (int i = tid; i <= n_done; i += kThreads) p.done[i] = 0u;
 }
 
@@ -552,36 +521,11 @@ __global__ void __launch_bounds__(kThreads, 1) whisper_head_kernel(const __grid_
     }
     p.best[blockIdx.x * kWhisperStepBatch + tid] = make_float2(v, __int_as_float(i));
   }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    sm.dead = atomicAdd(p.head_done, 1u) == gridDim.x - 1 ? 1 : 0;
-    __threadfence();
-  }
-  __syncthreads();
-  if (!sm.dead) return;
+  if (!last_block(p.head_done, &sm.dead)) return;
   for (int b = warp; b < p.B; b += kWarps) {
-    float v = -CUDART_INF_F;
-    int i = 0x7fffffff;
-    for (int c = lane; c < (int)gridDim.x; c += 32) {
-      const float2 o = __ldcg(p.best + c * kWhisperStepBatch + b);
-      const int oi = __float_as_int(o.y);
-      if (o.x > v || (o.x == v && oi < i)) { v = o.x; i = oi; }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const float o = __shfl_xor_sync(0xffffffffu, v, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-      if (o > v || (o == v && oi < i)) { v = o; i = oi; }
-    }
+    const int id = best_of_blocks(p.best + b, kWhisperStepBatch, lane);
     if (lane == 0) {
-      const int eot = p.stop[0];                           // stop: end-of-text id or -1, sequences that produced it, whether sequence b did
-      if (eot >= 0) {
-        if (p.stop[2 + b]) i = eot;
-        else if (i == eot) { p.stop[2 + b] = 1; atomicAdd(&p.stop[1], 1); }
-      }
-      p.tokens[b] = i;
-      p.hist[(int64_t)(*p.step_ctr) * p.B + b] = i;
+      keep_token(id, b, p.B, p.tokens, p.hist, p.step_ctr, p.stop);
       if (p.pos[b] < p.limit[b]) p.pos[b] += 1;
     }
   }
