@@ -31,6 +31,7 @@ for _v in ("OMP_NUM_THREADS", "OPENBLAS_NUM_THREADS", "MKL_NUM_THREADS"):
 
 import argparse  # noqa: E402
 import json  # noqa: E402
+import math  # noqa: E402
 import subprocess  # noqa: E402
 import sys  # noqa: E402
 import threading  # noqa: E402
@@ -477,7 +478,7 @@ def run_decode(args):
         e2e_regions = timed_regions(D, stream, min(args.repeats, 3), e2e_prep, e2e_run)
     e2e_ms = median(e2e_regions)
 
-    # ---- dominant kernel alone: split-KV decode attention, one launch per layer ------------------
+    # ---- the launched split-KV decode attention alone, one launch per layer -----------------------
     peaks = load_peaks()
     T_mid = ctx_start + steps // 2
     Hl = CFG["n_heads"] // tp_size
@@ -503,6 +504,22 @@ def run_decode(args):
         step_gbs = step_bytes / (ms_total / steps * 1e-3) / 1e9
         attn_gbs = attn_bytes / (attn_ms * 1e-3) / 1e9
         traffic, traffic_src = attention_traffic(KVl, T_mid, BATCH, Dh)
+        attention = {"kernel": f"attn_decode_bf16_kernel<{Dh}> (per layer; the last CTA of each sequence and kv head merges the splits)",
+                     "bound": "hbm", "achieved": attn_gbs, "peak": peaks["hbm"], "unit": "GB/s",
+                     "frac": attn_gbs / peaks["hbm"], "peak_kind": peaks["kind"],
+                     "traffic": traffic, "traffic_source": traffic_src,
+                     "bytes_per_launch": attn_bytes, "ms_per_launch": attn_ms}
+        # fewer launches than layers: every projection and attention is a link of a chain, and the chains are all of the step but its first and last kernels
+        per_step = launches / steps
+        chained = per_step < cfg["n_layers"]
+        roofline = attention
+        if chained:
+            links = math.ceil(5 * cfg["n_layers"] / 40)
+            roofline = {"kernel": f"gemv_chain_kernel<{16 if BATCH <= 16 else 32}, {Dh}>: every layer's projections and attention, {links} launches a step, timed as the "
+                                  f"whole step ({per_step:g} launches: embedding, head, token and position beside them)",
+                        "bound": "hbm", "achieved": step_gbs, "peak": peaks["hbm"], "unit": "GB/s", "frac": step_gbs / peaks["hbm"],
+                        "peak_kind": peaks["kind"], "traffic": None, "traffic_source": None, "bytes_per_launch": step_bytes / links,
+                        "ms_per_launch": ms_total / steps / links}
         line = {
             "metric": METRIC, "value": tokens / (ms_total * 1e-3), "unit": "tokens/s", "n_gpus": world,
             "steps": steps, "warmup": warm, "ms_per_step": ms_total / steps, "higher_is_better": True,
@@ -518,11 +535,9 @@ def run_decode(args):
                     "h2d_bytes_per_step": BATCH * 4, "d2h_bytes_per_step": BATCH * 4, "ms_per_step": e2e_ms / steps},
             "gpu_launches": int(launches),
             "clocks": clocks,
-            "roofline": {"kernel": f"attn_decode_bf16_kernel<{Dh}> (per layer; the last CTA of each sequence and kv head merges the splits)",
-                         "bound": "hbm", "achieved": attn_gbs, "peak": peaks["hbm"], "unit": "GB/s",
-                         "frac": attn_gbs / peaks["hbm"], "peak_kind": peaks["kind"],
-                         "traffic": traffic, "traffic_source": traffic_src,
-                         "bytes_per_launch": attn_bytes, "ms_per_launch": attn_ms},
+            "roofline": roofline,
+            # the launched attention alone; a step whose chains attend (chained_attention) does not launch it
+            "attention_launched": attention, "chained_attention": chained,
             "step_hbm": {"bytes_per_step_per_gpu": step_bytes, "achieved": step_gbs, "peak": peaks["hbm"], "unit": "GB/s",
                          "frac": step_gbs / peaks["hbm"]},
         }
@@ -624,7 +639,7 @@ def run_small_llama(args):
         "repeats": {"n": len(regions), "statistic": "median", "min_ms": regions[0], "max_ms": regions[-1]},
         "config": {"workload": "small llama (4 layers, hidden 256, 8 heads x 32, MLP 688, vocab 1024), float32, batch 1, "
                                "32-token prompt + 64 greedy steps; the time includes the prompt", "name": "small_llama",
-                   "l2": "the model (13.7 MB) is L2-resident by nature of the configuration: launch-bound"},
+                   "l2": "the model (13.7 MB) is L2-resident by nature of the configuration: latency-bound"},
         "e2e": {"value": steps / (ms * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 4,
                 "note": "the timed call takes the prompt from host memory and returns the tokens to it"},
         "gpu_launches": int(launches),
@@ -743,7 +758,7 @@ def run_whisper(args):
         "config": {"workload": "whisper-base shape (d_model 512, 8 heads, 6 + 6 layers, FFN 2048, vocab 51865), bf16, random "
                                "weights ~N(0, 0.02), mel [8, 80, 3000] ~N(0,1): encoder + cross K/V projection + 128 greedy steps",
                    "name": "whisper_base", "batch": batch,
-                   "l2": "decoder weights (97 MB) and cross K/V (147 MB) exceed L2 together; the step is launch-bound"},
+                   "l2": "decoder weights (97 MB) and cross K/V (147 MB) exceed L2 together; the step is latency-bound"},
         "e2e": {"value": batch * steps / (ms_whole * 1e-3), "unit": "tokens/s", "ms_whole_pipeline": ms_whole,
                 "ms_encoder_and_cross_kv": ms_whole - ms_dec, "h2d_bytes_per_step": int(mel.nbytes / steps),
                 "d2h_bytes_per_step": batch * 4,

@@ -324,7 +324,7 @@ class CompiledGraph:
         return self.results
 
     def kernel_count(self):
-        """Steps of one call: a kernel each where they run one by one; a replay runs chains of small steps as one kernel."""
+        """Steps of one call: a kernel each where they run one by one; a replay may run many of them as one kernel."""
         return len(self.steps)
 
     def buffer_bytes(self):

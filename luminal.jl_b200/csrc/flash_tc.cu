@@ -26,7 +26,9 @@
 // all operands from shared memory, 160 KB of operand reads per 128 keys and tile -- ran at 709
 // TFLOP/s on [4, 32, 4096, 128]; 128-key tiles with P in tensor memory 729; two softmax threads
 // per row 948; packed float32 pairs and three-input maxima in the softmax 959; MMAs issued under an elected branch (tc::elect_one) 983 -> 1049
-// on one box; what follows 1047 -> 1126; scores held in registers and P in parts 1126 -> 1203.)
+// on one box; what follows 1047 -> 1126; scores held in registers and P in parts 1126 -> 1203.  These are
+// single calls with pauses, near 1.9 GHz; called back to back the card's power limit takes the same call to 1000-1020: 1082-1102 us for [4, 32, 4096, 128], where those
+// before this paragraph's last two changes took 1239.)
 // A CTA holds the SM alone, so what it does outside its key loop is not hidden by another: 17000 clocks of
 // 136000 with 4096 keys, of 25000 with 256.  Q by TMA before the block's first barrier instead of by copies of
 // 16 bytes (any number of threads: the load path took 14 bytes a clock) has the first scores there after 3600
@@ -376,8 +378,7 @@ flash_tc_kernel(__nv_bfloat16* __restrict__ out, const __grid_constant__ CUtenso
       mbar_wait(&s_full[t], (j - j0) & 1, dead, err);          // S(j) is complete, and with it (pipe order) P V(j - 1): O is at rest
       fence_after();
       const int key0 = j * kBN + h * 64, last_seen = key_hi - key0;
-      // is key key0 + i visible?  One comparison and a select: as a chain of conditions every masked key was a branch of its own, and a
-      // tile on the diagonal took 5 us longer than one inside
+      // is key key0 + i visible?  One comparison and a select: as a chain of conditions a tile on the diagonal took 5 us longer than one inside
       auto seen = [&](int i) { return WIN ? (unsigned)(key0 + i - key_lo) <= key_span : i <= last_seen; };
       const bool inside = (j + 1) * kBN <= Sk && (!causal || (j + 1) * kBN - 1 <= q_off + q0 + t * kBM) &&
                           (!WIN || ex.window == 0 || j * kBN > q_off + q0 + t * kBM + kBM - 1 - ex.window);   // no key of the tile is masked

@@ -1507,8 +1507,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemv_cl_kernel(const GemvParams
 //   Measured (8 layers, per step, one launch per GEMV -> chained): Llama-3-8B shape at 1031 keys, batch 1 1044 -> 955 us, batch 32
 //   1252 -> 1143 us; Phi-3-mini batch 16 at 2052 keys 760 -> 693 us; Kevatar width 2048 batch 16 825 -> 734 us.  gemv_chain_clusters has the rule.
 //   Since then the links take less: one release and one acquire per dependency, the proxy fence on the reading side only, parameters a link
-//   ahead in shared memory, and the layers' decode attention as a link (chain_attend).  Whole steps, 32 layers: Llama-3-8B batch 1
-//   3.33 -> 3.05 ms, batch 32 9.2 -> 8.3; Phi-3-mini batch 16 2.68 -> 2.29.
+//   ahead in shared memory, and the layers' decode attention as a link (chain_attend).  Whole steps through the host, 32 layers: Llama-3-8B batch 1, 1031 keys
+//   3.34 -> 3.05 ms, batch 32, 8184 keys 9.37 -> 8.82; Phi-3-mini batch 16, 2052 keys 2.69 -> 2.29.
 //   LayerNorms (sums of x beside those of squares) are not built in: the Whisper decoder, which needs them, was slower chained at width 512,
 //   327 -> 350 us a step, one unit of k per tile; up to 16 sequences its step is a kernel of its own instead (whisper_step.cu, 189 us).
 //   warp 0 weights, 1 MMA, 2..5 epilogue (and attention), 6 activations.

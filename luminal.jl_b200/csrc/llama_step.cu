@@ -4,8 +4,8 @@
 // work at a few hundred features.  As launches (two norms, four products, attention and its merge per layer, then head, token and position) a step of the
 // small Llama (hidden 256, four layers, vocabulary 1024) is 36 of them, 1.5 to 4 us each.  Here one CTA per SM takes a fixed share of every piece's
 // units -- 16 rows of a matrix, or one sequence's query head -- and counts finished units through L2; the weights a unit needs are in registers before it
-// starts to wait: 132 -> 61 us a step at 100 keys (108 us through the host, 178 before; hidden 1024, 16 layers, ffn 4096, four sequences of 1000 keys
-// 2946 -> 1156; at every size that llama_step_fits lets in 1.3 to 2.5 times faster).  The norms are computed by every unit that reads their row: cheaper than another trip through L2.  Products: a lane holds 8 k of two
+// starts to wait: 132 -> 58 us a step at 100 keys, one step behind the other (97 us through the host with the logits; hidden 1024, 16 layers, ffn 4096, four sequences of 1000 keys
+// 2946 -> 1156; of the 160 sizes measured those that llama_step_fits lets in are 1.09 to 2.8 times faster).  The norms are computed by every unit that reads their row: cheaper than another trip through L2.  Products: a lane holds 8 k of two
 // rows (the layout of the launched kernel's tiles), a warp every eighth chunk of 32 k; lanes, then warps, are added in order.
 #include "llama_step.cuh"
 

@@ -2,11 +2,11 @@
 //
 // A traced graph of the reference is a chain of hundreds of steps of a microsecond's work or less.  As one graph node per step a replay is bound by
 // the time from one node to the next (404 nodes of a small Llama's 32-token graph: 2.4 us each, 985 us), and most of these nodes only move
-// elements.  At capture_end the runs of such steps become ONE kernel each (vm_kernel): a CTA per SM walks through its own list of (step, tile)
+// elements.  At capture_end the runs of such steps become ONE kernel each (vm_kernel) where that is estimated to be faster (own_us, plan_run): a CTA per SM walks through its own list of (step, tile)
 // entries and waits for the steps its entry reads by their tile counters, so what counts is the dependency chain, not the number of steps.  Two things
 // shorten that chain:
 //   * a movement step (permute, expand, slice, most reshapes) is an affine view of what it reads.  A step that reads such a step's output reads the
-//     source through the view instead (resolve()), so movements are still written out -- every buffer holds what it held -- but nobody waits for them;
+//     source through the view instead (plan_steps), so movements are still written out -- every buffer holds what it held -- but nobody waits for them;
 //   * a product whose tiles of 32 x 32 would leave SMs idle takes tiles of 32 x 8.
 // The arithmetic of every step is that of its own kernel in prims.cu, sums in the same order: a replay gives the bits of the calls it records.
 // Measured: the comment at vm_kernel.
@@ -425,7 +425,7 @@ __device__ __forceinline__ void vm_run(const VmOp& q, int tile, float* buf) {
 
 // One CTA per SM (launched cooperatively: they wait for one another).  Bound by the dependency chain: per link one counter through L2 (release, acquire),
 // the operands' trip from L2 and the step itself.  The next entry's step is fetched while the present one waits and runs.
-// The small Llama's 32-token graph (404 steps, a longest chain of 90): 255 us a replay, 2.0 us per element-wise link and 2.2 to 4 us per product, 960 us
+// The small Llama's 32-token graph (404 steps, a longest chain of 90): 237 us a replay, 2.0 us per element-wise link and 2.2 to 4 us per product, 950 us
 // as 404 nodes.  Of an element-wise link 1.1 us is the step with its release; a second fence in front of the release made that 1.4.
 __global__ void __launch_bounds__(kVmThreads, 1) vm_kernel(const VmParams P) {
   extern __shared__ __align__(16) float buf[];

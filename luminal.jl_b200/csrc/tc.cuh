@@ -80,9 +80,8 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One thread of a converged warp, known as such to the compiler: a loop that waits for operands and issues MMAs is written under ONE such branch.  Under
-// `lane == 0` every tcgen05 instruction is wrapped in a loop over the lanes that might be active, and its descriptors change registers each time: eight
-// MMAs of 128 x 16 x 16 with their wait and commit took 713 clocks to issue, 377 under this (47 each is what the tensor core takes).
+// One thread of a converged warp, for loops that wait for operands and issue MMAs: they are written under ONE such branch.  Under `lane == 0` around each group of
+// tcgen05 instructions eight MMAs of 128 x 16 x 16 with their wait and commit took 713 clocks to issue, under this 377 (47 each is what the tensor core takes).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
