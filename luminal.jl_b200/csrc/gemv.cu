@@ -2544,6 +2544,8 @@ int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMaxAttend + 1) * kCh
 // 28 (2450) +4.4, batch 17 (2914) +12.  With a key head per head the launched kernel has a quarter of the parts to merge and is harder to beat: 8190 keys, batch 8 (298) -5.4, 16
 // (1193) +13.5, 20 (1491) -9, 26 (3703) +32.  Head dimension 64 is bound by the work per stage, not by its bytes: 1031 keys, batch 1, 16, 17 -2.1, -2.7, +4.1; 4096
 // keys, batch 1, 16 +1.2, +3.0; 8190 keys, batch 32 +20.
+//   A short context in a large cache leaves most of a head's parts empty, and a CTA still looks at each: from four rounds of parts on that costs more than the
+// launch (22 sequences, 100 keys in a cache of 8256: 426 -> 441 us).
 //   Narrow models are chained up to three row groups, where an attention between is launched: at width 256 and 384 a link gained 5 % at 64 keys and lost up to
 // 12 % at 1031.
 bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, int D, int capacity, int* keys_per_cta, int* nsplit) {
@@ -2560,11 +2562,12 @@ bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, i
   }
   *keys_per_cta = (int)best;
   *nsplit = (int)ceil_div(cap, best);
-  const int64_t even = pairs * cap / ctas, over = best_cost - even, slack = std::min<int64_t>(even, 16000) * 2 / 25;
   if (e) return true;
+  const int64_t even = pairs * cap / ctas, over = best_cost - even, kept = std::min<int64_t>(even, 16000);
   if (D == 64) return best_cost <= 1050 || (over <= 200 && best_cost <= 2300);
-  if (G < 4 && Layout<__nv_bfloat16>::batch_pad(B) == 16) return over <= 950;
-  return over <= (G < 4 ? 900 : 1050) + slack;
+  if (*nsplit > 1 && pairs * *nsplit > 3 * ctas) return false;
+  if (G < 4) return over <= (Layout<__nv_bfloat16>::batch_pad(B) == 16 ? 950 : 900 + kept / 20);
+  return over <= 1050 + kept * 2 / 25;
 }
 
 int32_t GemvChain::add(const GemvParams& p) {
