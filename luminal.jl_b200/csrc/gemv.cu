@@ -18,6 +18,7 @@
 // the parity path.
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "gemv.cuh"
 #include "pdl.cuh"
@@ -2532,6 +2533,14 @@ int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms) {
 }
 int64_t gemv_chain_scratch_bytes() { return (int64_t)(kChainMaxAttend + 1) * kChainLine * 4; }
 
+// Whether an attention link gains: the keys' time its busiest CTA takes, and what an even spread over the CTAs would take (gemv_chain_attention_plan's comment).
+static bool link_pays(int64_t busiest, int64_t even, int B, int G, int D) {
+  const int64_t over = busiest - even, kept = std::min<int64_t>(even, 16000);
+  if (D == 64) return busiest <= 1050 || (over <= 200 && busiest <= 2300);
+  if (G < 4) return over <= (Layout<__nv_bfloat16>::batch_pad(B) == 16 ? 950 : 900 + kept / 20);
+  return over <= 1050 + kept * 2 / 25;
+}
+
 // One unit per CTA and round; a unit costs about 48 keys' time beside its keys (queries, the four warps' merge), and one of several parts 100 more (partial
 // results out, a counter).  The merge at the end takes 4 us, in which a CTA streams some 640 keys (Llama-3-8B shape, one sequence of 1031 keys, nine parts: the
 // last one 11.8 us after q/k/v, the others 4.6).  Without the 100 a head was cut into too many parts (28 sequences of 8190 keys: 17 rounds of units; the step
@@ -2563,11 +2572,29 @@ bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, i
   *keys_per_cta = (int)best;
   *nsplit = (int)ceil_div(cap, best);
   if (e) return true;
-  const int64_t even = pairs * cap / ctas, over = best_cost - even, kept = std::min<int64_t>(even, 16000);
-  if (D == 64) return best_cost <= 1050 || (over <= 200 && best_cost <= 2300);
-  if (*nsplit > 1 && pairs * *nsplit > 3 * ctas) return false;
-  if (G < 4) return over <= (Layout<__nv_bfloat16>::batch_pad(B) == 16 ? 950 : 900 + kept / 20);
-  return over <= 1050 + kept * 2 / 25;
+  if (D != 64 && *nsplit > 1 && pairs * *nsplit > 3 * ctas) return false;
+  return link_pays(best_cost, pairs * cap / ctas, B, G, D);
+}
+
+// The units as chain_unit makes them at these positions, CTA by CTA.  One sequence far longer than the others is a few CTAs' work in the link, while the launched
+// kernel cuts it for all: 16 sequences in a cache of 8256, one of 8190 keys and the others of 60, 456 -> 624 us a step (Llama-3-8B shape, four layers), half of them
+// long 573 -> 625, all within 40 keys of one another 737 -> 697.
+bool gemv_chain_attention_spreads(int clusters, int B, int KVl, int G, int D, int keys_per_cta, int nsplit, const int* pos) {
+  const char* e = getenv("LMB200_CHAIN_ATTENTION");
+  if (e) return atoi(e) != 0;
+  const int64_t pairs = (int64_t)B * KVl, ctas = (int64_t)clusters * kChainC;
+  std::vector<int64_t> load(ctas, 0);
+  int64_t total = 0;
+  bool split = false;
+  for (int64_t u = 0; u < pairs * nsplit; ++u) {
+    const int T = pos[u % pairs / KVl] + 1, per = (int)std::min<int64_t>(round_up(ceil_div(T, nsplit), 64), keys_per_cta);
+    const int64_t begin = u / pairs * per;
+    if (begin >= T) continue;
+    split = split || T > per;
+    total += std::min<int64_t>(T - begin, per);
+    load[u % ctas] += std::min<int64_t>(T - begin, per) + (T > per ? 148 : 48);
+  }
+  return link_pays(*std::max_element(load.begin(), load.end()) + (split ? 640 : 0), total / ctas, B, G, D);
 }
 
 int32_t GemvChain::add(const GemvParams& p) {

@@ -201,5 +201,7 @@ int gemv_chain_clusters(int B, int width, int per_chain, bool output_norms);
 int64_t gemv_chain_scratch_bytes();
 // Whether a step's attentions are links of its chains, and then their split of the keys (AttnParams::keys_per_cta, nsplit) for a cache of `capacity` positions
 bool gemv_chain_attention_plan(int clusters, int width, int B, int KVl, int G, int D, int capacity, int* keys_per_cta, int* nsplit);
+// Whether they still are with the sequences at these (host) positions, which differ
+bool gemv_chain_attention_spreads(int clusters, int B, int KVl, int G, int D, int keys_per_cta, int nsplit, const int* pos);
 
 }  // namespace lmb

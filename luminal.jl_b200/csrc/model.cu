@@ -1261,7 +1261,7 @@ GemvParams gemv_params(Session* S, const void* W, const WMap& m, const GemvPlan&
 
 GemvChain gemv_chain(Session* S, cudaStream_t st) {
   GemvChain ch;
-  ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done; ch.attention = S->chain_attention;
+  ch.ctx = S->m->ctx; ch.stream = st; ch.clusters = S->chain_clusters; ch.done = S->chain_done; ch.attention = S->chain_link;
   return ch;
 }
 
@@ -1960,7 +1960,7 @@ int32_t lmb::run_step(Session* S, bool with_head, bool want_logits) {
 }
 
 // Positions live on the device, one per sequence; the host keeps a copy for its bounds checks.  `ragged`
-// (the positions differ) selects the per-sequence RoPE path of the kernels, so changing it drops the graphs.
+// (the positions differ) selects the per-sequence RoPE path of the kernels and may take attention out of the chains, so changing it drops the graphs.
 int32_t lmb::push_positions(Session* S) {
   Ctx* ctx = S->m->ctx;
   bool ragged = false;
@@ -1972,9 +1972,13 @@ int32_t lmb::push_positions(Session* S) {
   LMB_CUDA(cudaMemcpyAsync(S->pos, S->host_pos_v.data(), (size_t)S->B * 4, cudaMemcpyHostToDevice, ctx->stream));
   LMB_CUDA(cudaStreamSynchronize(ctx->stream));
   S->host_pos = mx;
-  if (ragged != S->ragged) {
+  // all positions move on together: what holds for them here holds until they are set again
+  const bool link = S->chain_attention &&
+                    (!ragged || gemv_chain_attention_spreads(S->chain_clusters, S->B, S->m->KVl, S->m->G, S->m->D, S->chain_keys, S->chain_nsplit, S->host_pos_v.data()));
+  if (ragged != S->ragged || link != S->chain_link) {
     drop_graphs(S);
     S->ragged = ragged;
+    S->chain_link = link;
   }
   return LMB200_OK;
 }
@@ -2073,7 +2077,7 @@ extern "C" int32_t lmb200_session_create(lmb200_model hm, int32_t batch, int32_t
   int64_t po, pml;
   attn_plan(ctx, batch, M->KVl, M->G, M->D, S->cap, &S->keys_per_cta, &S->nsplit, &po, &pml);
   if (gemv_chain_attention_plan(S->chain_clusters, c.hidden, batch, M->KVl, M->G, M->D, S->cap, &S->chain_keys, &S->chain_nsplit)) {
-    S->chain_attention = true;
+    S->chain_attention = S->chain_link = true;
     po = std::max(po, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * M->D);
     pml = std::max(pml, (int64_t)batch * M->KVl * S->chain_nsplit * M->G * 2);
   }

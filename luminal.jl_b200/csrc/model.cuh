@@ -165,6 +165,7 @@ struct Session {
   unsigned* chain_done = nullptr;      // GemvChain::done
   int chain_clusters = 0;              // > 0: the fused step runs its GEMVs in chains
   bool chain_attention = false;        // ... with the attention among them, and its split of the keys
+  bool chain_link = false;             // ... at the present positions too
   int chain_keys = 0, chain_nsplit = 0;
   float* part_o = nullptr;
   float* part_ml = nullptr;

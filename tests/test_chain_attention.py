@@ -68,6 +68,36 @@ def test_launched_where_whole_heads_spread_badly(lib_built, device, batch, capac
     sess.close(); model.close()
 
 
+def test_unequal_positions_choose_anew(lib_built, device, monkeypatch):
+    """One long sequence among short ones launches its attention, positions close to one another keep it in the chain, back and forth in one session; the same
+    results as with the attention launched throughout."""
+    L = lib_built
+    model = L.Model(device, dtype="bf16", n_layers=4, hidden=2048, n_heads=16, n_kv_heads=4, intermediate=512, vocab=300, eps=1e-5, rope_base=10000.0)
+    model.init_random(seed=6, sigma=0.02)
+    batch, capacity = 16, 4096
+    places = [([4000] + [60] * 15, False), (list(range(3000, 3016)), True), ([100] * 16, True), ([60] * 15 + [4000], False), ([2000] * 16, True)]
+    got = {}
+    for env in (None, "0"):
+        monkeypatch.delenv("LMB200_CHAIN_ATTENTION", raising=False)
+        if env:
+            monkeypatch.setenv("LMB200_CHAIN_ATTENTION", env)
+        sess = L.Session(model, batch, capacity)
+        sess.fill_kv_random(4000, 7)
+        got[env] = []
+        for pos, link in places:
+            sess.set_positions(np.array(pos, np.int32))
+            tok = O.synth_tokens(8, 1, (batch,), 300).astype(np.int32)
+            for _ in range(3):
+                before = device.launch_count()
+                tok, lg = sess.decode_step(tok, want_logits=True)
+                assert (device.launch_count() - before == 4) is (link and env is None), pos[:2]
+                got[env].append(lg)
+                tok = O.synth_tokens(8, len(got[env]), (batch,), 300).astype(np.int32)
+        sess.close()
+    assert rel_err(np.stack(got[None]), np.stack(got["0"])) <= BF16_REL_TOL / 2
+    model.close()
+
+
 def test_deep_model_against_oracle(lib_built, device):
     """More links than one launch takes (nine layers: 46), from an empty cache."""
     L = lib_built
