@@ -140,7 +140,7 @@ def test_short_stage_reads_past_a_large_movement(lib_built, device, tail, fuse, 
 
 
 def stages_graph(G, rng, steps):
-    """Steps around the sizes (2^19 elements, 592 product tiles) from which one keeps its own kernel: runs fall apart into stages of one step and more, and
+    """Steps around the sizes (2^19 elements, or 16 us longer here) from which one keeps its own kernel: runs fall apart into stages of one step and more, and
     small steps read large movements."""
     g = G.Graph()
     n = 720                                                        # n x n is just below 2^19, n x 800 above
